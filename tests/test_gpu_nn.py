@@ -107,6 +107,26 @@ def test_backward_routing_network(dev):
         assert _rel(gp[name][1], rp[name][1]) < 1e-4, (name, "b", _rel(gp[name][1], rp[name][1]))
 
 
+@pytest.mark.parametrize("n,h,w", [(1, 8, 8), (3, 24, 40), (5, 72, 8)])
+def test_weight_gradient_ragged_tiles(dev, n, h, w):
+    """Grids whose levels end inside a pixel tile of the weight-gradient
+    kernel (down to one pixel), against the oracle."""
+    from aerojax_gb300.nn import WarmStartNet
+    flat = _routing_params(n + h)
+    net = WarmStartNet(device=dev, params=flat)
+    rng = np.random.default_rng(n * h + w)
+    x = rng.standard_normal((n, h, w, 16)).astype(np.float32)
+    dy = rng.standard_normal((n, h, w, 16)).astype(np.float32)
+    net.forward(torch.as_tensor(x, device=dev), n, h, w)
+    g = net.backward(torch.as_tensor(dy, device=dev), n, h, w).cpu().numpy().astype(np.float64)
+    ref = sum(N.backward(flat.astype(np.float64), x[s].astype(np.float64),
+                         dy[s].astype(np.float64), emulate_bf16=True) for s in range(n))
+    gp, rp = N.unflatten(g), N.unflatten(ref)
+    for name, _, _, _ in N.LAYERS:
+        assert _rel(gp[name][0], rp[name][0]) < 1e-4, (name, "W", _rel(gp[name][0], rp[name][0]))
+        assert _rel(gp[name][1], rp[name][1]) < 1e-4, (name, "b", _rel(gp[name][1], rp[name][1]))
+
+
 def test_backward_matches_oracle(dev):
     from aerojax_gb300.nn import WarmStartNet
     n, h, w = 2, 16, 16

@@ -818,8 +818,8 @@ int step_vjp_kernel_count(const AjStepParams& p, const Layout& L) {
   const int nst = p.fast_mode ? 2 : 3;
   int n = 1 + nst;                                  // dt + forward predictor stages
   const bool fused = parity_coarsest_fused(L);
-  if (p.v_cycles > 1)                               // rhs, forward solve
-    n += 1 + 1 + p.v_cycles * (2 * L.nlev + (fused ? 1 : 10));
+  if (p.v_cycles > 1)                               // rhs, forward solve (no statistics)
+    n += 1 + parity_kernel_count(p, L) - (parity_cluster_level(p, L) > 0);
   n += 2;                                           // correction, gradient
   n += p.v_cycles * (3 * L.nlev + (fused ? 1 : 10));  // reversed V-cycles
   n += 1 + 1 + nst + 1;                             // divergence, output, stages, scalars

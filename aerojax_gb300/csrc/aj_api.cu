@@ -732,16 +732,11 @@ int32_t aj_kernel_count(const AjStepParams* prm, int32_t cycles) {
   if (tile_predictor_params_ok(p)) n += tile_predictor_kernels();   // stages + rhs in tile kernels
   else n += (p.fast_mode ? 2 : 3) + (nn_forms_rhs(p, p.nn_factor > 0) ? 0 : 1);   // stages, rhs
   if (p.mg_mode == AJ_MG_PARITY) {
-    const int coarse = parity_coarsest_fused(L) ? 1 : 10;
-    int per_cycle = 2 * L.nlev + coarse;                        // levels, coarsest
-    if (p.flow_type == AJ_FLOW_TAYLOR_GREEN) per_cycle = 6 * L.nlev + coarse + 1;   // unfused
-    n += 1 + p.v_cycles * per_cycle;                            // begin + cycles
-    if (p.flow_type == AJ_FLOW_LID_DRIVEN_CAVITY) n += 4;       // mean and centre pin
+    n += parity_kernel_count(p, L);
   } else {
     int body = 2 * L.lc + 1 + (L.ld > 0 ? 2 : 0);               // downs, coarse solve, ups
     n += 2 + (cycles > 1 ? cycles : 1) * body + 1;              // init, resid, loop, out+stats
   }
-  if (p.mg_mode == AJ_MG_PARITY) n += 1;                        // stats
   n += 1;                                                       // correction
   // features, scales, the convolutions (12, or 10 with the two
   // full-resolution layer pairs fused), correction

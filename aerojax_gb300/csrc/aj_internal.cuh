@@ -307,6 +307,14 @@ int launch_cfl(const AjStepParams& p, void* ws, const float* u, const float* v,
                float* dt_out, cudaStream_t st);
 int launch_set_dt(const AjStepParams& p, void* ws, cudaStream_t st);
 bool parity_coarsest_fused(const Layout& L);   // coarsest sweeps on one cluster (aj_pressure.cu)
+// the lower levels of a parity cycle, or the whole solve, on one cluster
+// (aj_parity_cluster.cu)
+int parity_cluster_level(const AjStepParams& p, const Layout& L);
+int launch_parity_cluster(const AjStepParams& p, const Layout& L, void* ws, int lt,
+                          const float* const* masks, const float* b, const float* x0, float* x,
+                          const int* skip, AjStats* stats, cudaStream_t st);
+// launches of one parity solve, its statistics included
+int parity_kernel_count(const AjStepParams& p, const Layout& L);
 // reverse mode of the collocated step_pure (aj_adjoint.cu)
 size_t step_vjp_workspace(const AjStepParams& p, const Layout& L);
 int launch_step_vjp(const AjStepParams& p, const Layout& L, void* ws, void* aws, const float* u,

@@ -6,8 +6,8 @@
 // unscaled 2x2-average restriction, a prolongation that leaves the last fine
 // row and column zero, 10 coarsest sweeps, outlet row reset after each smoothing
 // phase, and the absolute early exit sum(r^2) dx dy < tol^2 after each cycle.
-// The second post-smoothing sweep and the prolongation are fused (the sweep
-// evaluates p + P(e) on the fly), so each level costs five kernels.
+// A tiled kernel per direction on the finest levels; the levels below (every
+// level and every cycle on small grids) on one cluster (aj_parity_cluster.cu).
 //
 // The converging mode lives in aj_converge.cu; this file dispatches to it.
 #include "aj_internal.cuh"
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(256) k_tg_norm(const float* __restrict__ x,
 }
 
 static int parity_solve(const AjStepParams& p, const Layout& L, void* ws, const float* mask,
-                        const float* p0, float* pout, cudaStream_t st) {
+                        const float* p0, float* pout, AjStats* stats, cudaStream_t st) {
   DevScalars* sc = at<DevScalars>(ws, 0);
   const int mac = p.grid_type == AJ_GRID_MAC;
   const float ax = (float)(1.0 / (p.dx * p.dx)), ay = (float)(1.0 / (p.dy * p.dy));
@@ -503,8 +503,9 @@ static int parity_solve(const AjStepParams& p, const Layout& L, void* ws, const 
   const int* skip = &sc->mg_skip;
   dim3 blk(32, 8);
   const long N0 = (long)p.nx * p.ny;
-  k_par_begin<<<1, 1, 0, st>>>(sc);
-  if (p0) k_copy<<<cdiv(N0, 256), 256, 0, st>>>(p0, pout, N0);
+  const int lt = parity_cluster_level(p, L);   // levels lt.. run on a cluster
+  if (lt > 0) k_par_begin<<<1, 1, 0, st>>>(sc);
+  if (lt > 0 && p0) k_copy<<<cdiv(N0, 256), 256, 0, st>>>(p0, pout, N0);
   if (p.flow_type == AJ_FLOW_LID_DRIVEN_CAVITY) {   // b -= mean(b) (multigrid_solver.py:78-80)
     k_mean_partials<<<kMeanBlocks, 256, 0, st>>>(b0, N0, sc, at<double>(ws, L.part));
     k_sub_mean<<<cdiv(N0, 256), 256, 0, st>>>(b0, N0, sc);
@@ -518,9 +519,18 @@ static int parity_solve(const AjStepParams& p, const Layout& L, void* ws, const 
     return l == 0 ? mask : at<float>(ws, L.M[l]);
   };
   const int vk = p.flow_type == AJ_FLOW_VON_KARMAN;
+  const float* masks[AJ_MAX_LEVELS + 1];
+  for (int l = 0; l <= nl; ++l) masks[l] = M(l);
+  int rc = AJ_OK;
+  // levels lt.. of one cycle on the cluster (with lt = 0 the whole solve)
+  auto cluster = [&](const int* sk) {
+    rc |= launch_parity_cluster(p, L, ws, lt, masks, B(lt), p0, X(lt), sk, stats, st);
+  };
   // the coarsest level's 10 sweeps from zero, ending in X(nl)
   auto coarsest = [&](const int* sk) {
-    if (parity_coarsest_fused(L)) {
+    if (lt == nl) {
+      cluster(sk);
+    } else if (parity_coarsest_fused(L)) {
       const int n = L.ln[nl], m = L.lm[nl];
       const size_t csm = (size_t)coarse_band_rows(n) * m * 12;
       cudaFuncSetAttribute(k_par_coarsest, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -583,16 +593,19 @@ static int parity_solve(const AjStepParams& p, const Layout& L, void* ws, const 
       k_tg_norm<<<kMeanBlocks, 256, 0, st>>>(X(0), B(0), p.nx, p.ny, ax, ay, sc, p.dx * p.dy,
                                              tol * tol, cyc == 0, sk);
     }
-    return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
+    if (stats) k_stats<<<1, 1, 0, st>>>(sc, stats, 0);
+    return rc == AJ_OK && cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
   }
+  const int nt = lt < nl ? lt : nl;   // levels 0 .. nt-1 by the tiled kernels
+  if (lt == 0) cluster(nullptr);
   auto tile_grid = [&](int l) {
     return l == 0 ? dim3(cdiv(L.lm[l], 64), cdiv(L.ln[l], 16)) : dim3(cdiv(L.lm[l], 32), cdiv(L.ln[l], 8));
   };
-  for (int cyc = 0; cyc < p.v_cycles; ++cyc) {
+  for (int cyc = 0; cyc < p.v_cycles && lt > 0; ++cyc) {
     const int* sk = cyc == 0 ? nullptr : skip;   // the first cycle always runs
-    // down the V: levels 0..nl-1; each level's pre-smoothed state goes to T,
+    // down the V: levels 0..nt-1; each level's pre-smoothed state goes to T,
     // its restricted residual to the next level's b
-    for (int l = 0; l < nl; ++l) {
+    for (int l = 0; l < nt; ++l) {
       ParTile a{};
       a.xin = (l == 0 && !(cyc == 0 && !p0)) ? X(0) : nullptr;
       a.b = B(l);
@@ -612,12 +625,13 @@ static int parity_solve(const AjStepParams& p, const Layout& L, void* ws, const 
       if (l == 0) k_par_down<16, 64><<<tile_grid(l), kPtThreads, 0, st>>>(a);
       else k_par_down<8, 32><<<tile_grid(l), kPtThreads, 0, st>>>(a);
     }
-    // coarsest: 10 sweeps from zero, ending in X
-    coarsest(sk);
+    // below: the cluster, or the coarsest level's 10 sweeps from zero, into X(nt)
+    if (lt < nl) cluster(sk);
+    else coarsest(sk);
     // up the V: T + P(coarser X), two post-sweeps, into X; level 0 also
     // forms the residual norm and its last block runs the early-exit test
     // (multigrid_solver.py:222-232)
-    for (int l = nl - 1; l >= 0; --l) {
+    for (int l = nt - 1; l >= 0; --l) {
       ParTile a{};
       a.xin = T(l);
       a.xc = X(l + 1);
@@ -646,7 +660,17 @@ static int parity_solve(const AjStepParams& p, const Layout& L, void* ws, const 
     k_store_center<<<1, 1, 0, st>>>(pout, (long)(p.nx / 2) * p.ny + p.ny / 2, sc);
     k_sub_center<<<cdiv(N0, 256), 256, 0, st>>>(pout, N0, sc);
   }
-  return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
+  if (stats && lt > 0) k_stats<<<1, 1, 0, st>>>(sc, stats, 0);   // the whole solve files its own
+  return rc == AJ_OK && cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
+}
+
+int parity_kernel_count(const AjStepParams& p, const Layout& L) {
+  const int lt = parity_cluster_level(p, L), nt = lt < L.nlev ? lt : L.nlev;
+  const int below = lt <= L.nlev || parity_coarsest_fused(L) ? 1 : 10;
+  int n = p.flow_type == AJ_FLOW_LID_DRIVEN_CAVITY ? 4 : 0;     // mean and centre pin
+  if (p.flow_type == AJ_FLOW_TAYLOR_GREEN) return 2 + p.v_cycles * (6 * L.nlev + below + 1);
+  if (lt == 0) return n + 1;                                    // the whole solve
+  return n + 2 + p.v_cycles * (2 * nt + below);                 // begin, cycles, statistics
 }
 
 int prepare_pressure(const AjStepParams& p, const Layout& L, void* ws, const float* mask,
@@ -673,9 +697,8 @@ int launch_pressure(const AjStepParams& p, const Layout& L, void* ws, const floa
                     const NnWarm* nn, bool init_done) {
   int rc;
   if (p.mg_mode == AJ_MG_PARITY) {
-    rc = parity_solve(p, L, ws, mask, p0, pout, st);
+    rc = parity_solve(p, L, ws, mask, p0, pout, stats, st);
     if (rc != AJ_OK) return rc;
-    if (stats) k_stats<<<1, 1, 0, st>>>(at<DevScalars>(ws, 0), stats, 0);
   } else {
     rc = converge_solve(p, L, ws, p0, pout, st, nn, stats, init_done);   // k_cv_out: stats
     if (rc != AJ_OK) return rc;

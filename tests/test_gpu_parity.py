@@ -37,6 +37,28 @@ def test_multigrid_parity(cuda_lib, name):
     assert rel(pm, g["p_mac"]) < TOL
 
 
+@pytest.mark.parametrize("nx,ny,guess", [(64, 32, True), (48, 80, False), (272, 48, False),
+                                         (96, 2048, False), (1008, 368, True)])
+def test_multigrid_parity_bands(cuda_lib, nx, ny, guess):
+    """Grids that put all, some or only the lower levels of the V-cycle on the
+    cluster, with bands that end inside the last blocks."""
+    import aerojax_gb300 as aj
+    from oracle import ref_np as R
+    rng = np.random.default_rng(nx + ny)
+    dx, dy = 0.02, 0.025
+    rhs = rng.standard_normal((nx, ny)).astype(np.float32)
+    mask = (rng.random((nx, ny)) > 0.05).astype(np.float32)
+    p0 = rng.standard_normal((nx, ny)).astype(np.float32) * 1e-3 if guess else None
+    for mac in (False, True):
+        fn = aj.poisson_multigrid_mac if mac else aj.poisson_multigrid
+        p, st = fn(T(rhs), T(mask), dx, dy, v_cycles=3, p0=T(p0) if guess else None,
+                   return_stats=True)
+        ref = R.poisson_multigrid(rhs.astype(np.float64), mask.astype(np.float64), dx, dy,
+                                  v_cycles=3, mac=mac, p0=None if p0 is None else p0.astype(np.float64))
+        assert rel(p, ref) < TOL, (mac, rel(p, ref))
+        assert st["cycles"] == 3 and st["err"] == 0
+
+
 @pytest.mark.parametrize("name", ["rk3", "rk2", "rk3_hyper", "rk3_field"])
 def test_predictor_collocated(cuda_lib, name):
     import aerojax_gb300 as aj

@@ -164,9 +164,10 @@ bool make_layout(const AjStepParams& p, Layout& L) {
     L.ld = converge_direct_level(L);
     if (L.ld > 0) {
       L.lc = L.ld;
-      L.dcy = take((size_t)L.lm[L.ld] * L.lm[L.ld] * 4);
+      L.dcy = take((size_t)L.lm[L.ld] * L.lm[L.ld] * 8);
       L.dly = take((size_t)L.lm[L.ld] * 4);
       L.dtmp = take((size_t)L.ln[L.ld] * L.lm[L.ld] * 4);
+      L.dpf = take(converge_direct_floats(L.ln[L.ld], L.lm[L.ld]) * 4);
     } else {
       L.lc = converge_first_block_level(L);
     }

@@ -980,8 +980,8 @@ __global__ void __launch_bounds__(CV_BLOCK_THREADS) k_cv_block(CvBlock a) {
 // tridiagonal systems (ax Tx + ay lambda_k) e_k = r_k in x, one per cosine
 // mode, solved here by parallel cyclic reduction.  The whole coarse part of
 // the V-cycle below level ld is replaced by this exact solve: a cosine
-// transform (k_cv_dfwd), the m tridiagonal solves (k_cv_dpcr) and the inverse
-// transform (k_cv_dbwd).
+// transform (k_cv_dct<true>), the m tridiagonal solves (k_cv_dpcr) and the
+// inverse transform (k_cv_dct<false>).
 constexpr int CV_DIRECT_MAX_CELLS = 65536;
 constexpr int CV_DIRECT_MAX_M = 128;
 constexpr int CV_DIRECT_MAX_N = 1024;
@@ -990,8 +990,11 @@ struct CvDirect {
   int n, m;
   float ax, g;
   const float* r;      // level-ld rhs [n][m]
-  const float* cy;     // cosine basis Cy[k][j] (orthonormal DCT-II)
+  const float* cy;     // cosine basis Cy[k][j] (orthonormal DCT-II), then its transpose
   const float* ly;     // ay * lambda_k
+  float2* kk;          // cyclic reduction's multipliers [m][steps][n] (k_cv_dfactor)
+  float* dd;           // and its final diagonals [m][n]
+  int steps;
   float* rhat;         // mode coefficients of r, transposed [m][n]
   float* ehat;         // mode coefficients of e, transposed [m][n]
   float* e;            // level-ld correction [n][m]
@@ -1008,137 +1011,189 @@ int converge_direct_level(const Layout& L) {
   return 0;
 }
 
-// rhat[k][i] = sum_j Cy[k][j] r[i][j]: 32 x 32 output tiles; both operand
-// panels (32 x m, m <= 128) are staged whole, so the block waits for global
-// memory once; thread (tx, ty) owns i = i0 + tx and the modes k0 + ty + 8q
-constexpr int CV_DT = 32;
-constexpr int CV_DK = CV_DIRECT_MAX_M + 1;
-__global__ void __launch_bounds__(256) k_cv_dfwd(CvDirect a) {
+// The cosine transforms: FWD rhat[k][i] = sum_j Cy[k][j] r[i][j], else
+// e[i][j] = sum_k ehat[k][i] Cy[k][j] (with the transposed basis both are row
+// by row products).  16 x 32 output tiles, 2 outputs a thread: at 512 x 128
+// that is 128 blocks, and since the three kernels of this solve are bound by
+// their own latency (one block's staging round, its product and a launch),
+// more and lighter blocks win: 32 x 32 tiles with 4-byte reads took 8 us each
+// cold, 16-byte reads of both panels and of the shared rows 5.2 -> TIME us.
+// The basis is staged before the wait for the previous kernel.
+constexpr int CV_DI = 16, CV_DC = 32;
+constexpr int CV_DK = CV_DIRECT_MAX_M + 4;   // row stride: 16-byte rows, free of bank conflicts
+template <bool FWD>
+__global__ void __launch_bounds__(256) k_cv_dct(CvDirect a) {
+  __shared__ __align__(16) float As[CV_DI][CV_DK];   // a row of r, or a column of ehat
+  __shared__ __align__(16) float Cs[CV_DC][CV_DK];   // rows of the basis
+  const int n = a.n, m = a.m, m4 = (m + 3) & ~3;
+  const int i0 = blockIdx.x * CV_DI, c0 = blockIdx.y * CV_DC;
+  const int t = threadIdx.x;
+  const float* __restrict__ basis = a.cy + (FWD ? 0 : (long)m * m);
+  const bool vec = (m & 3) == 0;   // 16-byte rows (the buffers are 256-byte aligned)
+  if (vec) {
+    for (int q = t; q < CV_DC * (m >> 2); q += 256) {
+      const int row = q / (m >> 2), c = (q - row * (m >> 2)) * 4;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c0 + row < m) v = __ldg(reinterpret_cast<const float4*>(basis + (long)(c0 + row) * m + c));
+      *reinterpret_cast<float4*>(&Cs[row][c]) = v;
+    }
+  } else {
+    for (int q = t; q < CV_DC * m4; q += 256) {
+      const int row = q / m4, c = q - row * m4;
+      Cs[row][c] = c0 + row < m && c < m ? ldg(basis + (long)(c0 + row) * m + c) : 0.f;
+    }
+  }
   pdl_wait();
   if (*a.done) return;
-  __shared__ float Cs[CV_DT][CV_DK];
-  __shared__ float Rs[CV_DT][CV_DK];
-  const int n = a.n, m = a.m;
-  const int i0 = blockIdx.x * CV_DT, k0 = blockIdx.y * CV_DT;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int rr = ty; rr < CV_DT; rr += 8) {
-    const int k = k0 + rr, i = i0 + rr;
-    for (int j = tx; j < m; j += CV_DT) {
-      Cs[rr][j] = k < m ? ldg(a.cy + (long)k * m + j) : 0.f;
-      Rs[rr][j] = i < n ? ldg(a.r + (long)i * m + j) : 0.f;
+  if (FWD && vec) {
+    for (int q = t; q < CV_DI * (m >> 2); q += 256) {
+      const int row = q / (m >> 2), c = (q - row * (m >> 2)) * 4;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i0 + row < n) v = __ldg(reinterpret_cast<const float4*>(a.r + (long)(i0 + row) * m + c));
+      *reinterpret_cast<float4*>(&As[row][c]) = v;
+    }
+  } else if (FWD) {
+    for (int q = t; q < CV_DI * m4; q += 256) {
+      const int row = q / m4, c = q - row * m4;
+      As[row][c] = i0 + row < n && c < m ? ldg(a.r + (long)(i0 + row) * m + c) : 0.f;
+    }
+  } else {   // [mode][row] in global memory: transposed on the way
+#pragma unroll 4
+    for (int q = t; q < CV_DI * m4; q += 256) {
+      const int row = q & (CV_DI - 1), c = q / CV_DI;
+      As[row][c] = i0 + row < n && c < m ? ldg(a.ehat + (long)c * n + i0 + row) : 0.f;
     }
   }
   __syncthreads();
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  // thread: row t & 15 and columns t >> 4 and 16 + (t >> 4) forward (rhat is
+  // stored row by row), else column t & 31 and rows t >> 5 and 8 + (t >> 5)
+  const int ri = FWD ? (t & 15) : (t >> 5), rc = FWD ? (t >> 4) : (t & 31);
+  const float* pa0 = As[ri];
+  const float* pa1 = As[FWD ? ri : ri + 8];
+  const float* pc0 = Cs[rc];
+  const float* pc1 = Cs[FWD ? rc + 16 : rc];
+  float s0 = 0.f, s1 = 0.f;
 #pragma unroll 8
-  for (int j = 0; j < m; ++j) {
-    const float rv = Rs[tx][j];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[q] = fmaf(Cs[ty + 8 * q][j], rv, acc[q]);
+  for (int j = 0; j < m4; j += 4) {
+    const float4 x0 = *reinterpret_cast<const float4*>(pa0 + j);
+    const float4 y0 = *reinterpret_cast<const float4*>(pc0 + j);
+    const float4 x1 = FWD ? x0 : *reinterpret_cast<const float4*>(pa1 + j);
+    const float4 y1 = FWD ? *reinterpret_cast<const float4*>(pc1 + j) : y0;
+    s0 = fmaf(x0.x, y0.x, s0);
+    s1 = fmaf(x1.x, y1.x, s1);
+    s0 = fmaf(x0.y, y0.y, s0);
+    s1 = fmaf(x1.y, y1.y, s1);
+    s0 = fmaf(x0.z, y0.z, s0);
+    s1 = fmaf(x1.z, y1.z, s1);
+    s0 = fmaf(x0.w, y0.w, s0);
+    s1 = fmaf(x1.w, y1.w, s1);
   }
-  const int i = i0 + tx;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int k = k0 + ty + 8 * q;
-    if (i < n && k < m) a.rhat[(long)k * n + i] = acc[q];
+  if (FWD) {
+    const int i = i0 + ri, k = c0 + rc;
+    if (i < n && k < m) a.rhat[(long)k * n + i] = s0;
+    if (i < n && k + 16 < m) a.rhat[(long)(k + 16) * n + i] = s1;
+  } else {
+    const int i = i0 + ri, j = c0 + rc;
+    if (i < n && j < m) a.e[(long)i * m + j] = s0;
+    if (i + 8 < n && j < m) a.e[(long)(i + 8) * m + j] = s1;
   }
 }
 
-// one block per cosine mode k: parallel cyclic reduction of
-// (ax Tx + ay lambda_k) ehat_k = rhat_k, n unknowns along x
-__global__ void __launch_bounds__(1024) k_cv_dpcr(CvDirect a) {
-  pdl_wait();
-  if (*a.done) return;
+// Parallel cyclic reduction of (ax Tx + ay lambda_k) ehat_k = rhat_k, n
+// unknowns along x, one block per cosine mode k.  Everything but the
+// right-hand side depends on the grid alone, so aj_prepare runs the
+// reduction of the matrix once and keeps each step's two multipliers and the
+// final diagonals (k_cv_dfactor): a solve then reads them in one round trip,
+// before the wait for the transform, and a step is two products where it was
+// two divisions and eight shared reads.
+__global__ void __launch_bounds__(1024) k_cv_dfactor(CvDirect a) {
   extern __shared__ __align__(16) float sh[];
-  const int n = a.n, k = blockIdx.x;
-  float* A0 = sh;
-  float* B0 = A0 + n;
-  float* C0 = B0 + n;
-  float* D0 = C0 + n;
-  float* A1 = D0 + n;
-  float* B1 = A1 + n;
-  float* C1 = B1 + n;
-  float* D1 = C1 + n;
-  const int i = threadIdx.x;
-  const float lyk = ldg(a.ly + k);
+  const int n = a.n, k = blockIdx.x, i = threadIdx.x;
+  float *Ac = sh, *Bc = Ac + n, *Cc = Bc + n, *An = Cc + n, *Bn = An + n, *Cn = Bn + n;
   if (i < n) {
     float dx = -2.f;
     if (i == 0) dx += 1.f;
     if (i == n - 1) dx += a.g;
-    A0[i] = i > 0 ? a.ax : 0.f;
-    C0[i] = i < n - 1 ? a.ax : 0.f;
-    B0[i] = fmaf(a.ax, dx, lyk);
-    D0[i] = ldg(a.rhat + (long)k * n + i);
+    Ac[i] = i > 0 ? a.ax : 0.f;
+    Cc[i] = i < n - 1 ? a.ax : 0.f;
+    Bc[i] = fmaf(a.ax, dx, ldg(a.ly + k));
   }
   __syncthreads();
-  float *Ac = A0, *Bc = B0, *Cc = C0, *Dc = D0, *An = A1, *Bn = B1, *Cn = C1, *Dn = D1;
-  for (int st = 1; st < n; st <<= 1) {
+  for (int st = 1, s = 0; st < n; st <<= 1, ++s) {
     if (i < n) {
-      const float ai = Ac[i], bi = Bc[i], ci = Cc[i], di = Dc[i];
-      float an = 0.f, bn = bi, cn = 0.f, dn = di;
+      float an = 0.f, bn = Bc[i], cn = 0.f, k1 = 0.f, k2 = 0.f;
       if (i - st >= 0) {
-        const float k1 = ai / Bc[i - st];
+        k1 = Ac[i] / Bc[i - st];
         an = -Ac[i - st] * k1;
         bn -= Cc[i - st] * k1;
-        dn -= Dc[i - st] * k1;
       }
       if (i + st < n) {
-        const float k2 = ci / Bc[i + st];
+        k2 = Cc[i] / Bc[i + st];
         cn = -Cc[i + st] * k2;
         bn -= Ac[i + st] * k2;
-        dn -= Dc[i + st] * k2;
       }
       An[i] = an;
       Bn[i] = bn;
       Cn[i] = cn;
-      Dn[i] = dn;
+      a.kk[((long)k * a.steps + s) * n + i] = make_float2(k1, k2);
     }
     __syncthreads();
     float* t;
     t = Ac; Ac = An; An = t;
     t = Bc; Bc = Bn; Bn = t;
     t = Cc; Cc = Cn; Cn = t;
-    t = Dc; Dc = Dn; Dn = t;
   }
-  if (i < n) a.ehat[(long)k * n + i] = Dc[i] / Bc[i];
+  if (i < n) a.dd[(long)k * n + i] = Bc[i];
 }
 
-// e[i][j] = sum_k ehat[k][i] Cy[k][j]: 32 x 32 output tiles, both m x 32
-// operand panels staged whole; thread (tx, ty) owns j = j0 + tx and the rows
-// i0 + ty + 8q
-__global__ void __launch_bounds__(256) k_cv_dbwd(CvDirect a) {
+template <int STEPS>
+__global__ void __launch_bounds__(1024) k_cv_dpcr(CvDirect a) {
+  __shared__ float D[2][CV_DIRECT_MAX_N];
+  const int n = a.n, k = blockIdx.x, i = threadIdx.x;
+  const bool in = i < n;
+  float2 kk[STEPS];
+  float dd = 1.f;
+#pragma unroll
+  for (int s = 0; s < STEPS; ++s)
+    kk[s] = in ? __ldg(a.kk + ((long)k * STEPS + s) * n + i) : make_float2(0.f, 0.f);
+  if (in) dd = ldg(a.dd + (long)k * n + i);
   pdl_wait();
   if (*a.done) return;
-  __shared__ float Es[CV_DIRECT_MAX_M][CV_DT + 1];
-  __shared__ float Cs[CV_DIRECT_MAX_M][CV_DT + 1];
-  const int n = a.n, m = a.m;
-  const int j0 = blockIdx.x * CV_DT, i0 = blockIdx.y * CV_DT;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int k = ty; k < m; k += 8) {
-    const int i = i0 + tx, j = j0 + tx;
-    Es[k][tx] = i < n ? ldg(a.ehat + (long)k * n + i) : 0.f;
-    Cs[k][tx] = j < m ? ldg(a.cy + (long)k * m + j) : 0.f;
-  }
-  __syncthreads();
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-  for (int k = 0; k < m; ++k) {
-    const float cv = Cs[k][tx];
+  float d = in ? ldg(a.rhat + (long)k * n + i) : 0.f;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[q] = fmaf(Es[k][ty + 8 * q], cv, acc[q]);
+  for (int s = 0; s < STEPS; ++s) {
+    const int st = 1 << s;
+    float* b = D[s & 1];
+    if (in) b[i] = d;
+    __syncthreads();
+    if (in && i - st >= 0) d -= b[i - st] * kk[s].x;
+    if (in && i + st < n) d -= b[i + st] * kk[s].y;
   }
-  const int j = j0 + tx;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int i = i0 + ty + 8 * q;
-    if (i < n && j < m) a.e[(long)i * m + j] = acc[q];
-  }
+  if (in) a.ehat[(long)k * n + i] = d / dd;
+}
+
+static int direct_steps(int n) {
+  int s = 0;
+  for (int st = 1; st < n; st <<= 1) ++s;
+  return s;
+}
+size_t converge_direct_floats(int n, int m) {   // the multipliers, then the diagonals
+  return (size_t)n * m * (2 * direct_steps(n) + 1);
+}
+
+template <int STEPS>
+static void dpcr_launch(const CvDirect& d, cudaStream_t st) {
+  if (d.steps == STEPS)
+    launch_pdl(true, k_cv_dpcr<STEPS>, dim3(d.m), dim3(cdiv(d.n, 32) * 32), 0, st, d);
+  else if constexpr (STEPS > 1)
+    dpcr_launch<STEPS - 1>(d, st);
 }
 
 static void direct_launch(const CvDirect& d, cudaStream_t st) {
-  launch_pdl(true, k_cv_dfwd, dim3(cdiv(d.n, CV_DT), cdiv(d.m, CV_DT)), dim3(CV_DT, 8), 0, st, d);
-  launch_pdl(true, k_cv_dpcr, dim3(d.m), dim3(cdiv(d.n, 32) * 32), 8 * d.n * sizeof(float), st, d);
-  launch_pdl(true, k_cv_dbwd, dim3(cdiv(d.m, CV_DT), cdiv(d.n, CV_DT)), dim3(CV_DT, 8), 0, st, d);
+  const dim3 g(cdiv(d.n, CV_DI), cdiv(d.m, CV_DC));
+  launch_pdl(true, k_cv_dct<true>, dim3(g), dim3(256), 0, st, d);
+  dpcr_launch<10>(d, st);   // n <= CV_DIRECT_MAX_N = 2^10
+  launch_pdl(true, k_cv_dct<false>, dim3(g), dim3(256), 0, st, d);
 }
 
 static CvDirect direct_args(const AjStepParams& p, const Layout& L, void* ws, const int* done);
@@ -1414,6 +1469,9 @@ static CvDirect direct_args(const AjStepParams& p, const Layout& L, void* ws, co
   d.r = at<float>(ws, L.B[L.ld]);
   d.cy = at<float>(ws, L.dcy);
   d.ly = at<float>(ws, L.dly);
+  d.steps = direct_steps(d.n);
+  d.kk = at<float2>(ws, L.dpf);
+  d.dd = at<float>(ws, L.dpf) + 2 * (size_t)d.n * d.m * d.steps;
   d.rhat = at<float>(ws, L.X[L.ld]);
   d.ehat = at<float>(ws, L.dtmp);
   d.e = at<float>(ws, L.T[L.ld]);
@@ -1659,11 +1717,12 @@ int converge_prepare(const AjStepParams& p, const Layout& L, void* ws, cudaStrea
     const int m = L.lm[L.ld];
     const double hy = p.dy * (double)(1 << L.ld), ay = 1.0 / (hy * hy);
     const double pi = 3.14159265358979323846;
-    cy.resize((size_t)m * m);
+    cy.resize(2 * (size_t)m * m);
     ly.resize(m);
     for (int k = 0; k < m; ++k) {
       const double sk = k == 0 ? sqrt(1.0 / m) : sqrt(2.0 / m);
       for (int j = 0; j < m; ++j) cy[(size_t)k * m + j] = (float)(sk * cos(pi * k * (2 * j + 1) / (2.0 * m)));
+      for (int j = 0; j < m; ++j) cy[(size_t)m * m + (size_t)j * m + k] = cy[(size_t)k * m + j];
       const double sn = sin(pi * k / (2.0 * m));
       ly[k] = (float)(-4.0 * ay * sn * sn);
     }
@@ -1672,6 +1731,9 @@ int converge_prepare(const AjStepParams& p, const Layout& L, void* ws, cudaStrea
         cudaMemcpyAsync(at<float>(ws, L.dly), ly.data(), ly.size() * 4, cudaMemcpyHostToDevice,
                         st) != cudaSuccess)
       return AJ_ERR_CUDA;
+    const CvDirect d = direct_args(p, L, ws, nullptr);
+    k_cv_dfactor<<<d.m, cdiv(d.n, 32) * 32, 6 * d.n * sizeof(float), st>>>(d);
+    if (cudaGetLastError() != cudaSuccess) return AJ_ERR_CUDA;
   }
   if (cudaFuncSetAttribute(k_cv_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)kBlockSmemMax + 1024) != cudaSuccess)

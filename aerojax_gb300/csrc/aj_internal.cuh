@@ -56,6 +56,7 @@ struct Layout {
   int lc = 0;                                           // first level of the coarse solve
   int ld = 0;                                           // level of the separable direct solve (0: none)
   size_t dcy = 0, dly = 0, dtmp = 0;                    // its cosine basis, y eigenvalues, scratch
+  size_t dpf = 0;                                       // its factored tridiagonal systems
   size_t nn_act = 0;                                    // learned warm start: activations
   size_t part = 0;                                      // per-block partial sums (FP64)
   size_t total = 0;
@@ -369,6 +370,7 @@ int converge_init(const AjStepParams& p, const Layout& L, void* ws, const float*
 size_t converge_block_smem(const Layout& L, int lc);
 int converge_first_block_level(const Layout& L);
 int converge_direct_level(const Layout& L);
+size_t converge_direct_floats(int n, int m);
 // level-0 tile shape of a grid (0 until converge_autotune has run for it)
 int tile_variant(int nx, int ny);
 int converge_autotune(const AjStepParams& p, const Layout& L, void* ws, int reps, float* times_ms,

@@ -337,6 +337,13 @@ def test_converging_shapes(cuda_lib, shape):
     assert rel(p, pref) <= 2.0 * rel(p6, pref) + 2e-6
 
 
+@pytest.mark.parametrize("shape", [(36, 6), (68, 44), (100, 20), (2048, 16)])
+def test_converging_direct_solve_shapes(cuda_lib, shape):
+    """The separable coarse solve where its rows are not a multiple of 4 (18x3,
+    34x22, 50x10) and at its longest systems (1024x8)."""
+    test_converging_shapes(cuda_lib, shape)
+
+
 _PDL_SCRIPT = r"""
 import sys, numpy as np, torch
 sys.path.insert(0, sys.argv[1])

@@ -784,6 +784,9 @@ int32_t aj_ensemble_step(int32_t n, const AjStepParams* prms, const float* const
     key += make_key(4, P[i], {ws[i], u[i], v[i], mask[i], pg, u_out[i], v_out[i], p_out[i],
                               stats ? (const void*)(stats + i) : nullptr});
   }
+  double cells = 0.0;
+  for (int i = 0; i < n; ++i) cells += (double)P[i].nx * P[i].ny;
+  for (int i = 0; i < n; ++i) Ls[i].crowd = (float)(cells / ((double)P[i].nx * P[i].ny));
   // one graph: the instances are independent branches forked from the
   // capturing stream and joined back, so they run concurrently
   return run_captured(key, (cudaStream_t)stream, [&](cudaStream_t s) {

@@ -187,20 +187,34 @@ struct TileCfg {
   static_assert(TI % 2 == 0 && TJ % 2 == 0, "tile interiors must align with the coarse grid");
   static_assert(NTH % PAIRS == 0, "threads must fill whole rows of column pairs");
 };
-using T0 = TileCfg<48, 64, 256>;   // level 0: 38 x 54 interior (default)
-using T0b = TileCfg<32, 64, 256>;  // level 0: 22 x 54 interior (more, shorter tiles)
-using T0c = TileCfg<64, 32, 256>;  // level 0: 54 x 22 interior (narrow tiles)
-using T1 = TileCfg<32, 32, 256>;   // coarser levels: 22 x 22 interior
+// Tile shapes, chosen per level by its size (cv_shape): large tiles where the
+// grid fills the GPU several times and the halo's share of the work counts,
+// small ones (and more threads each) where a few blocks' own chains set the
+// time.
+template <int NS, bool VEC = false>
+using TileL = TileCfg<48, 64, 256, NS, VEC>;   // 38 x 54 interior (42 x 58 with one sweep)
+template <int NS, bool VEC = false>
+using TileM = TileCfg<32, 32, 256, NS, VEC>;   // 22 x 22 (26 x 26)
+template <int NS, bool VEC = false>
+using TileS = TileCfg<32, 32, 512, NS, VEC>;
 // Level 0 post-smooths with one sweep (a V(2,1) cycle on the fine grid,
 // V(2,2) below it): the same tiles with a halo of 3
 constexpr int CV_NS_UP0 = 1;
-using T0u = TileCfg<48, 64, 256, CV_NS_UP0>;    // 42 x 58 interior
-using T0bu = TileCfg<32, 64, 256, CV_NS_UP0>;   // 26 x 58 interior
-using T0cu = TileCfg<64, 32, 256, CV_NS_UP0>;   // 58 x 26 interior
-using T0uv = TileCfg<48, 64, 256, CV_NS_UP0, true>;
-using T0buv = TileCfg<32, 64, 256, CV_NS_UP0, true>;
-using T0cuv = TileCfg<64, 32, 256, CV_NS_UP0, true>;
 constexpr int CV_TILE_VARIANTS = 3;
+constexpr int CV_SMALL_TILES = 360, CV_LARGE_TILES = 450;
+// The shape (0 large, 1 medium, 2 small) of an n x m level, by its tiles of 32x32
+// and of 48x64.  Level-0 down and up kernels together, inside a stream, us
+// (48x64 with 256 threads / 32x32 with 256 / 32x32 with 512): 256x64 14.7 /
+// 7.2 / 5.8, 768x192 15.0 / 9.1 / 8.7, 1024x192 15.0 / 10.1 / 10.6, 1440x352
+// 18.9 / 16.8 / 18.9, 1728x448 23.3 / 21.8 / 25.6, 1792x512 24.8 / 25.3 /
+// 30.0, 2048x512 25.3 / 28.1 / 33.5, 4096x2048 143 / 183 / 242.
+// crowd: how many such levels run side by side (an ensemble's instances by
+// their cells): it is the tiles of all of them that fill the GPU (16 channels
+// of 256x64 to 1024x256 as one batch: 564 us by each one's own size, 544 so).
+static int cv_shape(int n, int m, float crowd = 1.f) {
+  const float small = crowd * cdiv(n, 22) * cdiv(m, 22), large = crowd * cdiv(n, 38) * cdiv(m, 54);
+  return small <= CV_SMALL_TILES ? 2 : large < CV_LARGE_TILES ? 1 : 0;
+}
 
 __device__ __forceinline__ float cv_diag(const CvLvl& L, int gi, int gj) {
   float d = -2.f * (L.ax + L.ay);
@@ -422,14 +436,16 @@ __global__ void __launch_bounds__(TC::NTH) k_cv_down(CvLvl L, const float* r0, c
   pdl_wait();
   constexpr int SJ = TC::SJ, TI = TC::TI, TJ = TC::TJ;
   static_assert(!TC::VEC, "the pre-smoothing indexes its tile with stride SJ");
-  if (*done) return;
+  // both flags in one round trip, the first tested while the tile is loaded
+  const int skip = *done, second = r1 ? *cur : 0;
   __shared__ float E[TC::NT];
   __shared__ float R[TC::NT];
   const int i0 = blockIdx.y * TI, j0 = blockIdx.x * TJ;
   const int gi0 = i0 - TC::H, gj0 = j0 - TC::H;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const float* r = (r1 && *cur) ? r1 : r0;
+  const float* r = second ? r1 : r0;
   cv_load_r<TC>(E, R, L, gi0, gj0, r);
+  if (skip) return;
   cv_sweeps<TC>(E, R, L, gi0, gj0);
   // store e and compute the residual on the tile interior (in place in R:
   // every residual of this thread first, then the stores, so that no store
@@ -515,7 +531,6 @@ __global__ void __launch_bounds__(TC::NTH) k_cv_up(CvLvl L, const float* __restr
 }
 
 struct CvCheck {
-  double rtol;
   int max_cycles;
   int use_handle;
   cudaGraphConditionalHandle h;
@@ -524,21 +539,20 @@ struct CvCheck {
 // convergence bookkeeping after a V-cycle (device scalars; one thread).  All
 // fields are loaded before any is stored: interleaved, every load waited for
 // the store before it (a chain of dependent round trips at the end of the
-// cycle's last kernel).
+// cycle's last kernel).  The test compares squares - sum r^2 against the
+// solve's target rtol^2 sum b^2 - so that no FP64 root or quotient (1/64 of
+// the FP32 rate) stands between two cycles; k_cv_out forms the norms.
 __device__ void cv_check_body(DevScalars* sc, const CvCheck& ck) {
   int done = sc->mg_done, cycles = sc->mg_cycles, err = sc->err, loops = sc->loops;
-  const double bnorm = sc->bnorm, a0 = sc->acc[0];
+  const double target = sc->target, a0 = sc->acc[0];
   const int was_done = done;
   if (!was_done) {
     cycles += 1;
-    const double nb = bnorm > 0.0 ? bnorm : 1.0;
-    const double rel = sqrt(a0) / nb;
-    sc->rel = rel;
     sc->abs_sq = a0;
-    if (!isfinite(rel)) {
+    if (!isfinite(a0)) {
       err = AJ_ERR_NONFINITE;
       done = 1;
-    } else if (rel <= ck.rtol) {
+    } else if (a0 <= target) {
       done = 1;
     } else if (cycles >= ck.max_cycles) {
       err = AJ_ERR_NOT_CONVERGED;
@@ -575,7 +589,7 @@ struct PState {
 // the current residual over its tile and halo while its neighbours write the
 // next one, so the two must never share a buffer.
 template <class TC>
-__global__ void __launch_bounds__(TC::NTH, 4) k_cv_up0(
+__global__ void __launch_bounds__(TC::NTH, 1024 / TC::NTH) k_cv_up0(
     CvLvl L, PState rs, const float* __restrict__ e_in,
     const float* __restrict__ ec, int nc, int mc, float gc, PState ps, const float* __restrict__ b,
     DevScalars* sc, DfCoef co, CvCheck ck, int profile) {
@@ -1362,14 +1376,13 @@ __global__ void __launch_bounds__(256) k_cv_resid(const float* __restrict__ ps,
     // every field first, then the stores (see cv_check_body)
     const HistView hv = hist_view(sc);
     const double a0 = sc->acc[0], a1 = sc->acc[1];
-    const double bnorm = sqrt(a1);
-    const double nb = bnorm > 0.0 ? bnorm : 1.0;
-    const double rel = sqrt(a0) / nb;
+    // ||r|| <= rtol ||b|| (rtol alone for b = 0), in squares
+    const double target = rtol * rtol * (a1 > 0.0 ? a1 : 1.0);
     int err = AJ_OK, done = 0;
-    if (!isfinite(rel)) {
+    if (!isfinite(a0) || !isfinite(target)) {
       err = AJ_ERR_NONFINITE;
       done = 1;
-    } else if (rel <= rtol) {
+    } else if (a0 <= target) {
       done = 1;
     }
     sc->hist_cur = hv.cur;
@@ -1380,8 +1393,8 @@ __global__ void __launch_bounds__(256) k_cv_resid(const float* __restrict__ ps,
     sc->mg_cycles = 0;
     sc->loops = 0;
     sc->pcur = 0;
-    sc->bnorm = bnorm;
-    sc->rel = rel;
+    sc->bsq = a1;
+    sc->target = target;
     sc->abs_sq = a0;
     sc->acc[0] = 0.0;
     sc->acc[1] = 0.0;
@@ -1410,7 +1423,8 @@ __global__ void k_cv_out(PState ps, DevScalars* sc, float* __restrict__ p, long 
     // every field first, then the stores (stats may alias nothing the
     // compiler can prove, so interleaved each load waited for a store)
     const int cycles = sc->mg_cycles, done = sc->mg_done, err = sc->err;
-    const double rel = sc->rel, bnorm = sc->bnorm, abs_sq = sc->abs_sq;
+    const double bsq = sc->bsq, abs_sq = sc->abs_sq;
+    const double bnorm = sqrt(bsq), rel = sqrt(abs_sq) / (bnorm > 0.0 ? bnorm : 1.0);
     const float dt = sc->dt;
     if (hist) {
       sc->hist_pending = 1;
@@ -1510,26 +1524,45 @@ static void level0_up(const AjStepParams& p, const CvLvl& c, const Layout& L, vo
              at<float>(ws, L.b0), sc, df_coef(1.0 / (p.dx * p.dx), 1.0 / (p.dy * p.dy)), ck,
              profile);
 }
-static void level0_down_v(int v, const CvLvl& c, const Layout& L, void* ws, const int* done,
+// variant v of a level: 0 the shape that its size gives, the others the
+// autotuner's alternatives
+static int variant_shape(int v, const CvLvl& c) { return (cv_shape(c.n, c.m) + v) % CV_TILE_VARIANTS; }
+static void level0_down_s(int sh, const CvLvl& c, const Layout& L, void* ws, const int* done,
                           cudaStream_t st) {
-  if (v == 1) level0_down<T0b>(c, L, ws, done, st);
-  else if (v == 2) level0_down<T0c>(c, L, ws, done, st);
-  else level0_down<T0>(c, L, ws, done, st);
+  if (sh == 2) level0_down<TileS<CV_NS>>(c, L, ws, done, st);
+  else if (sh == 1) level0_down<TileM<CV_NS>>(c, L, ws, done, st);
+  else level0_down<TileL<CV_NS>>(c, L, ws, done, st);
 }
 // the 16-byte staged tiles need rows of a multiple of 4 floats and every
 // staged buffer 16-byte aligned (workspace offsets are multiples of 256)
 static bool level0_vec_ok(const CvLvl& c, const void* ws) {
   return c.m % 4 == 0 && (reinterpret_cast<uintptr_t>(ws) & 15) == 0;
 }
-static void level0_up_v(int v, const AjStepParams& p, const CvLvl& c, const Layout& L, void* ws,
+static void level0_up_s(int sh, const AjStepParams& p, const CvLvl& c, const Layout& L, void* ws,
                         DevScalars* sc, const CvCheck& ck, int profile, cudaStream_t st) {
-  const bool vec = level0_vec_ok(c, ws);
-  if (v == 1) vec ? level0_up<T0buv>(p, c, L, ws, sc, ck, profile, st)
-                  : level0_up<T0bu>(p, c, L, ws, sc, ck, profile, st);
-  else if (v == 2) vec ? level0_up<T0cuv>(p, c, L, ws, sc, ck, profile, st)
-                       : level0_up<T0cu>(p, c, L, ws, sc, ck, profile, st);
-  else vec ? level0_up<T0uv>(p, c, L, ws, sc, ck, profile, st)
-           : level0_up<T0u>(p, c, L, ws, sc, ck, profile, st);
+  auto run = [&](auto plain, auto vec) {
+    if (level0_vec_ok(c, ws)) level0_up<decltype(vec)>(p, c, L, ws, sc, ck, profile, st);
+    else level0_up<decltype(plain)>(p, c, L, ws, sc, ck, profile, st);
+  };
+  if (sh == 2) run(TileS<CV_NS_UP0>{}, TileS<CV_NS_UP0, true>{});
+  else if (sh == 1) run(TileM<CV_NS_UP0>{}, TileM<CV_NS_UP0, true>{});
+  else run(TileL<CV_NS_UP0>{}, TileL<CV_NS_UP0, true>{});
+}
+
+// the kernels of a level >= 1 in its size's shape
+template <class TC>
+static void level_down(const CvLvl& c, const Layout& L, void* ws, int l, const int* done,
+                       cudaStream_t st) {
+  launch_pdl(true, k_cv_down<TC>, dim3(tiles<TC>(c)), dim3(tile_threads<TC>()), 0, st, c,
+             at<float>(ws, L.B[l]), nullptr, done, at<float>(ws, L.X[l]),
+             at<float>(ws, L.B[l + 1]), done);
+}
+template <class TC>
+static void level_up(const CvLvl& c, const Layout& L, void* ws, int l, const int* done,
+                     cudaStream_t st) {
+  launch_pdl(true, k_cv_up<TC>, dim3(tiles<TC>(c)), dim3(tile_threads<TC>()), 0, st, c,
+             at<float>(ws, L.B[l]), at<float>(ws, L.X[l]), at<float>(ws, L.T[l + 1]), L.ln[l + 1],
+             L.lm[l + 1], (float)ghost_factor(l + 1), at<float>(ws, L.T[l]), done);
 }
 
 // one refinement iteration
@@ -1538,14 +1571,17 @@ static void cv_body(const AjStepParams& p, const Layout& L, void* ws,
   DevScalars* sc = at<DevScalars>(ws, 0);
   const int* done = &sc->mg_done;
   const int lc = L.lc;
+  // level 0: the autotuned shape, but beside other instances the rule's
+  const CvLvl c0 = cv_level(p, L, 0);
+  const int sh0 = L.crowd > 1.f ? cv_shape(c0.n, c0.m, L.crowd)
+                                : variant_shape(tile_variant(p.nx, p.ny), c0);
   for (int l = 0; l < lc; ++l) {
     CvLvl c = cv_level(p, L, l);
-    if (l == 0)
-      level0_down_v(tile_variant(p.nx, p.ny), c, L, ws, done, st);
-    else
-      launch_pdl(true, k_cv_down<T1>, dim3(tiles<T1>(c)), dim3(tile_threads<T1>()), 0, st, c,
-                 at<float>(ws, L.B[l]), nullptr, done, at<float>(ws, L.X[l]),
-                 at<float>(ws, L.B[l + 1]), done);
+    const int sh = cv_shape(c.n, c.m, L.crowd);
+    if (l == 0) level0_down_s(sh0, c, L, ws, done, st);
+    else if (sh == 2) level_down<TileS<CV_NS>>(c, L, ws, l, done, st);
+    else if (sh == 1) level_down<TileM<CV_NS>>(c, L, ws, l, done, st);
+    else level_down<TileL<CV_NS>>(c, L, ws, l, done, st);
   }
   if (L.ld > 0) {
     direct_launch(direct_args(p, L, ws, done), st);
@@ -1554,14 +1590,21 @@ static void cv_body(const AjStepParams& p, const Layout& L, void* ws,
   }
   for (int l = lc - 1; l >= 1; --l) {
     CvLvl c = cv_level(p, L, l);
-    launch_pdl(true, k_cv_up<T1>, dim3(tiles<T1>(c)), dim3(tile_threads<T1>()), 0, st, c,
-               at<float>(ws, L.B[l]), at<float>(ws, L.X[l]), at<float>(ws, L.T[l + 1]), L.ln[l + 1],
-               L.lm[l + 1], (float)ghost_factor(l + 1), at<float>(ws, L.T[l]), done);
+    const int sh = cv_shape(c.n, c.m, L.crowd);
+    if (sh == 2) level_up<TileS<CV_NS>>(c, L, ws, l, done, st);
+    else if (sh == 1) level_up<TileM<CV_NS>>(c, L, ws, l, done, st);
+    else level_up<TileL<CV_NS>>(c, L, ws, l, done, st);
   }
-  CvLvl c0 = cv_level(p, L, 0);
-  CvCheck ck{p.mg_rtol, p.max_cycles, use_handle, h};
-  level0_up_v(tile_variant(p.nx, p.ny), p, c0, L, ws, sc, ck, 0, st);
+  CvCheck ck{p.max_cycles, use_handle, h};
+  level0_up_s(sh0, p, c0, L, ws, sc, ck, 0, st);
 }
+
+// Cycles recorded in line before the while node.  An iteration of the node
+// costs ~4 us beyond its kernels (a cycle at 2048x512 49 us in line, 53 us in
+// the node), a cycle skipped in line ~1 us a kernel, so as many are unrolled as
+// nearly every solve runs: two from a warm start (two or three run), four
+// from zero (four or five).
+constexpr int CV_INLINE_WARM = 2, CV_INLINE_ZERO = 4;
 
 static cudaStream_t side_stream() {
   static cudaStream_t s = nullptr;
@@ -1618,9 +1661,15 @@ int converge_solve(const AjStepParams& p, const Layout& L, void* ws, const float
     int unroll = eager_unroll(p.max_cycles);
     for (int k = 0; k < unroll; ++k) cv_body(p, L, ws, 0, 0, st);
   } else {
-    // the refinement loop: a while node appended to the graph being captured
+    // the refinement loop: the first cycles in line (each of a cycle's
+    // kernels skips its work once the target is met), the others in a while
+    // node appended to the graph being captured
     cudaGraphConditionalHandle h;
     if (cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) != cudaSuccess)
+      return AJ_ERR_CUDA;
+    const int inline_cycles = p.warm_start == AJ_WARM_ZERO ? CV_INLINE_ZERO : CV_INLINE_WARM;
+    for (int k = 0; k < inline_cycles && k < p.max_cycles; ++k) cv_body(p, L, ws, h, 1, st);
+    if (cudaStreamGetCaptureInfo(st, &cs, &id, &g, &deps, &ed, &nd) != cudaSuccess)
       return AJ_ERR_CUDA;
     // the params union has no default constructor: zero-initialised storage
     alignas(cudaGraphNodeParams) unsigned char npbuf[sizeof(cudaGraphNodeParams)];
@@ -1755,13 +1804,13 @@ int profile_pressure_kernel(const AjStepParams& p, const Layout& L, void* ws, in
   DevScalars* sc = at<DevScalars>(ws, 0);
   const int* never = reinterpret_cast<const int*>(&sc->pad_[0]);   // always 0
   CvLvl c = cv_level(p, L, 0);
-  const int v = tile_variant(p.nx, p.ny);
+  const int sh = variant_shape(tile_variant(p.nx, p.ny), c);
   if (which == 0) {
-    level0_down_v(v, c, L, ws, never, st);
+    level0_down_s(sh, c, L, ws, never, st);
   } else if (which == 1) {
-    CvCheck ck{p.mg_rtol, p.max_cycles, 0, 0};
+    CvCheck ck{p.max_cycles, 0, 0};
     // profile mode reads the current state buffer and writes only the other one
-    level0_up_v(v, p, c, L, ws, sc, ck, 1, st);
+    level0_up_s(sh, p, c, L, ws, sc, ck, 1, st);
   } else if (which == 2) {
     if (L.ld > 0) {
       direct_launch(direct_args(p, L, ws, never), st);
@@ -1808,7 +1857,7 @@ int converge_autotune(const AjStepParams& p, const Layout& L, void* ws, int reps
   DevScalars* sc = at<DevScalars>(ws, 0);
   const int* never = reinterpret_cast<const int*>(&sc->pad_[0]);   // always 0
   const CvLvl c = cv_level(p, L, 0);
-  const CvCheck ck{p.mg_rtol, p.max_cycles, 0, 0};
+  const CvCheck ck{p.max_cycles, 0, 0};
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
     return AJ_ERR_CUDA;
@@ -1816,13 +1865,13 @@ int converge_autotune(const AjStepParams& p, const Layout& L, void* ws, int reps
   float best_ms = 1e30f;
   for (int v = 0; v < CV_TILE_VARIANTS; ++v) {
     for (int w = 0; w < 2; ++w) {   // warm-up
-      level0_down_v(v, c, L, ws, never, st);
-      level0_up_v(v, p, c, L, ws, sc, ck, 1, st);
+      level0_down_s(variant_shape(v, c), c, L, ws, never, st);
+      level0_up_s(variant_shape(v, c), p, c, L, ws, sc, ck, 1, st);
     }
     cudaEventRecord(e0, st);
     for (int r = 0; r < reps; ++r) {
-      level0_down_v(v, c, L, ws, never, st);
-      level0_up_v(v, p, c, L, ws, sc, ck, 1, st);
+      level0_down_s(variant_shape(v, c), c, L, ws, never, st);
+      level0_up_s(variant_shape(v, c), p, c, L, ws, sc, ck, 1, st);
     }
     cudaEventRecord(e1, st);
     if (cudaEventSynchronize(e1) != cudaSuccess) {

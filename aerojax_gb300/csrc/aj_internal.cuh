@@ -24,8 +24,9 @@ struct DevScalars {
   int mg_done;         // converging mode: target met (later cycles skip)
   int err;             // device-side AjStatus
   double acc[4];       // reduction accumulators (residual, rhs, spare)
-  double rel;          // last relative residual
-  double bnorm;        // ||b||
+  double rel;          // parity: last relative residual
+  double bnorm;        // parity: ||b||
+  double bsq, target;  // converging: sum b^2, and the sum r^2 that ends the solve
   double abs_sq;       // sum r^2 dx dy
   unsigned int red_count;
   int loops;           // converging mode: executions of the while body
@@ -64,6 +65,7 @@ struct Layout {
   int nlev = 0;                 // parity: max_levels (coarsest index); converge: depth
   int ln[AJ_MAX_LEVELS + 1] = {0}, lm[AJ_MAX_LEVELS + 1] = {0};
   int ncoarse = 0;              // converging: coarsest cell count
+  float crowd = 1.f;            // instances of this size running side by side
 };
 
 // Number of dynamic-LES temporaries (nx*ny floats each).

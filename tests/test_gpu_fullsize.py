@@ -344,6 +344,12 @@ def test_converging_direct_solve_shapes(cuda_lib, shape):
     test_converging_shapes(cuda_lib, shape)
 
 
+@pytest.mark.parametrize("shape", [(1440, 352), (1056, 576), (132, 24)])
+def test_converging_tile_shapes(cuda_lib, shape):
+    """Levels in the medium and small tiles whose last tiles are partial."""
+    test_converging_shapes(cuda_lib, shape)
+
+
 _PDL_SCRIPT = r"""
 import sys, numpy as np, torch
 sys.path.insert(0, sys.argv[1])

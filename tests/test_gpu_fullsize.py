@@ -286,6 +286,34 @@ def test_post_step_dye_matches_reference(cuda_lib):
                                             diagnostics=False), cn)
 
 
+@pytest.mark.parametrize("shape", [(2, 4), (5, 8), (33, 132), (130, 260), (37, 41)])
+@pytest.mark.parametrize("flow", ["von_karman", "taylor_green"])
+@pytest.mark.parametrize("grid", ["collocated", "mac"])
+def test_post_step_shapes(cuda_lib, shape, flow, grid):
+    """The epilogue four columns a thread (rows of a multiple of 4) and one
+    cell a thread, at the ends of their tiles, against the oracle; the dye
+    alone gives the same dye."""
+    import torch
+    import aerojax_gb300 as aj
+    from oracle import ref_np as R
+    nx, ny = shape
+    mac, per = grid == "mac", flow == "taylor_green"
+    rng = np.random.default_rng(nx * ny)
+    f = lambda *s: rng.standard_normal(s).astype(np.float32)
+    u, v = f(nx + mac, ny), f(nx, ny + mac)
+    c = rng.random((nx, ny)).astype(np.float32)
+    dx, dy, dt, kappa = 0.03, 0.02, 1e-3, 1e-2
+    t = [torch.as_tensor(a, device="cuda") for a in (u, v, c)]
+    out = aj.post_step(*t, dt, dx, dy, kappa, grid_type=grid, flow_type=flow)
+    alone = aj.post_step(*t, dt, dx, dy, kappa, grid_type=grid, flow_type=flow, diagnostics=False)
+    u, v, c = (a.astype(np.float64) for a in (u, v, c))
+    ref = (R.scalar_advection_diffusion(c, u, v, dt, dx, dy, kappa, mac, per),
+           *R.diagnostics(u, v, dx, dy, mac, per))
+    for name, a, b in zip(("dye", "vorticity", "divergence", "speed"), out, ref):
+        assert rel(a, b) < 1e-6 or float(np.max(np.abs(b))) == 0.0 == float(a.abs().max()), name
+    assert torch.equal(alone, out[0])
+
+
 def test_training_data_file(cuda_lib, tmp_path):
     """generate_training_data writes the reference's .npz layout
     (training_utils.py:12-81) and the recorded fields are the solver's."""

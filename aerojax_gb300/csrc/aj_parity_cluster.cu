@@ -26,10 +26,9 @@
 // cluster barriers (~0.3 us) on 16 SMs - hence the limit on a thread's run:
 // above it the tiled kernels, which use all SMs, are the faster ones.
 // Measured: a step_pure step at 512x96 with 3 cycles 130 -> 73 us (the solve
-// in one launch instead of 28), a five-cycle solve at 1008x368 276 -> 237 us
-// and a MAC step at 2048x512 with five cycles 459 -> 400 us (levels 1 or 2 and
-// below on the cluster).
-#include "aj_internal.cuh"
+// in one launch instead of 28); a cycle at 256x64 38.7 -> 16.8 us, at 512x128
+// 39.0 -> 19.5 us.
+#include "aj_parity_pair.cuh"
 
 #include <cooperative_groups.h>
 #include <math.h>
@@ -66,37 +65,21 @@ struct ParCluster {
   const int* skip;     // not whole: cycles after convergence are skipped
   DevScalars* sc;
   AjStats* stats;      // whole solve: nullable
-  float ax, ay, den, rden;
+  PairCoef co;
   double dxdy, tol2;
 };
-
-// s / den for the sweeps' constant divisor with rden = 1 / den: s rden and one
-// Newton correction of the quotient by its exact residual (Markstein 1990),
-// three operations instead of a division per cell
-__device__ __forceinline__ float pc_div(float s, float den, float rden) {
-  const float q = s * rden;
-  return fmaf(fmaf(-q, den, s), rden, q);
-}
-__device__ __forceinline__ float2 pc_div2(float2 s, float den, float rden) {
-  const float2 q = mul2(s, f2(rden));
-  return fma2(fma2(q, f2(-den), s), f2(rden), q);
-}
 
 // a barrier of a level's active warps (the others wait at the level's end)
 __device__ __forceinline__ void pc_sync(const PcLvl& L) {
   asm volatile("bar.sync 1, %0;\n" ::"r"(L.active) : "memory");
 }
 
-__device__ __forceinline__ float2 pc_ld2(const float* p) {
-  return *reinterpret_cast<const float2*>(p);
-}
-__device__ __forceinline__ void pc_st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
-
-// A thread's cells of a level: W columns from c, rows [ga, ga + cnt) with
-// array index q; [glo, ghi): the rows of the band and its halo in the domain.
-struct PcOwn {
-  int c, ga, cnt, q, glo, ghi;
+// A thread's cells of a level: W columns from c
+struct PcOwn : PairOwn {
+  int c;
 };
+__device__ __forceinline__ bool pair_lf(const PcLvl&, const PcOwn& o) { return o.c > 0; }
+__device__ __forceinline__ bool pair_rt(const PcLvl& L, const PcOwn& o) { return o.c + 2 < L.m; }
 template <int W>
 __device__ __forceinline__ PcOwn pc_own(const PcLvl& L, int rank) {
   PcOwn o;
@@ -113,87 +96,6 @@ __device__ __forceinline__ PcOwn pc_own(const PcLvl& L, int rank) {
   return o;
 }
 
-// What a sweep or residual of the column pair needs of its neighbours, read
-// from S: the rows above and below the run, and each row's sides (edge
-// ghosts: the cell itself).  All reads are issued before any is used; rows
-// past cnt hold anything.
-struct PcNb {
-  float2 above, below;
-  float lf[PC_RUN], rt[PC_RUN];
-  bool last;   // no row below the run
-};
-__device__ __forceinline__ PcNb pc_nb(const PcLvl& L, const PcOwn& o, const float* S,
-                                      const float2* x) {
-  const int m = L.m;
-  PcNb t;
-  t.last = o.ga + o.cnt >= o.ghi;
-  t.above = o.cnt > 0 && o.ga > o.glo ? pc_ld2(S + o.q - m) : x[0];
-  t.below = o.cnt > 0 && !t.last ? pc_ld2(S + o.q + o.cnt * m) : x[0];
-#pragma unroll
-  for (int r = 0; r < PC_RUN; ++r) {
-    t.lf[r] = r < o.cnt && o.c > 0 ? S[o.q + r * m - 1] : x[r].x;
-    t.rt[r] = r < o.cnt && o.c + 2 < m ? S[o.q + r * m + 2] : x[r].y;
-  }
-  return t;
-}
-__device__ __forceinline__ float2 pc_next(const PcOwn& o, const PcNb& t, const float2* x, int r) {
-  const float2 end = t.last ? x[r] : t.below;
-  return r + 1 < PC_RUN && r + 1 < o.cnt ? x[r + 1 < PC_RUN ? r + 1 : r] : end;
-}
-
-// one undamped Jacobi sweep of the pair, the reference's order of operations
-template <bool MAC>
-__device__ __forceinline__ void pc_sweep(const ParCluster& a, const PcLvl& L, const PcOwn& o,
-                                         const float* S, const float2* b, const float* M,
-                                         bool zero_last, float2* x) {
-  const PcNb t = pc_nb(L, o, S, x);
-  float2 prev = t.above;
-#pragma unroll
-  for (int r = 0; r < PC_RUN; ++r) {
-    const float2 cur = x[r], next = pc_next(o, t, x, r);
-    const float2 sx = mul2(f2(a.ax), add2(next, prev));
-    const float2 sy = add2(make_float2(cur.y, t.rt[r]), make_float2(t.lf[r], cur.x));
-    float2 p = pc_div2(sub2(fma2(f2(a.ay), sy, sx), b[r]), a.den, a.rden);
-    if (MAC && r < o.cnt) p = mul2(p, pc_ld2(M + o.q + r * L.m));
-    if (zero_last && o.ga + r == L.n - 1) p = make_float2(0.f, 0.f);
-    x[r] = p;
-    prev = cur;
-  }
-}
-
-// b - A x of the column pair (the MAC variant zeroes A x on the outlet row):
-// f(r, value pair) for the rows it owns
-template <typename F>
-__device__ __forceinline__ void pc_resid(const ParCluster& a, const PcLvl& L, const PcOwn& o,
-                                         const float* S, const float2* b, const float2* x,
-                                         F&& f) {
-  const PcNb t = pc_nb(L, o, S, x);
-  float2 prev = t.above;
-#pragma unroll
-  for (int r = 0; r < PC_RUN; ++r) {
-    const float2 cur = x[r], next = pc_next(o, t, x, r), two = mul2(cur, f2(2.f));
-    const float2 sx = mul2(f2(a.ax), sub2(add2(next, prev), two));
-    const float2 sy = sub2(add2(make_float2(cur.y, t.rt[r]), make_float2(t.lf[r], cur.x)), two);
-    float2 lap = fma2(f2(a.ay), sy, sx);
-    if (a.mac_outlet && o.ga + r == L.n - 1) lap = make_float2(0.f, 0.f);
-    if (r < o.cnt) f(r, sub2(b[r], lap));
-    prev = cur;
-  }
-}
-
-// the pair's cells from shared memory
-__device__ __forceinline__ void pc_load(const PcLvl& L, const PcOwn& o, const float* S, float2* v) {
-#pragma unroll
-  for (int r = 0; r < PC_RUN; ++r)
-    v[r] = r < o.cnt ? pc_ld2(S + o.q + r * L.m) : make_float2(0.f, 0.f);
-}
-__device__ __forceinline__ void pc_store(const PcLvl& L, const PcOwn& o, float* S,
-                                         const float2* v) {
-#pragma unroll
-  for (int r = 0; r < PC_RUN; ++r)
-    if (r < o.cnt) pc_st2(S + o.q + r * L.m, v[r]);
-}
-
 // Stores a thread's values of own rows in the halos of the blocks that reach
 // them within h rows: f(peer's array, offset to add to an index here, first
 // row, end row).  Every block's array has the same layout R rows further on,
@@ -207,19 +109,6 @@ __device__ __forceinline__ void pc_push(cg::cluster_group& cl, float* arr, const
     if (rank + d < C) f(cl.map_shared_rank(arr, rank + d), -off, r0 + d * L.R - h, L.n);
     if (rank >= d) f(cl.map_shared_rank(arr, rank - d), off, 0, r0 - (d - 1) * L.R + h);
   }
-}
-
-// sums of (hi, lo) pairs whose lo collects the TwoSum errors of hi
-__device__ __forceinline__ df pc_add(df a, df b) {
-  const df t = two_sum(a.hi, b.hi);
-  return {t.hi, t.lo + (a.lo + b.lo)};
-}
-template <int LANES>
-__device__ __forceinline__ df pc_lanes(df s) {
-#pragma unroll
-  for (int o = LANES / 2; o > 0; o >>= 1)
-    s = pc_add(s, df{__shfl_xor_sync(~0u, s.hi, o), __shfl_xor_sync(~0u, s.lo, o)});
-  return s;
 }
 
 template <bool MAC>
@@ -264,30 +153,30 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
       const PcLvl& L = a.lv[l];
       const PcLvl& Lc = a.lv[l + 1];
       float *A = arr(l, 1), *D = arr(l, 2), *Bc = arr(l + 1, 0);
+      auto none = [](int) { return false; };
       if (tid < L.active) {
         const PcOwn o = pc_own<2>(L, rank);
         const float* M = msk(l);
+        auto mask = [&](int r) { return pair_ld(M + o.q + r * L.m); };
+        auto last = [&](int r) { return a.zero_last && o.ga + r == L.n - 1; };
         float2 x[PC_RUN], b[PC_RUN];
-        pc_load(L, o, arr(l, 0), b);
+        pair_load<PC_RUN>(L, o, arr(l, 0), b);
         if (l == 0 && (cyc > 0 || a.have_x0)) {
-          pc_load(L, o, arr(0, 3), x);
-          pc_sweep<MAC>(a, L, o, arr(0, 3), b, M, false, x);
+          pair_load<PC_RUN>(L, o, arr(0, 3), x);
+          pair_sweep<MAC, PC_RUN>(a.co, L, o, arr(0, 3), b, mask, none, x);
         } else {   // from zero
-#pragma unroll
-          for (int r = 0; r < PC_RUN; ++r) {
-            x[r] = pc_div2(sub2(f2(0.f), b[r]), a.den, a.rden);
-            if (MAC && r < o.cnt) x[r] = mul2(x[r], pc_ld2(M + o.q + r * L.m));
-          }
+          pair_sweep0<MAC, PC_RUN>(a.co, o, b, mask, x);
         }
-        pc_store(L, o, A, x);
+        pair_store<PC_RUN>(L, o, A, x);
         pc_sync(L);
-        pc_sweep<MAC>(a, L, o, A, b, M, a.zero_last, x);
-        pc_store(L, o, D, x);
+        pair_sweep<MAC, PC_RUN>(a.co, L, o, A, b, mask, last, x);
+        pair_store<PC_RUN>(L, o, D, x);
         pc_sync(L);
         const int I0 = lo(l + 1, 0), I1 = hi(l + 1, 0), bc = base(l + 1), mc = Lc.m, J = o.c >> 1;
+        auto outlet = [&](int r) { return a.mac_outlet && o.ga + r == L.n - 1; };
         float2 ra{0.f, 0.f};
         float w[PC_RUN / 2];   // the coarse rows of the run
-        pc_resid(a, L, o, D, b, x, [&](int r, float2 v) {
+        pair_resid<PC_RUN>(a.co, L, o, D, b, outlet, x, [&](int r, float2 v) {
           // runs start at even rows: rows r - 1 and r of a 2x2 block; summed in
           // the order (0,0), (1,0), (0,1), (1,1)
           if (r & 1) w[r / 2] = 0.25f * (ra.x + v.x + ra.y + v.y);
@@ -315,7 +204,7 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
         const bool in = r < o.cnt;
         b[r] = in ? arr(nl, 0)[o.q + r * m] : 0.f;
         k[r] = MAC && in ? msk(nl)[o.q + r * m] : 1.f;
-        x[r] = pc_div(0.f - b[r], a.den, a.rden);
+        x[r] = pair_div(0.f - b[r], a.co);
         if (MAC) x[r] = x[r] * k[r];
       }
       const bool last = o.ga + o.cnt >= o.ghi;
@@ -336,7 +225,7 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
           const float next =
               r + 1 < PC_RUN_COARSE && r + 1 < o.cnt ? x[r + 1 < PC_RUN_COARSE ? r + 1 : r] : end;
           const float yp = o.c + 1 < m ? S[q + 1] : cur, ym = o.c > 0 ? S[q - 1] : cur;
-          const float p = pc_div(fmaf(a.ay, yp + ym, a.ax * (next + prev)) - b[r], a.den, a.rden);
+          const float p = pair_div(fmaf(a.co.ay, yp + ym, a.co.ax * (next + prev)) - b[r], a.co);
           x[r] = MAC ? p * k[r] : p;
           prev = cur;
         }
@@ -355,53 +244,32 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
       const float* E = arr(l + 1, l + 1 == nl ? 2 : 3);
       float *A = arr(l, 1), *D = arr(l, 2), *F = arr(l, 3);
       const int ga = lo(l, 0), gb = hi(l, 0);
+      auto none = [](int) { return false; };
       float2 x[PC_RUN], b[PC_RUN];
       PcOwn o;
       if (tid < L.active) {
         o = pc_own<2>(L, rank);
         const float* M = msk(l);
-        pc_load(L, o, arr(l, 0), b);
-        pc_load(L, o, D, x);
-        // columns c (even) and c + 1 of the prolongation: a coarse column and
-        // its mean with the next (0 past the last); odd rows the mean of their
-        // two coarse rows, the last one 0.  Rows outside the coarse halo (only
-        // fine halo rows that no sweep needs) stay as they are.  A run of four
-        // or two rows, even first, reads run / 2 + 1 coarse rows.
-        const int J = o.c >> 1, I0 = o.ga >> 1, Elo = lo(l + 1, 2), Ehi = hi(l + 1, 2);
-        const bool in = J <= mc - 2;
-        const float* e = E + (I0 - bc) * mc + J;
-        float2 w[PC_RUN / 2 + 1];
-#pragma unroll
-        for (int i = 0; i <= PC_RUN / 2; ++i) {
-          const bool ok = 2 * i <= o.cnt && o.cnt > 0 && I0 + i >= Elo && I0 + i < Ehi;
-          w[i].x = ok ? e[i * mc] : 0.f;
-          w[i].y = ok && in ? e[i * mc + 1] : 0.f;
-        }
-#pragma unroll
-        for (int r = 0; r < PC_RUN; ++r) {
-          const float2 u = w[r / 2], v = w[r / 2 + 1];
-          float2 p;
-          if (r & 1) {
-            const bool mid = I0 + r / 2 <= nc - 2;
-            p.x = mid ? 0.5f * (u.x + v.x) : 0.f;
-            p.y = mid && in ? 0.25f * (u.x + v.x + u.y + v.y) : 0.f;
-          } else {
-            p.x = u.x;
-            p.y = in ? 0.5f * (u.x + u.y) : 0.f;
-          }
-          x[r] = add2(x[r], p);
-        }
-        pc_store(L, o, A, x);
+        auto mask = [&](int r) { return pair_ld(M + o.q + r * L.m); };
+        auto last = [&](int r) { return a.zero_last && o.ga + r == L.n - 1; };
+        pair_load<PC_RUN>(L, o, arr(l, 0), b);
+        pair_load<PC_RUN>(L, o, D, x);
+        // (the coarse array holds every row this reads; those past its valid
+        // halo go into fine halo rows that no sweep needs)
+        const int J = o.c >> 1;
+        const float* e = E + ((o.ga >> 1) - bc) * mc + J;
+        pair_prolong<PC_RUN>(o, nc, J <= mc - 2, [&](int i, int d) { return e[i * mc + d]; }, x);
+        pair_store<PC_RUN>(L, o, A, x);
         pc_sync(L);
-        pc_sweep<MAC>(a, L, o, A, b, M, false, x);
-        pc_store(L, o, D, x);
+        pair_sweep<MAC, PC_RUN>(a.co, L, o, A, b, mask, none, x);
+        pair_store<PC_RUN>(L, o, D, x);
         pc_sync(L);
-        pc_sweep<MAC>(a, L, o, D, b, M, a.zero_last, x);
+        pair_sweep<MAC, PC_RUN>(a.co, L, o, D, b, mask, last, x);
         if (l == lt && !a.whole) {   // straight to global memory (m is even)
 #pragma unroll
           for (int r = 0; r < PC_RUN; ++r) {
             const int gi = o.ga + r;
-            if (r < o.cnt && gi >= ga && gi < gb) pc_st2(a.x + (long)gi * L.m + o.c, x[r]);
+            if (r < o.cnt && gi >= ga && gi < gb) pair_st(a.x + (long)gi * L.m + o.c, x[r]);
           }
         } else {
           // own rows, and what the neighbours' halos need of them: two rows for
@@ -411,7 +279,7 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
             for (int r = 0; r < PC_RUN; ++r) {
               const int gi = o.ga + r;
               if (r < o.cnt && gi >= max(ga, from) && gi < min(gb, to))
-                pc_st2(dst + o.q + off + r * L.m, x[r]);
+                pair_st(dst + o.q + off + r * L.m, x[r]);
             }
           };
           put(F, 0, ga, gb);
@@ -423,33 +291,29 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
       // level 0: the residual norm (multigrid_solver.py:222-232): exact
       // squares, their sums compensated (TwoSum), one FP64 value per block
       if (l > 0 || tid >= L.active) continue;
-      pc_load(L, o, F, x);   // the halo rows too, as the neighbours stored them
-      auto add = [](df& s, float v) { s = pc_add(s, two_prod(v, v)); };
-      pc_resid(a, L, o, F, b, x, [&](int r, float2 v) {
+      auto outlet = [&](int r) { return a.mac_outlet && o.ga + r == L.n - 1; };
+      pair_load<PC_RUN>(L, o, F, x);   // the halo rows too, as the neighbours stored them
+      pair_resid<PC_RUN>(a.co, L, o, F, b, outlet, x, [&](int r, float2 v) {
         const int gi = o.ga + r;
         if (gi < ga || gi >= gb) return;
-        add(rr, v.x);
-        add(rr, v.y);
-        if (cyc == 0) {
-          add(bb, b[r].x);
-          add(bb, b[r].y);
-        }
+        rr = pair_add_sq(rr, v);
+        if (cyc == 0) bb = pair_add_sq(bb, b[r]);
       });
     }
     if (!a.whole) break;   // the coarsest level alone
     // the early-exit test, the blocks' sums added by every block alike
     // (FP32 pairs throughout: FP64 runs at 1/64 of the FP32 rate, and 512
     // threads adding doubles took 7 us a cycle)
-    rr = pc_lanes<32>(rr);
-    if (cyc == 0) bb = pc_lanes<32>(bb);
+    rr = pair_lanes<32>(rr);
+    if (cyc == 0) bb = pair_lanes<32>(bb);
     if ((tid & 31) == 0) {
       wsum[tid >> 5] = rr;
       wsum[PC_WARPS + (tid >> 5)] = bb;
     }
     __syncthreads();
     if (tid < 32) {   // the warps' sums; lane q files the block's in block q
-      rr = pc_lanes<32>(wsum[tid]);
-      if (cyc == 0) bb = pc_lanes<32>(wsum[PC_WARPS + tid]);
+      rr = pair_lanes<32>(wsum[tid]);
+      if (cyc == 0) bb = pair_lanes<32>(wsum[PC_WARPS + tid]);
       if (tid < C) {
         df* d = cl.map_shared_rank(nrm, tid);
         d[rank] = rr;
@@ -458,9 +322,9 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
     }
     cl.sync();
     if (tid < 32) {
-      const df t = pc_lanes<PC_MAX_CTAS>(tid < C ? nrm[tid] : df{0.f, 0.f});
+      const df t = pair_lanes<PC_MAX_CTAS>(tid < C ? nrm[tid] : df{0.f, 0.f});
       if (cyc == 0)
-        bb = pc_lanes<PC_MAX_CTAS>(tid < C ? nrm[PC_MAX_CTAS + tid] : df{0.f, 0.f});
+        bb = pair_lanes<PC_MAX_CTAS>(tid < C ? nrm[PC_MAX_CTAS + tid] : df{0.f, 0.f});
       if (tid == 0) {
         if (cyc == 0) bsq = (double)bb.hi + (double)bb.lo;
         rsq = (double)t.hi + (double)t.lo;
@@ -570,14 +434,22 @@ static int pc_ctas(const Layout& L) {
   return C;
 }
 
-// The first level the cluster takes: the finest one whose bands fit in shared
-// memory and in the threads' runs; nl + 1 if not even the coarsest level does.
+// The first level the cluster takes; nl + 1 if not even the coarsest one's
+// bands fit in shared memory and in the threads' runs.  The whole solve where
+// level 0 fits (a cycle, collocated: 384x96 18.4 us against 20.5 us with tiled
+// level-0 kernels, 512x128 19.5 against 20.4); else the levels whose bands,
+// halo included, are at most PC_TAIL_CELLS cells: below that a level's two
+// launches cost more than its share of the cluster's time (limits of 1000 /
+// 1800 / none: 1008x368 25.8 / 25.8 / 28.3 us a cycle, 2048x512 37.1 / 35.7 /
+// 35.9).
+constexpr int PC_TAIL_CELLS = 1800;
 int parity_cluster_level(const AjStepParams& p, const Layout& L) {
   const int C = pc_ctas(L), nl = L.nlev;
   PcLvl lv[AJ_MAX_LEVELS + 1];
   for (int lt = p.flow_type == AJ_FLOW_TAYLOR_GREEN ? nl : 0; lt <= nl; ++lt) {
     const size_t bytes = pc_levels(L, lt, C, p.grid_type == AJ_GRID_MAC, lv);
-    if (bytes > 0 && bytes <= kBlockSmemMax) return lt;
+    if (bytes == 0 || bytes > kBlockSmemMax) continue;
+    if (lt == 0 || lt == nl || (lv[lt].R + 2 * lv[lt].H) * lv[lt].m <= PC_TAIL_CELLS) return lt;
   }
   return nl + 1;
 }
@@ -608,10 +480,7 @@ int launch_parity_cluster(const AjStepParams& p, const Layout& L, void* ws, int 
   a.skip = skip;
   a.sc = at<DevScalars>(ws, 0);
   a.stats = stats;
-  a.ax = (float)(1.0 / (p.dx * p.dx));
-  a.ay = (float)(1.0 / (p.dy * p.dy));
-  a.den = (float)(2.0 * (1.0 / (p.dx * p.dx) + 1.0 / (p.dy * p.dy)));
-  a.rden = 1.f / a.den;
+  a.co = parity_coef(p);
   a.dxdy = p.dx * p.dy;
   const double tol = p.mg_tolerance > 0 ? p.mg_tolerance : AJ_PARITY_TOL_DEFAULT;
   a.tol2 = tol * tol;

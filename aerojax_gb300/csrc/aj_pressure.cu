@@ -10,7 +10,7 @@
 // level and every cycle on small grids) on one cluster (aj_parity_cluster.cu).
 //
 // The converging mode lives in aj_converge.cu; this file dispatches to it.
-#include "aj_internal.cuh"
+#include "aj_parity_pair.cuh"
 
 #include <cooperative_groups.h>
 #include <math.h>
@@ -140,7 +140,6 @@ __global__ void k_par_begin(DevScalars* sc) {
   sc->err = AJ_OK;
 }
 
-// converged = sum r^2 dx dy < tol^2 (multigrid_solver.py:222-232)
 // converged = sum r^2 dx dy < tol^2 (multigrid_solver.py:222-232), run by the
 // last block of the level-0 up kernel once every block's norm is in
 __device__ void par_check_body(DevScalars* sc, double dxdy, double tol2, int first) {
@@ -209,10 +208,16 @@ bool parity_coarsest_fused(const Layout& L) {
 }
 
 // ---- one level of the V-cycle per launch, on tiles
-// (multigrid_solver.py:173-211).  A tile stages what its output needs with
-// halos in shared memory; edge ghosts map to the cell itself; cells outside
-// the domain are never read by cells inside it.  Each block writes only its
-// own cells, and no output aliases an input another block reads.
+// (multigrid_solver.py:173-211).  A block stages a region of 4 G rows by 64
+// columns - its 4 (G - 2) x 56 output cells and a halo of four - in one round
+// trip, a thread holding a column pair over four rows in registers
+// (aj_parity_pair.cuh), and shared memory carries only what neighbouring
+// threads read.  Each block writes only its own cells, and no output aliases
+// an input another block reads.  What bounds it: on the coarser grids a
+// block's own chain (the staging round and four barriers), on the finest one
+// issue (1.3 region cells per output cell).  A whole MAC cycle at 2048x512
+// 77.8 -> 38.7 us, at 4096x2048 407 -> 143 us (before: a division and two global
+// reads a cell and sweep, and every level on its own launches).
 struct ParTile {
   const float* xin;   // down: the cycle's input state (null: zero); up: the level's down result
   const float* xc;    // up: the coarser level's result (prolonged on the fly)
@@ -223,170 +228,177 @@ struct ParTile {
   DevScalars* sc;     // up on level 0: the residual norm (multigrid_solver.py:229-231)
   const int* skip;
   int n, m, nc, mc, zero_last, mac_outlet, also_b;
-  float ax, ay, den;
+  int pairs;          // every level array is 8-byte aligned (rows are even)
+  PairCoef co;
   double dxdy, tol2;  // up on level 0: the early-exit test
 };
-// Output tiles: 16 x 64 on the finest level (4 cells per thread: fewer halo
-// cells per output, more loads in flight), 8 x 32 on the coarser ones (their
-// grids have few blocks, and a block's dependent phases set the time).
-constexpr int kPtThreads = 256;
+constexpr unsigned PT_BIG_BLOCKS = 304;   // two of 512 threads on each of 152 SMs
+constexpr int PT_RUN = 4, PT_W = 64, PT_H = 4, PT_OUT = PT_W - 2 * PT_H;
 
-// Jacobi value at tile cell (r, c) from the staged iterate S (same arithmetic
-// as k_par_jacobi); (gi, gj) its global index
-template <int RJ>
-__device__ __forceinline__ float tile_jacobi(float (*S)[RJ], int r, int c, int gi, int gj,
-                                             const ParTile& a) {
-  const int rp = gi + 1 < a.n ? r + 1 : r, rm = gi > 0 ? r - 1 : r;
-  const int cp = gj + 1 < a.m ? c + 1 : c, cm = gj > 0 ? c - 1 : c;
-  const long k = (long)gi * a.m + gj;
-  float pn = (a.ax * (S[rp][c] + S[rm][c]) + a.ay * (S[r][cp] + S[r][cm]) - ldg(a.b + k)) / a.den;
-  if (a.mask) pn = pn * ldg(a.mask + k);
-  return pn;
+// two adjacent cells of a global array
+__device__ __forceinline__ float2 pt_ld(const ParTile& a, const float* p) {
+  return a.pairs ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(ldg(p), ldg(p + 1));
+}
+__device__ __forceinline__ void pt_st(const ParTile& a, float* p, float2 v) {
+  if (a.pairs) {
+    pair_st(p, v);
+  } else {
+    p[0] = v.x;
+    p[1] = v.y;
+  }
 }
 
-// b - A x at tile cell (r, c) of the staged x (the MAC variant zeroes A x on
-// the outlet row)
-template <int RJ>
-__device__ __forceinline__ float tile_resid(float (*S)[RJ], int r, int c, int gi, int gj,
-                                            const ParTile& a) {
-  const int rp = gi + 1 < a.n ? r + 1 : r, rm = gi > 0 ? r - 1 : r;
-  const int cp = gj + 1 < a.m ? c + 1 : c, cm = gj > 0 ? c - 1 : c;
-  const float x = S[r][c];
-  float lap = a.ax * (S[rp][c] + S[rm][c] - 2.f * x) + a.ay * (S[r][cp] + S[r][cm] - 2.f * x);
-  if (a.mac_outlet && gi == a.n - 1) lap = 0.f;
-  return ldg(a.b + (long)gi * a.m + gj) - lap;
+// this thread's cells of its block's region, clipped to the domain; mine:
+// whether they are output cells; k0: the global index of the first
+struct PtOwn : PairOwn {
+  bool mine, left, right;
+  int gj;
+  long k0;
+};
+struct PtGeo {
+  static constexpr int m = PT_W;
+};
+__device__ __forceinline__ bool pair_lf(const PtGeo&, const PtOwn& o) { return o.left; }
+__device__ __forceinline__ bool pair_rt(const PtGeo&, const PtOwn& o) { return o.right; }
+template <int G>
+__device__ __forceinline__ PtOwn pt_own(const ParTile& a) {
+  PtOwn o;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int gi0 = blockIdx.y * (PT_RUN * (G - 2)) - PT_H, gj0 = blockIdx.x * PT_OUT - PT_H;
+  o.gj = gj0 + 2 * tx;
+  o.ga = gi0 + PT_RUN * ty;
+  o.glo = max(gi0, 0);
+  o.ghi = min(gi0 + PT_RUN * G, a.n);
+  // tiles start at multiples of 4 rows and even columns: a run or a pair is
+  // never cut by the domain's first row or column, nor a pair by its last
+  const bool in = o.ga >= 0 && o.gj >= 0 && o.gj < a.m;
+  o.cnt = in ? max(min(PT_RUN, a.n - o.ga), 0) : 0;
+  o.left = o.gj > max(gj0, 0);
+  o.right = o.gj + 2 < min(gj0 + PT_W, a.m);
+  o.q = PT_RUN * ty * PT_W + 2 * tx;
+  o.mine = o.cnt > 0 && tx >= PT_H / 2 && tx < (PT_H + PT_OUT) / 2 && ty >= 1 && ty < G - 1;
+  o.k0 = (long)o.ga * a.m + o.gj;
+  return o;
+}
+__device__ __forceinline__ void pt_load(const ParTile& a, const PtOwn& o, const float* src,
+                                        float2* v) {
+#pragma unroll
+  for (int r = 0; r < PT_RUN; ++r)
+    v[r] = r < o.cnt ? pt_ld(a, src + o.k0 + (long)r * a.m) : make_float2(0.f, 0.f);
 }
 
 // down: two pre-sweeps (the second resets the outlet row), the residual and
 // its 2x2 average onto the coarser level (multigrid_solver.py:182-201)
-template <int kPtBY, int kPtBX>
-__global__ void __launch_bounds__(kPtThreads) k_par_down(ParTile a) {
+template <int G, bool MAC>
+__global__ void __launch_bounds__(32 * G, 1024 / (32 * G)) k_par_down(ParTile a) {
+  pdl_wait();
   if (a.skip && *a.skip) return;
-  __shared__ float X0[kPtBY + 6][kPtBX + 6];   // input, halo 3
-  __shared__ float X1[kPtBY + 4][kPtBX + 4];   // first sweep, halo 2
-  __shared__ float X2[kPtBY + 2][kPtBX + 2];   // second sweep, halo 1
-  __shared__ float R[kPtBY][kPtBX];            // residual
-  const int ti0 = blockIdx.y * kPtBY, tj0 = blockIdx.x * kPtBX;
-  const int tid = threadIdx.x, nt = kPtThreads;
-  auto inside = [&](int gi, int gj) { return gi >= 0 && gi < a.n && gj >= 0 && gj < a.m; };
-  for (int q = tid; q < (kPtBY + 6) * (kPtBX + 6); q += nt) {
-    const int r = q / (kPtBX + 6), c = q - r * (kPtBX + 6);
-    const int gi = ti0 - 3 + r, gj = tj0 - 3 + c;
-    X0[r][c] = (a.xin && inside(gi, gj)) ? ldg(a.xin + (long)gi * a.m + gj) : 0.f;
+  __shared__ __align__(8) float A[PT_RUN * G * PT_W], D[PT_RUN * G * PT_W];
+  const PtOwn o = pt_own<G>(a);
+  constexpr PtGeo geo{};
+  float2 x[PT_RUN], b[PT_RUN], k[PT_RUN];
+  pt_load(a, o, a.b, b);
+  if (MAC) pt_load(a, o, a.mask, k);
+  auto mask = [&](int r) { return k[r]; };
+  auto none = [](int) { return false; };
+  auto last = [&](int r) { return a.zero_last && o.ga + r == a.n - 1; };
+  auto outlet = [&](int r) { return a.mac_outlet && o.ga + r == a.n - 1; };
+  if (a.xin) {
+    pt_load(a, o, a.xin, x);
+    pair_store<PT_RUN>(geo, o, A, x);
+    __syncthreads();
+    pair_sweep<MAC, PT_RUN>(a.co, geo, o, A, b, mask, none, x);
+  } else {
+    pair_sweep0<MAC, PT_RUN>(a.co, o, b, mask, x);
   }
+  pair_store<PT_RUN>(geo, o, D, x);
   __syncthreads();
-  for (int q = tid; q < (kPtBY + 4) * (kPtBX + 4); q += nt) {
-    const int r = q / (kPtBX + 4), c = q - r * (kPtBX + 4);
-    const int gi = ti0 - 2 + r, gj = tj0 - 2 + c;
-    X1[r][c] = inside(gi, gj) ? tile_jacobi<kPtBX + 6>(X0, r + 1, c + 1, gi, gj, a) : 0.f;
-  }
+  pair_sweep<MAC, PT_RUN>(a.co, geo, o, D, b, mask, last, x);
+  pair_store<PT_RUN>(geo, o, A, x);
   __syncthreads();
-  for (int q = tid; q < (kPtBY + 2) * (kPtBX + 2); q += nt) {
-    const int r = q / (kPtBX + 2), c = q - r * (kPtBX + 2);
-    const int gi = ti0 - 1 + r, gj = tj0 - 1 + c;
-    float x = 0.f;
-    if (inside(gi, gj))
-      x = (a.zero_last && gi == a.n - 1) ? 0.f : tile_jacobi<kPtBX + 4>(X1, r + 1, c + 1, gi, gj, a);
-    X2[r][c] = x;
-  }
-  __syncthreads();
-  for (int q = tid; q < kPtBY * kPtBX; q += nt) {
-    const int r = q / kPtBX, c = q - r * kPtBX;
-    const int gi = ti0 + r, gj = tj0 + c;
-    float res = 0.f;
-    if (inside(gi, gj)) {
-      a.xout[(long)gi * a.m + gj] = X2[r + 1][c + 1];
-      res = tile_resid<kPtBX + 2>(X2, r + 1, c + 1, gi, gj, a);
-    }
-    R[r][c] = res;
-  }
-  __syncthreads();
-  for (int q = tid; q < (kPtBY / 2) * (kPtBX / 2); q += nt) {
-    const int I = q / (kPtBX / 2), J = q - I * (kPtBX / 2);
-    const int gI = ti0 / 2 + I, gJ = tj0 / 2 + J;
-    if (gI < a.nc && gJ < a.mc)   // summed in the order (0,0), (1,0), (0,1), (1,1)
-      a.bc[(long)gI * a.mc + gJ] =
-          0.25f * (R[2 * I][2 * J] + R[2 * I + 1][2 * J] + R[2 * I][2 * J + 1] + R[2 * I + 1][2 * J + 1]);
-  }
+  if (!o.mine) return;
+#pragma unroll
+  for (int r = 0; r < PT_RUN; ++r)
+    if (r < o.cnt) pt_st(a, a.xout + o.k0 + (long)r * a.m, x[r]);
+  float2 ra{0.f, 0.f};
+  float* bc = a.bc + (long)(o.ga >> 1) * a.mc + (o.gj >> 1);
+  pair_resid<PT_RUN>(a.co, geo, o, A, b, outlet, x, [&](int r, float2 v) {
+    // summed in the order (0,0), (1,0), (0,1), (1,1)
+    if (r & 1) bc[(long)(r / 2) * a.mc] = 0.25f * (ra.x + v.x + ra.y + v.y);
+    ra = v;
+  });
 }
 
 // up: p + P(e) and two post-sweeps (the second resets the outlet row,
 // multigrid_solver.py:203-211); with NORM (level 0) also sum (b - A p)^2 and,
-// on the first cycle, b^2 (double-FP32 per block, FP64 across blocks)
-template <int kPtBY, int kPtBX, bool NORM>
-__global__ void __launch_bounds__(kPtThreads) k_par_up(ParTile a) {
+// on the first cycle, b^2 (exact squares, compensated sums, FP64 across
+// blocks)
+template <int G, bool MAC, bool NORM>
+__global__ void __launch_bounds__(32 * G, 1024 / (32 * G)) k_par_up(ParTile a) {
+  pdl_wait();
   if (a.skip && *a.skip) return;
-  constexpr int H = NORM ? 3 : 2;                       // halo of the corrected iterate
-  __shared__ float Y[kPtBY + 2 * H][kPtBX + 2 * H];
-  __shared__ float X1[kPtBY + 2 * H - 2][kPtBX + 2 * H - 2];
-  __shared__ float X2[NORM ? kPtBY + 2 : 1][NORM ? kPtBX + 2 : 1];
-  const int ti0 = blockIdx.y * kPtBY, tj0 = blockIdx.x * kPtBX;
-  const int tid = threadIdx.x, nt = kPtThreads;
-  auto inside = [&](int gi, int gj) { return gi >= 0 && gi < a.n && gj >= 0 && gj < a.m; };
-  for (int q = tid; q < (kPtBY + 2 * H) * (kPtBX + 2 * H); q += nt) {
-    const int r = q / (kPtBX + 2 * H), c = q - r * (kPtBX + 2 * H);
-    const int gi = ti0 - H + r, gj = tj0 - H + c;
-    float y = 0.f;
-    if (inside(gi, gj)) {
-      y = ldg(a.xin + (long)gi * a.m + gj);
-      y = y + prolong_ref(a.xc, a.nc, a.mc, gi, gj);
+  __shared__ __align__(8) float A[PT_RUN * G * PT_W], D[PT_RUN * G * PT_W];
+  const PtOwn o = pt_own<G>(a);
+  constexpr PtGeo geo{};
+  float2 x[PT_RUN], b[PT_RUN], k[PT_RUN];
+  pt_load(a, o, a.xin, x);
+  pt_load(a, o, a.b, b);
+  if (MAC) pt_load(a, o, a.mask, k);
+  auto mask = [&](int r) { return k[r]; };
+  auto none = [](int) { return false; };
+  auto last = [&](int r) { return a.zero_last && o.ga + r == a.n - 1; };
+  auto outlet = [&](int r) { return a.mac_outlet && o.ga + r == a.n - 1; };
+  const int I0 = o.ga >> 1, J = o.gj >> 1;
+  const float* e = a.xc + (long)I0 * a.mc + J;
+  pair_prolong<PT_RUN>(
+      o, a.nc, J <= a.mc - 2,
+      [&](int i, int d) { return I0 + i < a.nc ? ldg(e + (long)i * a.mc + d) : 0.f; }, x);
+  pair_store<PT_RUN>(geo, o, A, x);
+  __syncthreads();
+  pair_sweep<MAC, PT_RUN>(a.co, geo, o, A, b, mask, none, x);
+  pair_store<PT_RUN>(geo, o, D, x);
+  __syncthreads();
+  pair_sweep<MAC, PT_RUN>(a.co, geo, o, D, b, mask, last, x);
+  if (o.mine) {
+#pragma unroll
+    for (int r = 0; r < PT_RUN; ++r)
+      if (r < o.cnt) pt_st(a, a.xout + o.k0 + (long)r * a.m, x[r]);
+  }
+  if constexpr (NORM) {
+    pair_store<PT_RUN>(geo, o, A, x);
+    __syncthreads();
+    df rr{0.f, 0.f}, bb{0.f, 0.f};
+    if (o.mine)
+      pair_resid<PT_RUN>(a.co, geo, o, A, b, outlet, x, [&](int r, float2 v) {
+        // (b - A p) in FP32 as the reference evaluates it; its square exactly
+        rr = pair_add_sq(rr, v);
+        if (a.also_b) bb = pair_add_sq(bb, b[r]);
+      });
+    __shared__ df ws[2 * G];
+    rr = pair_lanes<32>(rr);
+    if (a.also_b) bb = pair_lanes<32>(bb);
+    if (threadIdx.x == 0) {
+      ws[threadIdx.y] = rr;
+      ws[G + threadIdx.y] = bb;
     }
-    Y[r][c] = y;
-  }
-  __syncthreads();
-  for (int q = tid; q < (kPtBY + 2 * H - 2) * (kPtBX + 2 * H - 2); q += nt) {
-    const int r = q / (kPtBX + 2 * H - 2), c = q - r * (kPtBX + 2 * H - 2);
-    const int gi = ti0 - H + 1 + r, gj = tj0 - H + 1 + c;
-    X1[r][c] = inside(gi, gj) ? tile_jacobi<kPtBX + 2 * H>(Y, r + 1, c + 1, gi, gj, a) : 0.f;
-  }
-  __syncthreads();
-  auto second = [&](int r, int c, int gi, int gj) {   // (r, c) in X1 coordinates
-    return (a.zero_last && gi == a.n - 1) ? 0.f : tile_jacobi<kPtBX + 2 * H - 2>(X1, r, c, gi, gj, a);
-  };
-  if constexpr (!NORM) {
-    for (int q = tid; q < kPtBY * kPtBX; q += nt) {
-      const int r = q / kPtBX, c = q - r * kPtBX;
-      const int gi = ti0 + r, gj = tj0 + c;
-      if (inside(gi, gj)) a.xout[(long)gi * a.m + gj] = second(r + 1, c + 1, gi, gj);
+    __syncthreads();
+    if (threadIdx.y > 0) return;
+    const int l = threadIdx.x;
+    rr = pair_lanes<G>(ws[l % G]);
+    if (a.also_b) bb = pair_lanes<G>(ws[G + l % G]);
+    if (l == 0) {
+      atomicAdd(&a.sc->acc[0], (double)rr.hi + (double)rr.lo);
+      if (a.also_b) atomicAdd(&a.sc->acc[1], (double)bb.hi + (double)bb.lo);
+      __threadfence();
+      // every block's sums are in: the early-exit test
+      if (atomicAdd(&a.sc->red_count, 1u) == gridDim.x * gridDim.y - 1) {
+        __threadfence();
+        a.sc->red_count = 0u;
+        par_check_body(a.sc, a.dxdy, a.tol2, a.also_b);
+      }
     }
-  } else {
-  for (int q = tid; q < (kPtBY + 2) * (kPtBX + 2); q += nt) {
-    const int r = q / (kPtBX + 2), c = q - r * (kPtBX + 2);
-    const int gi = ti0 - 1 + r, gj = tj0 - 1 + c;
-    X2[r][c] = inside(gi, gj) ? second(r + 1, c + 1, gi, gj) : 0.f;
-  }
-  __syncthreads();
-  df rr{0.f, 0.f}, bb{0.f, 0.f};
-  for (int q = tid; q < kPtBY * kPtBX; q += nt) {
-    const int r = q / kPtBX, c = q - r * kPtBX;
-    const int gi = ti0 + r, gj = tj0 + c;
-    if (inside(gi, gj)) {
-      a.xout[(long)gi * a.m + gj] = X2[r + 1][c + 1];
-      const float bv = ldg(a.b + (long)gi * a.m + gj);
-      const float res = tile_resid<kPtBX + 2>(X2, r + 1, c + 1, gi, gj, a);
-      // (b - A p) in FP32 as the reference evaluates it; its square exactly
-      rr = df_add(rr, two_prod(res, res));
-      bb = df_add(bb, two_prod(bv, bv));
-    }
-  }
-  const double s = block_sum_df(rr);
-  const double sb = a.also_b ? block_sum_df(bb) : 0.0;
-  __shared__ int am_last;
-  if (tid == 0) {
-    atomicAdd(&a.sc->acc[0], s);
-    if (a.also_b) atomicAdd(&a.sc->acc[1], sb);
-    __threadfence();
-    am_last = atomicAdd(&a.sc->red_count, 1u) == gridDim.x * gridDim.y - 1;
-  }
-  __syncthreads();
-  if (am_last && tid == 0) {   // every block's sums are in: the early-exit test
-    __threadfence();
-    a.sc->red_count = 0u;
-    par_check_body(a.sc, a.dxdy, a.tol2, a.also_b);
-  }
   }
 }
-
 
 __global__ void k_copy(const float* __restrict__ s, float* __restrict__ d, long n) {
   long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -598,8 +610,16 @@ static int parity_solve(const AjStepParams& p, const Layout& L, void* ws, const 
   }
   const int nt = lt < nl ? lt : nl;   // levels 0 .. nt-1 by the tiled kernels
   if (lt == 0) cluster(nullptr);
-  auto tile_grid = [&](int l) {
-    return l == 0 ? dim3(cdiv(L.lm[l], 64), cdiv(L.ln[l], 16)) : dim3(cdiv(L.lm[l], 32), cdiv(L.ln[l], 8));
+  auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 7) == 0; };
+  const int pairs = aligned(pout) && (!mac || aligned(mask));   // the workspace's arrays are
+  // a level's kernel on regions of 64 rows where those fill the GPU twice over
+  // (less of their work is halo), else of 32 rows (more and shorter blocks)
+  auto launch = [&](int l, auto big, auto small, const ParTile& a) {
+    const unsigned gx = cdiv(L.lm[l], PT_OUT), g16 = cdiv(L.ln[l], PT_RUN * 14);
+    if (gx * g16 >= PT_BIG_BLOCKS)
+      launch_pdl(true, big, dim3(gx, g16), dim3(32, 16), 0, st, a);
+    else
+      launch_pdl(true, small, dim3(gx, cdiv(L.ln[l], PT_RUN * 6)), dim3(32, 8), 0, st, a);
   };
   for (int cyc = 0; cyc < p.v_cycles && lt > 0; ++cyc) {
     const int* sk = cyc == 0 ? nullptr : skip;   // the first cycle always runs
@@ -619,11 +639,10 @@ static int parity_solve(const AjStepParams& p, const Layout& L, void* ws, const 
       a.mc = L.lm[l + 1];
       a.zero_last = vk;
       a.mac_outlet = mac && vk;
-      a.ax = ax;
-      a.ay = ay;
-      a.den = den;
-      if (l == 0) k_par_down<16, 64><<<tile_grid(l), kPtThreads, 0, st>>>(a);
-      else k_par_down<8, 32><<<tile_grid(l), kPtThreads, 0, st>>>(a);
+      a.pairs = pairs;
+      a.co = parity_coef(p);
+      if (mac) launch(l, k_par_down<16, true>, k_par_down<8, true>, a);
+      else launch(l, k_par_down<16, false>, k_par_down<8, false>, a);
     }
     // below: the cluster, or the coarsest level's 10 sweeps from zero, into X(nt)
     if (lt < nl) cluster(sk);
@@ -647,13 +666,14 @@ static int parity_solve(const AjStepParams& p, const Layout& L, void* ws, const 
       a.zero_last = vk;
       a.mac_outlet = mac && vk;
       a.also_b = cyc == 0;
-      a.ax = ax;
-      a.ay = ay;
-      a.den = den;
+      a.pairs = pairs;
+      a.co = parity_coef(p);
       a.dxdy = p.dx * p.dy;
       a.tol2 = tol * tol;
-      if (l == 0) k_par_up<16, 64, true><<<tile_grid(l), kPtThreads, 0, st>>>(a);
-      else k_par_up<8, 32, false><<<tile_grid(l), kPtThreads, 0, st>>>(a);
+      if (l == 0 && mac) launch(l, k_par_up<16, true, true>, k_par_up<8, true, true>, a);
+      else if (l == 0) launch(l, k_par_up<16, false, true>, k_par_up<8, false, true>, a);
+      else if (mac) launch(l, k_par_up<16, true, false>, k_par_up<8, true, false>, a);
+      else launch(l, k_par_up<16, false, false>, k_par_up<8, false, false>, a);
     }
   }
   if (p.flow_type == AJ_FLOW_LID_DRIVEN_CAVITY) {   // p -= p[nx/2, ny/2]

@@ -163,371 +163,258 @@ static DfCoef df_coef(double ax, double ay) {
 }
 
 // ---------------------------------------------------------------- tiles
-// A tile is SI x SJ cells of shared memory: the TI x TJ interior plus a halo
-// of H = 2 NS + 1 cells (NS red-black sweeps, one cell for the residual).
-// Threads form a (SJ/2) x RG grid: thread (tx, ty) owns the column pair
-// {2tx, 2tx+1} and walks the rows ty, ty+RG, ...; in a red-black half-sweep
-// exactly one cell of its pair per row has the colour being updated, so no
-// index needs a division.
-// VEC tiles (k_cv_up0 on a level whose rows are a multiple of 4 floats) are
-// staged in 16-byte chunks: their shared rows start at the 16-byte column at
-// or left of the tile's first one and are SJS = SJ + 4 floats long (the
-// pressure window's rows, PJS, cover its TJ + 2 columns from the 16-byte
-// column at or left of its first, in whole chunks), and the kernel indexes
-// them through base pointers shifted by the offsets from those columns.
-template <int SI_, int SJ_, int NTH_, int NS_ = CV_NS, bool VEC_ = false>
-struct TileCfg {
-  static constexpr int SI = SI_, SJ = SJ_, NTH = NTH_, NS = NS_, H = 2 * NS_ + 1;
-  static constexpr bool VEC = VEC_;
-  static constexpr int TI = SI - 2 * H, TJ = SJ - 2 * H;
-  static constexpr int SJS = VEC ? SJ + 4 : SJ;
-  static constexpr int PJS = VEC ? (TJ + 2 + 3 + 3) / 4 * 4 : TJ + 2;
-  static constexpr int PAIRS = SJ / 2, RG = NTH / PAIRS, NT = SI * SJS;
-  static_assert(!VEC || SJ % 4 == 0, "a 16-byte staged row is whole chunks");
-  static_assert(TI % 2 == 0 && TJ % 2 == 0, "tile interiors must align with the coarse grid");
-  static_assert(NTH % PAIRS == 0, "threads must fill whole rows of column pairs");
-};
-// Tile shapes, chosen per level by its size (cv_shape): large tiles where the
-// grid fills the GPU several times and the halo's share of the work counts,
-// small ones (and more threads each) where a few blocks' own chains set the
-// time.
-template <int NS, bool VEC = false>
-using TileL = TileCfg<48, 64, 256, NS, VEC>;   // 38 x 54 interior (42 x 58 with one sweep)
-template <int NS, bool VEC = false>
-using TileM = TileCfg<32, 32, 256, NS, VEC>;   // 22 x 22 (26 x 26)
-template <int NS, bool VEC = false>
-using TileS = TileCfg<32, 32, 512, NS, VEC>;
-// Level 0 post-smooths with one sweep (a V(2,1) cycle on the fine grid,
-// V(2,2) below it): the same tiles with a halo of 3
-constexpr int CV_NS_UP0 = 1;
-constexpr int CV_TILE_VARIANTS = 3;
-constexpr int CV_SMALL_TILES = 360, CV_LARGE_TILES = 450;
-// The shape (0 large, 1 medium, 2 small) of an n x m level, by its tiles of 32x32
-// and of 48x64.  Level-0 down and up kernels together, inside a stream, us
-// (48x64 with 256 threads / 32x32 with 256 / 32x32 with 512): 256x64 14.7 /
-// 7.2 / 5.8, 768x192 15.0 / 9.1 / 8.7, 1024x192 15.0 / 10.1 / 10.6, 1440x352
-// 18.9 / 16.8 / 18.9, 1728x448 23.3 / 21.8 / 25.6, 1792x512 24.8 / 25.3 /
-// 30.0, 2048x512 25.3 / 28.1 / 33.5, 4096x2048 143 / 183 / 242.
-// crowd: how many such levels run side by side (an ensemble's instances by
-// their cells): it is the tiles of all of them that fill the GPU (16 channels
-// of 256x64 to 1024x256 as one batch: 564 us by each one's own size, 544 so).
-static int cv_shape(int n, int m, float crowd = 1.f) {
-  const float small = crowd * cdiv(n, 22) * cdiv(m, 22), large = crowd * cdiv(n, 38) * cdiv(m, 54);
-  return small <= CV_SMALL_TILES ? 2 : large < CV_LARGE_TILES ? 1 : 0;
-}
+// A smoothing block covers a region of 4 G rows by 64 columns - its output
+// cells and a halo - in one round trip of 8-byte reads.  A thread owns a column
+// pair over four rows: those cells' e, right-hand side and inverse diagonal
+// live in registers for the whole kernel, and shared memory carries only what
+// neighbouring threads read, the even columns in one plane and the odd ones in
+// another (unit stride for every access).  A red-black half-sweep updates one
+// cell of each row: its vertical neighbours but the run's two ends are the
+// thread's own, of the horizontal ones one is, so four updates cost six
+// shared reads and four writes, and a half-sweep reads only the other colour,
+// so one barrier separates two of them.
+// Cells outside the level, and level 0's pinned outlet row, hold 0 and an
+// inverse diagonal of 0, so every cell is updated alike (the diagonal carries
+// the ghost rule).  The region's border is bordered by zeros: after half-sweep
+// h the cells at distance h + 1 or more from it hold exact red-black values,
+// and the output cells lie far enough inside (CP_H_DOWN, CP_H_UP; even, so that
+// a column pair or a 2x2 block is never cut, and regions start at even
+// coordinates: a cell's colour is (row + column) & 1 in the region too).
+// Level-0 down and up kernels together in a stream, against tiles with every
+// cell in shared memory: 1024x256 10.9 -> 7.0 us, 2048x512 25.0 -> 16.1 us,
+// 4096x2048 143 -> 84 us (down 51 -> 24, up 89 -> 59: 4.7 TB/s).
+constexpr int CP_RUN = 4, CP_COLS = 64, CP_PAIRS = CP_COLS / 2;
+constexpr int CP_H_DOWN = 6;   // four half-sweeps and the residual need 5
+constexpr int CP_H_UP = 4;     // four half-sweeps (level 0: two, and p + e one cell further)
+// Threads an SM holds at once (the kernels' register bound: 56).  1152 against
+// 768 for level 0's up kernel: 4096x2048 64.5 -> 58.9 us; 1536 spill.
+constexpr int CP_THREADS_SM = 1152;
+constexpr int CP_LD = CP_PAIRS + 1;   // plane row: one zero beside the first (odd columns) or last pair
 
-__device__ __forceinline__ float cv_diag(const CvLvl& L, int gi, int gj) {
-  float d = -2.f * (L.ax + L.ay);
-  if (gi == 0) d += L.ax;
-  if (gj == 0) d += L.ay;
-  if (gj == L.m - 1) d += L.ay;
-  if (gi == L.n - 1) d += (L.level == 0) ? L.ax : L.ax * L.g;
-  return d;
+__device__ __forceinline__ float2 cp_ldg2(const float* p) {
+  return __ldg(reinterpret_cast<const float2*>(p));
 }
+__device__ __forceinline__ void cp_st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
 
-// red-black half-sweeps over the whole shared-memory tile; cells outside the
-// domain hold 0 and never change (the diagonal carries the ghost rule).  After
-// half-sweep h the cells at distance >= h+1 from the tile border hold exact
-// red-black values; the cells nearer the border are never stored.  Tiles start
-// at even global coordinates, so a cell's colour is (ti + tj) & 1.
-template <class TC, bool INTERIOR>
-__device__ __forceinline__ void cv_sweeps_t(float* E, const float* R, const CvLvl& L, int gi0,
-                                            int gj0) {
-  constexpr int SJ = TC::SJ, SI = TC::SI;
-  constexpr int ROWS = (SI - 2 + TC::RG - 1) / TC::RG;   // rows of a thread per half-sweep
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const float inv_int = 1.f / (-2.f * (L.ax + L.ay));
-  for (int h = 0; h < 2 * TC::NS; ++h) {
-    const int color = h & 1;
-    // every new value of this thread's rows first, then the stores: a
-    // half-sweep reads only the other colour, so no store can feed a load of
-    // the same half-sweep, and the loads of all rows are in flight together
-    float val[ROWS];
-    int cc[ROWS];
+template <int G, int H>
+struct CpTile {
+  static constexpr int ROWS = CP_RUN * G, OUT_I = ROWS - 2 * H, OUT_J = CP_COLS - 2 * H;
+  static constexpr int PLANE = (ROWS + 2) * CP_LD;   // a zero row above and below
+  int tx, ty, gi, gj;   // the thread's first cell in the level (possibly outside)
+  int n, m;
+  long k;               // its index
+  float* X;             // this thread's place in the planes of even and odd columns
+  float* Y;
+  __device__ __forceinline__ CpTile(const CvLvl& L, float* planes)
+      : tx(threadIdx.x), ty(threadIdx.y), n(L.n), m(L.m) {
+    gi = blockIdx.y * OUT_I - H + CP_RUN * ty;
+    gj = blockIdx.x * OUT_J - H + 2 * tx;
+    k = (long)gi * m + gj;
+    X = planes + (CP_RUN * ty + 1) * CP_LD + tx;
+    Y = planes + PLANE + (CP_RUN * ty + 1) * CP_LD + 1 + tx;
+  }
+  // row r of the thread lies in the level (m is even: a pair is never cut)
+  __device__ __forceinline__ bool in(int r) const {
+    return (unsigned)(gi + r) < (unsigned)n && (unsigned)gj < (unsigned)m;
+  }
+  // row r belongs to the block's output
+  __device__ __forceinline__ bool mine(int r) const {
+    const int i = CP_RUN * ty + r;
+    return i >= H && i < ROWS - H && tx >= H / 2 && tx < CP_PAIRS - H / 2 && in(r);
+  }
+  __device__ __forceinline__ void zero_planes(float* planes) const {
+    for (int t = ty * CP_PAIRS + tx; t < 2 * PLANE; t += CP_PAIRS * G) planes[t] = 0.f;
+  }
+  __device__ __forceinline__ void load(const float* src, float2* v) const {
 #pragma unroll
-    for (int q = 0; q < ROWS; ++q) {
-      const int ti = 1 + ty + q * TC::RG;
-      const int tj = 2 * tx + ((color + ti) & 1);
-      const int gi = gi0 + ti, gj = gj0 + tj;
-      const bool upd = ti < SI - 1 &&
-                       (INTERIOR ? (tj >= 1 && tj < SJ - 1)
-                                 : (tj >= 1 && tj < SJ - 1 && (unsigned)gi < (unsigned)L.n &&
-                                    (unsigned)gj < (unsigned)L.m &&
-                                    !(L.level == 0 && gi == L.n - 1)));
-      cc[q] = -1;
-      val[q] = 0.f;
-      if (upd) {
-        const int c = ti * TC::SJS + tj;
-        const float nb = L.ax * (E[c + TC::SJS] + E[c - TC::SJS]) + L.ay * (E[c + 1] + E[c - 1]);
-        float inv = inv_int;
-        if (!INTERIOR && (gi == 0 || gj == 0 || gi == L.n - 1 || gj == L.m - 1))
-          inv = 1.f / cv_diag(L, gi, gj);
-        val[q] = (R[c] - nb) * inv;
-        cc[q] = c;
+    for (int r = 0; r < CP_RUN; ++r)
+      v[r] = in(r) ? cp_ldg2(src + k + (long)r * m) : make_float2(0.f, 0.f);
+  }
+  __device__ __forceinline__ void put(const float2* x) const {
+#pragma unroll
+    for (int r = 0; r < CP_RUN; ++r) {
+      X[r * CP_LD] = x[r].x;
+      Y[r * CP_LD] = x[r].y;
+    }
+  }
+  // the cells of one colour: even rows' even columns and odd rows' odd ones are red (0)
+  template <int COLOR>
+  __device__ __forceinline__ void put_color(const float2* x) const {
+#pragma unroll
+    for (int r = 0; r < CP_RUN; ++r) {
+      if ((r + COLOR) & 1) Y[r * CP_LD] = x[r].y;
+      else X[r * CP_LD] = x[r].x;
+    }
+  }
+  // ax (up + down) + ay (left + right) of the cell of row r that has colour COLOR
+  template <int COLOR>
+  __device__ __forceinline__ float nb(const CvLvl& L, const float2* x, int r) const {
+    float up, dn, sides;
+    if ((r + COLOR) & 1) {
+      up = r > 0 ? x[r > 0 ? r - 1 : 0].y : Y[-CP_LD];
+      dn = r + 1 < CP_RUN ? x[r + 1 < CP_RUN ? r + 1 : r].y : Y[CP_RUN * CP_LD];
+      sides = X[r * CP_LD + 1] + x[r].x;
+    } else {
+      up = r > 0 ? x[r > 0 ? r - 1 : 0].x : X[-CP_LD];
+      dn = r + 1 < CP_RUN ? x[r + 1 < CP_RUN ? r + 1 : r].x : X[CP_RUN * CP_LD];
+      sides = x[r].y + Y[r * CP_LD - 1];
+    }
+    return fmaf(L.ax, dn + up, L.ay * sides);
+  }
+  template <int COLOR>
+  __device__ __forceinline__ void half_sweep(const CvLvl& L, const float2* b, const float2* inv,
+                                             float2* x) const {
+    float v[CP_RUN];
+#pragma unroll
+    for (int r = 0; r < CP_RUN; ++r) v[r] = nb<COLOR>(L, x, r);
+#pragma unroll
+    for (int r = 0; r < CP_RUN; ++r) {
+      if ((r + COLOR) & 1) x[r].y = (b[r].y - v[r]) * inv[r].y;
+      else x[r].x = (b[r].x - v[r]) * inv[r].x;
+    }
+  }
+  // the diagonals of row r's pair
+  __device__ __forceinline__ float2 diag(const CvLvl& L, int r) const {
+    float d = -2.f * (L.ax + L.ay);
+    if (gi + r == 0) d += L.ax;
+    if (gi + r == n - 1) d += L.level == 0 ? L.ax : L.ax * L.g;
+    return make_float2(gj == 0 ? d + L.ay : d, gj + 1 == m - 1 ? d + L.ay : d);
+  }
+  // their inverses, 0 for cells that stay 0
+  __device__ __forceinline__ void inverse(const CvLvl& L, float2* inv) const {
+    const float c = 1.f / (-2.f * (L.ax + L.ay));
+    if (gi >= 1 && gi + CP_RUN <= n - 1 && gj >= 1 && gj + 2 <= m - 1) {
+#pragma unroll
+      for (int r = 0; r < CP_RUN; ++r) inv[r] = f2(c);
+    } else {
+#pragma unroll
+      for (int r = 0; r < CP_RUN; ++r) {
+        const float2 d = diag(L, r);
+        const bool live = in(r) && !(L.level == 0 && gi + r == n - 1);
+        inv[r] = live ? make_float2(1.f / d.x, 1.f / d.y) : f2(0.f);
       }
     }
-#pragma unroll
-    for (int q = 0; q < ROWS; ++q)
-      if (cc[q] >= 0) E[cc[q]] = val[q];
-    __syncthreads();
   }
-}
-// A tile whose every cell is an interior cell of the level (no boundary row
-// or column, not the pinned outlet row) takes the sweep without the checks.
-template <class TC>
-__device__ __forceinline__ void cv_sweeps(float* E, const float* R, const CvLvl& L, int gi0,
-                                          int gj0) {
-  if (gi0 >= 1 && gj0 >= 1 && gi0 + TC::SI <= L.n - 1 && gj0 + TC::SJ <= L.m - 1)
-    cv_sweeps_t<TC, true>(E, R, L, gi0, gj0);
-  else
-    cv_sweeps_t<TC, false>(E, R, L, gi0, gj0);
-}
-
-// The coarse cells a tile's cell-centred bilinear prolongation reads, with the
-// ghost rules folded in: row -1 copies row 0 (inlet Neumann), row nc is
-// g * row nc-1 (outlet ghost), columns clamp (wall Neumann).
-template <class TC>
-struct CoarseWin {
-  static constexpr int R = TC::SI / 2 + 3, C = TC::SJ / 2 + 3;
+  // x += P(e_coarse) inside the level: the cell-centred bilinear prolongation
+  // (weights 9/16, 3/16, 3/16, 1/16), first along the rows.  Ghosts: row -1
+  // copies row 0 (inlet Neumann), row nc is g times row nc - 1 (outlet ghost),
+  // columns clamp (wall Neumann).
+  __device__ __forceinline__ void prolong(const CvLvl& L, const float* __restrict__ ec, int nc,
+                                          int mc, float g, float2* x) const {
+    const int I0 = (gi >> 1) - 1, J = gj >> 1;
+    const int Jl = min(max(J - 1, 0), mc - 1), Jc = min(max(J, 0), mc - 1),
+              Jr = min(max(J + 1, 0), mc - 1);
+    float2 h[CP_RUN / 2 + 2];
+#pragma unroll
+    for (int i = 0; i < CP_RUN / 2 + 2; ++i) {
+      const int I = min(max(I0 + i, 0), nc - 1);
+      const float* e = ec + (long)I * mc;
+      const float c = 3.f * ldg(e + Jc), f = I0 + i >= nc ? g : 1.f;
+      h[i] = make_float2(f * (c + ldg(e + Jl)), f * (c + ldg(e + Jr)));
+    }
+#pragma unroll
+    for (int r = 0; r < CP_RUN; ++r) {
+      const float2 a = h[r / 2 + 1], o = (r & 1) ? h[r / 2 + 2] : h[r / 2];
+      if (in(r) && !(L.level == 0 && gi + r == n - 1))
+        x[r] = fma2(fma2(a, f2(3.f), o), f2(1.f / 16.f), x[r]);
+    }
+  }
 };
-
-template <class TC>
-__device__ __forceinline__ void cv_load_coarse(float* W, int gi0, int gj0,
-                                               const float* __restrict__ ec, int nc, int mc,
-                                               float g) {
-  using CW = CoarseWin<TC>;
-  const int I0 = (gi0 >> 1) - 1, J0 = (gj0 >> 1) - 1;
-  for (int t = threadIdx.y * blockDim.x + threadIdx.x; t < CW::R * CW::C;
-       t += blockDim.x * blockDim.y) {
-    const int a = t / CW::C, b = t - a * CW::C;
-    int I = I0 + a;
-    const int J = min(max(J0 + b, 0), mc - 1);
-    float f = 1.f;
-    if (I < 0) I = 0;
-    if (I >= nc) {
-      I = nc - 1;
-      f = g;
-    }
-    float v = 0.f;
-    if (I0 + a >= -1 && I0 + a <= nc) v = ldg(ec + (long)I * mc + J);
-    W[t] = f == 1.f ? v : f * v;
-  }
-}
-
-// tile + halo load for a pre-smoothing: E = 0, R = r; each row is read as
-// two coalesced runs of SJ/2 floats
-template <class TC>
-__device__ __forceinline__ void cv_load_r(float* E, float* R, const CvLvl& L, int gi0, int gj0,
-                                          const float* __restrict__ r) {
-  constexpr int SJ = TC::SJ;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-#pragma unroll
-  for (int ti = ty; ti < TC::SI; ti += TC::RG) {
-    const int gi = gi0 + ti;
-    const bool row_in = (unsigned)gi < (unsigned)L.n;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int tj = tx + q * TC::PAIRS;
-      const int gj = gj0 + tj;
-      const bool in = row_in && (unsigned)gj < (unsigned)L.m;
-      E[ti * SJ + tj] = 0.f;
-      R[ti * SJ + tj] = in ? ldg(r + (long)gi * L.m + gj) : 0.f;
-    }
-  }
-  __syncthreads();
-}
-
-// 4-byte asynchronous global-to-shared copy; zero-fill when !in (the source
-// is then not read)
-__device__ __forceinline__ void cv_cp4(float* dst, const float* src, bool in) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src),
-               "r"(in ? 4 : 0));
-}
-
-// tile + halo of a post-smoothing, requested without waiting: R = r and
-// E = e_in by cp.async (zero outside the level, e also on level 0's pinned
-// outlet row), so that their round trip overlaps the coarse window's; the
-// caller commits, waits, synchronises and then adds the prolongation
-template <class TC>
-__device__ __forceinline__ void cv_stage_async(float* E, float* R, const CvLvl& L, int gi0,
-                                               int gj0, const float* __restrict__ r,
-                                               const float* __restrict__ e_in) {
-  const int tx = threadIdx.x, ty = threadIdx.y;
-#pragma unroll
-  for (int ti = ty; ti < TC::SI; ti += TC::RG) {
-    const int gi = gi0 + ti;
-    const bool row_in = (unsigned)gi < (unsigned)L.n;
-    const bool row_e = row_in && !(L.level == 0 && gi == L.n - 1);
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int tj = tx + q * TC::PAIRS;
-      const int gj = gj0 + tj;
-      const bool in = row_in && (unsigned)gj < (unsigned)L.m;
-      const long k = in ? (long)gi * L.m + gj : 0;
-      cv_cp4(R + ti * TC::SJS + tj, r + k, in);
-      cv_cp4(E + ti * TC::SJS + tj, e_in + k, in && row_e);
-    }
-  }
-}
-
-// 16-byte asynchronous copy, zero-filled when !in; both addresses 16-byte
-// aligned (the caller's VEC tiles guarantee it)
-__device__ __forceinline__ void cv_cp16(float* dst, const float* src, bool in) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src),
-               "r"(in ? 16 : 0));
-}
-
-// cv_stage_async of a VEC tile: rows of SJS floats from global column x0 (a
-// multiple of 4; the level's row length m is one too, so a chunk is wholly
-// inside or outside the level)
-template <class TC>
-__device__ __forceinline__ void cv_stage_async_v(float* E, float* R, const CvLvl& L, int gi0,
-                                                 int x0, const float* __restrict__ r,
-                                                 const float* __restrict__ e_in, int tid) {
-  constexpr int CH = TC::SJS / 4;
-  for (int t = tid; t < TC::SI * CH; t += TC::NTH) {
-    const int ti = t / CH, ch = t - ti * CH;
-    const int gi = gi0 + ti, gx = x0 + 4 * ch;
-    const bool in = (unsigned)gi < (unsigned)L.n && gx >= 0 && gx < L.m;
-    const bool ine = in && !(L.level == 0 && gi == L.n - 1);
-    const long k = in ? (long)gi * L.m + gx : 0;
-    cv_cp16(R + ti * TC::SJS + 4 * ch, r + k, in);
-    cv_cp16(E + ti * TC::SJS + 4 * ch, e_in + k, ine);
-  }
-}
-
-// e += P(e_coarse) on the cells this thread staged: the cell-centred
-// bilinear prolongation (weights 9/16, 3/16, 3/16, 1/16) from the coarse
-// window W (after cv_load_coarse, the copies' wait and a barrier)
-template <class TC>
-__device__ __forceinline__ void cv_add_prolong(float* E, const CvLvl& L, int gi0, int gj0,
-                                               const float* W) {
-  using CW = CoarseWin<TC>;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int I0 = (gi0 >> 1) - 1, J0 = (gj0 >> 1) - 1;
-#pragma unroll
-  for (int ti = ty; ti < TC::SI; ti += TC::RG) {
-    const int gi = gi0 + ti;
-    if ((unsigned)gi >= (unsigned)L.n || (L.level == 0 && gi == L.n - 1)) continue;
-    const int a = (gi >> 1) - I0, ai = (gi & 1) ? a + 1 : a - 1;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int tj = tx + q * TC::PAIRS;
-      const int gj = gj0 + tj;
-      if ((unsigned)gj >= (unsigned)L.m) continue;
-      const int b = (gj >> 1) - J0, bj = (gj & 1) ? b + 1 : b - 1;
-      const float c0 = W[a * CW::C + b], cx = W[ai * CW::C + b];
-      const float cy = W[a * CW::C + bj], cxy = W[ai * CW::C + bj];
-      float* e = E + ti * TC::SJS + tj;
-      *e = *e + (9.f * c0 + 3.f * cx + 3.f * cy + cxy) * (1.f / 16.f);
-    }
-  }
-}
 
 // pre-smoothing from e = 0, residual, 2x2 average onto the coarse rhs.  On
 // level 0 the residual alternates between two buffers (r0, r1) with the
-// pressure state: *cur selects the one the last iteration wrote.
-template <class TC>
-__global__ void __launch_bounds__(TC::NTH) k_cv_down(CvLvl L, const float* r0, const float* r1,
-                                                     const int* cur, float* __restrict__ e_out,
-                                                     float* __restrict__ rc, const int* done) {
+// pressure state: *cur selects the one the last iteration wrote.  The first
+// half-sweep from zero needs no neighbours, and after the last one the black
+// cells' residuals are 0 by construction, so only the red cells' are formed.
+template <int G>
+__global__ void __launch_bounds__(32 * G, CP_THREADS_SM / (32 * G)) k_cv_down(
+    CvLvl L, const float* r0, const float* r1, const int* cur, float* __restrict__ e_out,
+    float* __restrict__ rc, const int* done) {
   pdl_wait();
-  constexpr int SJ = TC::SJ, TI = TC::TI, TJ = TC::TJ;
-  static_assert(!TC::VEC, "the pre-smoothing indexes its tile with stride SJ");
+  using T = CpTile<G, CP_H_DOWN>;
+  __shared__ float planes[2 * T::PLANE];
   // both flags in one round trip, the first tested while the tile is loaded
   const int skip = *done, second = r1 ? *cur : 0;
-  __shared__ float E[TC::NT];
-  __shared__ float R[TC::NT];
-  const int i0 = blockIdx.y * TI, j0 = blockIdx.x * TJ;
-  const int gi0 = i0 - TC::H, gj0 = j0 - TC::H;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const float* r = second ? r1 : r0;
-  cv_load_r<TC>(E, R, L, gi0, gj0, r);
+  const T t(L, planes);
+  float2 b[CP_RUN], x[CP_RUN], inv[CP_RUN];
+  t.load(second ? r1 : r0, b);
+  t.zero_planes(planes);
+  t.inverse(L, inv);
   if (skip) return;
-  cv_sweeps<TC>(E, R, L, gi0, gj0);
-  // store e and compute the residual on the tile interior (in place in R:
-  // every residual of this thread first, then the stores, so that no store
-  // holds back the next cell's loads)
-  constexpr int DR = (TI + TC::RG - 1) / TC::RG;
-  float res[DR][2];
-  int rc_[DR][2];
+  __syncthreads();
 #pragma unroll
-  for (int it = 0; it < DR; ++it) {
-    const int ti = TC::H + ty + it * TC::RG;
-    const int gi = gi0 + ti;
+  for (int r = 0; r < CP_RUN; ++r)
+    x[r] = (r & 1) ? make_float2(0.f, b[r].y * inv[r].y) : make_float2(b[r].x * inv[r].x, 0.f);
+  t.template put_color<0>(x);
+  __syncthreads();
+  t.template half_sweep<1>(L, b, inv, x);
+  t.template put_color<1>(x);
+  __syncthreads();
+  t.template half_sweep<0>(L, b, inv, x);
+  t.template put_color<0>(x);
+  __syncthreads();
+  t.template half_sweep<1>(L, b, inv, x);
+  t.template put_color<1>(x);
+  __syncthreads();
+  float res[CP_RUN];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int tj = TC::H + tx + q * TC::PAIRS;
-      const int gj = gj0 + tj;
-      rc_[it][q] = -1;
-      res[it][q] = 0.f;
-      if (ti >= TC::H + TI || gi >= L.n || tj >= TC::H + TJ || gj >= L.m) continue;
-      const int c = ti * SJ + tj;
-      e_out[(long)gi * L.m + gj] = E[c];
-      if (!(L.level == 0 && gi == L.n - 1)) {
-        const float nb = L.ax * (E[c + SJ] + E[c - SJ]) + L.ay * (E[c + 1] + E[c - 1]);
-        res[it][q] = R[c] - (nb + cv_diag(L, gi, gj) * E[c]);
-      }
-      rc_[it][q] = c;
-    }
+  for (int r = 0; r < CP_RUN; ++r) {
+    const float2 d = t.diag(L, r);
+    const float nb = t.template nb<0>(L, x, r);
+    const float v = (r & 1) ? b[r].y - fmaf(d.y, x[r].y, nb) : b[r].x - fmaf(d.x, x[r].x, nb);
+    res[r] = L.level == 0 && t.gi + r == t.n - 1 ? 0.f : v;
   }
 #pragma unroll
-  for (int it = 0; it < DR; ++it)
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-      if (rc_[it][q] >= 0) R[rc_[it][q]] = res[it][q];
-  __syncthreads();
-  const int mc = L.m >> 1, nc = L.n >> 1;
-  for (int ci = ty; ci < TI / 2; ci += TC::RG) {
-    const int I = (i0 >> 1) + ci;
-    if (I >= nc) break;
-    for (int cj = tx; cj < TJ / 2; cj += TC::PAIRS) {
-      const int J = (j0 >> 1) + cj;
-      if (J >= mc) break;
-      const int c = (TC::H + 2 * ci) * SJ + TC::H + 2 * cj;
-      rc[(long)I * mc + J] = 0.25f * (R[c] + R[c + SJ] + R[c + 1] + R[c + SJ + 1]);
-    }
+  for (int r = 0; r < CP_RUN; r += 2) {
+    if (!t.mine(r)) continue;
+    cp_st2(e_out + t.k + (long)r * t.m, x[r]);
+    cp_st2(e_out + t.k + (long)(r + 1) * t.m, x[r + 1]);
+    rc[(long)((t.gi + r) >> 1) * (t.m >> 1) + (t.gj >> 1)] = 0.25f * (res[r] + res[r + 1]);
   }
 }
 
 // e + P(e_coarse), post-smoothing, store (levels >= 1)
-template <class TC>
-__global__ void __launch_bounds__(TC::NTH) k_cv_up(CvLvl L, const float* __restrict__ r,
-                                                   const float* __restrict__ e_in,
-                                                   const float* __restrict__ ec, int nc, int mc,
-                                                   float gc, float* __restrict__ e_out,
-                                                   const int* done) {
+template <int G>
+__global__ void __launch_bounds__(32 * G, CP_THREADS_SM / (32 * G)) k_cv_up(
+    CvLvl L, const float* __restrict__ r, const float* __restrict__ e_in,
+    const float* __restrict__ ec, int nc, int mc, float gc, float* __restrict__ e_out,
+    const int* done) {
   pdl_wait();
-  constexpr int SJ = TC::SJ, TI = TC::TI, TJ = TC::TJ;
-  static_assert(!TC::VEC, "the level >= 1 post-smoothing indexes its tile with stride SJ");
-  if (*done) return;
-  __shared__ float E[TC::NT];
-  __shared__ float R[TC::NT];
-  const int i0 = blockIdx.y * TI, j0 = blockIdx.x * TJ;
-  const int gi0 = i0 - TC::H, gj0 = j0 - TC::H;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  cv_stage_async<TC>(E, R, L, gi0, gj0, r, e_in);
-  asm volatile("cp.async.commit_group;\n" ::);
-  __shared__ float W[CoarseWin<TC>::R * CoarseWin<TC>::C];
-  cv_load_coarse<TC>(W, gi0, gj0, ec, nc, mc, gc);
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  using T = CpTile<G, CP_H_UP>;
+  __shared__ float planes[2 * T::PLANE];
+  const int skip = *done;
+  const T t(L, planes);
+  float2 b[CP_RUN], x[CP_RUN], inv[CP_RUN];
+  t.load(r, b);
+  t.load(e_in, x);
+  t.zero_planes(planes);
+  t.prolong(L, ec, nc, mc, gc, x);
+  t.inverse(L, inv);
+  if (skip) return;
   __syncthreads();
-  cv_add_prolong<TC>(E, L, gi0, gj0, W);
+  t.put(x);
   __syncthreads();
-  cv_sweeps<TC>(E, R, L, gi0, gj0);
-  for (int ti = TC::H + ty; ti < TC::H + TI; ti += TC::RG) {
-    const int gi = gi0 + ti;
-    if (gi >= L.n) break;
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int tj = TC::H + tx + q * TC::PAIRS;
-      const int gj = gj0 + tj;
-      if (tj >= TC::H + TJ || gj >= L.m) continue;
-      e_out[(long)gi * L.m + gj] = E[ti * SJ + tj];
-    }
+  for (int s = 0; s < CV_NS; ++s) {
+    t.template half_sweep<0>(L, b, inv, x);
+    t.template put_color<0>(x);
+    __syncthreads();
+    t.template half_sweep<1>(L, b, inv, x);
+    if (s + 1 == CV_NS) break;
+    t.template put_color<1>(x);
+    __syncthreads();
   }
+#pragma unroll
+  for (int q = 0; q < CP_RUN; ++q)
+    if (t.mine(q)) cp_st2(e_out + t.k + (long)q * t.m, x[q]);
+}
+
+// asynchronous 8-byte global-to-shared copy; zeros when !in (the source is
+// then not read)
+__device__ __forceinline__ void cv_cp8(float* dst, const float* src, bool in) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src),
+               "r"(in ? 8 : 0));
 }
 
 struct CvCheck {
@@ -586,18 +473,19 @@ struct PState {
 // residual of the reference operator for the next iteration (double-FP32), its
 // FP64 norm, and the convergence test in the last block to finish.  The
 // residual ping-pongs with the pressure (rs.a pairs with ps.a): a block reads
-// the current residual over its tile and halo while its neighbours write the
-// next one, so the two must never share a buffer.
-template <class TC>
-__global__ void __launch_bounds__(TC::NTH, 1024 / TC::NTH) k_cv_up0(
-    CvLvl L, PState rs, const float* __restrict__ e_in,
-    const float* __restrict__ ec, int nc, int mc, float gc, PState ps, const float* __restrict__ b,
-    DevScalars* sc, DfCoef co, CvCheck ck, int profile) {
+// the current residual over its region while its neighbours write the next
+// one, so the two must never share a buffer.  The pressure of the region goes
+// to shared memory beside the other reads (8-byte asynchronous copies of the
+// thread's own pairs, zero outside the level and on the pinned outlet row).
+template <int G>
+__global__ void __launch_bounds__(32 * G, CP_THREADS_SM / (32 * G)) k_cv_up0(
+    CvLvl L, PState rs, const float* __restrict__ e_in, const float* __restrict__ ec, int nc,
+    int mc, float gc, PState ps, const float* __restrict__ b0, DevScalars* sc, DfCoef co,
+    CvCheck ck, int profile) {
   pdl_wait();
-  constexpr int TI = TC::TI, TJ = TC::TJ, SJS = TC::SJS;
-  constexpr int PI = TI + 2, PJ = TJ + 2, PJS = TC::PJS;
-  static_assert(PJ <= 2 * TC::PAIRS, "the pressure window must fit two column runs");
-  if (!profile && sc->mg_done) {
+  using T = CpTile<G, CP_H_UP>;
+  const int met = sc->mg_done, cur = sc->pcur;   // one round trip
+  if (!profile && met) {
     // met before this body ran (the initial guess already satisfied the
     // tolerance, or the rhs is zero): every kernel of the body skipped its
     // work and no block reaches the convergence test, so end the loop here
@@ -607,183 +495,99 @@ __global__ void __launch_bounds__(TC::NTH, 1024 / TC::NTH) k_cv_up0(
       cudaGraphSetConditional(ck.h, 0u);
     return;
   }
-  __shared__ __align__(16) float E[TC::NT];
-  __shared__ __align__(16) float R[TC::NT];
-  __shared__ __align__(16) float PH[PI * PJS];
-  __shared__ __align__(16) float PL[PI * PJS];
-  __shared__ int am_last;
-  const int i0 = blockIdx.y * TI, j0 = blockIdx.x * TJ;
-  const int gi0 = i0 - TC::H, gj0 = j0 - TC::H;
-  // the tile's and the window's first logical cells (VEC: the shared rows
-  // start at the 16-byte column at or left of them)
-  const int xe = TC::VEC ? (gj0 & ~3) : gj0;
-  const int xw = TC::VEC ? ((j0 - 1) & ~3) : j0 - 1;
-  float* const Es = E + (gj0 - xe);
-  float* const Rs = R + (gj0 - xe);
-  float* const PHs = PH + (j0 - 1 - xw);
-  float* const PLs = PL + (j0 - 1 - xw);
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int tid = ty * TC::PAIRS + tx;
+  __shared__ float planes[2 * T::PLANE];
+  __shared__ __align__(8) float PH[T::ROWS * CP_COLS];
+  __shared__ __align__(8) float PL[T::ROWS * CP_COLS];
+  const T t(L, planes);
   const long N = (long)L.n * L.m;
-  const int cur = sc->pcur;
   const float* __restrict__ pin = cur ? ps.b : ps.a;
   float* __restrict__ pout = cur ? ps.a : ps.b;
-  const float* __restrict__ r = cur ? rs.b : rs.a;
   float* __restrict__ r_next = cur ? rs.a : rs.b;
-  // Every global read is requested before the first wait, so that the block
-  // pays one round trip: the tile of r and e (tile and halo) and the pressure
-  // window (interior + 1) by cp.async straight into R, E, PH and PL, b into
-  // registers (this thread's residual cells: rows ty + RG q, columns tx and
-  // tx + PAIRS), the coarse window by plain loads; the prolongation is then
-  // added to E in shared memory.
-  if constexpr (TC::VEC) {
-    cv_stage_async_v<TC>(E, R, L, gi0, xe, r, e_in, tid);
-    constexpr int PCH = PJS / 4;
-    for (int t = tid; t < PI * PCH; t += TC::NTH) {
-      const int pi = t / PCH, ch = t - pi * PCH;
-      const int gi = i0 - 1 + pi, gx = xw + 4 * ch;
-      const bool in = (unsigned)gi < (unsigned)L.n && gi != L.n - 1 && gx >= 0 && gx < L.m;
-      const long k = in ? (long)gi * L.m + gx : 0;
-      cv_cp16(PH + pi * PJS + 4 * ch, pin + k, in);
-      cv_cp16(PL + pi * PJS + 4 * ch, pin + N + k, in);
-    }
-  } else {
-    cv_stage_async<TC>(E, R, L, gi0, gj0, r, e_in);
-    for (int pi = ty; pi < PI; pi += TC::RG) {
-      const int gi = i0 - 1 + pi;
-      const bool row_in = (unsigned)gi < (unsigned)L.n && gi != L.n - 1;
+  const int q0 = CP_RUN * t.ty * CP_COLS + 2 * t.tx;   // the thread's place in PH and PL
+  float2 b[CP_RUN], x[CP_RUN], inv[CP_RUN];
+  t.load(cur ? rs.b : rs.a, b);
+  t.load(e_in, x);
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int pj = tx + q * TC::PAIRS;
-        if (pj >= PJ) continue;
-        const int gj = j0 - 1 + pj;
-        const bool in = row_in && (unsigned)gj < (unsigned)L.m;
-        const long k = in ? (long)gi * L.m + gj : 0;
-        cv_cp4(PH + pi * PJS + pj, pin + k, in);
-        cv_cp4(PL + pi * PJS + pj, pin + N + k, in);
-      }
-    }
+  for (int r = 0; r < CP_RUN; ++r) {
+    const bool in = t.in(r) && t.gi + r != L.n - 1;
+    const long k = in ? t.k + (long)r * L.m : 0;
+    cv_cp8(PH + q0 + r * CP_COLS, pin + k, in);
+    cv_cp8(PL + q0 + r * CP_COLS, pin + N + k, in);
+    if (t.gi + r == L.n - 1) x[r] = f2(0.f);   // the outlet row's error is 0
   }
   asm volatile("cp.async.commit_group;\n" ::);
-  constexpr int RQ = (TI + TC::RG - 1) / TC::RG;
-  float bpre[RQ][2];
-#pragma unroll
-  for (int it = 0; it < RQ; ++it) {
-    const int ti = ty + it * TC::RG, gi = i0 + ti;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int tj = tx + q * TC::PAIRS, gj = j0 + tj;
-      bpre[it][q] = (ti < TI && gi < L.n && tj < TJ && gj < L.m) ? ldg(b + (long)gi * L.m + gj) : 0.f;
-    }
-  }
-  __shared__ float W[CoarseWin<TC>::R * CoarseWin<TC>::C];
-  cv_load_coarse<TC>(W, gi0, gj0, ec, nc, mc, gc);
+  t.zero_planes(planes);
+  t.prolong(L, ec, nc, mc, gc, x);
+  t.inverse(L, inv);
+  __syncthreads();
+  t.put(x);
+  __syncthreads();
+  t.template half_sweep<0>(L, b, inv, x);
+  t.template put_color<0>(x);
+  __syncthreads();
+  t.template half_sweep<1>(L, b, inv, x);
+  // p + e on the region's cells; what the residual reads of them is exact
+  t.load(b0, b);
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  __syncthreads();
-  cv_add_prolong<TC>(Es, L, gi0, gj0, W);
-  __syncthreads();
-  cv_sweeps<TC>(Es, Rs, L, gi0, gj0);
-  // new pressure on the interior and one cell around it, the thread's two
-  // columns of a row as one pair (all of this thread's sums first, then the
-  // stores)
-  constexpr int PR = (PI + TC::RG - 1) / TC::RG;
-  df2 pv[PR];
-  int pt[PR][2];
 #pragma unroll
-  for (int it = 0; it < PR; ++it) {
-    const int pi = ty + it * TC::RG;
-    const int gi = i0 - 1 + pi;
-    const bool row_in = pi < PI && (unsigned)gi < (unsigned)L.n && gi != L.n - 1;
-    float h[2], l[2], e[2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int pj = tx + q * TC::PAIRS;
-      const int gj = j0 - 1 + pj;
-      pt[it][q] = -1;
-      h[q] = l[q] = e[q] = 0.f;
-      if (row_in && pj < PJ && (unsigned)gj < (unsigned)L.m) {
-        const int t = pi * PJS + pj;
-        h[q] = PHs[t];
-        l[q] = PLs[t];
-        e[q] = Es[(TC::H - 1 + pi) * SJS + (TC::H - 1 + pj)];
-        pt[it][q] = t;
-      }
-    }
-    pv[it] = df2_add_f(df2{make_float2(h[0], h[1]), make_float2(l[0], l[1])},
-                       make_float2(e[0], e[1]));
-  }
-#pragma unroll
-  for (int it = 0; it < PR; ++it) {
-    if (pt[it][0] >= 0) {
-      PHs[pt[it][0]] = pv[it].hi.x;
-      PLs[pt[it][0]] = pv[it].lo.x;
-    }
-    if (pt[it][1] >= 0) {
-      PHs[pt[it][1]] = pv[it].hi.y;
-      PLs[pt[it][1]] = pv[it].lo.y;
-    }
+  for (int r = 0; r < CP_RUN; ++r) {
+    float* ph = PH + q0 + r * CP_COLS;
+    float* pl = PL + q0 + r * CP_COLS;
+    const df2 v = df2_add_f(df2{*reinterpret_cast<float2*>(ph), *reinterpret_cast<float2*>(pl)}, x[r]);
+    cp_st2(ph, v.hi);
+    cp_st2(pl, v.lo);
   }
   __syncthreads();
-  const df ax{co.axh, co.axl}, ay{co.ayh, co.ayl};
   float acc = 0.f;
+  if (t.mine(0)) {
+    const df ax{co.axh, co.axl}, ay{co.ayh, co.ayl};
+    auto row = [&](int r) {
+      const int q = q0 + r * CP_COLS;
+      return df2{*reinterpret_cast<const float2*>(PH + q), *reinterpret_cast<const float2*>(PL + q)};
+    };
+    df2 c = row(0), xm = t.gi > 0 ? row(-1) : c;   // Neumann ghost at the inlet
 #pragma unroll
-  for (int it = 0; it < RQ; ++it) {
-    const int ti = ty + it * TC::RG;
-    const int gi = i0 + ti;
-    if (ti >= TI || gi >= L.n) break;
-    // the row's two columns tx and tx + PAIRS; a column outside the tile or
-    // the grid reads the row's first window cell (in bounds) and stores nothing
-    bool ok[2];
-    long k[2];
-    df pc[2], xp[2], xm[2], yp[2], ym[2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int tj = tx + q * TC::PAIRS;
-      const int gj = j0 + tj;
-      ok[q] = tj < TJ && gj < L.m;
-      k[q] = (long)gi * L.m + gj;
-      const int c = (ti + 1) * PJS + (ok[q] ? tj + 1 : 1);
-      pc[q] = df{PHs[c], PLs[c]};
-      xp[q] = df{PHs[c + PJS], PLs[c + PJS]};                    // row n-1 holds the pinned 0
-      xm[q] = gi > 0 ? df{PHs[c - PJS], PLs[c - PJS]} : pc[q];   // Neumann ghosts
-      yp[q] = gj < L.m - 1 ? df{PHs[c + 1], PLs[c + 1]} : pc[q];
-      ym[q] = gj > 0 ? df{PHs[c - 1], PLs[c - 1]} : pc[q];
-      if (ok[q]) {
-        pout[k[q]] = pc[q].hi;
-        pout[N + k[q]] = pc[q].lo;
+    for (int r = 0; r < CP_RUN; ++r) {
+      if (!t.mine(r)) break;
+      const int q = q0 + r * CP_COLS;
+      const df2 xp = row(r + 1);   // row n - 1 holds the pinned 0
+      // the pair's left and right neighbours, the cell itself at the walls
+      const bool lw = t.gj == 0, rw = t.gj + 2 >= L.m;
+      const df2 yp{make_float2(c.hi.y, rw ? c.hi.y : PH[q + 2]),
+                   make_float2(c.lo.y, rw ? c.lo.y : PL[q + 2])};
+      const df2 ym{make_float2(lw ? c.hi.x : PH[q - 1], c.hi.x),
+                   make_float2(lw ? c.lo.x : PL[q - 1], c.lo.x)};
+      const long k = t.k + (long)r * L.m;
+      cp_st2(pout + k, c.hi);
+      cp_st2(pout + N + k, c.lo);
+      float2 rr{0.f, 0.f};
+      if (t.gi + r != L.n - 1) {
+        const df2 res = df2_residual(b[r], c, xp, xm, yp, ym, ax, ay);
+        rr = add2(res.hi, res.lo);
       }
-    }
-    float rr[2] = {0.f, 0.f};
-    if (gi != L.n - 1) {
-      auto pair = [](const df* v) {
-        return df2{make_float2(v[0].hi, v[1].hi), make_float2(v[0].lo, v[1].lo)};
-      };
-      const df2 res = df2_residual(make_float2(bpre[it][0], bpre[it][1]), pair(pc), pair(xp),
-                                   pair(xm), pair(yp), pair(ym), ax, ay);
-      const float2 s = add2(res.hi, res.lo);
-      rr[0] = s.x;
-      rr[1] = s.y;
-    }
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      if (!ok[q]) continue;
-      if (!profile) r_next[k[q]] = rr[q];
-      acc = fmaf(rr[q], rr[q], acc);
+      if (!profile) cp_st2(r_next + k, rr);
+      acc = fmaf(rr.x, rr.x, acc);
+      acc = fmaf(rr.y, rr.y, acc);
+      xm = c;
+      c = xp;
     }
   }
   if (profile) return;
-  block_sum_atomic_f(acc, &sc->acc[0]);
-  if (tid == 0) {
-    __threadfence();
-    unsigned int ticket = atomicAdd(&sc->red_count, 1u);
-    am_last = ticket == gridDim.x * gridDim.y - 1;
-  }
+  __shared__ df ws[G];
+  const df s = sum_lanes<32>(df{acc, 0.f});
+  if (t.tx == 0) ws[t.ty] = s;
   __syncthreads();
-  if (am_last && tid == 0) {
+  if (t.ty > 0) return;
+  const df total = sum_lanes<32>(t.tx < G ? ws[t.tx] : df{0.f, 0.f});
+  if (t.tx == 0) {
+    atomicAdd(&sc->acc[0], (double)total.hi + (double)total.lo);
     __threadfence();
-    sc->red_count = 0u;
-    sc->pcur = 1 - cur;
-    cv_check_body(sc, ck);
+    if (atomicAdd(&sc->red_count, 1u) == gridDim.x * gridDim.y - 1) {
+      __threadfence();
+      sc->red_count = 0u;
+      sc->pcur = 1 - cur;
+      cv_check_body(sc, ck);
+    }
   }
 }
 
@@ -1497,28 +1301,37 @@ static PState pstate(const Layout& L, void* ws) {
   return PState{at<float>(ws, L.p64), at<float>(ws, L.p64b)};
 }
 
-template <class TC>
-static dim3 tiles(const CvLvl& c) {
-  return dim3(cdiv(c.m, TC::TJ), cdiv(c.n, TC::TI));
-}
-template <class TC>
-static dim3 tile_threads() {
-  return dim3(TC::PAIRS, TC::RG);
+// The shape of an n x m level: regions of 48 rows (0), of 32 rows (1: more and
+// shorter blocks, where those are no more than the SMs) or of 64 rows (2, for
+// the autotuner; level 0's up kernel has 48).  Level-0 down and up kernels
+// together in a stream, us, 48 / 32 / 64 rows: 256x64 6.7 / 6.0 / 6.9, 512x96
+// 6.8 / 6.0 / 7.1, 1024x256 7.0 / 7.7 / 7.2, 2048x512 16.1 / 16.1 / 16.4,
+// 4096x2048 84 / 88 / 87.  crowd: how many such levels run side by side (an
+// ensemble's instances by their cells): all their blocks share the SMs.
+constexpr int CV_TILE_VARIANTS = 3, CV_SMALL_BLOCKS = 152;
+static int cv_shape(int n, int m, float crowd = 1.f) {
+  using T = CpTile<8, CP_H_DOWN>;
+  return crowd * cdiv(n, T::OUT_I) * cdiv(m, T::OUT_J) <= CV_SMALL_BLOCKS ? 1 : 0;
 }
 
-// level-0 kernels of tile variant v (chosen per grid shape by the autotuner)
-template <class TC>
+template <int G, int H>
+static dim3 tiles(const CvLvl& c) {
+  return dim3(cdiv(c.m, CpTile<G, H>::OUT_J), cdiv(c.n, CpTile<G, H>::OUT_I));
+}
+
+// level-0 kernels with G row groups
+template <int G>
 static void level0_down(const CvLvl& c, const Layout& L, void* ws, const int* done,
                         cudaStream_t st) {
   const DevScalars* sc = at<DevScalars>(ws, 0);
-  launch_pdl(true, k_cv_down<TC>, dim3(tiles<TC>(c)), dim3(tile_threads<TC>()), 0, st, c,
+  launch_pdl(true, k_cv_down<G>, tiles<G, CP_H_DOWN>(c), dim3(CP_PAIRS, G), 0, st, c,
              at<float>(ws, L.B[0]), at<float>(ws, L.T[0]), &sc->pcur, at<float>(ws, L.X[0]),
              at<float>(ws, L.B[1]), done);
 }
-template <class TC>
+template <int G>
 static void level0_up(const AjStepParams& p, const CvLvl& c, const Layout& L, void* ws,
                       DevScalars* sc, const CvCheck& ck, int profile, cudaStream_t st) {
-  launch_pdl(true, k_cv_up0<TC>, dim3(tiles<TC>(c)), dim3(tile_threads<TC>()), 0, st, c,
+  launch_pdl(true, k_cv_up0<G>, tiles<G, CP_H_UP>(c), dim3(CP_PAIRS, G), 0, st, c,
              PState{at<float>(ws, L.B[0]), at<float>(ws, L.T[0])}, at<float>(ws, L.X[0]),
              at<float>(ws, L.T[1]), L.ln[1], L.lm[1], (float)ghost_factor(1), pstate(L, ws),
              at<float>(ws, L.b0), sc, df_coef(1.0 / (p.dx * p.dx), 1.0 / (p.dy * p.dy)), ck,
@@ -1529,38 +1342,28 @@ static void level0_up(const AjStepParams& p, const CvLvl& c, const Layout& L, vo
 static int variant_shape(int v, const CvLvl& c) { return (cv_shape(c.n, c.m) + v) % CV_TILE_VARIANTS; }
 static void level0_down_s(int sh, const CvLvl& c, const Layout& L, void* ws, const int* done,
                           cudaStream_t st) {
-  if (sh == 2) level0_down<TileS<CV_NS>>(c, L, ws, done, st);
-  else if (sh == 1) level0_down<TileM<CV_NS>>(c, L, ws, done, st);
-  else level0_down<TileL<CV_NS>>(c, L, ws, done, st);
-}
-// the 16-byte staged tiles need rows of a multiple of 4 floats and every
-// staged buffer 16-byte aligned (workspace offsets are multiples of 256)
-static bool level0_vec_ok(const CvLvl& c, const void* ws) {
-  return c.m % 4 == 0 && (reinterpret_cast<uintptr_t>(ws) & 15) == 0;
+  if (sh == 2) level0_down<16>(c, L, ws, done, st);
+  else if (sh == 1) level0_down<8>(c, L, ws, done, st);
+  else level0_down<12>(c, L, ws, done, st);
 }
 static void level0_up_s(int sh, const AjStepParams& p, const CvLvl& c, const Layout& L, void* ws,
                         DevScalars* sc, const CvCheck& ck, int profile, cudaStream_t st) {
-  auto run = [&](auto plain, auto vec) {
-    if (level0_vec_ok(c, ws)) level0_up<decltype(vec)>(p, c, L, ws, sc, ck, profile, st);
-    else level0_up<decltype(plain)>(p, c, L, ws, sc, ck, profile, st);
-  };
-  if (sh == 2) run(TileS<CV_NS_UP0>{}, TileS<CV_NS_UP0, true>{});
-  else if (sh == 1) run(TileM<CV_NS_UP0>{}, TileM<CV_NS_UP0, true>{});
-  else run(TileL<CV_NS_UP0>{}, TileL<CV_NS_UP0, true>{});
+  if (sh == 1) level0_up<8>(p, c, L, ws, sc, ck, profile, st);
+  else level0_up<12>(p, c, L, ws, sc, ck, profile, st);
 }
 
 // the kernels of a level >= 1 in its size's shape
-template <class TC>
+template <int G>
 static void level_down(const CvLvl& c, const Layout& L, void* ws, int l, const int* done,
                        cudaStream_t st) {
-  launch_pdl(true, k_cv_down<TC>, dim3(tiles<TC>(c)), dim3(tile_threads<TC>()), 0, st, c,
+  launch_pdl(true, k_cv_down<G>, tiles<G, CP_H_DOWN>(c), dim3(CP_PAIRS, G), 0, st, c,
              at<float>(ws, L.B[l]), nullptr, done, at<float>(ws, L.X[l]),
              at<float>(ws, L.B[l + 1]), done);
 }
-template <class TC>
+template <int G>
 static void level_up(const CvLvl& c, const Layout& L, void* ws, int l, const int* done,
                      cudaStream_t st) {
-  launch_pdl(true, k_cv_up<TC>, dim3(tiles<TC>(c)), dim3(tile_threads<TC>()), 0, st, c,
+  launch_pdl(true, k_cv_up<G>, tiles<G, CP_H_UP>(c), dim3(CP_PAIRS, G), 0, st, c,
              at<float>(ws, L.B[l]), at<float>(ws, L.X[l]), at<float>(ws, L.T[l + 1]), L.ln[l + 1],
              L.lm[l + 1], (float)ghost_factor(l + 1), at<float>(ws, L.T[l]), done);
 }
@@ -1579,9 +1382,8 @@ static void cv_body(const AjStepParams& p, const Layout& L, void* ws,
     CvLvl c = cv_level(p, L, l);
     const int sh = cv_shape(c.n, c.m, L.crowd);
     if (l == 0) level0_down_s(sh0, c, L, ws, done, st);
-    else if (sh == 2) level_down<TileS<CV_NS>>(c, L, ws, l, done, st);
-    else if (sh == 1) level_down<TileM<CV_NS>>(c, L, ws, l, done, st);
-    else level_down<TileL<CV_NS>>(c, L, ws, l, done, st);
+    else if (sh == 1) level_down<8>(c, L, ws, l, done, st);
+    else level_down<12>(c, L, ws, l, done, st);
   }
   if (L.ld > 0) {
     direct_launch(direct_args(p, L, ws, done), st);
@@ -1591,9 +1393,8 @@ static void cv_body(const AjStepParams& p, const Layout& L, void* ws,
   for (int l = lc - 1; l >= 1; --l) {
     CvLvl c = cv_level(p, L, l);
     const int sh = cv_shape(c.n, c.m, L.crowd);
-    if (sh == 2) level_up<TileS<CV_NS>>(c, L, ws, l, done, st);
-    else if (sh == 1) level_up<TileM<CV_NS>>(c, L, ws, l, done, st);
-    else level_up<TileL<CV_NS>>(c, L, ws, l, done, st);
+    if (sh == 1) level_up<8>(c, L, ws, l, done, st);
+    else level_up<12>(c, L, ws, l, done, st);
   }
   CvCheck ck{p.max_cycles, use_handle, h};
   level0_up_s(sh0, p, c0, L, ws, sc, ck, 0, st);

@@ -188,6 +188,21 @@ __device__ __forceinline__ df df_add(df a, df b) {
   return quick_two_sum(s.hi, s.lo);
 }
 
+// Sums as (hi, lo) pairs whose lo collects the TwoSum errors of hi: a third of
+// df_add's operations where terms of one sign are added (and FP64 runs at
+// 1/64 of the FP32 rate); the sum of LANES neighbouring lanes in each of them
+__device__ __forceinline__ df sum_add(df a, df b) {
+  const df t = two_sum(a.hi, b.hi);
+  return {t.hi, t.lo + (a.lo + b.lo)};
+}
+template <int LANES>
+__device__ __forceinline__ df sum_lanes(df s) {
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1)
+    s = sum_add(s, df{__shfl_xor_sync(~0u, s.hi, o), __shfl_xor_sync(~0u, s.lo, o)});
+  return s;
+}
+
 // Block-wide sum of one double-FP32 value per thread, in a fixed order (the
 // result is bit-reproducible): a TwoSum butterfly inside each warp, one FP64
 // value per warp, the warps summed by thread 0, which gets the total.  Every

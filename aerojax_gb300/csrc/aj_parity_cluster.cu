@@ -304,16 +304,16 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
     // the early-exit test, the blocks' sums added by every block alike
     // (FP32 pairs throughout: FP64 runs at 1/64 of the FP32 rate, and 512
     // threads adding doubles took 7 us a cycle)
-    rr = pair_lanes<32>(rr);
-    if (cyc == 0) bb = pair_lanes<32>(bb);
+    rr = sum_lanes<32>(rr);
+    if (cyc == 0) bb = sum_lanes<32>(bb);
     if ((tid & 31) == 0) {
       wsum[tid >> 5] = rr;
       wsum[PC_WARPS + (tid >> 5)] = bb;
     }
     __syncthreads();
     if (tid < 32) {   // the warps' sums; lane q files the block's in block q
-      rr = pair_lanes<32>(wsum[tid]);
-      if (cyc == 0) bb = pair_lanes<32>(wsum[PC_WARPS + tid]);
+      rr = sum_lanes<32>(wsum[tid]);
+      if (cyc == 0) bb = sum_lanes<32>(wsum[PC_WARPS + tid]);
       if (tid < C) {
         df* d = cl.map_shared_rank(nrm, tid);
         d[rank] = rr;
@@ -322,9 +322,9 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
     }
     cl.sync();
     if (tid < 32) {
-      const df t = pair_lanes<PC_MAX_CTAS>(tid < C ? nrm[tid] : df{0.f, 0.f});
+      const df t = sum_lanes<PC_MAX_CTAS>(tid < C ? nrm[tid] : df{0.f, 0.f});
       if (cyc == 0)
-        bb = pair_lanes<PC_MAX_CTAS>(tid < C ? nrm[PC_MAX_CTAS + tid] : df{0.f, 0.f});
+        bb = sum_lanes<PC_MAX_CTAS>(tid < C ? nrm[PC_MAX_CTAS + tid] : df{0.f, 0.f});
       if (tid == 0) {
         if (cyc == 0) bsq = (double)bb.hi + (double)bb.lo;
         rsq = (double)t.hi + (double)t.lo;

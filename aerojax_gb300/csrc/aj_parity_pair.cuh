@@ -169,21 +169,8 @@ __device__ __forceinline__ void pair_store(const G& L, const O& o, float* S, con
     if (r < o.cnt) pair_st(S + o.q + r * L.m, v[r]);
 }
 
-// sums of exact squares as (hi, lo) pairs whose lo collects the TwoSum errors
-// of hi (FP32 pairs: FP64 runs at 1/64 of the FP32 rate)
-__device__ __forceinline__ df pair_add(df a, df b) {
-  const df t = two_sum(a.hi, b.hi);
-  return {t.hi, t.lo + (a.lo + b.lo)};
-}
 __device__ __forceinline__ df pair_add_sq(df s, float2 v) {
-  return pair_add(pair_add(s, two_prod(v.x, v.x)), two_prod(v.y, v.y));
-}
-template <int LANES>
-__device__ __forceinline__ df pair_lanes(df s) {
-#pragma unroll
-  for (int o = LANES / 2; o > 0; o >>= 1)
-    s = pair_add(s, df{__shfl_xor_sync(~0u, s.hi, o), __shfl_xor_sync(~0u, s.lo, o)});
-  return s;
+  return sum_add(sum_add(s, two_prod(v.x, v.x)), two_prod(v.y, v.y));
 }
 
 }  // namespace aj

@@ -375,8 +375,8 @@ __global__ void __launch_bounds__(32 * G, 1024 / (32 * G)) k_par_up(ParTile a) {
         if (a.also_b) bb = pair_add_sq(bb, b[r]);
       });
     __shared__ df ws[2 * G];
-    rr = pair_lanes<32>(rr);
-    if (a.also_b) bb = pair_lanes<32>(bb);
+    rr = sum_lanes<32>(rr);
+    if (a.also_b) bb = sum_lanes<32>(bb);
     if (threadIdx.x == 0) {
       ws[threadIdx.y] = rr;
       ws[G + threadIdx.y] = bb;
@@ -384,8 +384,8 @@ __global__ void __launch_bounds__(32 * G, 1024 / (32 * G)) k_par_up(ParTile a) {
     __syncthreads();
     if (threadIdx.y > 0) return;
     const int l = threadIdx.x;
-    rr = pair_lanes<G>(ws[l % G]);
-    if (a.also_b) bb = pair_lanes<G>(ws[G + l % G]);
+    rr = sum_lanes<G>(ws[l % G]);
+    if (a.also_b) bb = sum_lanes<G>(ws[G + l % G]);
     if (l == 0) {
       atomicAdd(&a.sc->acc[0], (double)rr.hi + (double)rr.lo);
       if (a.also_b) atomicAdd(&a.sc->acc[1], (double)bb.hi + (double)bb.lo);

@@ -471,6 +471,47 @@ __device__ __forceinline__ float weno_d(const float* __restrict__ f, int i, int 
   return weno5(up ? d0 : d5, up ? d1 : d4, up ? d2 : d3, up ? d3 : d2, up ? d4 : d1);
 }
 
+// the Laplacian's Laplacian at a cell two or more from every edge, from the 13
+// values it touches (first letter: row i + 1 (p) or i - 1 (m), second: column)
+__device__ __forceinline__ float bih13(const RkArgs& a, float fc, float fxp, float fxm, float fyp,
+                                       float fym, float xp2, float xm2, float yp2, float ym2,
+                                       float pp, float pm, float mp, float mm, float lap) {
+  const float lxp = lap5(xp2, fc, pp, pm, fxp, a.idx2, a.idy2);    // lap_at(i + 1, j)
+  const float lxm = lap5(fc, xm2, mp, mm, fxm, a.idx2, a.idy2);    // lap_at(i - 1, j)
+  const float lyp = lap5(pp, mp, yp2, fc, fyp, a.idx2, a.idy2);    // lap_at(i, j + 1)
+  const float lym = lap5(pm, mm, fc, ym2, fym, a.idx2, a.idy2);    // lap_at(i, j - 1)
+  return (lxp + lxm - 2.f * lap) * a.idx2 + (lyp + lym - 2.f * lap) * a.idy2;
+}
+// first-order upwind advection
+__device__ __forceinline__ float upwind5(const RkArgs& a, float fc, float fxp, float fxm,
+                                         float fyp, float fym, float uc, float vc) {
+  float fx = uc > 0.f ? uc * (fc - fxm) * a.idx : uc * (fxp - fc) * a.idx;
+  float fy = vc > 0.f ? vc * (fc - fym) * a.idy : vc * (fyp - fc) * a.idy;
+  return fx + fy;
+}
+// the right-hand side from its terms; s: nu_sgs (0 without)
+template <bool HYPER>
+__device__ __forceinline__ float rhs_sum(const RkArgs& a, float adv, float lap, float bih, float s) {
+  float nu_arg = a.dc ? a.nu + s : a.nu;              // the GUI passes nu + nu_sgs as nu
+  float nut = a.nsg ? nu_arg + s : nu_arg;            // rk: nu + nu_sgs
+  float r = -adv + nut * lap;
+  if (HYPER) r -= nu_arg * a.nuh_fac * bih;
+  return r;
+}
+// the stage's update of x0 with slope r (k1: the first slope, RK2's last stage)
+__device__ __forceinline__ float stage_sum(const RkArgs& a, float x0, float r, float chi, float k1,
+                                           float dt) {
+  float den = 1.f + dt * chi * a.inv_eta;
+  if (a.rk2) {
+    if (a.stage == 1) return brinkman_div(x0 + dt * r, den);
+    return brinkman_div(x0 + 0.5f * dt * (k1 + r), den);
+  }
+  if (a.stage == 1) return brinkman_div(x0 + dt * r, den);
+  float xs = x0 + dt * r;
+  if (a.stage == 2) return brinkman_div(0.75f * x0 + 0.25f * xs, den);
+  return brinkman_div((1.f / 3.f) * x0 + (2.f / 3.f) * xs, den);
+}
+
 // explicit right-hand side for one velocity component f at (i, j)
 // (rk3_simple_new.py:284-313)
 template <bool PER, bool HYPER, int ADV>
@@ -497,11 +538,7 @@ __device__ __forceinline__ float rhs_comp(const RkArgs& a, const float* __restri
       const float xp2 = ldg(q + 2 * ny), xm2 = ldg(q - 2 * ny), yp2 = ldg(q + 2), ym2 = ldg(q - 2);
       const float pp = ldg(q + ny + 1), pm = ldg(q + ny - 1), mp = ldg(q - ny + 1),
                   mm = ldg(q - ny - 1);
-      const float lxp = lap5(xp2, fc, pp, pm, fxp, a.idx2, a.idy2);    // lap_at(i + 1, j)
-      const float lxm = lap5(fc, xm2, mp, mm, fxm, a.idx2, a.idy2);    // lap_at(i - 1, j)
-      const float lyp = lap5(pp, mp, yp2, fc, fyp, a.idx2, a.idy2);    // lap_at(i, j + 1)
-      const float lym = lap5(pm, mm, fc, ym2, fym, a.idx2, a.idy2);    // lap_at(i, j - 1)
-      bih = (lxp + lxm - 2.f * lap) * a.idx2 + (lyp + lym - 2.f * lap) * a.idy2;
+      bih = bih13(a, fc, fxp, fxm, fyp, fym, xp2, xm2, yp2, ym2, pp, pm, mp, mm, lap);
     }
   } else {
     fc = ldg(f + k);
@@ -526,16 +563,9 @@ __device__ __forceinline__ float rhs_comp(const RkArgs& a, const float* __restri
     adv = uc * weno_d<PER, 0>(f, i, j, nx, ny, a.idx, uc) +
           vc * weno_d<PER, 1>(f, i, j, nx, ny, a.idy, vc);
   } else {
-    float fx = uc > 0.f ? uc * (fc - fxm) * a.idx : uc * (fxp - fc) * a.idx;
-    float fy = vc > 0.f ? vc * (fc - fym) * a.idy : vc * (fyp - fc) * a.idy;
-    adv = fx + fy;
+    adv = upwind5(a, fc, fxp, fxm, fyp, fym, uc, vc);
   }
-  float s = a.nsg ? ldg(a.nsg + k) : 0.f;
-  float nu_arg = a.dc ? a.nu + s : a.nu;              // the GUI passes nu + nu_sgs as nu
-  float nut = a.nsg ? nu_arg + s : nu_arg;            // rk: nu + nu_sgs
-  float r = -adv + nut * lap;
-  if (HYPER) r -= nu_arg * a.nuh_fac * bih;
-  return r;
+  return rhs_sum<HYPER>(a, adv, lap, bih, a.nsg ? ldg(a.nsg + k) : 0.f);
 }
 
 // stage update of one component at (i, j); returns the stage output
@@ -545,29 +575,14 @@ __device__ __forceinline__ float stage_val(const RkArgs& a, const float* f, cons
                                            float dt) {
   long k = (long)i * a.ny + j;
   float r = rhs_comp<PER, HYPER, ADV>(a, f, i, j);
-  float x0 = ldg(f0 + k);
-  float den = 1.f + dt * ldg(a.chi + k) * a.inv_eta;
-  if (a.rk2) {
-    if (a.stage == 1) {
-      if (k1_out) k1_out[k] = r;
-      return brinkman_div(x0 + dt * r, den);
-    }
-    return brinkman_div(x0 + 0.5f * dt * (ldg(k1 + k) + r), den);
-  }
-  if (a.stage == 1) return brinkman_div(x0 + dt * r, den);
-  float xs = x0 + dt * r;
-  if (a.stage == 2) return brinkman_div(0.75f * x0 + 0.25f * xs, den);
-  return brinkman_div((1.f / 3.f) * x0 + (2.f / 3.f) * xs, den);
+  if (a.rk2 && a.stage == 1 && k1_out) k1_out[k] = r;
+  return stage_sum(a, ldg(f0 + k), r, ldg(a.chi + k), a.rk2 && a.stage == 2 ? ldg(k1 + k) : 0.f, dt);
 }
 
+// one cell of a stage
 template <bool PER, bool HYPER, int ADV>
-__global__ void __launch_bounds__(256) k_rk_col(RkArgs a) {
-  pdl_wait();
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
+__device__ __forceinline__ void rk_col_cell(const RkArgs& a, int i, int j, float dt) {
   const int nx = a.nx, ny = a.ny;
-  if (i >= nx || j >= ny) return;
-  const float dt = a.sc->dt;
   long k = (long)i * ny + j;
   bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
   if (!last) {
@@ -608,8 +623,116 @@ __global__ void __launch_bounds__(256) k_rk_col(RkArgs a) {
   a.vout[k] = vo;
 }
 
+template <bool PER, bool HYPER, int ADV>
+__global__ void __launch_bounds__(256) k_rk_col(RkArgs a) {
+  pdl_wait();
+  int j = blockIdx.x * blockDim.x + threadIdx.x;
+  int i = blockIdx.y * blockDim.y + threadIdx.y;
+  if (i >= a.nx || j >= a.ny) return;
+  rk_col_cell<PER, HYPER, ADV>(a, i, j, a.sc->dt);
+}
+
+// The upwind stage four columns a thread: 16-byte reads of the five rows that
+// the Laplacian and the bi-Laplacian touch serve four cells where each cell
+// read its 13 values by itself (27 reads for four cells instead of 120; the
+// stage waited on them, at half the SM's warps).  Cells that lie within two
+// of an edge, and their vectors' others, go cell by cell on the first blocks.
+__host__ __device__ inline int rk4_edge_blocks(int nx, int ny) {
+  return (4 * ny + 8 * (nx - 4) + 255) / 256;
+}
+template <bool HYPER>
+__global__ void __launch_bounds__(256) k_rk_col4(RkArgs a) {
+  pdl_wait();
+  const int nx = a.nx, ny = a.ny;
+  const float dt = a.sc->dt;
+  const int edge = rk4_edge_blocks(nx, ny);
+  if ((int)blockIdx.x < edge) {   // a cell each: two rows, four columns at each end
+    const int e = blockIdx.x * 256 + threadIdx.y * 32 + threadIdx.x, f = e - 4 * ny;
+    if (f < 0) rk_col_cell<false, HYPER, AJ_ADV_UPWIND>(a, e < 2 * ny ? e / ny : nx - 4 + e / ny, e % ny, dt);
+    else if (f < 8 * (nx - 4))
+      rk_col_cell<false, HYPER, AJ_ADV_UPWIND>(a, 2 + f / 8, f % 8 < 4 ? f % 8 : ny - 8 + f % 8, dt);
+    return;
+  }
+  const int bj = (ny + 127) / 128, b = blockIdx.x - edge;
+  const int j = (b % bj * 32 + threadIdx.x) * 4, i = b / bj * 8 + threadIdx.y;
+  if (i < 2 || i > nx - 3 || j < 4 || j > ny - 8) return;
+  const long k = (long)i * ny + j;
+  const bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
+  struct F4 {
+    float v[4];
+  };
+  auto ld = [&](const float* p) {
+    const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+    return F4{t.x, t.y, t.z, t.w};
+  };
+  const F4 uc = ld(a.uin + k), vc = ld(a.vin + k), chi = ld(a.chi + k);
+  const F4 sg = a.nsg ? ld(a.nsg + k) : F4{0.f, 0.f, 0.f, 0.f};
+  const F4 mk = last ? ld(a.mask + k) : F4{1.f, 1.f, 1.f, 1.f};
+  auto component = [&](const float* f, const F4& fc, const float* f0, const float* k1,
+                       float* k1_out, float* out) {
+    const float* q = f + k;
+    const F4 xm = ld(q - ny), xp = ld(q + ny), x0 = ld(f0 + k);
+    const F4 g = a.rk2 && last ? ld(k1 + k) : F4{0.f, 0.f, 0.f, 0.f};
+    // columns j - 2 .. j + 5 of row i, j - 1 .. j + 4 of rows i - 1 and i + 1
+    float c[8] = {0.f, 0.f, fc.v[0], fc.v[1], fc.v[2], fc.v[3], 0.f, 0.f};
+    float m[6] = {0.f, xm.v[0], xm.v[1], xm.v[2], xm.v[3], 0.f};
+    float p[6] = {0.f, xp.v[0], xp.v[1], xp.v[2], xp.v[3], 0.f};
+    F4 xm2{}, xp2{};
+    if (HYPER) {
+      const float2 l = __ldg(reinterpret_cast<const float2*>(q - 2));
+      const float2 r = __ldg(reinterpret_cast<const float2*>(q + 4));
+      c[0] = l.x, c[1] = l.y, c[6] = r.x, c[7] = r.y;
+      m[0] = ldg(q - ny - 1), m[5] = ldg(q - ny + 4);
+      p[0] = ldg(q + ny - 1), p[5] = ldg(q + ny + 4);
+      xm2 = ld(q - 2 * (long)ny);
+      xp2 = ld(q + 2 * (long)ny);
+    } else {
+      c[1] = ldg(q - 1), c[6] = ldg(q + 4);
+    }
+    float o[4], slope[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float w = c[t + 2], yp = c[t + 3], ym = c[t + 1];
+      const float lap = lap5(p[t + 1], m[t + 1], yp, ym, w, a.idx2, a.idy2);
+      const float bih = HYPER ? bih13(a, w, p[t + 1], m[t + 1], yp, ym, xp2.v[t], xm2.v[t],
+                                      c[t + 4], c[t], p[t + 2], p[t], m[t + 2], m[t], lap)
+                              : 0.f;
+      const float adv = upwind5(a, w, p[t + 1], m[t + 1], yp, ym, uc.v[t], vc.v[t]);
+      slope[t] = rhs_sum<HYPER>(a, adv, lap, bih, sg.v[t]);
+      const float x = stage_sum(a, x0.v[t], slope[t], chi.v[t], g.v[t], dt);
+      o[t] = mk.v[t] > 0.5f ? x : 0.f;
+    }
+    if (a.rk2 && !last && k1_out)
+      *reinterpret_cast<float4*>(k1_out + k) = make_float4(slope[0], slope[1], slope[2], slope[3]);
+    *reinterpret_cast<float4*>(out + k) = make_float4(o[0], o[1], o[2], o[3]);
+  };
+  component(a.uin, uc, a.u0, a.k1u, a.k1u_out, a.uout);
+  component(a.vin, vc, a.v0, a.k1v, a.k1v_out, a.vout);
+}
+constexpr int RK4_MIN_NY = 64;
+constexpr long RK4_MIN_CELLS = 1 << 17;
+// whether a stage runs four columns a thread: whole 16-byte rows, every array
+// aligned, and a grid large enough that the blocks' number does not set the
+// time.  Three stages, plain / with hyperviscosity, us, a cell a thread ->
+// four: 512x128 7.5 / 11.2 -> 8.0 / 10.5, 1024x256 12.2 / 19.0 -> 9.4 / 12.1,
+// 2048x512 28.1 / 45.7 -> 19.7 / 27.6, 4096x2048 294 / 392 -> 147 / 200.
+static bool rk_col4_ok(const RkArgs& a) {
+  if (a.ny % 4 || a.ny < RK4_MIN_NY || a.nx < 8 || (long)a.nx * a.ny < RK4_MIN_CELLS) return false;
+  for (const void* p : {(const void*)a.uin, (const void*)a.vin, (const void*)a.u0,
+                        (const void*)a.v0, (const void*)a.chi, (const void*)a.mask,
+                        (const void*)a.nsg, (const void*)a.uout, (const void*)a.vout})
+    if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+  return true;
+}
+
 template <bool PER>
 static void dispatch_rk_col(const RkArgs& a, bool hyper, int adv, dim3 g, dim3 b, cudaStream_t st) {
+  if (!PER && adv == AJ_ADV_UPWIND && rk_col4_ok(a)) {
+    const dim3 g4(rk4_edge_blocks(a.nx, a.ny) + cdiv(a.ny, 128) * cdiv(a.nx, 8));
+    if (hyper) launch_pdl(true, k_rk_col4<true>, dim3(g4), dim3(32, 8), 0, st, a);
+    else launch_pdl(true, k_rk_col4<false>, dim3(g4), dim3(32, 8), 0, st, a);
+    return;
+  }
   if (hyper) {
     if (adv == AJ_ADV_WENO5) launch_pdl(true, k_rk_col<PER, true, AJ_ADV_WENO5>, dim3(g), dim3(b),
                                         0, st, a);

@@ -59,6 +59,28 @@ def test_multigrid_parity_bands(cuda_lib, nx, ny, guess):
         assert st["cycles"] == 3 and st["err"] == 0
 
 
+@pytest.mark.parametrize("hyper,fast,slip,flow", [(0.0, False, True, "von_karman"),
+                                                  (0.05, False, False, "von_karman"),
+                                                  (0.05, True, True, "von_karman"),
+                                                  (0.02, False, True, "lid_driven_cavity")])
+def test_predictor_collocated_wide(cuda_lib, hyper, fast, slip, flow):
+    """The stage kernel that takes four columns a thread (grids of 2^17 cells
+    and rows of a multiple of 4), its edge cells and partial blocks."""
+    import aerojax_gb300 as aj
+    from oracle import ref_np as R
+    nx, ny = 517, 260
+    rng = np.random.default_rng(5)
+    f = lambda a, s: (a + s * rng.standard_normal((nx, ny))).astype(np.float32)
+    u, v, sgs = f(1.0, 0.3), f(0.0, 0.3), np.abs(f(0.0, 1e-3))
+    mask = (rng.random((nx, ny)) > 0.02).astype(np.float32)
+    kw = dict(U_inf=1.1, nu_hyper_ratio=hyper, slip_walls=slip, fast_mode=fast,
+              brinkman_eta=1e-3, flow_type=flow)
+    us, vs = aj.rk_step_unified(T(u), T(v), 2e-3, 1e-2, 0.02, 0.025, T(mask), nu_sgs=T(sgs), **kw)
+    d = lambda a: a.astype(np.float64)
+    ur, vr = R.rk_step_unified(d(u), d(v), 2e-3, 1e-2, 0.02, 0.025, d(mask), nu_sgs=d(sgs), **kw)
+    assert rel(us, ur) < TOL and rel(vs, vr) < TOL
+
+
 def test_multigrid_parity_unaligned(cuda_lib):
     """A mask and a result that start on 4-byte boundaries only: the tiled
     kernels' pairs fall back to single cells and give the same bits."""

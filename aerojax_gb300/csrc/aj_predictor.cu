@@ -471,6 +471,50 @@ __device__ __forceinline__ float weno_d(const float* __restrict__ f, int i, int 
   return weno5(up ? d0 : d5, up ? d1 : d4, up ? d2 : d3, up ? d3 : d2, up ? d4 : d1);
 }
 
+// weno5 in the two lanes of paired FP32 instructions, every operation in the
+// order and with the contractions of the scalar function in the collocated
+// kernel: the two kernels give the same bits there.  The weights' reciprocals are single instructions: their
+// arguments are at least 1e-12, and 0 beyond 2^126 as in the scalar function.
+__device__ __forceinline__ float rcp_norm(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float2 weno5_pair(float2 v1, float2 v2, float2 v3, float2 v4,
+                                             float2 v5) {
+  const float2 m2 = f2(-2.f), m4 = f2(-4.f), c13 = f2(13.f / 12.f), c4 = f2(0.25f);
+  const float2 s1 = add2(fma2(m2, v2, v1), v3), s2 = add2(fma2(m2, v3, v2), v4),
+               s3 = add2(fma2(m2, v4, v3), v5), t = mul2(f2(3.f), v3);
+  const float2 e1 = add2(fma2(m4, v2, v1), t), e2 = sub2(v2, v4), e3 = add2(fma2(m4, v4, t), v5);
+  const float2 b1 = fma2(mul2(c13, s1), s1, mul2(mul2(c4, e1), e1));
+  const float2 b2 = fma2(mul2(c4, e2), e2, mul2(mul2(c13, s2), s2));
+  const float2 b3 = fma2(mul2(c13, s3), s3, mul2(mul2(c4, e3), e3));
+  auto weight = [](float w, float2 b) {
+    const float2 d = add2(f2(1e-6f), b), q = mul2(d, d);
+    return mul2(f2(w), make_float2(rcp_norm(q.x), rcp_norm(q.y)));
+  };
+  const float2 a1 = weight(0.1f, b1), a2 = weight(0.6f, b2), a3 = weight(0.3f, b3);
+  const float2 third = f2(1.f / 3.f), m6 = f2(-1.f / 6.f), c56 = f2(5.f / 6.f);
+  const float2 q1 = fma2(f2(11.f / 6.f), v3, fma2(v1, third, mul2(f2(-7.f / 6.f), v2)));
+  const float2 q2 = fma2(v4, third, fma2(c56, v3, mul2(v2, m6)));
+  const float2 q3 = fma2(v5, m6, fma2(v3, third, mul2(c56, v4)));
+  const float2 num = fma2(a3, q3, fma2(a2, q2, mul2(a1, q1))), den = add2(add2(a1, a2), a3);
+  return make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
+}
+
+// weno_d7 in pairs: g[0..6] the samples -3 .. 3 of each lane
+__device__ __forceinline__ float2 weno_d7_pair(const float2 (&g)[7], float ih, float2 vel) {
+  float2 d[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) d[q] = mul2(sub2(g[q + 1], g[q]), f2(ih));
+  const bool ux = vel.x > 0.f, uy = vel.y > 0.f;
+  float2 v[5];
+#pragma unroll
+  for (int q = 0; q < 5; ++q)
+    v[q] = make_float2(ux ? d[q].x : d[5 - q].x, uy ? d[q].y : d[5 - q].y);
+  return weno5_pair(v[0], v[1], v[2], v[3], v[4]);
+}
+
 // the Laplacian's Laplacian at a cell two or more from every edge, from the 13
 // values it touches (first letter: row i + 1 (p) or i - 1 (m), second: column)
 __device__ __forceinline__ float bih13(const RkArgs& a, float fc, float fxp, float fxm, float fyp,
@@ -579,48 +623,51 @@ __device__ __forceinline__ float stage_val(const RkArgs& a, const float* f, cons
   return stage_sum(a, ldg(f0 + k), r, ldg(a.chi + k), a.rk2 && a.stage == 2 ? ldg(k1 + k) : 0.f, dt);
 }
 
-// one cell of a stage
+// one stage of component COMP at (i, j).  The last stage applies the hard mask
+// (rk3_simple_new.py:334-335), then the boundary conditions (:250-280): a
+// value, or the stage at the cell that the boundary copies from.  One
+// evaluation for all of them: with one at each branch the kernel waited on
+// instruction fetches (WENO5 128x32 three stages 21 us).
+template <bool PER, bool HYPER, int ADV, int COMP>
+__device__ __forceinline__ void rk_col_one(const RkArgs& a, int i, int j, float dt) {
+  const int nx = a.nx, ny = a.ny;
+  const bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
+  int ii = i, jj = j;
+  float o = 0.f;
+  bool set = false;
+  if (last) {
+    const bool wall = j == 0 || j == ny - 1, end = i == 0 || i == nx - 1;
+    if (a.flow == AJ_FLOW_VON_KARMAN) {
+      ii = i == nx - 1 ? nx - 2 : i;
+      if (COMP == 0) {
+        set = i == 0 || (!a.slip && wall);
+        if (i == 0 && (a.slip || !wall)) o = a.U;
+        if (a.slip) jj = j == 0 ? 1 : (j == ny - 1 ? ny - 2 : j);
+      } else {
+        set = i == 0 || wall;
+      }
+    } else if (a.flow == AJ_FLOW_LID_DRIVEN_CAVITY) {
+      set = end || wall;
+      if (COMP == 0 && !end && j == ny - 1 && j != 0) o = a.U;
+    }
+    if (!set) set = !(ldg(a.mask + (long)ii * ny + jj) > 0.5f);
+  }
+  if (!set)
+    o = COMP == 0 ? stage_val<PER, HYPER, ADV>(a, a.uin, a.u0, a.k1u, last ? nullptr : a.k1u_out, ii, jj, dt)
+                  : stage_val<PER, HYPER, ADV>(a, a.vin, a.v0, a.k1v, last ? nullptr : a.k1v_out, ii, jj, dt);
+  (COMP == 0 ? a.uout : a.vout)[(long)i * ny + j] = o;
+}
 template <bool PER, bool HYPER, int ADV>
 __device__ __forceinline__ void rk_col_cell(const RkArgs& a, int i, int j, float dt) {
-  const int nx = a.nx, ny = a.ny;
-  long k = (long)i * ny + j;
-  bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
-  if (!last) {
+  if (ADV != AJ_ADV_WENO5 && (a.rk2 ? a.stage != 2 : a.stage != 3)) {
+    // both components in one scope share their loads
+    const long k = (long)i * a.ny + j;
     a.uout[k] = stage_val<PER, HYPER, ADV>(a, a.uin, a.u0, a.k1u, a.k1u_out, i, j, dt);
     a.vout[k] = stage_val<PER, HYPER, ADV>(a, a.vin, a.v0, a.k1v, a.k1v_out, i, j, dt);
     return;
   }
-  // final stage: hard mask (rk3_simple_new.py:334-335) then boundary
-  // conditions (:250-280), evaluated at the cell each boundary copies from.
-  float uo, vo;
-  if (a.flow == AJ_FLOW_VON_KARMAN) {
-    int ai = (i == nx - 1) ? nx - 2 : i;
-    int bj = a.slip ? (j == 0 ? 1 : (j == ny - 1 ? ny - 2 : j)) : j;
-    if (!a.slip && (j == 0 || j == ny - 1)) uo = 0.f;
-    else if (i == 0) uo = a.U;
-    else {
-      long q = (long)ai * ny + bj;
-      uo = ldg(a.mask + q) > 0.5f ? stage_val<PER, HYPER, ADV>(a, a.uin, a.u0, a.k1u, nullptr, ai, bj, dt) : 0.f;
-    }
-    if (i == 0 || j == 0 || j == ny - 1) vo = 0.f;
-    else {
-      long q = (long)ai * ny + j;
-      vo = ldg(a.mask + q) > 0.5f ? stage_val<PER, HYPER, ADV>(a, a.vin, a.v0, a.k1v, nullptr, ai, j, dt) : 0.f;
-    }
-  } else if (a.flow == AJ_FLOW_LID_DRIVEN_CAVITY) {
-    bool edge_x = (i == 0 || i == nx - 1);
-    if (edge_x || j == 0) uo = 0.f;
-    else if (j == ny - 1) uo = a.U;
-    else uo = ldg(a.mask + k) > 0.5f ? stage_val<PER, HYPER, ADV>(a, a.uin, a.u0, a.k1u, nullptr, i, j, dt) : 0.f;
-    if (edge_x || j == 0 || j == ny - 1) vo = 0.f;
-    else vo = ldg(a.mask + k) > 0.5f ? stage_val<PER, HYPER, ADV>(a, a.vin, a.v0, a.k1v, nullptr, i, j, dt) : 0.f;
-  } else {
-    bool m = ldg(a.mask + k) > 0.5f;
-    uo = m ? stage_val<PER, HYPER, ADV>(a, a.uin, a.u0, a.k1u, nullptr, i, j, dt) : 0.f;
-    vo = m ? stage_val<PER, HYPER, ADV>(a, a.vin, a.v0, a.k1v, nullptr, i, j, dt) : 0.f;
-  }
-  a.uout[k] = uo;
-  a.vout[k] = vo;
+  rk_col_one<PER, HYPER, ADV, 0>(a, i, j, dt);
+  rk_col_one<PER, HYPER, ADV, 1>(a, i, j, dt);
 }
 
 template <bool PER, bool HYPER, int ADV>
@@ -725,12 +772,87 @@ static bool rk_col4_ok(const RkArgs& a) {
   return true;
 }
 
+// WENO5 stages, non-periodic, a run of rows a thread: the thread walks R cells
+// in x with its column's seven u and v in registers, and the two components
+// are the lanes of paired FP32 instructions, reconstructions included (both
+// components share the advecting velocity).  What bounds it: instructions
+// issued.  Cells within three of an edge go one component a thread on the
+// first blocks.  Three stages, us, a cell a thread -> this: 128x32 10.4 -> 9.9,
+// 512x128 12.4 -> 10.6, 1024x256 24.7 -> 17.1, 2048x512 68 -> 47.
+struct ColRows {
+  static constexpr int HB = 3, R = 2;
+  __host__ __device__ static int edge_blocks(int nx, int ny) {
+    return (2 * 2 * HB * (ny + nx - 2 * HB) + 255) / 256;
+  }
+};
+__global__ void __launch_bounds__(256, 4) k_rk_col_rows(RkArgs a) {
+  pdl_wait();
+  constexpr int HB = ColRows::HB, R = ColRows::R, E = 2 * HB;
+  const int nx = a.nx, ny = a.ny;
+  const float dt = a.sc->dt;
+  const int edge = ColRows::edge_blocks(nx, ny);
+  if ((int)blockIdx.x < edge) {
+    const int cells = E * (ny + nx - 2 * HB);
+    int e = blockIdx.x * 256 + threadIdx.y * 32 + threadIdx.x;
+    if (e >= 2 * cells) return;
+    const bool comp = e >= cells;
+    if (comp) e -= cells;
+    const int f = e - E * ny, q = f < 0 ? e / ny : f % E;
+    const int i = f < 0 ? (q < HB ? q : nx - E + q) : HB + f / E;
+    const int j = f < 0 ? e % ny : (q < HB ? q : ny - E + q);
+    if (comp) rk_col_one<false, false, AJ_ADV_WENO5, 1>(a, i, j, dt);
+    else rk_col_one<false, false, AJ_ADV_WENO5, 0>(a, i, j, dt);
+    return;
+  }
+  const int bj = (ny + 31) / 32, b = blockIdx.x - edge;
+  const int j = b % bj * 32 + threadIdx.x, i0 = HB + (b / bj * 8 + threadIdx.y) * R;
+  if (j < HB || j > ny - 1 - HB || i0 > nx - 1 - HB) return;
+  const bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
+  long k = (long)i0 * ny + j;
+  auto at = [&](long q) { return make_float2(ldg(a.uin + q), ldg(a.vin + q)); };
+  float2 x[7];   // column j, rows i - 3 .. i + 3
+#pragma unroll
+  for (int q = 1; q < 7; ++q) x[q] = at(k + (long)(q - 4) * ny);
+#pragma unroll
+  for (int r = 0; r < R; ++r, k += ny) {
+    if (i0 + r > nx - 1 - HB) break;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) x[q] = x[q + 1];
+    x[6] = at(k + 3 * (long)ny);
+    const float2 c = x[3];
+    const float2 y[7] = {at(k - 3), at(k - 2), at(k - 1), c, at(k + 1), at(k + 2), at(k + 3)};
+    const float2 adv = fma2(f2(c.y), weno_d7_pair(y, a.idy, f2(c.y)),
+                            mul2(f2(c.x), weno_d7_pair(x, a.idx, f2(c.x))));
+    const float s = a.nsg ? ldg(a.nsg + k) : 0.f, chi = ldg(a.chi + k);
+    const float lu = lap5(x[4].x, x[2].x, y[4].x, y[2].x, c.x, a.idx2, a.idy2);
+    const float lv = lap5(x[4].y, x[2].y, y[4].y, y[2].y, c.y, a.idx2, a.idy2);
+    const float ru = rhs_sum<false>(a, adv.x, lu, 0.f, s), rv = rhs_sum<false>(a, adv.y, lv, 0.f, s);
+    if (a.rk2 && !last && a.k1u_out) {
+      a.k1u_out[k] = ru;
+      a.k1v_out[k] = rv;
+    }
+    const bool two = a.rk2 && last;
+    float uo = stage_sum(a, ldg(a.u0 + k), ru, chi, two ? ldg(a.k1u + k) : 0.f, dt);
+    float vo = stage_sum(a, ldg(a.v0 + k), rv, chi, two ? ldg(a.k1v + k) : 0.f, dt);
+    if (last && !(ldg(a.mask + k) > 0.5f)) uo = vo = 0.f;
+    a.uout[k] = uo;
+    a.vout[k] = vo;
+  }
+}
+
 template <bool PER>
 static void dispatch_rk_col(const RkArgs& a, bool hyper, int adv, dim3 g, dim3 b, cudaStream_t st) {
   if (!PER && adv == AJ_ADV_UPWIND && rk_col4_ok(a)) {
     const dim3 g4(rk4_edge_blocks(a.nx, a.ny) + cdiv(a.ny, 128) * cdiv(a.nx, 8));
     if (hyper) launch_pdl(true, k_rk_col4<true>, dim3(g4), dim3(32, 8), 0, st, a);
     else launch_pdl(true, k_rk_col4<false>, dim3(g4), dim3(32, 8), 0, st, a);
+    return;
+  }
+  if (!PER && !hyper && adv == AJ_ADV_WENO5 && a.nx > 4 * ColRows::HB && a.ny > 4 * ColRows::HB) {
+    const unsigned rows = cdiv(a.nx - 2 * ColRows::HB, 8 * ColRows::R);
+    launch_pdl(true, k_rk_col_rows,
+               dim3(ColRows::edge_blocks(a.nx, a.ny) + rows * cdiv(a.ny, 32)), dim3(32, 8), 0, st,
+               a);
     return;
   }
   if (hyper) {
@@ -1129,177 +1251,286 @@ __device__ __forceinline__ float stage_mac_v_int(const RkMac& a, int i, int j, f
   return finish_mac<1>(a, k, r, chi, dt, k1o);
 }
 
-// stage_mac_u_int and stage_mac_v_int (without hyperviscosity) for the two
-// faces of one interior cell as the lanes of paired FP32 instructions: lane
-// x the u-face (i, j), lane y the v-face (i, j).  "Along" is a face's own
-// direction (x for u, y for v, the upwinded difference), "across" the other
-// (the central difference); the cross velocity is v at the u-face and u at
-// the v-face.  Every lane evaluates its face's expressions in the same order
-// as the scalar functions (products added by fma where those contract).
+// The values that the two faces of one interior cell read, u-face (i, j) in
+// lane x and v-face (i, j) in lane y.  "Along" is a face's own direction (x
+// for u, y for v), "across" the other.
+struct FacePair {
+  float2 c, am, ap, cm, cp;   // the face, its neighbours along and across
+  float2 q2, q3;              // the cross velocity's far faces: v at (i-1, j+1), (i-1, j); u at
+                              // (i+1, j-1), (i, j-1); its near ones are (vyp, vw) and (uxp, uw)
+  float2 mc, mo;              // mask of the cell and of its neighbour across each face
+  float2 sc, so;              // eddy viscosity, likewise
+};
+
+__device__ __forceinline__ float2 pair_cross(const FacePair& f) {
+  const float2 half = f2(0.5f);
+  const float2 q0 = make_float2(f.ap.y, f.ap.x), q1 = make_float2(f.c.y, f.c.x);
+  return mul2(half, add2(mul2(half, add2(q0, q1)), mul2(half, add2(f.q2, f.q3))));
+}
+
+// right-hand side of both faces from the advection before its mask; chi out.
+// Every lane evaluates its face's expressions in the order of stage_mac_u_int
+// and stage_mac_v_int (products added by fma where those contract).
+__device__ __forceinline__ float2 pair_rhs(const RkMac& a, const FacePair& f, float2 adv,
+                                           float2& chi) {
+  const float2 half = f2(0.5f);
+  adv = mul2(adv, mul2(half, add2(f.mc, f.mo)));
+  // Laplacian: x terms are u's along and v's across sums, y terms the others
+  const float2 s_al = add2(f.ap, f.am), s_ac = add2(f.cp, f.cm);
+  const float2 two_c = mul2(f2(2.f), f.c);
+  const float2 lap = fma2(sub2(make_float2(s_al.x, s_ac.y), two_c), f2(a.idx2),
+                          mul2(sub2(make_float2(s_ac.x, s_al.y), two_c), f2(a.idy2)));
+  float2 nut = f2(a.nu);
+  if (a.nsg) nut = add2(nut, mul2(half, add2(f.sc, f.so)));
+  chi = mul2(half, add2(sub2(f2(1.f), f.mc), sub2(f2(1.f), f.mo)));
+  return fma2(nut, lap, make_float2(-adv.x, -adv.y));
+}
+
+// the blended upwind advection of both faces
+__device__ __forceinline__ float2 pair_upwind(const RkMac& a, const FacePair& f) {
+  const float2 cross = pair_cross(f);
+  const float2 h_al = make_float2(a.idx, a.idy);
+  const float2 back = mul2(sub2(f.c, f.am), h_al), fwd = mul2(sub2(f.ap, f.c), h_al);
+  const float2 al = make_float2(upwind_weight(f.c.x), upwind_weight(f.c.y));
+  const float2 adv_al = mul2(f.c, fma2(al, back, mul2(sub2(f2(1.f), al), fwd)));
+  const float2 d_ac = mul2(sub2(f.cp, f.cm), make_float2(0.5f * a.idy, 0.5f * a.idx));
+  return fma2(cross, d_ac, adv_al);
+}
+
+// both faces of interior cell (i, j), one cell a thread
 __device__ __forceinline__ float2 stage_mac_uv_int(const RkMac& a, int i, int j, float dt,
                                                    float* k1u, float* k1v) {
   const int ny = a.ny, nyv = ny + 1;
   const long ku = (long)i * ny + j, kv = (long)i * nyv + j;
   const float* u = a.uin + ku;
   const float* v = a.vin + kv;
-  const float uw = ldg(u), uxm = ldg(u - ny), uxp = ldg(u + ny), uym = ldg(u - 1),
-              uyp = ldg(u + 1);
-  const float vw = ldg(v), vym = ldg(v - 1), vyp = ldg(v + 1), vxm = ldg(v - nyv),
-              vxp = ldg(v + nyv);
-  const float2 c = make_float2(uw, vw);
-  const float2 am = make_float2(uxm, vym), ap = make_float2(uxp, vyp);
-  const float2 cm = make_float2(uym, vxm), cp = make_float2(uyp, vxp);
-  const float2 half = f2(0.5f);
-  // 0.5 (0.5 (v[j+1] + v[j]) + 0.5 (v[i-1, j+1] + v[i-1, j])) and
-  // 0.5 (0.5 (u[i+1] + u[i]) + 0.5 (u[i+1, j-1] + u[i, j-1]))
-  const float2 q0 = make_float2(ldg(v + 1), uxp), q1 = make_float2(vw, uw);
-  const float2 q2 = make_float2(ldg(v - nyv + 1), ldg(u + ny - 1)), q3 = make_float2(vxm, uym);
-  const float2 cross = mul2(half, add2(mul2(half, add2(q0, q1)), mul2(half, add2(q2, q3))));
-  const float2 h_al = make_float2(a.idx, a.idy);
-  const float2 back = mul2(sub2(c, am), h_al), fwd = mul2(sub2(ap, c), h_al);
-  const float2 al = make_float2(upwind_weight(uw), upwind_weight(vw));
-  const float2 adv_al = mul2(c, fma2(al, back, mul2(sub2(f2(1.f), al), fwd)));
-  const float2 d_ac = mul2(sub2(cp, cm), make_float2(0.5f * a.idy, 0.5f * a.idx));
-  // the cell's mask and its neighbour across the face (i-1 for u, j-1 for v)
-  const float2 mc = f2(ldg(a.mask + ku));
-  const float2 mo = make_float2(ldg(a.mask + ku - ny), ldg(a.mask + ku - 1));
-  const float2 adv = mul2(fma2(cross, d_ac, adv_al), mul2(half, add2(mc, mo)));
-  // Laplacian: x terms are u's along and v's across sums, y terms the others
-  const float2 s_al = add2(ap, am), s_ac = add2(cp, cm);
-  const float2 two_c = mul2(f2(2.f), c);
-  const float2 lap = fma2(sub2(make_float2(s_al.x, s_ac.y), two_c), f2(a.idx2),
-                          mul2(sub2(make_float2(s_ac.x, s_al.y), two_c), f2(a.idy2)));
-  float2 nut = f2(a.nu);
+  FacePair f;
+  f.c = make_float2(ldg(u), ldg(v));
+  f.am = make_float2(ldg(u - ny), ldg(v - 1));
+  f.ap = make_float2(ldg(u + ny), ldg(v + 1));
+  f.cm = make_float2(ldg(u - 1), ldg(v - nyv));
+  f.cp = make_float2(ldg(u + 1), ldg(v + nyv));
+  f.q2 = make_float2(ldg(v - nyv + 1), ldg(u + ny - 1));
+  f.q3 = make_float2(f.cm.y, f.cm.x);
+  f.mc = f2(ldg(a.mask + ku));
+  f.mo = make_float2(ldg(a.mask + ku - ny), ldg(a.mask + ku - 1));
+  f.sc = f.so = f2(0.f);
   if (a.nsg) {
-    const float2 no = make_float2(ldg(a.nsg + ku - ny), ldg(a.nsg + ku - 1));
-    nut = add2(nut, mul2(half, add2(f2(ldg(a.nsg + ku)), no)));
+    f.sc = f2(ldg(a.nsg + ku));
+    f.so = make_float2(ldg(a.nsg + ku - ny), ldg(a.nsg + ku - 1));
   }
-  const float2 r = fma2(nut, lap, make_float2(-adv.x, -adv.y));
-  const float2 chi = mul2(half, add2(sub2(f2(1.f), mc), sub2(f2(1.f), mo)));
+  float2 chi;
+  const float2 r = pair_rhs(a, f, pair_upwind(a, f), chi);
   return make_float2(finish_mac<0>(a, ku, r.x, chi.x, dt, k1u),
                      finish_mac<1>(a, kv, r.y, chi.y, dt, k1v));
+}
+
+// one stage of face (i, j) of u (COMP 0) or v; the last one rewrites the
+// boundary rows: a value, or the stage of the interior face they copy
+template <int COMP, bool HYPER, int ADV>
+__device__ __forceinline__ void rk_mac_face(const RkMac& a, int i, int j, float dt) {
+  const int nx = a.nx, ny = a.ny, m = COMP == 0 ? ny : ny + 1;
+  if (i >= (COMP == 0 ? nx + 1 : nx) || j >= m) return;
+  const bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
+  int ii = i, jj = j;
+  float o = 0.f;
+  bool fixed = false;
+  if (last && a.flow == AJ_FLOW_VON_KARMAN) {
+    if (COMP == 0) {
+      fixed = (!a.slip && (j == 0 || j == ny - 1)) || i == 0;
+      if (i == 0 && (a.slip || (j != 0 && j != ny - 1))) o = a.U;
+      ii = i == nx ? nx - 1 : i;
+      jj = a.slip ? (j == 0 ? 1 : (j == ny - 1 ? ny - 2 : j)) : j;
+    } else {
+      fixed = i == 0 || j == 0 || j == ny;
+      ii = i == nx - 1 ? nx - 2 : i;
+    }
+  } else if (last && a.flow == AJ_FLOW_LID_DRIVEN_CAVITY) {
+    if (COMP == 0) {
+      fixed = i == 0 || i == nx || j == 0 || j == ny - 1;
+      if (i != 0 && i != nx && j == ny - 1 && j != 0) o = a.U;
+    } else {
+      fixed = i == 0 || i == nx - 1 || j == 0 || j == ny;
+    }
+  }
+  if (!fixed)
+    o = stage_mac_any<COMP, HYPER, ADV>(a, ii, jj, dt,
+                                        last ? nullptr : (COMP == 0 ? a.k1u_out : a.k1v_out));
+  (COMP == 0 ? a.uout : a.vout)[(long)i * m + j] = o;
+}
+
+// one stage of face (i, j) of one component, 0 <= i <= nx, 0 <= j <= ny: the
+// interior faces of the slip-wall channel without the index logic.  WENO5's
+// 7-point stencils and the face velocities stay off the rows that the boundary
+// conditions rewrite (u 4 <= i <= nx-4, 4 <= j <= ny-5; v 4 <= i <= nx-5,
+// 4 <= j <= ny-4)
+template <int COMP, bool HYPER, int ADV>
+__device__ __forceinline__ void rk_mac_one(const RkMac& a, int i, int j, float dt) {
+  constexpr int HB = ADV == AJ_ADV_WENO5 ? 4 : 2;
+  const int ei = COMP == 0 ? a.nx - HB : a.nx - 1 - HB, ej = COMP == 0 ? a.ny - 1 - HB : a.ny - HB;
+  if (!(a.flow == AJ_FLOW_VON_KARMAN && a.slip && i >= HB && i <= ei && j >= HB && j <= ej))
+    return rk_mac_face<COMP, HYPER, ADV>(a, i, j, dt);
+  const bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
+  float* k1o = last ? nullptr : (COMP == 0 ? a.k1u_out : a.k1v_out);
+  const float o = ADV == AJ_ADV_WENO5 ? stage_mac_any<COMP, HYPER, ADV, true>(a, i, j, dt, k1o)
+                  : COMP == 0         ? stage_mac_u_int<HYPER>(a, i, j, dt, k1o)
+                                      : stage_mac_v_int<HYPER>(a, i, j, dt, k1o);
+  (COMP == 0 ? a.uout : a.vout)[(long)i * (COMP == 0 ? a.ny : a.ny + 1) + j] = o;
 }
 
 template <bool HYPER, int ADV>
 __global__ void __launch_bounds__(256) k_rk_mac(RkMac a) {
   pdl_wait();
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  const int nx = a.nx, ny = a.ny;
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.y * blockDim.y + threadIdx.y;
   const float dt = a.sc->dt;
-  bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
-  const bool fast = a.flow == AJ_FLOW_VON_KARMAN && a.slip;
-  if (ADV == AJ_ADV_WENO5) {
-    // interior faces: u 4 <= i <= nx-4, 4 <= j <= ny-5; v 4 <= i <= nx-5,
-    // 4 <= j <= ny-4 (the 7-point stencils and the face velocities stay off
-    // the rows the boundary conditions rewrite)
-    if (i <= nx && j < ny) {
-      const long k = (long)i * ny + j;
-      float o;
-      if (fast && i >= 4 && i <= nx - 4 && j >= 4 && j <= ny - 5) {
-        o = stage_mac_any<0, HYPER, ADV, true>(a, i, j, dt, last ? nullptr : a.k1u_out);
-      } else if (!last) {
-        o = stage_mac_any<0, HYPER, ADV>(a, i, j, dt, a.k1u_out);
-      } else if (a.flow == AJ_FLOW_VON_KARMAN) {
-        if (!a.slip && (j == 0 || j == ny - 1)) o = 0.f;
-        else if (i == 0) o = a.U;
-        else {
-          int ii = i == nx ? nx - 1 : i;
-          int jj = a.slip ? (j == 0 ? 1 : (j == ny - 1 ? ny - 2 : j)) : j;
-          o = stage_mac_any<0, HYPER, ADV>(a, ii, jj, dt, nullptr);
-        }
-      } else if (a.flow == AJ_FLOW_LID_DRIVEN_CAVITY) {
-        if (i == 0 || i == nx || j == 0) o = 0.f;
-        else if (j == ny - 1) o = a.U;
-        else o = stage_mac_any<0, HYPER, ADV>(a, i, j, dt, nullptr);
-      } else {
-        o = stage_mac_any<0, HYPER, ADV>(a, i, j, dt, nullptr);
-      }
-      a.uout[k] = o;
-    }
-    if (i < nx && j <= ny) {
-      const long k = (long)i * (ny + 1) + j;
-      float o;
-      if (fast && i >= 4 && i <= nx - 5 && j >= 4 && j <= ny - 4) {
-        o = stage_mac_any<1, HYPER, ADV, true>(a, i, j, dt, last ? nullptr : a.k1v_out);
-      } else if (!last) {
-        o = stage_mac_any<1, HYPER, ADV>(a, i, j, dt, a.k1v_out);
-      } else if (a.flow == AJ_FLOW_VON_KARMAN) {
-        if (i == 0 || j == 0 || j == ny) o = 0.f;
-        else o = stage_mac_any<1, HYPER, ADV>(a, i == nx - 1 ? nx - 2 : i, j, dt, nullptr);
-      } else if (a.flow == AJ_FLOW_LID_DRIVEN_CAVITY) {
-        if (i == 0 || i == nx - 1 || j == 0 || j == ny) o = 0.f;
-        else o = stage_mac_any<1, HYPER, ADV>(a, i, j, dt, nullptr);
-      } else {
-        o = stage_mac_any<1, HYPER, ADV>(a, i, j, dt, nullptr);
-      }
-      a.vout[k] = o;
-    }
+  if (ADV != AJ_ADV_WENO5 && !HYPER && a.flow == AJ_FLOW_VON_KARMAN && a.slip && i >= 2 &&
+      i <= a.nx - 3 && j >= 2 && j <= a.ny - 3) {
+    // both faces of an interior cell share the paired FP32 instructions
+    const bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
+    const float2 o = stage_mac_uv_int(a, i, j, dt, last ? nullptr : a.k1u_out,
+                                      last ? nullptr : a.k1v_out);
+    a.uout[(long)i * a.ny + j] = o.x;
+    a.vout[(long)i * (a.ny + 1) + j] = o.y;
     return;
   }
-  if (fast && i >= 2 && i <= nx - 3 && j >= 2 && j <= ny - 3) {
-    // both faces of the cell interior: one scope, so the loads they share
-    // (u at (i,j), (i+1,j), (i,j-1); v at (i,j), (i,j+1), (i-1,j); mask and
-    // nu_sgs at (i,j)) are issued once; without hyperviscosity the two faces
-    // share the paired FP32 instructions
-    float uo, vo;
-    if (HYPER) {
-      uo = stage_mac_u_int<HYPER>(a, i, j, dt, last ? nullptr : a.k1u_out);
-      vo = stage_mac_v_int<HYPER>(a, i, j, dt, last ? nullptr : a.k1v_out);
-    } else {
-      const float2 o = stage_mac_uv_int(a, i, j, dt, last ? nullptr : a.k1u_out,
-                                        last ? nullptr : a.k1v_out);
-      uo = o.x;
-      vo = o.y;
-    }
-    a.uout[(long)i * ny + j] = uo;
-    a.vout[(long)i * (ny + 1) + j] = vo;
+  rk_mac_one<0, HYPER, ADV>(a, i, j, dt);
+  rk_mac_one<1, HYPER, ADV>(a, i, j, dt);
+}
+
+// The stage of the slip-wall von Karman channel a run of rows a thread: the
+// thread walks R cells in x with its columns' values in registers, so a cell
+// reads 12 values (WENO5: 21) where one by itself read 20 (58), and both
+// faces share the paired FP32 instructions, WENO5's reconstructions too.
+// Cells within HB of an edge, where the boundary conditions' index logic
+// applies, go one face a thread on the first blocks.  What bounds it:
+// instructions issued (WENO5), L2 reads (upwind).  Two rows a thread; one was
+// 3 to 5 % slower, four and eight ran out of threads below 2048x512.  Three
+// stages, us, a cell a thread -> this, upwind / WENO5: 128x32 13.2 / 21.9 ->
+// 11.5 / 14.2, 512x128 15.1 / 26.3 -> 11.8 / 16.0, 1021x509 26.7 / 66 ->
+// 18.2 / 33, 2048x512 40 / 113 -> 30 / 58, 4096x2048 236 / 699 -> 223 / 441.
+template <int ADV>
+struct MacRows {
+  static constexpr int HB = ADV == AJ_ADV_WENO5 ? 4 : 2;   // edge cells: i < HB, i > nx-1-HB, ...
+  static constexpr int R = 2;
+  static constexpr int BLOCKS = ADV == AJ_ADV_WENO5 ? 4 : 5;   // blocks an SM (64, 48 registers)
+  __host__ __device__ static int edge_blocks(int nx, int ny) {
+    return (2 * (2 * HB + 1) * (ny + 1 + nx - 2 * HB) + 255) / 256;   // u and v faces
+  }
+};
+template <int ADV>
+__global__ void __launch_bounds__(256, MacRows<ADV>::BLOCKS) k_rk_mac_rows(RkMac a) {
+  pdl_wait();
+  using M = MacRows<ADV>;
+  constexpr int HB = M::HB, R = M::R;
+  const int nx = a.nx, ny = a.ny, nyv = ny + 1;
+  const float dt = a.sc->dt;
+  const int edge = M::edge_blocks(nx, ny);
+  if ((int)blockIdx.x < edge) {
+    constexpr int E = 2 * HB + 1;   // rows (columns) at both ends
+    const int cells = E * (nyv + nx - 2 * HB);
+    int e = blockIdx.x * 256 + threadIdx.y * 32 + threadIdx.x;
+    if (e >= 2 * cells) return;
+    const bool comp = e >= cells;
+    if (comp) e -= cells;
+    const int f = e - E * nyv, q = f < 0 ? e / nyv : f % E;
+    const int i = f < 0 ? (q < HB ? q : nx - 2 * HB + q) : HB + f / E;
+    const int j = f < 0 ? e % nyv : (q < HB ? q : ny - 2 * HB + q);
+    if (comp) rk_mac_one<1, false, ADV>(a, i, j, dt);
+    else rk_mac_one<0, false, ADV>(a, i, j, dt);
     return;
   }
-  // u faces
-  if (i <= nx && j < ny) {
-    long k = (long)i * ny + j;
-    float o;
-    if (fast && i >= 2 && i <= nx - 2 && j >= 2 && j <= ny - 3) {
-      o = stage_mac_u_int<HYPER>(a, i, j, dt, last ? nullptr : a.k1u_out);
-    } else if (!last) {
-      o = stage_mac<0, HYPER>(a, i, j, dt, a.k1u_out);
-    } else if (a.flow == AJ_FLOW_VON_KARMAN) {
-      if (!a.slip && (j == 0 || j == ny - 1)) o = 0.f;
-      else if (i == 0) o = a.U;
-      else {
-        int ii = i == nx ? nx - 1 : i;
-        int jj = a.slip ? (j == 0 ? 1 : (j == ny - 1 ? ny - 2 : j)) : j;
-        o = stage_mac<0, HYPER>(a, ii, jj, dt, nullptr);
-      }
-    } else if (a.flow == AJ_FLOW_LID_DRIVEN_CAVITY) {
-      if (i == 0 || i == nx || j == 0) o = 0.f;
-      else if (j == ny - 1) o = a.U;
-      else o = stage_mac<0, HYPER>(a, i, j, dt, nullptr);
-    } else {
-      o = stage_mac<0, HYPER>(a, i, j, dt, nullptr);
+  const int bj = (ny + 31) / 32, b = blockIdx.x - edge;
+  const int j = b % bj * 32 + threadIdx.x, i0 = HB + (b / bj * 8 + threadIdx.y) * R;
+  if (j < HB || j > ny - 1 - HB || i0 > nx - 1 - HB) return;
+  const bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
+  float* k1u = last ? nullptr : a.k1u_out;
+  float* k1v = last ? nullptr : a.k1v_out;
+  const float* u = a.uin + (long)i0 * ny + j;
+  const float* v = a.vin + (long)i0 * nyv + j;
+  const float* m = a.mask + (long)i0 * ny + j;
+  const float* sg = a.nsg ? a.nsg + (long)i0 * ny + j : nullptr;
+  constexpr int XW = ADV == AJ_ADV_WENO5 ? 7 : 3, XH = XW / 2;
+  float2 x[XW];   // column j of u and v, rows i - XH .. i + XH
+#pragma unroll
+  for (int q = 1; q < XW; ++q)
+    x[q] = make_float2(ldg(u + (long)(q - 1 - XH) * ny), ldg(v + (long)(q - 1 - XH) * nyv));
+  float um = ldg(u - 1);           // u at (i, j - 1)
+  float v_mp = ldg(v - nyv + 1);   // v at (i - 1, j + 1)
+  float m_im = ldg(m - ny), s_im = sg ? ldg(sg - ny) : 0.f;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = i0 + r;
+    if (i > nx - 1 - HB) break;
+#pragma unroll
+    for (int q = 0; q + 1 < XW; ++q) x[q] = x[q + 1];
+    x[XW - 1] = make_float2(ldg(u + (long)XH * ny), ldg(v + (long)XH * nyv));
+    const float u_pm = ldg(u + ny - 1);
+    FacePair f;
+    f.c = x[XH];
+    const float up = ldg(u + 1), vm = ldg(v - 1), vp = ldg(v + 1);
+    f.am = make_float2(x[XH - 1].x, vm);
+    f.ap = make_float2(x[XH + 1].x, vp);
+    f.cm = make_float2(um, x[XH - 1].y);
+    f.cp = make_float2(up, x[XH + 1].y);
+    f.q2 = make_float2(v_mp, u_pm);
+    f.q3 = make_float2(f.cm.y, f.cm.x);
+    const float m_c = ldg(m);
+    f.mc = f2(m_c);
+    f.mo = make_float2(m_im, ldg(m - 1));
+    f.sc = f.so = f2(0.f);
+    if (sg) {
+      const float s_c = ldg(sg);
+      f.sc = f2(s_c);
+      f.so = make_float2(s_im, ldg(sg - 1));
+      s_im = s_c;
+      sg += ny;
     }
-    a.uout[k] = o;
-  }
-  // v faces
-  if (i < nx && j <= ny) {
-    long k = (long)i * (ny + 1) + j;
-    float o;
-    if (fast && i >= 2 && i <= nx - 3 && j >= 2 && j <= ny - 2) {
-      o = stage_mac_v_int<HYPER>(a, i, j, dt, last ? nullptr : a.k1v_out);
-    } else if (!last) {
-      o = stage_mac<1, HYPER>(a, i, j, dt, a.k1v_out);
-    } else if (a.flow == AJ_FLOW_VON_KARMAN) {
-      if (i == 0 || j == 0 || j == ny) o = 0.f;
-      else o = stage_mac<1, HYPER>(a, i == nx - 1 ? nx - 2 : i, j, dt, nullptr);
-    } else if (a.flow == AJ_FLOW_LID_DRIVEN_CAVITY) {
-      if (i == 0 || i == nx - 1 || j == 0 || j == ny) o = 0.f;
-      else o = stage_mac<1, HYPER>(a, i, j, dt, nullptr);
+    float2 adv;
+    if constexpr (ADV == AJ_ADV_WENO5) {
+      // u in lane x, v in lane y; both derivatives in x, then both in y
+      const float2 cross = pair_cross(f);
+      const float2 vx = make_float2(f.c.x, cross.y), vy = make_float2(cross.x, f.c.y);
+      const float2 y[7] = {make_float2(ldg(u - 3), ldg(v - 3)), make_float2(ldg(u - 2), ldg(v - 2)),
+                           make_float2(um, vm), f.c, make_float2(up, vp),
+                           make_float2(ldg(u + 2), ldg(v + 2)), make_float2(ldg(u + 3), ldg(v + 3))};
+      adv = fma2(vy, weno_d7_pair(y, a.idy, vy), mul2(vx, weno_d7_pair(x, a.idx, vx)));
     } else {
-      o = stage_mac<1, HYPER>(a, i, j, dt, nullptr);
+      adv = pair_upwind(a, f);
     }
-    a.vout[k] = o;
+    float2 chi;
+    const float2 rhs = pair_rhs(a, f, adv, chi);
+    const long ku = (long)i * ny + j, kv = (long)i * nyv + j;
+    a.uout[ku] = finish_mac<0>(a, ku, rhs.x, chi.x, dt, k1u);
+    a.vout[kv] = finish_mac<1>(a, kv, rhs.y, chi.y, dt, k1v);
+    um = u_pm;
+    v_mp = vp;
+    m_im = m_c;
+    u += ny;
+    v += nyv;
+    m += ny;
   }
+}
+
+template <int ADV>
+static bool mac_rows_ok(const RkMac& a, bool hyper) {
+  return !hyper && a.flow == AJ_FLOW_VON_KARMAN && a.slip && a.nx > 4 * MacRows<ADV>::HB &&
+         a.ny > 4 * MacRows<ADV>::HB;
+}
+template <int ADV>
+static void dispatch_rk_mac(const RkMac& a, bool hyper, cudaStream_t st) {
+  if (mac_rows_ok<ADV>(a, hyper)) {
+    using M = MacRows<ADV>;
+    const unsigned rows = cdiv(a.nx - 2 * M::HB, 8 * M::R);
+    launch_pdl(true, k_rk_mac_rows<ADV>, dim3(M::edge_blocks(a.nx, a.ny) + rows * cdiv(a.ny, 32)),
+               dim3(32, 8), 0, st, a);
+    return;
+  }
+  // 16 x 16 blocks: measured 4.5 us per step faster than 32 x 8 (and than
+  // 64 x 4, 8 x 32) on the 2048x512 workload
+  const dim3 blk(16, 16), grd(cdiv(a.ny + 1, 16), cdiv(a.nx + 1, 16));
+  if (hyper) launch_pdl(true, k_rk_mac<true, ADV>, dim3(grd), dim3(blk), 0, st, a);
+  else launch_pdl(true, k_rk_mac<false, ADV>, dim3(grd), dim3(blk), 0, st, a);
 }
 
 // ============================================================ driver
@@ -1386,9 +1617,6 @@ int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const flo
     a.rk2 = rk2;
     a.flow = p.flow_type;
     a.slip = p.slip_walls;
-    // 16 x 16 blocks: measured 4.5 us per step faster than 32 x 8 (and than
-    // 64 x 4, 8 x 32) on the 2048x512 workload
-    dim3 blk(16, 16), grd(cdiv(ny + 1, 16), cdiv(nx + 1, 16));
     const float* in_u = u;
     const float* in_v = v;
     for (int s = 1; s <= nstage; ++s) {
@@ -1401,11 +1629,8 @@ int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const flo
       a.vout = last ? vs : dst[1];
       a.k1u_out = (rk2 && s == 1) ? K[0] : nullptr;
       a.k1v_out = (rk2 && s == 1) ? K[1] : nullptr;
-      const bool weno = p.advection == AJ_ADV_WENO5;
-      if (hyper && weno) launch_pdl(true, k_rk_mac<true, AJ_ADV_WENO5>, dim3(grd), dim3(blk), 0, st, a);
-      else if (hyper) launch_pdl(true, k_rk_mac<true, AJ_ADV_UPWIND>, dim3(grd), dim3(blk), 0, st, a);
-      else if (weno) launch_pdl(true, k_rk_mac<false, AJ_ADV_WENO5>, dim3(grd), dim3(blk), 0, st, a);
-      else launch_pdl(true, k_rk_mac<false, AJ_ADV_UPWIND>, dim3(grd), dim3(blk), 0, st, a);
+      if (p.advection == AJ_ADV_WENO5) dispatch_rk_mac<AJ_ADV_WENO5>(a, hyper, st);
+      else dispatch_rk_mac<AJ_ADV_UPWIND>(a, hyper, st);
       in_u = a.uout;
       in_v = a.vout;
     }

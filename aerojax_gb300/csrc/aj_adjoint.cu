@@ -157,8 +157,9 @@ __device__ __forceinline__ void bc_gather_T(const float* __restrict__ gu_o,
 struct AdjCorr {
   const float *gu_o, *gv_o, *gp_o, *mask;
   float *gus, *gvs, *gdpx, *gdpy, *pbar;
-  const DevScalars* sc;
-  int nx, ny, gui;
+  DevScalars* sc;
+  int nx, ny, gui, set_dt;         // set_dt: write dt, dtc to sc (nothing before this kernel did)
+  float dt, dtc;                   // the step's dt and the correction's
   float idx, idy, h2x, h2y, thresh;
 };
 
@@ -172,6 +173,10 @@ __global__ void __launch_bounds__(256) k_adj_correct(AdjCorr c) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = blockIdx.y * blockDim.y + threadIdx.y;
   const int nx = c.nx, ny = c.ny;
+  if (c.set_dt && i == 0 && j == 0) {
+    c.sc->dt = c.dt;
+    c.sc->dt_corr = c.dtc;
+  }
   if (i >= nx || j >= ny) return;
   const long k = (long)i * ny + j;
   float gu, gv;
@@ -179,7 +184,7 @@ __global__ void __launch_bounds__(256) k_adj_correct(AdjCorr c) {
   if (!c.gui && !live_at(c.mask, k)) gu = gv = 0.f;            // step.py:348-349
   c.gus[k] = gu;
   c.gvs[k] = gv;
-  const float dt = c.sc->dt_corr;
+  const float dt = c.dtc;
   float ax = -dt * gu, ay = -dt * gv;                           // (row 0: gu = 0, :341)
   if (c.gui) {
     c.gdpx[k] = ax;
@@ -654,7 +659,6 @@ int launch_step_vjp(const AjStepParams& p, const Layout& L, void* ws, void* aws,
   // nothing before the predictor's reverse pass reads them: the predictor
   // runs on a side branch joined before k_adj_rk_out.  With more cycles the
   // forward solve counts the cycles the reverse pass replays, in line.
-  if ((rc = launch_set_dt(p, ws, st)) != AJ_OK) return rc;
   const bool branch = p.v_cycles == 1;
   if (branch) {
     if (cudaEventRecord(fk->fork, st) != cudaSuccess ||
@@ -662,7 +666,7 @@ int launch_step_vjp(const AjStepParams& p, const Layout& L, void* ws, void* aws,
       return AJ_ERR_CUDA;
   }
   rc = launch_predictor(p, L, ws, u, v, mask, nullptr, 0, F(A.wnu), F(A.wnv),
-                        branch ? fk->side : st);
+                        branch ? fk->side : st, branch ? DtFrom::host_unwritten : DtFrom::host);
   if (rc != AJ_OK) return rc;
   if (branch && cudaEventRecord(fk->join, fk->side) != cudaSuccess) return AJ_ERR_CUDA;
   const int* ncyc = nullptr;
@@ -693,6 +697,9 @@ int launch_step_vjp(const AjStepParams& p, const Layout& L, void* ws, void* aws,
   c.h2y = (float)(1.0 / (2.0 * p.dy));
   c.thresh = (float)(0.1 / p.dx);
   c.gui = p.variant == AJ_VARIANT_GUI;
+  c.set_dt = branch;
+  c.dt = (float)p.dt;
+  c.dtc = (float)p.dt_correction > 0.f ? (float)p.dt_correction : c.dt;
   launch_pdl(true, k_adj_correct, grd, blk, 0, st, c);
   launch_pdl(true, k_adj_grad, grd, blk, 0, st, c);
   // ---- multigrid, reversed (cycles from the last to the first)
@@ -816,7 +823,7 @@ int launch_step_vjp(const AjStepParams& p, const Layout& L, void* ws, void* aws,
 
 int step_vjp_kernel_count(const AjStepParams& p, const Layout& L) {
   const int nst = p.fast_mode ? 2 : 3;
-  int n = 1 + nst;                                  // dt + forward predictor stages
+  int n = nst;                                      // forward predictor stages
   const bool fused = parity_coarsest_fused(L);
   if (p.v_cycles > 1)                               // rhs, forward solve (no statistics)
     n += 1 + parity_kernel_count(p, L) - (parity_cluster_level(p, L) > 0);

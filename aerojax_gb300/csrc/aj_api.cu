@@ -365,7 +365,12 @@ static int enqueue_step(const AjStepParams& p, const Layout& L, void* ws, const 
     nsg = f;
     dc = (p.variant == AJ_VARIANT_GUI && !mac) ? 1 : 0;
   }
-  rc = p.cfl_dt ? launch_cfl(p, ws, u, v, nullptr, st) : launch_set_dt(p, ws, st);
+  // a fixed dt is written by the predictor's first stage, unless the
+  // converging solve's initial state or the tile kernel read it before
+  const bool tile = tile_predictor_ok(p, u, mask, nsg);
+  const bool stage_sets_dt = !p.cfl_dt && !conv && !tile;
+  rc = p.cfl_dt ? launch_cfl(p, ws, u, v, nullptr, st)
+                : (stage_sets_dt ? (int)AJ_OK : launch_set_dt(p, ws, st));
   if (rc != AJ_OK) return rc;
   if (conv) {
     if (cudaEventRecord(fk->dt_done, st) != cudaSuccess ||
@@ -381,14 +386,15 @@ static int enqueue_step(const AjStepParams& p, const Layout& L, void* ws, const 
   if (les && cudaStreamWaitEvent(st, fk->les_done, 0) != cudaSuccess) return AJ_ERR_CUDA;
   float* us = at<float>(ws, L.sS_u);
   float* vs = at<float>(ws, L.sS_v);
-  if (tile_predictor_ok(p, u, mask, nsg)) {
+  if (tile) {
     // the three stages, boundary rows and the pressure rhs in one tile kernel
     const float* sb[4] = {at<float>(ws, L.sA_u), at<float>(ws, L.sA_v), at<float>(ws, L.sB_u),
                           at<float>(ws, L.sB_v)};
     rc = launch_predictor_tile(p, ws, u, v, mask, nsg, us, vs, at<float>(ws, L.b0), sb, st);
     if (rc != AJ_OK) return rc;
   } else {
-    rc = launch_predictor(p, L, ws, u, v, mask, nsg, dc, us, vs, st);
+    rc = launch_predictor(p, L, ws, u, v, mask, nsg, dc, us, vs, st,
+                          stage_sets_dt ? DtFrom::host : DtFrom::device);
     if (rc != AJ_OK) return rc;
     // with the learned warm start on the MAC grid, the network's features
     // kernel forms the right-hand side (one launch fewer before the network)
@@ -404,7 +410,7 @@ static int enqueue_step(const AjStepParams& p, const Layout& L, void* ws, const 
   nw.packed = nn.packed;
   nw.master = nn.master;
   nw.mask = mask;
-  if (nn_forms_rhs(p, nn.packed != nullptr) && !tile_predictor_ok(p, u, mask, nsg)) {
+  if (nn_forms_rhs(p, nn.packed != nullptr) && !tile) {
     nw.us = us;
     nw.vs = vs;
   }
@@ -688,9 +694,9 @@ int32_t aj_predictor(const AjStepParams* prm, const float* u, const float* v, co
   make_layout(p, L);
   if ((rc = ws_ok(L, ws, bytes)) != AJ_OK) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  rc = p.cfl_dt ? launch_cfl(p, ws, u, v, nullptr, st) : launch_set_dt(p, ws, st);
-  if (rc != AJ_OK) return rc;
-  return launch_predictor(p, L, ws, u, v, mask, nu_sgs, double_count, u_star, v_star, st);
+  if (p.cfl_dt && (rc = launch_cfl(p, ws, u, v, nullptr, st)) != AJ_OK) return rc;
+  return launch_predictor(p, L, ws, u, v, mask, nu_sgs, double_count, u_star, v_star, st,
+                          p.cfl_dt ? DtFrom::device : DtFrom::host);
 }
 
 int32_t aj_cfl_dt(const AjStepParams* prm, const float* u, const float* v, float* dt_out,
@@ -716,7 +722,7 @@ int32_t aj_profile_kernel(const AjStepParams* prm, int32_t which, const float* u
   if (which == 3) {   // the predictor (all stages) from (u, v) into the workspace
     if (!u || !v || !mask) return AJ_ERR_PARAM;
     return launch_predictor(p, L, ws, u, v, mask, nullptr, 0, at<float>(ws, L.sS_u),
-                            at<float>(ws, L.sS_v), st);
+                            at<float>(ws, L.sS_v), st, DtFrom::device);
   }
   return AJ_ERR_PARAM;
 }
@@ -727,7 +733,8 @@ int32_t aj_kernel_count(const AjStepParams* prm, int32_t cycles) {
   Layout L;
   if (!make_layout(p, L)) return -1;
   const bool mac = p.grid_type == AJ_GRID_MAC;
-  int n = 1;                                                    // cfl or set-dt
+  // cfl, or the dt's own launch where the first stage does not write it
+  int n = p.cfl_dt || p.mg_mode == AJ_MG_CONVERGE || tile_predictor_params_ok(p) ? 1 : 0;
   if (p.les_model != AJ_LES_NONE && (p.variant == AJ_VARIANT_GUI || mac))
     n += p.les_model == AJ_LES_DYNAMIC ? (mac ? 1 : 0) + 4 : 1;
   if (tile_predictor_params_ok(p)) n += tile_predictor_kernels();   // stages + rhs in tile kernels

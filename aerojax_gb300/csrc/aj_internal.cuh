@@ -304,9 +304,13 @@ inline cudaError_t launch_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim
 
 // ------------------------------------------------------------------ launchers
 // predictor (aj_predictor.cu)
+// where a predictor's dt comes from: the device's scalars (a CFL dt, or one
+// that is set already), the parameters, written to the scalars by the first
+// stage, or the parameters alone (the scalars are set on another stream)
+enum class DtFrom { device, host, host_unwritten };
 int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const float* u,
                      const float* v, const float* mask, const float* nsg, int double_count,
-                     float* us, float* vs, cudaStream_t st);
+                     float* us, float* vs, cudaStream_t st, DtFrom dt);
 // the MAC predictor's three stages, boundary rows and pressure rhs (b,
 // nullable) in one shared-memory tile kernel (aj_predictor_tile.cu)
 bool tile_predictor_params_ok(const AjStepParams& p);

@@ -53,6 +53,25 @@ int launch_set_dt(const AjStepParams& p, void* ws, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
 }
 
+// A stage's dt: read from the device, or known to the host.  A step with a
+// fixed dt needs no launch of its own to put it on the device: its first
+// stage writes it for the kernels after it.
+struct StageDt {
+  DevScalars* write = nullptr;   // first stage of a fixed-dt step
+  const DevScalars* sc = nullptr;
+  float dt = 0.f, dtc = 0.f;
+  int known = 0;
+};
+__device__ __forceinline__ float stage_dt(const StageDt& d) { return d.known ? d.dt : d.sc->dt; }
+// (the large kernels do it on their edge blocks' branch: before the loads it
+// cost the staggered upwind stages at 4096x2048 223 -> 281 us)
+__device__ __forceinline__ void stage_dt_write(const StageDt& d) {
+  if (d.write && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
+    d.write->dt = d.dt;
+    d.write->dt_corr = d.dtc > 0.f ? d.dtc : d.dt;
+  }
+}
+
 // compute_cfl_timestep (timestepping/cfl_adaptive_dt.py:6-71): block maxima,
 // atomicMax, and the last block to finish turns the maximum into dt.
 __global__ void k_cfl(const float* __restrict__ u, const float* __restrict__ v, long nu_,
@@ -399,7 +418,7 @@ int launch_les(const AjStepParams& p, const Layout& L, void* ws, int model, cons
 struct RkArgs {
   const float *uin, *vin, *u0, *v0, *chi, *mask, *nsg, *k1u, *k1v;
   float *uout, *vout, *k1u_out, *k1v_out;
-  const DevScalars* sc;
+  StageDt dt;
   int nx, ny;
   float idx, idy, idx2, idy2, nu, inv_eta, U, nuh_fac;
   int dc, stage, rk2, flow, slip;
@@ -676,7 +695,8 @@ __global__ void __launch_bounds__(256) k_rk_col(RkArgs a) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= a.nx || j >= a.ny) return;
-  rk_col_cell<PER, HYPER, ADV>(a, i, j, a.sc->dt);
+  stage_dt_write(a.dt);
+  rk_col_cell<PER, HYPER, ADV>(a, i, j, stage_dt(a.dt));
 }
 
 // The upwind stage four columns a thread: 16-byte reads of the five rows that
@@ -691,9 +711,10 @@ template <bool HYPER>
 __global__ void __launch_bounds__(256) k_rk_col4(RkArgs a) {
   pdl_wait();
   const int nx = a.nx, ny = a.ny;
-  const float dt = a.sc->dt;
+  const float dt = stage_dt(a.dt);
   const int edge = rk4_edge_blocks(nx, ny);
   if ((int)blockIdx.x < edge) {   // a cell each: two rows, four columns at each end
+    stage_dt_write(a.dt);
     const int e = blockIdx.x * 256 + threadIdx.y * 32 + threadIdx.x, f = e - 4 * ny;
     if (f < 0) rk_col_cell<false, HYPER, AJ_ADV_UPWIND>(a, e < 2 * ny ? e / ny : nx - 4 + e / ny, e % ny, dt);
     else if (f < 8 * (nx - 4))
@@ -789,9 +810,10 @@ __global__ void __launch_bounds__(256, 4) k_rk_col_rows(RkArgs a) {
   pdl_wait();
   constexpr int HB = ColRows::HB, R = ColRows::R, E = 2 * HB;
   const int nx = a.nx, ny = a.ny;
-  const float dt = a.sc->dt;
+  const float dt = stage_dt(a.dt);
   const int edge = ColRows::edge_blocks(nx, ny);
   if ((int)blockIdx.x < edge) {
+    stage_dt_write(a.dt);
     const int cells = E * (ny + nx - 2 * HB);
     int e = blockIdx.x * 256 + threadIdx.y * 32 + threadIdx.x;
     if (e >= 2 * cells) return;
@@ -871,7 +893,7 @@ static void dispatch_rk_col(const RkArgs& a, bool hyper, int adv, dim3 g, dim3 b
 struct RkMac {
   const float *uin, *vin, *u0, *v0, *mask, *nsg, *k1u, *k1v;
   float *uout, *vout, *k1u_out, *k1v_out;
-  const DevScalars* sc;
+  StageDt dt;
   int nx, ny;
   float idx, idy, idx2, idy2, nu, inv_eta, U, nuh;
   int stage, rk2, flow, slip;
@@ -1383,7 +1405,8 @@ __global__ void __launch_bounds__(256) k_rk_mac(RkMac a) {
   pdl_wait();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = blockIdx.y * blockDim.y + threadIdx.y;
-  const float dt = a.sc->dt;
+  const float dt = stage_dt(a.dt);
+  stage_dt_write(a.dt);
   if (ADV != AJ_ADV_WENO5 && !HYPER && a.flow == AJ_FLOW_VON_KARMAN && a.slip && i >= 2 &&
       i <= a.nx - 3 && j >= 2 && j <= a.ny - 3) {
     // both faces of an interior cell share the paired FP32 instructions
@@ -1424,9 +1447,14 @@ __global__ void __launch_bounds__(256, MacRows<ADV>::BLOCKS) k_rk_mac_rows(RkMac
   using M = MacRows<ADV>;
   constexpr int HB = M::HB, R = M::R;
   const int nx = a.nx, ny = a.ny, nyv = ny + 1;
-  const float dt = a.sc->dt;
+  // upwind reads the device's dt even where it is not used: without that read
+  // the compiler orders the loads after it differently, and three stages at
+  // 4096x2048 take 285 us instead of 223
+  const float read = ADV == AJ_ADV_WENO5 ? 0.f : a.dt.sc->dt;
+  const float dt = ADV == AJ_ADV_WENO5 ? stage_dt(a.dt) : (a.dt.known ? a.dt.dt : read);
   const int edge = M::edge_blocks(nx, ny);
   if ((int)blockIdx.x < edge) {
+    stage_dt_write(a.dt);
     constexpr int E = 2 * HB + 1;   // rows (columns) at both ends
     const int cells = E * (nyv + nx - 2 * HB);
     int e = blockIdx.x * 256 + threadIdx.y * 32 + threadIdx.x;
@@ -1536,8 +1564,12 @@ static void dispatch_rk_mac(const RkMac& a, bool hyper, cudaStream_t st) {
 // ============================================================ driver
 int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const float* u,
                      const float* v, const float* mask, const float* nsg, int double_count,
-                     float* us, float* vs, cudaStream_t st) {
-  const DevScalars* sc = at<DevScalars>(ws, 0);
+                     float* us, float* vs, cudaStream_t st, DtFrom dt) {
+  StageDt sdt;
+  sdt.sc = at<DevScalars>(ws, 0);
+  sdt.known = dt != DtFrom::device;
+  sdt.dt = (float)p.dt;
+  sdt.dtc = (float)p.dt_correction;
   const int nx = p.nx, ny = p.ny;
   const bool rk2 = p.fast_mode != 0;
   const int nstage = rk2 ? 2 : 3;
@@ -1557,7 +1589,6 @@ int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const flo
     a.nsg = nsg;
     a.k1u = K[0];
     a.k1v = K[1];
-    a.sc = sc;
     a.nx = nx;
     a.ny = ny;
     a.idx = (float)(1.0 / p.dx);
@@ -1577,6 +1608,8 @@ int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const flo
     const float* in_v = v;
     for (int s = 1; s <= nstage; ++s) {
       a.stage = s;
+      a.dt = sdt;
+      if (s == 1 && dt == DtFrom::host) a.dt.write = at<DevScalars>(ws, 0);
       a.uin = in_u;
       a.vin = in_v;
       bool last = s == nstage;
@@ -1593,6 +1626,7 @@ int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const flo
   } else {
     if (p.advection != AJ_ADV_UPWIND && p.advection != AJ_ADV_WENO5) return AJ_ERR_PARAM;
     if (tile_predictor_ok(p, u, mask, nsg)) {
+      if (dt != DtFrom::device) launch_set_dt(p, ws, st);
       const float* sb[4] = {A[0], A[1], B[0], B[1]};
       return launch_predictor_tile(p, ws, u, v, mask, nsg, us, vs, nullptr, sb, st);
     }
@@ -1603,7 +1637,6 @@ int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const flo
     a.nsg = nsg;
     a.k1u = K[0];
     a.k1v = K[1];
-    a.sc = sc;
     a.nx = nx;
     a.ny = ny;
     a.idx = (float)(1.0 / p.dx);
@@ -1621,6 +1654,8 @@ int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const flo
     const float* in_v = v;
     for (int s = 1; s <= nstage; ++s) {
       a.stage = s;
+      a.dt = sdt;
+      if (s == 1 && dt == DtFrom::host) a.dt.write = at<DevScalars>(ws, 0);
       a.uin = in_u;
       a.vin = in_v;
       bool last = s == nstage;

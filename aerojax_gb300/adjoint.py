@@ -55,7 +55,8 @@ class StepVjp:
         self.aws = torch.empty(nbytes, dtype=torch.uint8, device=device)
         shape = (cfg.nx, cfg.ny)
         z = lambda: torch.zeros(shape, dtype=torch.float32, device=device)
-        self.u_in, self.v_in = z(), z()
+        self.uv_in = torch.zeros((2, *shape), dtype=torch.float32, device=device)
+        self.u_in, self.v_in = self.uv_in[0], self.uv_in[1]
         self.g_in = (z(), z(), z())          # cotangents of the step's u, v, p
         self.g_out = (z(), z())              # cotangents of the step's input u, v
         self.gsdf = z()
@@ -67,11 +68,13 @@ class StepVjp:
     def kernel_count(self) -> int:
         return int(lib().aj_step_vjp_kernel_count(ctypes.byref(self.plan.params)))
 
-    def __call__(self, u, v, mask, gu, gv, gp=None, stream=None):
-        """Cotangents of one step's inputs, written to ``self.g_out``; the
-        SDF's cotangent is added to ``self.gsdf`` and (d/d nu, d/d U_inf) to
+    def __call__(self, u, v, mask, gu, gv, gp=None, stream=None, out=None):
+        """Cotangents of one step's inputs, written to ``self.g_out`` (or to
+        ``out``; ``self.g_in``'s first two may be overwritten); the SDF's
+        cotangent is added to ``self.gsdf`` and (d/d nu, d/d U_inf) to
         ``self.gscal``.  u, v, gu, gv, gp are copied into the staging buffers
         (skipped when they already are those buffers)."""
+        out = self.g_out if out is None else out
         for dst, src in ((self.u_in, u), (self.v_in, v), (self.g_in[0], gu), (self.g_in[1], gv)):
             if src.data_ptr() != dst.data_ptr():
                 dst.copy_(src)
@@ -83,11 +86,11 @@ class StepVjp:
         P = self.plan
         check("aj_step_vjp", lib().aj_step_vjp(
             ctypes.byref(P.params), self.u_in.data_ptr(), self.v_in.data_ptr(), mask.data_ptr(),
-            self.g_in[0].data_ptr(), self.g_in[1].data_ptr(), gp_ptr, self.g_out[0].data_ptr(),
-            self.g_out[1].data_ptr(), self.gsdf.data_ptr() if self.cfg.has_sdf else None,
+            self.g_in[0].data_ptr(), self.g_in[1].data_ptr(), gp_ptr, out[0].data_ptr(),
+            out[1].data_ptr(), self.gsdf.data_ptr() if self.cfg.has_sdf else None,
             self.gscal.data_ptr(), P.ws.data_ptr(), P.nbytes, self.aws.data_ptr(), self.adj_bytes,
             _stream(stream)))
-        return self.g_out
+        return out
 
     def zero_grad(self):
         self.gsdf.zero_()
@@ -178,8 +181,9 @@ def _cached(cache: dict, key, make):
 def _forward_plan(cfg: StepConfig, device):
     def make():
         shape = (cfg.nx, cfg.ny)
-        e = lambda: torch.empty(shape, dtype=torch.float32, device=device)
-        return (Plan(cfg, device), [(e(), e()), (e(), e())], e())
+        e = lambda *lead: torch.empty((*lead, *shape), dtype=torch.float32, device=device)
+        pair = lambda t: (t[0], t[1], t)
+        return (Plan(cfg, device), [pair(e(2)), pair(e(2))], e())
     ent = _cached(_FWD, (repr(replace(cfg, dt=0.0)), str(device)), make)
     ent[0].params.dt = float(cfg.dt)
     return ent
@@ -202,20 +206,20 @@ def differentiable_rollout(initial_state: SimState, mask, params: dict, num_step
     plan, bufs, p = _forward_plan(cfg, dev)
     plan.prepare(mask, sdf, stream)
     nx, ny = cfg.nx, cfg.ny
-    hu = torch.empty((num_steps, nx, ny), dtype=torch.float32, device=dev)
-    hv = torch.empty_like(hu)
+    # both histories in one allocation: a step's u and v are filed by one copy
+    hist = torch.empty((2, num_steps, nx, ny), dtype=torch.float32, device=dev)
+    hu, hv = hist[0], hist[1]
     # fixed ping-pong buffers: one cached graph serves every step
     bufs[0][0].copy_(initial_state.u)
     bufs[0][1].copy_(initial_state.v)
     cur = 0
     for k in range(num_steps):
-        (u, v), (uo, vo) = bufs[cur], bufs[1 - cur]
+        (u, v, _), (uo, vo, new) = bufs[cur], bufs[1 - cur]
         check("aj_step", lib().aj_step(ctypes.byref(plan.params), u.data_ptr(), v.data_ptr(),
                                        mask.data_ptr(), None, uo.data_ptr(), vo.data_ptr(),
                                        p.data_ptr(), plan.ws.data_ptr(), plan.nbytes,
                                        plan.stats_buf.data_ptr(), _stream(stream)))
-        hu[k].copy_(uo)
-        hv[k].copy_(vo)
+        hist[:, k].copy_(new)
         cur = 1 - cur
     prev_u = hu[-2] if num_steps > 1 else initial_state.u
     prev_v = hv[-2] if num_steps > 1 else initial_state.v
@@ -244,12 +248,21 @@ def rollout_vjp(initial_state: SimState, mask, params: dict, num_steps: int, g_u
     gA = (op.g_in[0], op.g_in[1])
     gA[0].copy_(g_u)
     gA[1].copy_(g_v)
+    # the two histories as one tensor, where differentiable_rollout made them:
+    # one copy stages a step's u and v.  The cotangents stay in place.
+    hist = hu._base if hu._base is not None and hu._base is hv._base else None
+    if hist is not None and not (hist.shape == (2, *hu.shape) and
+                                 hist[0].data_ptr() == hu.data_ptr() and
+                                 hist[1].data_ptr() == hv.data_ptr()):
+        hist = None
     for k in range(num_steps - 1, -1, -1):
-        u_k = initial_state.u if k == 0 else hu[k - 1]
-        v_k = initial_state.v if k == 0 else hv[k - 1]
-        gu, gv = op(u_k, v_k, mask, gA[0], gA[1], None, stream=stream)
-        gA[0].copy_(gu)
-        gA[1].copy_(gv)
+        if k > 0 and hist is not None:
+            op.uv_in.copy_(hist[:, k - 1])
+            u_k, v_k = op.u_in, op.v_in
+        else:
+            u_k = initial_state.u if k == 0 else hu[k - 1]
+            v_k = initial_state.v if k == 0 else hv[k - 1]
+        op(u_k, v_k, mask, gA[0], gA[1], None, stream=stream, out=gA)
     sc = op.gscal.cpu()
     return {"u": gA[0].clone(), "v": gA[1].clone(),
             "sdf": op.gsdf.clone() if sdf is not None else None,

@@ -9,7 +9,7 @@
 //   correction + interface projection + boundary rows + hard masks
 //     (solver/pure_functions/step.py:259-397)       -> k_adj_correct, k_adj_grad
 //   parity multigrid (pressure_solvers/multigrid_solver.py:173-241)
-//                                                    -> k_adj_pair/prolong/coarsest
+//                                                    -> k_adj_pair/prolong/tail
 //   rhs = div*mask/dt (step.py:182-199)              -> k_adj_div
 //   RK3/RK2 upwind predictor with implicit Brinkman (rk3_simple_new.py:284-358)
 //                                                    -> k_adj_rk_out, k_adj_rk_stage
@@ -27,6 +27,7 @@
 // first, so one transpose covers both.  Forward stage states are recomputed
 // by the forward predictor kernels (stage buffers of the step workspace).
 #include "aj_internal.cuh"
+#include <algorithm>
 
 #include <cooperative_groups.h>
 #include <mutex>
@@ -82,7 +83,7 @@ static bool make_adj_layout(const AjStepParams& p, const Layout& L, AdjLayout& A
     A.GB[l] = take(n);
   }
   A.nblk = cdiv(p.ny, kAdjBX) * cdiv(p.nx, kAdjBY);
-  A.part = take((size_t)A.nblk * 3 * 8);
+  A.part = take(((size_t)A.nblk * 3 + 1) * 8);   // the stages' blocks, the inlet rows
   A.total = off;
   return true;
 }
@@ -355,20 +356,13 @@ __global__ void __cluster_dims__(kCoarseCtas, 1, 1) __launch_bounds__(kCoarseThr
   for (int q = threadIdx.x; q < nr * m; q += blockDim.x) gb[(long)r0 * m + q] = G[q];
 }
 
-// transpose of the reference prolongation (multigrid_solver.py:134-156) onto
-// the coarse cell (I, J): even fine cells inject, odd interior ones average
-__global__ void __launch_bounds__(256) k_adj_prolong(const float* __restrict__ gf,
-                                                     float* __restrict__ gc, int nc, int mc,
-                                                     const int* ncyc, int cyc) {
-  pdl_wait();
-  if (ncyc && cyc >= *ncyc) return;
-  const int J = blockIdx.x * blockDim.x + threadIdx.x;
-  const int I = blockIdx.y * blockDim.y + threadIdx.y;
-  if (I >= nc || J >= mc) return;
-  const int mf = 2 * mc;
-  auto F = [&](int a, int b) { return ldg(gf + (long)a * mf + b); };
+// Transpose of the reference prolongation (multigrid_solver.py:134-156) at
+// coarse cell (I, J) from the fine field F: even fine cells inject, odd
+// interior ones average.
+template <class Fine>
+__device__ __forceinline__ float prolong_T(Fine F, int I, int J, int nc, int mc) {
   const bool iu = I <= nc - 2, id = I >= 1, ju = J <= mc - 2, jd = J >= 1;
-  float r = F(2 * I, 2 * J);
+  const float r = F(2 * I, 2 * J);
   float s = 0.f;
   if (iu) s += F(2 * I + 1, 2 * J);
   if (id) s += F(2 * I - 1, 2 * J);
@@ -379,7 +373,140 @@ __global__ void __launch_bounds__(256) k_adj_prolong(const float* __restrict__ g
   if (id && ju) q += F(2 * I - 1, 2 * J + 1);
   if (iu && jd) q += F(2 * I + 1, 2 * J - 1);
   if (id && jd) q += F(2 * I - 1, 2 * J - 1);
-  gc[(long)I * mc + J] = r + 0.5f * s + 0.25f * q;
+  return r + 0.5f * s + 0.25f * q;
+}
+
+// The reversed cycle's small levels in one block: level 0 of this tail has at
+// most kTailCells cells, and its levels' fields (the cotangent P, the second
+// sweep's Q, b's cotangent G) all lie in shared memory.  The operations are
+// k_adj_pair's, k_adj_prolong's and k_adj_coarsest's in their order.  What
+// bounds it: the chain of some 25 phases with a barrier each; it replaces
+// three launches of some 3 us for each level and the coarsest one's 7.  With
+// the parts' sum in the last stage and the cotangents kept in place, the
+// gradient of eight steps at 512x128 (tail from 128x32) 1100 -> 964 us, the
+// reverse pass of eight at 128x32 (tail from 64x16) 676 -> 511.  kTailCells is
+// four cells a thread: a larger level has more to gain from more blocks than
+// the launches cost.
+constexpr int kTailCells = 4096, kTailThreads = 1024, kTailLevels = 12;
+struct AdjTail {
+  const float* gx;   // cotangent of the tail's first level
+  float* gb;         // its b's cotangent, out
+  int levels;        // 1 .. kTailLevels, the coarsest included
+  int n[kTailLevels], m[kTailLevels], off[kTailLevels];   // sizes; first cell in P, Q, G
+  int cells;
+  float ax, ay, d;
+};
+__global__ void __launch_bounds__(kTailThreads) k_adj_tail(AdjTail a, const int* ncyc, int cyc) {
+  pdl_wait();
+  if (ncyc && cyc >= *ncyc) return;
+  extern __shared__ float tsm[];
+  float *P = tsm, *Q = tsm + a.cells, *G = tsm + 2 * a.cells;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const float ax = a.ax, ay = a.ay, d = a.d;
+  // every cell of level l once: f(i, j, index in the level)
+  auto cells = [&](int l, auto f) {
+    const int n = a.n[l], m = a.m[l];
+    for (int i = ty; i < n; i += kTailThreads / 32)
+      for (int j = tx; j < m; j += 32) f(i, j, i * m + j);
+    __syncthreads();
+  };
+  auto nsum = [&](const float* S, int l, int i, int j) {
+    const int n = a.n[l], m = a.m[l];
+    const int ip = i + 1 < n ? i + 1 : n - 1, im = i > 0 ? i - 1 : 0;
+    const int jp = j + 1 < m ? j + 1 : m - 1, jm = j > 0 ? j - 1 : 0;
+    return ax * (S[ip * m + j] + S[im * m + j]) + ay * (S[i * m + jp] + S[i * m + jm]);
+  };
+  const int last = a.levels - 1;
+  // up-sweep, reversed: the two post-sweeps, then the prolongation's transpose
+  for (int l = 0; l < last; ++l) {
+    float *p = P + a.off[l], *q = Q + a.off[l], *g = G + a.off[l];
+    const int n = a.n[l], m = a.m[l];
+    cells(l, [&](int i, int, int k) {
+      const float x = l == 0 ? ldg(a.gx + k) : p[k];
+      p[k] = i == n - 1 ? 0.f : x / d;
+    });
+    cells(l, [&](int i, int j, int k) {
+      const float h = nsum(p, l, i, j) / d;
+      q[k] = h;
+      g[k] = 0.f - p[k] - h;
+    });
+    cells(l, [&](int i, int j, int k) { p[k] = nsum(q, l, i, j); });
+    float* pc = P + a.off[l + 1];
+    cells(l + 1, [&](int i, int j, int k) {
+      pc[k] = prolong_T([&](int x, int y) { return p[x * m + y]; }, i, j, a.n[l + 1], a.m[l + 1]);
+    });
+  }
+  {  // coarsest: ten sweeps from zero
+    float *p = P + a.off[last], *q = Q + a.off[last], *g = G + a.off[last];
+    cells(last, [&](int, int, int k) {
+      const float h = p[k] / d;
+      p[k] = h;
+      g[k] = -h;
+    });
+    for (int s = 9; s >= 1; --s) {
+      cells(last, [&](int i, int j, int k) {
+        const float h = nsum(p, last, i, j) / d;
+        q[k] = h;
+        g[k] = g[k] - h;
+      });
+      float* t = p;
+      p = q;
+      q = t;
+    }
+  }
+  // down-sweep, reversed: the restriction's transpose and the two pre-sweeps
+  for (int l = last - 1; l >= 0; --l) {
+    float *p = P + a.off[l], *g = G + a.off[l];
+    const float* gc = G + a.off[l + 1];
+    const int n = a.n[l], m = a.m[l], mc = a.m[l + 1];
+    auto sres = [&](int i, int j) { return 0.25f * gc[(i >> 1) * mc + (j >> 1)]; };
+    cells(l, [&](int i, int j, int k) {
+      const int ip = i + 1 < n ? i + 1 : n - 1, im = i > 0 ? i - 1 : 0;
+      const int jp = j + 1 < m ? j + 1 : m - 1, jm = j > 0 ? j - 1 : 0;
+      const float sc = sres(i, j);
+      const float x = p[k] - (ax * (sres(ip, j) + sres(im, j) - 2.f * sc) +
+                              ay * (sres(i, jp) + sres(i, jm) - 2.f * sc));
+      p[k] = i == n - 1 ? 0.f : x / d;
+    });
+    cells(l, [&](int i, int j, int k) {
+      const float r = g[k] + sres(i, j) - p[k] - nsum(p, l, i, j) / d;
+      g[k] = r;
+      if (l == 0) a.gb[k] = r;
+    });
+  }
+}
+
+// the first level of the reversed cycle that runs in k_adj_tail (nlev + 1:
+// none).  At least two levels (the coarsest alone has k_adj_coarsest's
+// cluster), at most kTailCells cells on the first.
+static int adj_tail_level(const Layout& L) {
+  for (int l = 1; l < L.nlev; ++l)
+    if ((long)L.ln[l] * L.lm[l] <= kTailCells && L.nlev + 1 - l <= kTailLevels) return l;
+  return L.nlev + 1;
+}
+static AdjTail adj_tail(const Layout& L, int first) {
+  AdjTail t{};
+  t.levels = L.nlev + 1 - first;
+  for (int l = 0; l < t.levels; ++l) {
+    t.n[l] = L.ln[first + l];
+    t.m[l] = L.lm[first + l];
+    t.off[l] = t.cells;
+    t.cells += t.n[l] * t.m[l];
+  }
+  return t;
+}
+
+__global__ void __launch_bounds__(256) k_adj_prolong(const float* __restrict__ gf,
+                                                     float* __restrict__ gc, int nc, int mc,
+                                                     const int* ncyc, int cyc) {
+  pdl_wait();
+  if (ncyc && cyc >= *ncyc) return;
+  const int J = blockIdx.x * blockDim.x + threadIdx.x;
+  const int I = blockIdx.y * blockDim.y + threadIdx.y;
+  if (I >= nc || J >= mc) return;
+  const int mf = 2 * mc;
+  gc[(long)I * mc + J] =
+      prolong_T([&](int a, int b) { return ldg(gf + (long)a * mf + b); }, I, J, nc, mc);
 }
 
 // ------------------------------------------------------------------ rhs
@@ -419,6 +546,13 @@ struct AdjRk {
   float *gu, *gv;                  // last stage: cotangents of the step's u, v
   float *gsdf;                     // accumulated (nullable)
   double* part;                    // per-block d/d nu
+  // d/d nu, d/d U_inf (nullable): k_adj_rk_out's first block files the inlet
+  // rows' sum in inlet_part, the last stage's last block adds all parts in a
+  // fixed order to gscal
+  double *gscal, *parts, *inlet_part;
+  int nparts, corr_walls, pred_walls;
+  const float* gu_o;
+  unsigned int* count;
   const float* mask;
   const DevScalars* sc;
   int nx, ny, last, slip;
@@ -436,6 +570,20 @@ __global__ void __launch_bounds__(256) k_adj_rk_out(AdjRk a) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = blockIdx.y * blockDim.y + threadIdx.y;
   const int nx = a.nx, ny = a.ny;
+  if (a.gscal && blockIdx.x == 0 && blockIdx.y == 0) {
+    // d/d U_inf, the inlet rows: the correction's final row 0 where live (the
+    // GUI step leaves the two corners on the walls: corr_walls = 0) and the
+    // predictor output's row 0 (with no-slip walls its two corners are 0:
+    // pred_walls = 0)
+    double s = 0.0;
+    for (int q = threadIdx.y * blockDim.x + threadIdx.x; q < ny; q += blockDim.x * blockDim.y) {
+      const bool wall = q == 0 || q == ny - 1;
+      if (a.pred_walls || !wall) s += (double)ldg(a.gus + q);
+      if ((a.corr_walls || !wall) && live_at(a.mask, q)) s += (double)ldg(a.gu_o + q);
+    }
+    s = block_sum(s);
+    if (threadIdx.x == 0 && threadIdx.y == 0) *a.inlet_part = s;
+  }
   if (i >= nx || j >= ny) return;
   const long k = (long)i * ny + j;
   float gu, gv;
@@ -566,46 +714,37 @@ __global__ void __launch_bounds__(256) k_adj_rk_stage(AdjRk a) {
     }
   }
   const double t = block_sum_df(nub);
-  if (threadIdx.x == 0 && threadIdx.y == 0) a.part[blockIdx.y * gridDim.x + blockIdx.x] = t;
-}
-
-// d/d nu from the stage partials and d/d U_inf from the inlet rows (the
-// correction's final row 0 where live, and the predictor output's row 0),
-// summed in a fixed order and added to gscal[0], gscal[1]
-// (four independent accumulators per thread keep four loads in flight: one
-// accumulator left the block waiting on one partial at a time, 28 us)
-// The inlet rows: the correction's final row 0 where live (the GUI step
-// leaves the two corners on the walls: corr_walls = 0) and the predictor
-// output's row 0 (with no-slip walls its two corners are 0: pred_walls = 0).
-__global__ void __launch_bounds__(1024) k_adj_scalars(const double* __restrict__ part, int nparts,
-                                                      const float* __restrict__ gu_o,
-                                                      const float* __restrict__ gus,
-                                                      const float* __restrict__ mask, int ny,
-                                                      int corr_walls, int pred_walls,
-                                                      double* gscal) {
-  pdl_wait();
-  const int bd = blockDim.x;
-  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0, u = 0.0;
-  int q = threadIdx.x;
-  for (; q + 3 * bd < nparts; q += 4 * bd) {
-    const double a = part[q], b = part[q + bd], c = part[q + 2 * bd], d = part[q + 3 * bd];
-    s0 += a;
-    s1 += b;
-    s2 += c;
-    s3 += d;
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  if (!a.last || !a.gscal) {
+    if (tid == 0) a.part[blockIdx.y * gridDim.x + blockIdx.x] = t;
+    return;
   }
-  for (; q < nparts; q += bd) s0 += part[q];
-  double s = (s0 + s1) + (s2 + s3);
-  for (int q = threadIdx.x; q < ny; q += blockDim.x) {
-    const bool wall = q == 0 || q == ny - 1;
-    if (pred_walls || !wall) u += (double)ldg(gus + q);
-    if ((corr_walls || !wall) && live_at(mask, q)) u += (double)ldg(gu_o + q);
+  // the last block of the last stage adds all stages' parts (a launch of its
+  // own took 5 to 10 us: one block, two dependent round trips)
+  __shared__ int am_last;
+  if (tid == 0) {
+    a.part[blockIdx.y * gridDim.x + blockIdx.x] = t;
+    __threadfence();
+    am_last = atomicAdd(a.count, 1u) == gridDim.x * gridDim.y - 1;
   }
-  s = block_sum(s);
-  u = block_sum(u);
-  if (threadIdx.x == 0) {
-    gscal[0] += s;
-    gscal[1] += u;
+  __syncthreads();
+  if (!am_last) return;
+  __threadfence();
+  const int bd = blockDim.x * blockDim.y;
+  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+  int q = tid;
+  for (; q + 3 * bd < a.nparts; q += 4 * bd) {   // four loads in flight
+    s0 += __ldcg(a.parts + q);
+    s1 += __ldcg(a.parts + q + bd);
+    s2 += __ldcg(a.parts + q + 2 * bd);
+    s3 += __ldcg(a.parts + q + 3 * bd);
+  }
+  for (; q < a.nparts; q += bd) s0 += __ldcg(a.parts + q);
+  const double s = block_sum((s0 + s1) + (s2 + s3));
+  if (tid == 0) {
+    a.gscal[0] += s;
+    a.gscal[1] += *a.inlet_part;
+    *a.count = 0u;
   }
 }
 
@@ -703,7 +842,10 @@ int launch_step_vjp(const AjStepParams& p, const Layout& L, void* ws, void* aws,
   launch_pdl(true, k_adj_correct, grd, blk, 0, st, c);
   launch_pdl(true, k_adj_grad, grd, blk, 0, st, c);
   // ---- multigrid, reversed (cycles from the last to the first)
-  if (cudaMemsetAsync(F(A.GB[0]), 0, (size_t)N * 4, st) != cudaSuccess) return AJ_ERR_CUDA;
+  // (one cycle assigns b's cotangent; of several, the skipped ones leave it)
+  if (p.v_cycles > 1 &&
+      cudaMemsetAsync(F(A.GB[0]), 0, (size_t)N * 4, st) != cudaSuccess)
+    return AJ_ERR_CUDA;
   const float ax = (float)(1.0 / (p.dx * p.dx)), ay = (float)(1.0 / (p.dy * p.dy));
   const float den = (float)(2.0 * (1.0 / (p.dx * p.dx) + 1.0 / (p.dy * p.dy)));
   const int nl = L.nlev;
@@ -720,16 +862,28 @@ int launch_step_vjp(const AjStepParams& p, const Layout& L, void* ws, void* aws,
                dim3(kPairBX, kPairBY), 0, st, gin, gout, F(A.GB[l]), gbc, L.ln[l], L.lm[l], ax, ay,
                den, assign, nc, cyc);
   };
+  const int lt = std::min(adj_tail_level(L), nl);   // levels above the tail
   for (int cyc = p.v_cycles - 1; cyc >= 0; --cyc) {
     const int* nc = cyc == 0 ? nullptr : ncyc;                 // cycle 0 always ran
     // up-sweep, reversed: the two post-sweeps (GX -> GT), then the
     // prolongation's transpose onto the coarser level's GX
-    for (int l = 0; l < nl; ++l) {
-      pair(l, F(A.GX[l]), F(A.GT[l]), nullptr, l > 0, nc, cyc);
+    for (int l = 0; l < lt; ++l) {
+      pair(l, F(A.GX[l]), F(A.GT[l]), nullptr, l > 0 || p.v_cycles == 1, nc, cyc);
       launch_pdl(true, k_adj_prolong, lg(l + 1), blk, 0, st, F(A.GT[l]), F(A.GX[l + 1]),
                  L.ln[l + 1], L.lm[l + 1], nc, cyc);
     }
-    if (parity_coarsest_fused(L)) {                            // coarsest: 10 sweeps from zero
+    if (lt < nl) {                                             // the small levels
+      AdjTail t = adj_tail(L, lt);
+      t.gx = F(A.GX[lt]);
+      t.gb = F(A.GB[lt]);
+      t.ax = ax;
+      t.ay = ay;
+      t.d = den;
+      cudaFuncSetAttribute(k_adj_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kBlockSmemMax);
+      launch_pdl(true, k_adj_tail, dim3(1), dim3(kTailThreads), (size_t)t.cells * 12, st, t, nc,
+                 cyc);
+    } else if (parity_coarsest_fused(L)) {                     // coarsest: 10 sweeps from zero
       const int n = L.ln[nl], m = L.lm[nl];
       cudaFuncSetAttribute(k_adj_coarsest, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)kBlockSmemMax);
@@ -746,7 +900,7 @@ int launch_step_vjp(const AjStepParams& p, const Layout& L, void* ws, void* aws,
     // down-sweep, reversed: the restriction's transpose and the two
     // pre-sweeps on GT; the first pre-sweep's input is zero below level 0
     // and in the first cycle, else its cotangent goes to GX[0]
-    for (int l = nl - 1; l >= 0; --l)
+    for (int l = lt - 1; l >= 0; --l)
       pair(l, F(A.GT[l]), (l == 0 && cyc > 0) ? F(A.GX[0]) : nullptr, F(A.GB[l + 1]), 0, nc, cyc);
   }
   // ---- rhs and divergence, reversed
@@ -784,6 +938,14 @@ int launch_step_vjp(const AjStepParams& p, const Layout& L, void* ws, void* aws,
   r.slip = p.slip_walls;
   r.nuh_fac = (float)(p.nu_hyper_ratio * p.dx * p.dy);
   r.nuh = (float)p.nu * r.nuh_fac;
+  r.gscal = gscal;
+  r.nparts = (rk2 ? 2 : 3) * A.nblk;
+  r.parts = at<double>(aws, A.part);
+  r.inlet_part = r.parts + 3 * (size_t)A.nblk;
+  r.corr_walls = p.variant == AJ_VARIANT_PURE;
+  r.pred_walls = p.slip_walls != 0;
+  r.gu_o = gu_o;
+  r.count = &sc->red_count;
   const bool hyper = p.nu_hyper_ratio > 0.0;
   if (branch && cudaStreamWaitEvent(st, fk->join, 0) != cudaSuccess) return AJ_ERR_CUDA;
   launch_pdl(true, k_adj_rk_out, grd, blk, 0, st, r);
@@ -814,10 +976,6 @@ int launch_step_vjp(const AjStepParams& p, const Layout& L, void* ws, void* aws,
     else launch_pdl(true, k_adj_rk_stage<false>, grd, blk, 0, st, r);
     cur = 1 - cur;
   }
-  if (gscal)
-    launch_pdl(true, k_adj_scalars, dim3(1), dim3(1024), 0, st, at<double>(aws, A.part),
-               nst * A.nblk, gu_o, F(A.gus), mask, ny, (int)(p.variant == AJ_VARIANT_PURE),
-               (int)(p.slip_walls != 0), gscal);
   return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
 }
 
@@ -828,8 +986,9 @@ int step_vjp_kernel_count(const AjStepParams& p, const Layout& L) {
   if (p.v_cycles > 1)                               // rhs, forward solve (no statistics)
     n += 1 + parity_kernel_count(p, L) - (parity_cluster_level(p, L) > 0);
   n += 2;                                           // correction, gradient
-  n += p.v_cycles * (3 * L.nlev + (fused ? 1 : 10));  // reversed V-cycles
-  n += 1 + 1 + nst + 1;                             // divergence, output, stages, scalars
+  const int lt = adj_tail_level(L);                 // reversed V-cycles
+  n += p.v_cycles * (lt < L.nlev ? 3 * lt + 1 : 3 * L.nlev + (fused ? 1 : 10));
+  n += 1 + 1 + nst;                                 // divergence, output, stages
   return n;
 }
 

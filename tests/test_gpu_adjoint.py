@@ -193,3 +193,27 @@ def test_ragged_grid_parity_solve_and_reverse_mode(dev):
                             _t(gv, dev), _t(gp, dev), v_cycles=2)
     for name in ("u", "v", "sdf"):
         assert _rel(got[name].cpu(), ref[name]) <= 1e-4, name
+
+
+@pytest.mark.parametrize("nx,ny,cycles", [(32, 32, 1), (1040, 256, 1), (256, 64, 1), (272, 64, 2),
+                                          (128, 128, 1)])
+def test_step_vjp_small_levels(dev, nx, ny, cycles):
+    """The reversed cycle's small levels in one block: none (1040x256, level 3
+    of 130x32), from the second level at its largest (256x64), some rows beyond
+    it (272x64), square ones; results written over the incoming cotangents."""
+    from oracle import adjoint_np as A
+    from aerojax_gb300 import adjoint as ADJ
+    u, v, mask, s, rng = _case(nx, ny, nx + ny)
+    gu, gv = (rng.standard_normal((nx, ny)).astype(np.float32) for _ in range(2))
+    ref = A.step_pure_vjp(u, v, DT, mask, s, DX, DX, NU, U, gu, gv, np.zeros_like(gu),
+                          v_cycles=cycles)
+    op = ADJ.StepVjp(ADJ._config(nx, ny, DX, DX, NU, U, DT, True, cycles), dev)
+    tm, ts = _t(mask, dev), _t(s, dev)
+    op.prepare(tm, ts)
+    got = op(_t(u, dev), _t(v, dev), tm, _t(gu, dev), _t(gv, dev), out=op.g_in[:2])
+    assert _rel(got[0].cpu(), ref["u"]) <= 1e-4
+    assert _rel(got[1].cpu(), ref["v"]) <= 1e-4
+    assert _rel(op.gsdf.cpu(), ref["sdf"]) <= 1e-4
+    sc = op.gscal.cpu()
+    assert _scalar_ok(float(sc[0]), ref, "nu", 1e-4)
+    assert _scalar_ok(float(sc[1]), ref, "U_inf", 1e-4)

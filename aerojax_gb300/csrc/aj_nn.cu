@@ -19,6 +19,7 @@
 // gradient.
 #include "aj_internal.cuh"
 #include <cuda_bf16.h>
+#include <algorithm>
 #include <stdlib.h>
 #include <string.h>
 
@@ -110,18 +111,82 @@ struct ConvArgs {
   int relu;
   float* Yp;         // nullable: 2x2 average pool of Y
   const float* Xc;   // nullable: the input is up2(Xc) + X
-  const DevScalars* norm;   // nullable: scale input channels 0 and 2 by 1 / the
-                            // sample's RMS (the features' normalisation)
+  const DevScalars* norm = nullptr;   // nullable: scale input channels 0 and 2 by 1 / the
+                                      // sample's RMS (the features' normalisation)
+  // the backward pass: Y and Yp are kept where these are positive (the ReLU
+  // adjoint of the layer below), and Yp is the plain 2x2 sum (the adjoint of
+  // the up-sampling) with pool_scale 1
+  const float* gate = nullptr;
+  const float* gate_p = nullptr;
+  float pool_scale = 0.25f;
 };
 
-// The output side of one conv tile: outputs of one 8 x 8 pixel tile and
-// BN = NT * 8 channels from co0.
+// The output side of one conv tile: outputs of one pixel tile and BN = NT * 8
+// channels from co0.
 struct ConvOut {
   float* Y;
-  float* Yp;          // nullable: 2x2 average pool of Y
+  float* Yp;          // nullable: 2x2 average pool (or sum) of Y
   const float* bias;  // nullable
   int relu, H, W, Cout, n, h0, w0, co0;
+  const float* gate = nullptr;
+  const float* gate_p = nullptr;
+  float pool_scale = 0.25f;
 };
+
+// Epilogue of one warp's 16 pixels (tile rows ty0 and ty0 + 1 of eight
+// columns): bias, ReLU, gate, store; with Yp also the 2x2 pool of the output
+// before its gate (the warp holds both rows of a pooling window; the column
+// neighbour is 4 lanes up), summed in the order s00 + s10 + s01 + s11 of the
+// oracle's pool2.
+template <int NT>
+__device__ __forceinline__ void conv_finish(const float (&acc)[NT][4], const ConvOut& o, int ty0) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
+  const int gw = o.w0 + g;
+#pragma unroll
+  for (int q = 0; q < NT; ++q) {
+    const int col = o.co0 + q * 8 + tg * 2;
+    const float b0 = o.bias ? o.bias[col] : 0.f, b1 = o.bias ? o.bias[col + 1] : 0.f;
+    float y[2][2];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      y[half][0] = acc[q][half * 2] + b0;
+      y[half][1] = acc[q][half * 2 + 1] + b1;
+      if (o.relu) {
+        y[half][0] = fmaxf(y[half][0], 0.f);
+        y[half][1] = fmaxf(y[half][1], 0.f);
+      }
+      const int gh = o.h0 + ty0 + half;
+      if (gh < o.H && gw < o.W) {
+        const long e = (((long)o.n * o.H + gh) * o.W + gw) * o.Cout + col;
+        float2 v = make_float2(y[half][0], y[half][1]);
+        if (o.gate) {
+          const float2 k = __ldg(reinterpret_cast<const float2*>(o.gate + e));
+          v = make_float2(k.x > 0.f ? v.x : 0.f, k.y > 0.f ? v.y : 0.f);
+        }
+        *reinterpret_cast<float2*>(o.Y + e) = v;
+      }
+    }
+    if (o.Yp) {
+      float pv[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const float s01 = __shfl_down_sync(0xffffffffu, y[0][c], 4);
+        const float s11 = __shfl_down_sync(0xffffffffu, y[1][c], 4);
+        pv[c] = o.pool_scale * (((y[0][c] + y[1][c]) + s01) + s11);
+      }
+      const int ph = (o.h0 + ty0) >> 1, pw = gw >> 1;
+      if (!(g & 1) && o.h0 + ty0 + 1 < o.H && gw + 1 < o.W) {
+        const long e = (((long)o.n * (o.H / 2) + ph) * (o.W / 2) + pw) * o.Cout + col;
+        if (o.gate_p) {
+          const float2 k = __ldg(reinterpret_cast<const float2*>(o.gate_p + e));
+          pv[0] = k.x > 0.f ? pv[0] : 0.f;
+          pv[1] = k.y > 0.f ? pv[1] : 0.f;
+        }
+        *reinterpret_cast<float2*>(o.Yp + e) = make_float2(pv[0], pv[1]);
+      }
+    }
+  }
+}
 
 // The K loop and epilogue of one conv tile from shared memory: As holds the
 // tile's 10 x 10 halo in BF16 ([px][CIN + 8]), Bs the 9 taps' weights
@@ -146,12 +211,6 @@ __device__ __forceinline__ void conv_core(const __nv_bfloat16* As, const __nv_bf
   // (m >> 1) * 8, for B output channel 8 (m >> 1) + r of the pair of
   // 8-channel groups at channel offset (m & 1) * 8.
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, tg = lane & 3;
-  float* __restrict__ Y = o.Y;
-  float* __restrict__ Yp = o.Yp;
-  const float* __restrict__ bias = o.bias;
-  const int relu = o.relu, H = o.H, W = o.W, Cout = o.Cout, n = o.n, h0 = o.h0, w0 = o.w0,
-            co0 = o.co0;
   const int prow = warp & 3, kh = warp >> 2;
   const int ty0 = 2 * prow;
   const int lm = lane >> 3, lr = lane & 7;
@@ -197,43 +256,7 @@ __device__ __forceinline__ void conv_core(const __nv_bfloat16* As, const __nv_bf
   for (int q = 0; q < NT; ++q)
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[q][e] += red[((prow * NT + q) * 4 + e) * 32 + lane];
-  // epilogue: bias, ReLU, store; with Yp also the 2x2 average pool of the
-  // output (the warp holds both rows of a pooling window; the column
-  // neighbour is 4 lanes up), summed in the order s00 + s10 + s01 + s11 of the
-  // oracle's pool2
-  const int gw = w0 + g;
-#pragma unroll
-  for (int q = 0; q < NT; ++q) {
-    const int col = co0 + q * 8 + tg * 2;
-    const float b0 = bias ? bias[col] : 0.f, b1 = bias ? bias[col + 1] : 0.f;
-    float y[2][2];
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      y[half][0] = acc[q][half * 2] + b0;
-      y[half][1] = acc[q][half * 2 + 1] + b1;
-      if (relu) {
-        y[half][0] = fmaxf(y[half][0], 0.f);
-        y[half][1] = fmaxf(y[half][1], 0.f);
-      }
-      const int gh = h0 + ty0 + half;
-      if (gh < H && gw < W)
-        *reinterpret_cast<float2*>(&Y[(((long)n * H + gh) * W + gw) * Cout + col]) =
-            make_float2(y[half][0], y[half][1]);
-    }
-    if (Yp) {
-      float pv[2];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const float s01 = __shfl_down_sync(0xffffffffu, y[0][c], 4);
-        const float s11 = __shfl_down_sync(0xffffffffu, y[1][c], 4);
-        pv[c] = 0.25f * (((y[0][c] + y[1][c]) + s01) + s11);
-      }
-      const int ph = (h0 + ty0) >> 1, pw = gw >> 1;
-      if (!(g & 1) && h0 + ty0 + 1 < H && gw + 1 < W)
-        *reinterpret_cast<float2*>(&Yp[(((long)n * (H / 2) + ph) * (W / 2) + pw) * Cout + col]) =
-            make_float2(pv[0], pv[1]);
-    }
-  }
+  conv_finish<NT>(acc, o, ty0);
 }
 
 // One 8 x 8 pixel tile t (tiles ordered w fastest, then h, then sample) and
@@ -246,10 +269,6 @@ __device__ __forceinline__ void conv_tile(const ConvArgs& cv, int t, int co0,
   const float* __restrict__ X = cv.X;
   const int H = cv.H, W = cv.W, Cout = cv.Cout;
   const __nv_bfloat16* __restrict__ WT = cv.WT;
-  const float* __restrict__ bias = cv.bias;
-  float* __restrict__ Y = cv.Y;
-  const int relu = cv.relu;
-  float* __restrict__ Yp = cv.Yp;
   const float* __restrict__ Xc = cv.Xc;
   using S = ConvSmem<CIN, NT>;
   constexpr int AS = S::AS, BN = S::BN;
@@ -335,13 +354,146 @@ __device__ __forceinline__ void conv_tile(const ConvArgs& cv, int t, int co0,
   }
   cp_async_wait<0>();
   __syncthreads();
-  conv_core<CIN, NT>(As, Bs, conv_sm, ConvOut{Y, Yp, bias, relu, H, W, Cout, n, h0, w0, co0});
+  conv_core<CIN, NT>(As, Bs, conv_sm,
+                     ConvOut{cv.Y, cv.Yp, cv.bias, cv.relu, H, W, Cout, n, h0, w0, co0, cv.gate,
+                             cv.gate_p, cv.pool_scale});
 }
 
 template <int CIN, int NT>
 __global__ void __launch_bounds__(CONV_THREADS) k_conv3x3(ConvArgs a) {
   extern __shared__ __align__(16) unsigned char conv_sm[];
   conv_tile<CIN, NT, true>(a, blockIdx.x, blockIdx.y * NT * 8, conv_sm);
+}
+
+// The same convolution for batches: a block stages its channels' weights once
+// and walks a run of 16 x 8 pixel tiles.  A warp holds 32 pixels (two
+// 16-pixel fragments a weight fragment serves), warps 0-3 taps 0-4 and warps
+// 4-7 taps 5-8 as in conv_core; each half of K finishes one of the two
+// fragments, the other's partial sums go through shared memory.  Every sum
+// has conv_core's terms in its order.  The next tile's input is in flight
+// during a tile's epilogue.  What bounds it: instructions issued (45 % of the
+// slots at 16 warps an SM) and shared-memory reads of the fragments (57 %).
+// 16 samples of 256x64, cold: 32 -> 32 channels 41 -> 35 us, 64 -> 64 at
+// 128x32 35 -> 32, 16 -> 32 60 -> 27 (a block per 8 x 8 tile, each staging its
+// weights, before).
+constexpr int CR_TH = 16, CR_HALO = (CR_TH + 2) * (CT + 2);
+template <int CIN, int NT>
+struct RunSmem {
+  static constexpr int AS = CIN + 8, BN = NT * 8;
+  static constexpr size_t a_bytes = (size_t)CR_HALO * AS * 2, b_bytes = (size_t)9 * BN * AS * 2;
+  static constexpr size_t bytes = a_bytes + b_bytes + (size_t)8 * NT * 4 * 32 * 4;
+  static_assert(a_bytes % 16 == 0 && b_bytes % 16 == 0, "16-byte aligned sections");
+};
+template <int CIN, int NT, bool UP>
+__global__ void __launch_bounds__(CONV_THREADS, 2) k_conv_run(ConvArgs cv, int tiles, int run) {
+  using S = RunSmem<CIN, NT>;
+  constexpr int AS = S::AS, BN = S::BN, C8 = CIN / 8;
+  constexpr int NP = CR_HALO * C8, L = (NP + CONV_THREADS - 1) / CONV_THREADS;
+  extern __shared__ __align__(16) unsigned char run_sm[];
+  __nv_bfloat16* As = reinterpret_cast<__nv_bfloat16*>(run_sm);
+  __nv_bfloat16* Bs = reinterpret_cast<__nv_bfloat16*>(run_sm + S::a_bytes);
+  float* red = reinterpret_cast<float*>(run_sm + S::a_bytes + S::b_bytes);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int H = cv.H, W = cv.W, Cout = cv.Cout, co0 = blockIdx.y * BN;
+  const int tw = (W + CT - 1) / CT, th = (H + CR_TH - 1) / CR_TH;
+  const int t0 = blockIdx.x * run, t1 = min(t0 + run, tiles);
+  for (int e = tid; e < 9 * BN * C8; e += CONV_THREADS) {
+    const int row = e / C8, q = e - row * C8;
+    const int tap = row / BN, r = row - tap * BN;
+    cp_async16(Bs + row * AS + q * 8, cv.WT + ((long)tap * Cout + co0 + r) * CIN + q * 8);
+  }
+  cp_async_commit();
+  float4 xa[L], xb[L];
+  auto load = [&](int t) {
+    const int w0 = t % tw * CT, h0 = t / tw % th * CR_TH, n = t / (tw * th);
+#pragma unroll
+    for (int k = 0; k < L; ++k) {
+      const int e = tid + k * CONV_THREADS, px = e / C8, q = e - px * C8;
+      const int hy = px / (CT + 2), gh = h0 - 1 + hy, gw = w0 - 1 + px - hy * (CT + 2);
+      xa[k] = xb[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (e < NP && gh >= 0 && gh < H && gw >= 0 && gw < W) {
+        const float4* src =
+            reinterpret_cast<const float4*>(cv.X + (((long)n * H + gh) * W + gw) * CIN + q * 8);
+        xa[k] = __ldg(src);
+        xb[k] = __ldg(src + 1);
+        if (UP) {   // the decoder's up2(Xc) + X
+          const float4* cs = reinterpret_cast<const float4*>(
+              cv.Xc + (((long)n * (H >> 1) + (gh >> 1)) * (W >> 1) + (gw >> 1)) * CIN + q * 8);
+          const float4 ca = __ldg(cs), cb = __ldg(cs + 1);
+          xa[k] = make_float4(ca.x + xa[k].x, ca.y + xa[k].y, ca.z + xa[k].z, ca.w + xa[k].w);
+          xb[k] = make_float4(cb.x + xb[k].x, cb.y + xb[k].y, cb.z + xb[k].z, cb.w + xb[k].w);
+        }
+      }
+    }
+  };
+  const int prow = warp & 3, kh = warp >> 2;
+  const int lm = lane >> 3, lr = lane & 7;
+  const unsigned as0 = (unsigned)__cvta_generic_to_shared(As);
+  const unsigned bs0 = (unsigned)__cvta_generic_to_shared(Bs);
+  pdl_wait();
+  // (the decoder's input takes twice the registers: it is loaded at its use)
+  if (!UP && t0 < t1) load(t0);
+  cp_async_wait<0>();
+  for (int t = t0; t < t1; ++t) {
+    if (UP) load(t);
+#pragma unroll
+    for (int k = 0; k < L; ++k) {
+      const int e = tid + k * CONV_THREADS, px = e / C8, q = e - px * C8;
+      if (e < NP)
+        *reinterpret_cast<uint4*>(As + px * AS + q * 8) =
+            make_uint4(pack_bf16x2(xa[k].x, xa[k].y), pack_bf16x2(xa[k].z, xa[k].w),
+                       pack_bf16x2(xb[k].x, xb[k].y), pack_bf16x2(xb[k].z, xb[k].w));
+    }
+    __syncthreads();
+    float acc[2][NT][4], acc2[2][NT][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int q = 0; q < NT; ++q)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[m][q][e] = acc2[m][q][e] = 0.f;
+#pragma unroll 1
+    for (int tap = kh ? 5 : 0; tap < (kh ? 9 : 5); ++tap) {
+      const int dy = tap / 3, dx = tap % 3;
+      const unsigned a_row = as0 + (unsigned)((((4 * prow + dy + (lm & 1)) * (CT + 2) + lr + dx) * AS +
+                                               (lm >> 1) * 8) * 2);
+      const unsigned b_row = bs0 + (unsigned)(((tap * BN + (lm >> 1) * 8 + lr) * AS + (lm & 1) * 8) * 2);
+#pragma unroll
+      for (int ks = 0; ks < CIN / 16; ++ks) {
+        uint32_t f[2][4];
+        ldsm_x4(f[0], a_row + ks * 32);
+        ldsm_x4(f[1], a_row + (unsigned)(2 * (CT + 2) * AS * 2) + ks * 32);
+#pragma unroll
+        for (int qp = 0; qp < NT / 2; ++qp) {
+          uint32_t b[4];
+          ldsm_x4(b, b_row + (unsigned)(qp * 16 * AS * 2) + ks * 32);
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            mma_bf16((ks & 1) ? acc2[m][2 * qp] : acc[m][2 * qp], f[m], b);
+            mma_bf16((ks & 1) ? acc2[m][2 * qp + 1] : acc[m][2 * qp + 1], f[m], b + 2);
+          }
+        }
+      }
+    }
+    float own[NT][4];
+#pragma unroll
+    for (int q = 0; q < NT; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float s0 = acc[0][q][e] + acc2[0][q][e], s1 = acc[1][q][e] + acc2[1][q][e];
+        own[q][e] = kh ? s1 : s0;
+        red[((warp * NT + q) * 4 + e) * 32 + lane] = kh ? s0 : s1;
+      }
+    if (!UP && t + 1 < t1) load(t + 1);
+    __syncthreads();   // the partial sums are in place, and every warp is done with As
+#pragma unroll
+    for (int q = 0; q < NT; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) own[q][e] += red[(((warp ^ 4) * NT + q) * 4 + e) * 32 + lane];
+    const int w0 = t % tw * CT, h0 = t / tw % th * CR_TH, n = t / (tw * th);
+    conv_finish<NT>(own, ConvOut{cv.Y, cv.Yp, cv.bias, cv.relu, H, W, Cout, n, h0, w0, co0, cv.gate,
+                                 cv.gate_p, cv.pool_scale}, 4 * prow + 2 * kh);
+  }
 }
 
 // ---------------------------------------------------------------- layer pairs
@@ -557,20 +709,40 @@ static bool nn_pairs_enabled() {
 int nn_inference_conv_launches() { return nn_pairs_enabled() ? 10 : 12; }
 
 template <int CIN, int NT>
-static void conv_launch(const float* X, int N, int H, int W, int Cout, const __nv_bfloat16* WT,
-                        const float* bias, float* Y, int relu, float* Yp, const float* Xc,
-                        cudaStream_t st, bool pdl, const DevScalars* norm) {
+static void conv_launch(const ConvArgs& a, cudaStream_t st, bool pdl) {
   using S = ConvSmem<CIN, NT>;
-  const int tiles = ((W + CT - 1) / CT) * ((H + CT - 1) / CT) * N;
-  dim3 grid(tiles, Cout / S::BN);
-  launch_pdl(pdl, k_conv3x3<CIN, NT>, grid, dim3(CONV_THREADS), S::bytes, st,
-             ConvArgs{X, N, H, W, Cout, WT, bias, Y, relu, Yp, Xc, norm});
+  const int tiles = ((a.W + CT - 1) / CT) * ((a.H + CT - 1) / CT) * a.N;
+  launch_pdl(pdl, k_conv3x3<CIN, NT>, dim3(tiles, a.Cout / S::BN), dim3(CONV_THREADS), S::bytes, st,
+             a);
+}
+
+constexpr int CONV_RUNS = 304;   // blocks of k_conv_run, all channels: two per SM
+// 8 x 8 tiles times channel groups from which a layer goes to k_conv_run (at
+// the other kernel's one block an SM).  A training pass, us, without it and
+// from 152, 304, 608, 1216: one sample of 256x64 299, 295, 299, 299, 300; four
+// 484, 444, 445, 456, 485; sixteen 1096, 977, 977, 976, 1007; eight of 96x40
+// 385, 362, 367, 385, 385.
+constexpr long CONV_RUN_MIN = 152;
+template <int CIN, int NT, bool UP>
+static void run_launch(const ConvArgs& a, cudaStream_t st, bool pdl) {
+  using S = RunSmem<CIN, NT>;
+  const int tiles = ((a.W + CT - 1) / CT) * ((a.H + CR_TH - 1) / CR_TH) * a.N;
+  const int slabs = a.Cout / S::BN;
+  const int run = (int)cdiv(tiles, std::max(1, CONV_RUNS / slabs));
+  launch_pdl(pdl, k_conv_run<CIN, NT, UP>, dim3(cdiv(tiles, run), slabs), dim3(CONV_THREADS),
+             S::bytes, st, a, tiles, run);
 }
 
 template <int CIN, int NT>
 static void conv_attr() {
   cudaFuncSetAttribute(k_conv3x3<CIN, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)ConvSmem<CIN, NT>::bytes);
+  if constexpr (CIN <= 64) {
+    cudaFuncSetAttribute(k_conv_run<CIN, NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)RunSmem<CIN, NT>::bytes);
+    cudaFuncSetAttribute(k_conv_run<CIN, NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)RunSmem<CIN, NT>::bytes);
+  }
 }
 // the dynamic shared-memory opt-in of every convolution instance (once, before
 // any launch or capture)
@@ -590,40 +762,34 @@ static void conv_attrs() {
 }
 
 template <int CIN>
-static int conv_cin(const float* X, int N, int H, int W, int Cout, const __nv_bfloat16* WT,
-                    const float* bias, float* Y, int relu, float* Yp, const float* Xc,
-                    cudaStream_t st, bool pdl, const DevScalars* norm) {
+static int conv_cin(const ConvArgs& a, cudaStream_t st, bool pdl) {
   // 32 output channels per block, or 16 when that leaves fewer blocks than
   // SMs (the small grids of the deep layers are latency-bound: more, lighter
   // blocks load their weights sooner)
-  const long tiles = (long)((W + CT - 1) / CT) * ((H + CT - 1) / CT) * N;
-  const bool narrow = Cout == 16 || tiles * (Cout / 32) < 152;
-  switch (Cout) {
-    case 16:
-    case 32:
-    case 64:
-    case 128:
-      if (narrow) conv_launch<CIN, 2>(X, N, H, W, Cout, WT, bias, Y, relu, Yp, Xc, st, pdl, norm);
-      else conv_launch<CIN, 4>(X, N, H, W, Cout, WT, bias, Y, relu, Yp, Xc, st, pdl, norm);
-      break;
-    default: return AJ_ERR_PARAM;
+  const long tiles = (long)((a.W + CT - 1) / CT) * ((a.H + CT - 1) / CT) * a.N;
+  const bool narrow = a.Cout == 16 || tiles * (a.Cout / 32) < 152;
+  if (a.Cout != 16 && a.Cout != 32 && a.Cout != 64 && a.Cout != 128) return AJ_ERR_PARAM;
+  if constexpr (CIN <= 64) {
+    if (!a.norm && tiles * (narrow ? a.Cout / 16 : a.Cout / 32) >= CONV_RUN_MIN) {
+      if (narrow) a.Xc ? run_launch<CIN, 2, true>(a, st, pdl) : run_launch<CIN, 2, false>(a, st, pdl);
+      else a.Xc ? run_launch<CIN, 4, true>(a, st, pdl) : run_launch<CIN, 4, false>(a, st, pdl);
+      return AJ_OK;
+    }
   }
+  if (narrow) conv_launch<CIN, 2>(a, st, pdl);
+  else conv_launch<CIN, 4>(a, st, pdl);
   return AJ_OK;
 }
 
-// Y = conv(X, WT) (+ bias, ReLU); WT[tap][Cout][Cin] BF16; Yp (nullable,
-// H and W even) receives the 2x2 average pool of Y; with Xc (nullable) the
-// input is up2(Xc) + X.  pdl: dependent launch (the weights WT must be
-// complete before the chain of dependent launches started)
-static int conv3x3(const float* X, int N, int H, int W, int Cin, int Cout,
-                   const __nv_bfloat16* WT, const float* bias, float* Y, int relu,
-                   cudaStream_t st, float* Yp = nullptr, const float* Xc = nullptr,
-                   bool pdl = false, const DevScalars* norm = nullptr) {
-  switch (Cin) {
-    case 16: return conv_cin<16>(X, N, H, W, Cout, WT, bias, Y, relu, Yp, Xc, st, pdl, norm);
-    case 32: return conv_cin<32>(X, N, H, W, Cout, WT, bias, Y, relu, Yp, Xc, st, pdl, norm);
-    case 64: return conv_cin<64>(X, N, H, W, Cout, WT, bias, Y, relu, Yp, Xc, st, pdl, norm);
-    case 128: return conv_cin<128>(X, N, H, W, Cout, WT, bias, Y, relu, Yp, Xc, st, pdl, norm);
+// One layer: Y = conv(X, WT) (+ bias, ReLU, gate; ConvArgs).  Yp needs even H
+// and W.  pdl: dependent launch (the weights WT must be complete before the
+// chain of dependent launches started)
+static int conv3x3(int cin, const ConvArgs& a, cudaStream_t st, bool pdl = false) {
+  switch (cin) {
+    case 16: return conv_cin<16>(a, st, pdl);
+    case 32: return conv_cin<32>(a, st, pdl);
+    case 64: return conv_cin<64>(a, st, pdl);
+    case 128: return conv_cin<128>(a, st, pdl);
     default: return AJ_ERR_PARAM;
   }
 }
@@ -651,6 +817,7 @@ constexpr int DW_BLOCKS = 304;                // two per SM of a 152-SM GB300
 
 struct DwArgs {
   const float* X;    // NHWC [N][H][W][Cin]
+  const float* Xc;   // nullable: the layer's input is up2(Xc) + X
   const float* dZ;   // NHWC [N][H][W][Cout]
   int N, H, W, Cin, Cout;
   int tiles, run;    // pixel tiles in all, and per block
@@ -668,7 +835,8 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t* r, unsigned addr) {
 
 // TH: tile height, 16, or 8 where 64 accumulators leave no room to hold the
 // staged pieces of 16 rows in registers
-template <int CI, int CO, int TH>
+// UP: the input is up2(Xc) + X
+template <int CI, int CO, int TH, bool UP>
 __global__ void __launch_bounds__(DW_THREADS, 2) k_conv_dw(DwArgs a) {
   constexpr int XS = CI + 8, ZS = CO + 8;     // row strides: 16-byte aligned, bank-conflict free
   constexpr int XQ = CI / 4, ZQ = CO / 4;     // float4 pieces of a pixel
@@ -692,6 +860,7 @@ __global__ void __launch_bounds__(DW_THREADS, 2) k_conv_dw(DwArgs a) {
     for (int q = 0; q < 2 * NP; ++q)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[m][q][e] = 0.f;
+  pdl_wait();
   float4 bs = make_float4(0.f, 0.f, 0.f, 0.f);
   // this lane's rows: of A (pixels x ci) matrix j holds pixels 8 (j >> 1) ..
   // and channels 8 (j & 1) ..; of B (pixels x co) pixels 8 (j & 1) .. and
@@ -709,9 +878,15 @@ __global__ void __launch_bounds__(DW_THREADS, 2) k_conv_dw(DwArgs a) {
       const int e = tid + k * DW_THREADS, px = e / XQ, q = e - px * XQ;
       const int hy = px / DW_HW, gh = h0 - 1 + hy, gw = w0 - 1 + px - hy * DW_HW;
       xv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (e < XN && gh >= 0 && gh < H && gw >= 0 && gw < W)
+      if (e < XN && gh >= 0 && gh < H && gw >= 0 && gw < W) {
         xv[k] = __ldg(reinterpret_cast<const float4*>(
             a.X + (((long)n * H + gh) * W + gw) * a.Cin + ci0 + q * 4));
+        if (UP) {
+          const float4 c = __ldg(reinterpret_cast<const float4*>(
+              a.Xc + (((long)n * (H >> 1) + (gh >> 1)) * (W >> 1) + (gw >> 1)) * a.Cin + ci0 + q * 4));
+          xv[k] = make_float4(c.x + xv[k].x, c.y + xv[k].y, c.z + xv[k].z, c.w + xv[k].w);
+        }
+      }
     }
 #pragma unroll
     for (int k = 0; k < ZL; ++k) {
@@ -797,7 +972,9 @@ static void dw_launch(DwArgs a, cudaStream_t st) {
   const int chunks = DW_BLOCKS / slabs > 1 ? DW_BLOCKS / slabs : 1;
   a.run = (int)cdiv(a.tiles, chunks);
   a.pairs = (reinterpret_cast<uintptr_t>(a.dW) & 7) == 0;   // every offset into it is even
-  k_conv_dw<CI, CO, TH><<<dim3(cdiv(a.tiles, a.run), slabs), DW_THREADS, 0, st>>>(a);
+  const dim3 grid(cdiv(a.tiles, a.run), slabs);
+  if (a.Xc) launch_pdl(true, k_conv_dw<CI, CO, TH, true>, grid, dim3(DW_THREADS), 0, st, a);
+  else launch_pdl(true, k_conv_dw<CI, CO, TH, false>, grid, dim3(DW_THREADS), 0, st, a);
 }
 
 // the gradient of layer (cin, cout)'s weights and bias; the table's widths
@@ -811,71 +988,55 @@ static int conv_dw(const DwArgs& a, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------- element-wise
-// dX (fine, accumulated) += pool2 adjoint of dY (coarse)
-__global__ void k_pool2_bwd(const float* __restrict__ dY, float* __restrict__ dX, int N, int H,
-                            int W, int C) {   // H, W of dY
-  long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const long T = (long)N * 2 * H * 2 * W * C;
-  if (e >= T) return;
-  const int c = (int)(e % C);
-  long q = e / C;
-  const int w = (int)(q % (2 * W));
-  q /= 2 * W;
-  const int h = (int)(q % (2 * H));
-  const int n = (int)(q / (2 * H));
-  dX[e] += 0.25f * dY[(((long)n * H + h / 2) * W + w / 2) * C + c];
-}
-
-// Y (fine) = up2(X coarse) + S (fine)
-__global__ void k_up2_add(const float* __restrict__ X, const float* __restrict__ S,
-                          float* __restrict__ Y, int N, int H, int W, int C) {   // fine H, W
-  long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const long T = (long)N * H * W * C;
-  if (e >= T) return;
-  const int c = (int)(e % C);
-  long q = e / C;
+// The skip connection's gradient: dX (fine) += the pool2 adjoint of dY
+// (coarse), kept where the layer's output S is positive.  A thread takes four
+// channels of one window.  What bounds it: HBM (it reads two fine tensors and
+// writes one).
+__global__ void __launch_bounds__(256) k_pool2_bwd(const float4* __restrict__ dY,
+                                                   const float4* __restrict__ S, float4* dX, int N,
+                                                   int H, int W, int C4) {   // H, W of dY; C / 4
+  pdl_wait();
+  const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (e >= (long)N * H * W * C4) return;
+  const int c = (int)(e % C4);
+  const long q = e / C4;
   const int w = (int)(q % W);
-  q /= W;
-  const int h = (int)(q % H);
-  const int n = (int)(q / H);
-  Y[e] = X[(((long)n * (H / 2) + h / 2) * (W / 2) + w / 2) * C + c] + S[e];
-}
-
-// dX (coarse) = adjoint of nearest up2 applied to dY (fine)
-__global__ void k_up2_bwd(const float* __restrict__ dY, float* __restrict__ dX, int N, int H,
-                          int W, int C) {   // coarse H, W
-  long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const long T = (long)N * H * W * C;
-  if (e >= T) return;
-  const int c = (int)(e % C);
-  long q = e / C;
-  const int w = (int)(q % W);
-  q /= W;
-  const int h = (int)(q % H);
-  const int n = (int)(q / H);
-  const int W2 = 2 * W;
-  const long b = (((long)n * 2 * H + 2 * h) * W2 + 2 * w) * C + c;
-  dX[e] = dY[b] + dY[b + (long)W2 * C] + dY[b + C] + dY[b + (long)W2 * C + C];
-}
-
-// dZ = dOut * (Y > 0)   (ReLU adjoint)
-__global__ void k_relu_gate(const float* __restrict__ dOut, const float* __restrict__ Y,
-                            float* __restrict__ dZ, long T) {
-  long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (e < T) dZ[e] = Y[e] > 0.f ? dOut[e] : 0.f;
+  const long nh = q / W;   // n H + h: fine row 2 nh
+  const float4 g = __ldg(dY + e);
+  long k[4];
+  float4 s[4], d[4];
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    k[f] = ((2 * nh + (f >> 1)) * 2 * W + 2 * w + (f & 1)) * C4 + c;
+    s[f] = __ldg(S + k[f]);
+    d[f] = dX[k[f]];
+  }
+#pragma unroll
+  for (int f = 0; f < 4; ++f)
+    dX[k[f]] = make_float4(s[f].x > 0.f ? fmaf(0.25f, g.x, d[f].x) : 0.f,
+                           s[f].y > 0.f ? fmaf(0.25f, g.y, d[f].y) : 0.f,
+                           s[f].z > 0.f ? fmaf(0.25f, g.z, d[f].z) : 0.f,
+                           s[f].w > 0.f ? fmaf(0.25f, g.w, d[f].w) : 0.f);
 }
 
 // loss = mean over pixels of (y[.,0] - target)^2; dy = its gradient
+// (wide: dy is 16-byte aligned)
 __global__ void k_mse(const float* __restrict__ y, const float* __restrict__ target,
-                      float* __restrict__ dy, long P, double* loss) {
+                      float* __restrict__ dy, long P, double* loss, int wide) {
   float s = 0.f;
   const float inv = 1.f / (float)P;
   for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < P; p += (long)gridDim.x * blockDim.x) {
     const float d = y[p * 16] - target[p];
     s = fmaf(d, d, s);
-    dy[p * 16] = 2.f * d * inv;
+    const float g = 2.f * d * inv;
+    if (wide) {
+      float4* o = reinterpret_cast<float4*>(dy) + p * 4;
 #pragma unroll
-    for (int c = 1; c < 16; ++c) dy[p * 16 + c] = 0.f;
+      for (int c = 0; c < 4; ++c) o[c] = make_float4(c == 0 ? g : 0.f, 0.f, 0.f, 0.f);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 16; ++c) dy[p * 16 + c] = c == 0 ? g : 0.f;
+    }
   }
   block_sum_atomic((double)s * (double)inv, loss);
 }
@@ -937,7 +1098,7 @@ static PackTab pack_tab() {
 // Every tensor the backward pass needs, for batch n at the network grid h x w.
 struct NnActs {
   float *x, *a0, *s0, *p0, *a1, *s1, *p1, *a2, *s2, *p2, *a3, *bt;
-  float *u2, *o2, *u1, *o1, *u0, *o0, *y;
+  float *o2, *o1, *o0, *y;
   // backward: skip-connection gradients and two scratch buffers per resolution
   float *ds0, *ds1, *ds2, *sa0, *sa1, *sb1, *sa2, *sb2, *sa3, *sb3;
   size_t total;
@@ -965,11 +1126,8 @@ static NnActs act_layout(int n, int h, int w, void* base) {
   A.p2 = take(P3 * 128);
   A.a3 = take(P3 * 128);
   A.bt = take(P3 * 128);
-  A.u2 = take(P2 * 128);
   A.o2 = take(P2 * 64);
-  A.u1 = take(P1 * 64);
   A.o1 = take(P1 * 32);
-  A.u0 = take(P0 * 32);
   A.o0 = take(P0 * 32);
   A.y = take(P0 * 16);
   A.ds0 = take(P0 * 32);
@@ -998,17 +1156,20 @@ struct NnW {
 
 static inline unsigned ew_blocks(long T) { return cdiv(T, 256); }
 
-// The forward pass.  keep: materialise the decoder inputs u = up2(o) + s
-// (the backward pass needs them); else the decoder convolutions add the
-// up-sampled coarse input while staging their halo (inference).
+// The forward pass.  The decoder convolutions add the up-sampled coarse input
+// u = up2(o) + s while staging their halo; the backward pass does the same.
+// keep: every layer's output is kept for it (no layer pairs).
 int nn_forward(int n, int h, int w, const NnW& W, const NnActs& A, cudaStream_t st,
                bool keep = true, const DevScalars* norm = nullptr) {
   const int H0 = h, W0 = w, H1 = h / 2, W1 = w / 2, H2 = h / 4, W2 = w / 4, H3 = h / 8, W3 = w / 8;
-  // inference launches the convolutions as one chain of dependent launches
+  // one chain of dependent launches; training's first layer may follow the
+  // packing of the weights that it stages before it waits: a plain launch
   auto conv = [&](int l, const float* in, float* out, int H, int Wd, float* pooled = nullptr,
                   const float* coarse = nullptr) {
-    return conv3x3(in, n, H, Wd, kLayers[l].cin, kLayers[l].cout, W.wf(l), W.bias(l), out,
-                   kLayers[l].relu, st, pooled, coarse, !keep, l == E0A ? norm : nullptr);
+    return conv3x3(kLayers[l].cin,
+                   ConvArgs{in, n, H, Wd, kLayers[l].cout, W.wf(l), W.bias(l), out,
+                            kLayers[l].relu, pooled, coarse, l == E0A ? norm : nullptr},
+                   st, !keep || l != E0A);
   };
   int rc = AJ_OK;
   // inference on one sample: the full-resolution layer pairs in one launch each
@@ -1027,72 +1188,69 @@ int nn_forward(int n, int h, int w, const NnW& W, const NnActs& A, cudaStream_t 
   rc |= conv(E2B, A.a2, A.s2, H2, W2, A.p2);
   rc |= conv(E3A, A.p2, A.a3, H3, W3);
   rc |= conv(E3B, A.a3, A.bt, H3, W3);
-  if (keep) {
-    k_up2_add<<<ew_blocks((long)n * H2 * W2 * 128), 256, 0, st>>>(A.bt, A.s2, A.u2, n, H2, W2, 128);
-    rc |= conv(D2, A.u2, A.o2, H2, W2);
-    k_up2_add<<<ew_blocks((long)n * H1 * W1 * 64), 256, 0, st>>>(A.o2, A.s1, A.u1, n, H1, W1, 64);
-    rc |= conv(D1, A.u1, A.o1, H1, W1);
-    k_up2_add<<<ew_blocks((long)n * H0 * W0 * 32), 256, 0, st>>>(A.o1, A.s0, A.u0, n, H0, W0, 32);
-    rc |= conv(D0A, A.u0, A.o0, H0, W0);
-  } else {
-    rc |= conv(D2, A.s2, A.o2, H2, W2, nullptr, A.bt);
-    rc |= conv(D1, A.s1, A.o1, H1, W1, nullptr, A.o2);
-    if (pairs)
-      pair_launch<32, 32, 16>(PairArgs{A.s0, A.o1, nullptr, H0, W0, W.wf(D0A), W.bias(D0A),
-                                       kLayers[D0A].relu, W.wf(D0B), W.bias(D0B),
-                                       kLayers[D0B].relu, A.y, nullptr}, st);
-    else
-      rc |= conv(D0A, A.s0, A.o0, H0, W0, nullptr, A.o1);
-  }
+  rc |= conv(D2, A.s2, A.o2, H2, W2, nullptr, A.bt);
+  rc |= conv(D1, A.s1, A.o1, H1, W1, nullptr, A.o2);
+  if (pairs)
+    pair_launch<32, 32, 16>(PairArgs{A.s0, A.o1, nullptr, H0, W0, W.wf(D0A), W.bias(D0A),
+                                     kLayers[D0A].relu, W.wf(D0B), W.bias(D0B),
+                                     kLayers[D0B].relu, A.y, nullptr}, st);
+  else
+    rc |= conv(D0A, A.s0, A.o0, H0, W0, nullptr, A.o1);
   if (!pairs) rc |= conv(D0B, A.o0, A.y, H0, W0);
   if (rc != AJ_OK) return AJ_ERR_PARAM;
   return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
 }
 
-// gradient of one conv layer: dz = dout (* ReLU gate), dW, db, and (if dx) the
-// input gradient
-static void layer_bwd(int l, int n, int H, int Wd, const float* in, const float* out,
-                      const float* dout, float* dz, float* dx, const NnW& W, float* grad,
-                      cudaStream_t st) {
+// Gradient of one conv layer from g, the gradient of its output before the
+// ReLU: dW, db and (if dx) the input's gradient.  in (+ up2(in_c)): the
+// layer's input.  gate: dx is kept where it is positive (the ReLU adjoint of
+// the layer that made in); dx_c receives up2's adjoint of dx, kept where
+// gate_c is.
+static int layer_bwd(int l, int n, int H, int Wd, const float* in, const float* in_c,
+                     const float* g, float* dx, const float* gate, float* dx_c,
+                     const float* gate_c, const NnW& W, float* grad, cudaStream_t st) {
   const int cin = kLayers[l].cin, cout = kLayers[l].cout;
-  const long P = (long)n * H * Wd;
-  const float* g = dout;
-  if (kLayers[l].relu) {
-    k_relu_gate<<<ew_blocks(P * cout), 256, 0, st>>>(dout, out, dz, P * cout);
-    g = dz;
-  }
-  conv_dw(DwArgs{in, g, n, H, Wd, cin, cout, 0, 0, grad + w_off(l), grad + b_off(l), 0},
-          st);
-  if (dx) conv3x3(g, n, H, Wd, cout, cin, W.wb(l), nullptr, dx, 0, st);
+  int rc = conv_dw(DwArgs{in, in_c, g, n, H, Wd, cin, cout, 0, 0, grad + w_off(l),
+                          grad + b_off(l), 0}, st);
+  if (dx)
+    rc |= conv3x3(cout, ConvArgs{g, n, H, Wd, cin, W.wb(l), nullptr, dx, 0, dx_c, nullptr, nullptr,
+                                 gate, gate_c, 1.f}, st, true);
+  return rc;
 }
 
 int nn_backward(int n, int h, int w, const float* dy, const NnW& W, const NnActs& A, float* grad,
                 cudaStream_t st) {
   const int H0 = h, W0 = w, H1 = h / 2, W1 = w / 2, H2 = h / 4, W2 = w / 4, H3 = h / 8, W3 = w / 8;
-  const long P0 = (long)n * H0 * W0, P1 = P0 / 4, P2 = P0 / 16, P3 = P0 / 64;
   if (cudaMemsetAsync(grad, 0, n_params() * 4, st) != cudaSuccess) return AJ_ERR_CUDA;
-  // Each layer_bwd gates its incoming gradient in place and writes the input
-  // gradient to a different buffer.  Decoder first: y = d0b(o0),
-  // o0 = d0a(u0), u0 = up(o1) + s0, ...
-  layer_bwd(D0B, n, H0, W0, A.o0, A.y, dy, nullptr, A.sa0, W, grad, st);        // sa0 = d o0
-  layer_bwd(D0A, n, H0, W0, A.u0, A.o0, A.sa0, A.sa0, A.ds0, W, grad, st);      // ds0 = d u0
-  k_up2_bwd<<<ew_blocks(P1 * 32), 256, 0, st>>>(A.ds0, A.sa1, n, H1, W1, 32);   // sa1 = d o1
-  layer_bwd(D1, n, H1, W1, A.u1, A.o1, A.sa1, A.sa1, A.ds1, W, grad, st);       // ds1 = d u1
-  k_up2_bwd<<<ew_blocks(P2 * 64), 256, 0, st>>>(A.ds1, A.sa2, n, H2, W2, 64);   // sa2 = d o2
-  layer_bwd(D2, n, H2, W2, A.u2, A.o2, A.sa2, A.sa2, A.ds2, W, grad, st);       // ds2 = d u2
-  k_up2_bwd<<<ew_blocks(P3 * 128), 256, 0, st>>>(A.ds2, A.sa3, n, H3, W3, 128); // sa3 = d bt
-  // encoder: the skip gradients ds* accumulate the pooled paths
-  layer_bwd(E3B, n, H3, W3, A.a3, A.bt, A.sa3, A.sa3, A.sb3, W, grad, st);      // sb3 = d a3
-  layer_bwd(E3A, n, H3, W3, A.p2, A.a3, A.sb3, A.sb3, A.sa3, W, grad, st);      // sa3 = d p2
-  k_pool2_bwd<<<ew_blocks(P2 * 128), 256, 0, st>>>(A.sa3, A.ds2, n, H3, W3, 128);   // ds2 = d s2
-  layer_bwd(E2B, n, H2, W2, A.a2, A.s2, A.ds2, A.ds2, A.sa2, W, grad, st);      // sa2 = d a2
-  layer_bwd(E2A, n, H2, W2, A.p1, A.a2, A.sa2, A.sa2, A.sb2, W, grad, st);      // sb2 = d p1
-  k_pool2_bwd<<<ew_blocks(P1 * 64), 256, 0, st>>>(A.sb2, A.ds1, n, H2, W2, 64);     // ds1 = d s1
-  layer_bwd(E1B, n, H1, W1, A.a1, A.s1, A.ds1, A.ds1, A.sa1, W, grad, st);      // sa1 = d a1
-  layer_bwd(E1A, n, H1, W1, A.p0, A.a1, A.sa1, A.sa1, A.sb1, W, grad, st);      // sb1 = d p0
-  k_pool2_bwd<<<ew_blocks(P0 * 32), 256, 0, st>>>(A.sb1, A.ds0, n, H1, W1, 32);     // ds0 = d s0
-  layer_bwd(E0B, n, H0, W0, A.a0, A.s0, A.ds0, A.ds0, A.sa0, W, grad, st);      // sa0 = d a0
-  layer_bwd(E0A, n, H0, W0, A.x, A.a0, A.sa0, A.sa0, nullptr, W, grad, st);
+  // Each gradient is gated where it is made.  Decoder first: y = d0b(o0),
+  // o0 = d0a(up(o1) + s0), ...; d s0 (ds0) waits for the pooled path.
+  int rc = AJ_OK;
+  auto bwd = [&](int l, int H, int Wd, const float* in, const float* in_c, const float* g,
+                 float* dx, const float* gate, float* dx_c = nullptr,
+                 const float* gate_c = nullptr) {
+    rc |= layer_bwd(l, n, H, Wd, in, in_c, g, dx, gate, dx_c, gate_c, W, grad, st);
+  };
+  auto skip = [&](const float* dp, const float* s, float* ds, int H, int Wd, int C) {
+    launch_pdl(true, k_pool2_bwd, dim3(ew_blocks((long)n * H * Wd * C / 4)), dim3(256), 0, st,
+               reinterpret_cast<const float4*>(dp), reinterpret_cast<const float4*>(s),
+               reinterpret_cast<float4*>(ds), n, H, Wd, C / 4);
+  };
+  bwd(D0B, H0, W0, A.o0, nullptr, dy, A.sa0, A.o0);                  // sa0 = d o0
+  bwd(D0A, H0, W0, A.s0, A.o1, A.sa0, A.ds0, nullptr, A.sa1, A.o1);  // ds0, sa1 = d o1
+  bwd(D1, H1, W1, A.s1, A.o2, A.sa1, A.ds1, nullptr, A.sa2, A.o2);   // ds1, sa2 = d o2
+  bwd(D2, H2, W2, A.s2, A.bt, A.sa2, A.ds2, nullptr, A.sa3, A.bt);   // ds2, sa3 = d bt
+  bwd(E3B, H3, W3, A.a3, nullptr, A.sa3, A.sb3, A.a3);               // sb3 = d a3
+  bwd(E3A, H3, W3, A.p2, nullptr, A.sb3, A.sa3, nullptr);            // sa3 = d p2
+  skip(A.sa3, A.s2, A.ds2, H3, W3, 128);                             // ds2 = d s2
+  bwd(E2B, H2, W2, A.a2, nullptr, A.ds2, A.sa2, A.a2);               // sa2 = d a2
+  bwd(E2A, H2, W2, A.p1, nullptr, A.sa2, A.sb2, nullptr);            // sb2 = d p1
+  skip(A.sb2, A.s1, A.ds1, H2, W2, 64);                              // ds1 = d s1
+  bwd(E1B, H1, W1, A.a1, nullptr, A.ds1, A.sa1, A.a1);               // sa1 = d a1
+  bwd(E1A, H1, W1, A.p0, nullptr, A.sa1, A.sb1, nullptr);            // sb1 = d p0
+  skip(A.sb1, A.s0, A.ds0, H1, W1, 32);                              // ds0 = d s0
+  bwd(E0B, H0, W0, A.a0, nullptr, A.ds0, A.sa0, A.a0);               // sa0 = d a0
+  bwd(E0A, H0, W0, A.x, nullptr, A.sa0, nullptr, nullptr);
+  if (rc != AJ_OK) return AJ_ERR_PARAM;
   return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
 }
 
@@ -1310,13 +1468,24 @@ __global__ void k_nn_apply_guess(const float* __restrict__ y, int nx, int ny, in
   p0[k] = i == nx - 1 ? 0.f : pp[k] + nn_corr_at(y, nx, ny, F, sc->nn_out_scale, i, j);
 }
 
-// [n][h][w][3] -> [n][h][w][16] (zeros beyond the features)
-__global__ void k_nn_expand(const float* __restrict__ x3, float* __restrict__ x16, long cells) {
+// [n][h][w][3] -> [n][h][w][16] (zeros beyond the features), four channels a
+// thread (wide: x16 is 16-byte aligned)
+__global__ void k_nn_expand(const float* __restrict__ x3, float* __restrict__ x16, long cells,
+                            int wide) {
   const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (e >= cells * 16) return;
-  const long c = e / 16;
-  const int ch = (int)(e - c * 16);
-  x16[e] = ch < 3 ? x3[c * 3 + ch] : 0.f;
+  if (e >= cells * 4) return;
+  const long c = e >> 2;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if ((e & 3) == 0) v = make_float4(x3[c * 3], x3[c * 3 + 1], x3[c * 3 + 2], 0.f);
+  if (wide) {
+    reinterpret_cast<float4*>(x16)[e] = v;
+  } else {
+    float* o = x16 + e * 4;
+    o[0] = v.x;
+    o[1] = v.y;
+    o[2] = v.z;
+    o[3] = v.w;
+  }
 }
 
 // features (+ optional dataset copy and target) for one step's pressure solve
@@ -1449,14 +1618,15 @@ int32_t aj_nn_loss(int32_t n, int32_t h, int32_t w, const float* y, const float*
   const long P = (long)n * h * w;
   unsigned nb = cdiv(P, 256 * 4);
   if (nb > 1216) nb = 1216;
-  k_mse<<<nb, 256, 0, st>>>(y, target, dy, P, loss);
+  k_mse<<<nb, 256, 0, st>>>(y, target, dy, P, loss, (reinterpret_cast<uintptr_t>(dy) & 15) == 0);
   return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
 }
 
 int32_t aj_nn_expand(int32_t n, int32_t h, int32_t w, const float* x3, float* x16, void* stream) {
   if (!nn_shape_ok(n, h, w) || !x3 || !x16) return AJ_ERR_PARAM;
   const long cells = (long)n * h * w;
-  k_nn_expand<<<cdiv(cells * 16, 256), 256, 0, (cudaStream_t)stream>>>(x3, x16, cells);
+  k_nn_expand<<<cdiv(cells * 4, 256), 256, 0, (cudaStream_t)stream>>>(
+      x3, x16, cells, (reinterpret_cast<uintptr_t>(x16) & 15) == 0);
   return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
 }
 

@@ -127,6 +127,31 @@ def test_weight_gradient_ragged_tiles(dev, n, h, w):
         assert _rel(gp[name][1], rp[name][1]) < 1e-4, (name, "b", _rel(gp[name][1], rp[name][1]))
 
 
+@pytest.mark.parametrize("n,h,w", [(9, 72, 40), (19, 64, 8)])
+def test_batched_convolution_runs(dev, n, h, w):
+    """Batches whose layers walk runs of 16x8 tiles: partial tiles in both
+    directions on every level (72x40, 36x20, 18x10), and the smallest number
+    of tiles that does (19 samples of 64x8); forward and backward."""
+    from aerojax_gb300.nn import WarmStartNet
+    flat = _routing_params(n * 7 + h)
+    net = WarmStartNet(device=dev, params=flat)
+    rng = np.random.default_rng(n + h * w)
+    x = rng.standard_normal((n, h, w, 16)).astype(np.float32)
+    dy = rng.standard_normal((n, h, w, 16)).astype(np.float32)
+    y = net.forward(torch.as_tensor(x, device=dev), n, h, w).cpu().numpy()
+    g = net.backward(torch.as_tensor(dy, device=dev), n, h, w).cpu().numpy().astype(np.float64)
+    f64 = flat.astype(np.float64)
+    for s in range(n):
+        ref = N.forward(f64, x[s].astype(np.float64), emulate_bf16=True)
+        assert _rel(y[s], ref) < 1e-4, (s, _rel(y[s], ref))
+    ref = sum(N.backward(f64, x[s].astype(np.float64), dy[s].astype(np.float64), emulate_bf16=True)
+              for s in range(n))
+    gp, rp = N.unflatten(g), N.unflatten(ref)
+    for name, _, _, _ in N.LAYERS:
+        assert _rel(gp[name][0], rp[name][0]) < 1e-4, (name, "W", _rel(gp[name][0], rp[name][0]))
+        assert _rel(gp[name][1], rp[name][1]) < 1e-4, (name, "b", _rel(gp[name][1], rp[name][1]))
+
+
 def test_backward_matches_oracle(dev):
     from aerojax_gb300.nn import WarmStartNet
     n, h, w = 2, 16, 16

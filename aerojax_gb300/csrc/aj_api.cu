@@ -126,7 +126,7 @@ bool make_layout(const AjStepParams& p, Layout& L) {
   L.k1_u = take(nU * 4);
   L.k1_v = take(nV * 4);
   L.nu_sgs = take(N * 4);
-  L.dyn = take(16 * N * 4);
+  L.dyn = take(2 * N * 4);   // the dynamic model's cell-centred velocities (MAC)
   L.b0 = take(N * 4);
   L.T0 = take(N * 4);
   if (p.mg_mode == AJ_MG_PARITY) {
@@ -736,7 +736,7 @@ int32_t aj_kernel_count(const AjStepParams* prm, int32_t cycles) {
   // cfl, or the dt's own launch where the first stage does not write it
   int n = p.cfl_dt || p.mg_mode == AJ_MG_CONVERGE || tile_predictor_params_ok(p) ? 1 : 0;
   if (p.les_model != AJ_LES_NONE && (p.variant == AJ_VARIANT_GUI || mac))
-    n += p.les_model == AJ_LES_DYNAMIC ? (mac ? 1 : 0) + 4 : 1;
+    n += p.les_model == AJ_LES_DYNAMIC ? (mac ? 1 : 0) + 1 : 1;
   if (tile_predictor_params_ok(p)) n += tile_predictor_kernels();   // stages + rhs in tile kernels
   else n += (p.fast_mode ? 2 : 3) + (nn_forms_rhs(p, p.nn_factor > 0) ? 0 : 1);   // stages, rhs
   if (p.mg_mode == AJ_MG_PARITY) {

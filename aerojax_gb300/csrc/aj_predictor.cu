@@ -9,6 +9,7 @@
 // stage also applies the hard mask and the boundary conditions, by evaluating
 // the stage formula at the cell the boundary condition copies from.
 #include "aj_internal.cuh"
+#include <algorithm>
 #include <math.h>
 
 namespace aj {
@@ -224,149 +225,196 @@ __global__ void k_mac_to_center(const float* __restrict__ u, const float* __rest
   vc[(long)i * ny + j] = 0.5f * (v[(long)i * (ny + 1) + j + 1] + v[(long)i * (ny + 1) + j]);
 }
 
-// dynamic_smagorinsky (les_models.py:79-176) in four passes.
-// pass 1: |S| and |S| S_ij at every cell
-__global__ void k_dyn_strain(const float* __restrict__ u, const float* __restrict__ v, int nx,
-                             int ny, float h2x, float h2y, float* __restrict__ smag,
-                             float* __restrict__ ssxx, float* __restrict__ ssxy,
-                             float* __restrict__ ssyy) {
-  pdl_wait();
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= nx || j >= ny) return;
-  Strain s = strain_at(u, v, i, j, nx, ny, h2x, h2y);
-  long k = (long)i * ny + j;
-  smag[k] = s.smag;
-  ssxx[k] = s.smag * s.sxx;
-  ssxy[k] = s.smag * s.sxy;
-  ssyy[k] = s.smag * s.syy;
+// dynamic_smagorinsky (les_models.py:79-176) in one pass down the rows: the
+// strain |S|, S_ij; the 5x5 periodic box filters (les_models.py:57-76) of u,
+// v, uu, uv, vv and |S| S_ij, five columns, then five rows (the summation
+// order is not the reference's 25 rolls; in FP32 the separable sums are as
+// close to the FP64 result as the reference's own FP32 evaluation, or closer);
+// Leonard stress L_ij, model tensor M_ij and the contractions LM and MM; their
+// 3x3 interior averages, C_d = <LM>/(<MM>+1e-8) clipped to [0, 0.2] and
+// nu_sgs = C_d Delta^2 |S|.
+// A block owns a strip of columns, a thread a column, with five more at each
+// end (wrapped), and walks a run of rows.  Each stage works one row behind
+// the one before it, on rows that earlier steps left in shared memory for the
+// neighbouring columns and in registers for its own: one barrier a row.
+// What bounds it: instructions issued.  As four kernels (strain, filter, LM and
+// MM, average) it moved 33 arrays through memory; this reads two and writes
+// one, with the same bits.
+constexpr int DY_THREADS = 256, DY_HALO = 5, DY_LEAD = 7;   // rows from load to result
+// Rows a block: 12 of a run's rows are lead.  Up to four rows one block an SM
+// covers the grid, and the short chain is worth more than a second block;
+// longer runs are halved by two.  us at 152 / 304 blocks (four kernels):
+// 256x64 5.8 / 5.8 (6.2), 512x128 7.5 / 8.3 (7.3), 1024x256 16.5 / 11.4 (12.6),
+// 2048x512 19.5 at 304 (36), 4096x2048 106 at 304, 112 at 608 (294).
+static int dyn_rows(int nx, int strips) {
+  const int one = (int)cdiv((long)nx * strips, 152);
+  return one <= 4 ? std::max(one, 2) : (int)cdiv((long)nx * strips, 304);
 }
-
-// pass 2: 5x5 periodic box filter (les_models.py:57-76) of u, v, uu, uv, vv
-// and of the three |S| S_ij products, separably: a block stages its 8 x 32
-// output tile with a two-cell periodic halo of u, v and the three products,
-// sums five columns, then five rows - 8 additions per field and cell
-// instead of 24, every operand from shared memory.  (The summation order is
-// not the reference's 25 rolls; in FP32 the separable sums are as close to
-// the FP64 result as the reference's own FP32 evaluation, or closer.)
-constexpr int DF_TI = 8, DF_TJ = 32, DF_H = 2;
-constexpr int DF_SI = DF_TI + 2 * DF_H, DF_SJ = DF_TJ + 2 * DF_H;   // 12 x 36 staged cells
-__global__ void __launch_bounds__(256) k_dyn_filter(const float* __restrict__ u,
-                                                    const float* __restrict__ v,
-                                                    const float* __restrict__ ssxx,
-                                                    const float* __restrict__ ssxy,
-                                                    const float* __restrict__ ssyy, int nx,
-                                                    int ny, float* __restrict__ ut,
-                                                    float* __restrict__ vt,
-                                                    float* __restrict__ uut,
-                                                    float* __restrict__ uvt,
-                                                    float* __restrict__ vvt,
-                                                    float* __restrict__ fxx,
-                                                    float* __restrict__ fxy,
-                                                    float* __restrict__ fyy) {
+struct DynRow {
+  float2 uv[3][DY_THREADS + 4], pd[2][DY_THREADS + 4], ft[2][DY_THREADS + 4], lm[2][DY_THREADS + 4];
+  float po[2][DY_THREADS + 4];
+};
+__global__ void __launch_bounds__(DY_THREADS, 2) k_dyn(const float* __restrict__ u,
+                                                       const float* __restrict__ v, int nx, int ny,
+                                                       int width, int run, float h2x, float h2y,
+                                                       float a2, float delta2,
+                                                       float* __restrict__ nsg,
+                                                       float* __restrict__ cd) {
   pdl_wait();
-  __shared__ float S[5][DF_SI][DF_SJ];    // u, v, |S|Sxx, |S|Sxy, |S|Syy
-  __shared__ float Hs[8][DF_SI][DF_TJ];   // five-column sums of the eight fields
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * DF_TJ + tx;
-  const int i0 = blockIdx.y * DF_TI, j0 = blockIdx.x * DF_TJ;
-  for (int e = tid; e < DF_SI * DF_SJ; e += DF_TI * DF_TJ) {
-    const int r = e / DF_SJ, c = e - r * DF_SJ;
-    int gi = (i0 - DF_H + r) % nx, gj = (j0 - DF_H + c) % ny;
-    gi += gi < 0 ? nx : 0;
-    gj += gj < 0 ? ny : 0;
-    const long k = (long)gi * ny + gj;
-    S[0][r][c] = ldg(u + k);
-    S[1][r][c] = ldg(v + k);
-    S[2][r][c] = ldg(ssxx + k);
-    S[3][r][c] = ldg(ssxy + k);
-    S[4][r][c] = ldg(ssyy + k);
-  }
-  __syncthreads();
-  for (int e = tid; e < DF_SI * DF_TJ; e += DF_TI * DF_TJ) {
-    const int r = e / DF_TJ, c = e - r * DF_TJ;
-    float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int d = 0; d < 2 * DF_H + 1; ++d) {
-      const float uu = S[0][r][c + d], vv = S[1][r][c + d];
-      a[0] += uu;
-      a[1] += vv;
-      a[2] += uu * uu;
-      a[3] += uu * vv;
-      a[4] += vv * vv;
-      a[5] += S[2][r][c + d];
-      a[6] += S[3][r][c + d];
-      a[7] += S[4][r][c + d];
-    }
-#pragma unroll
-    for (int f = 0; f < 8; ++f) Hs[f][r][c] = a[f];
-  }
-  __syncthreads();
-  const int i = i0 + ty, j = j0 + tx;
-  if (i >= nx || j >= ny) return;
-  float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int d = 0; d < 2 * DF_H + 1; ++d)
-#pragma unroll
-    for (int f = 0; f < 8; ++f) a[f] += Hs[f][ty + d][tx];
+  __shared__ DynRow S;
+  const int t = threadIdx.x + 2;                       // two pad columns at each end
+  const int j = blockIdx.x * width + (int)threadIdx.x - DY_HALO;
+  const int jw = (j % ny + ny) % ny;
+  const int r0 = blockIdx.y * run, r1 = min(r0 + run, nx);
+  const bool mine = (int)threadIdx.x >= DY_HALO && (int)threadIdx.x < DY_HALO + width && j < ny;
+  const bool inside = j > 0 && j < ny - 1;
   const float inv = 1.0f / 25.0f;
-  const long k = (long)i * ny + j;
-  ut[k] = a[0] * inv;
-  vt[k] = a[1] * inv;
-  uut[k] = a[2] * inv;
-  uvt[k] = a[3] * inv;
-  vvt[k] = a[4] * inv;
-  fxx[k] = a[5] * inv;
-  fxy[k] = a[6] * inv;
-  fyy[k] = a[7] * inv;
-}
-
-// pass 3: Leonard stress L_ij, model tensor M_ij, contractions LM and MM
-__global__ void k_dyn_lm(const float* __restrict__ ut, const float* __restrict__ vt,
-                         const float* __restrict__ uut, const float* __restrict__ uvt,
-                         const float* __restrict__ vvt, const float* __restrict__ fxx,
-                         const float* __restrict__ fxy, const float* __restrict__ fyy, int nx,
-                         int ny, float h2x, float h2y, float a2, float* __restrict__ lm,
-                         float* __restrict__ mm) {
-  pdl_wait();
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= nx || j >= ny) return;
-  long k = (long)i * ny + j;
-  Strain st = strain_at(ut, vt, i, j, nx, ny, h2x, h2y);
-  float u_ = ut[k], v_ = vt[k];
-  float L11 = u_ * u_ - uut[k], L12 = u_ * v_ - uvt[k], L22 = v_ * v_ - vvt[k];
-  float M11 = a2 * st.smag * st.sxx - fxx[k];
-  float M12 = a2 * st.smag * st.sxy - fxy[k];
-  float M22 = a2 * st.smag * st.syy - fyy[k];
-  lm[k] = L11 * M11 + L12 * M12 + L22 * M22;
-  mm[k] = M11 * M11 + M12 * M12 + M22 * M22;
-}
-
-// pass 4: 3x3 interior average, C_d = <LM>/(<MM>+1e-8) clipped to [0, 0.2],
-// nu_sgs = C_d Delta^2 |S|
-__global__ void k_dyn_final(const float* __restrict__ lm, const float* __restrict__ mm,
-                            const float* __restrict__ smag, int nx, int ny, float delta2,
-                            float* __restrict__ nsg, float* __restrict__ cd) {
-  pdl_wait();
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= nx || j >= ny) return;
-  long k = (long)i * ny + j;
-  float alm = 0.f, amm = 0.f;
-  if (i > 0 && i < nx - 1 && j > 0 && j < ny - 1) {
-    for (int di = -1; di <= 1; ++di)
-      for (int dj = -1; dj <= 1; ++dj) {
-        long q = (long)(i + di) * ny + (j + dj);
-        alm += lm[q];
-        amm += mm[q];
-      }
-    alm *= (1.0f / 9.0f);
-    amm *= (1.0f / 9.0f);
+  int row = ((r0 - DY_HALO) % nx + nx) % nx;           // the row that the next load takes
+  auto next = [&]() {
+    const long k = (long)row * ny + jw;
+    row = row + 1 < nx ? row + 1 : 0;
+    return make_float2(ldg(u + k), ldg(v + k));
+  };
+  float2 c0 = make_float2(0.f, 0.f), c1 = c0, c2 = next();   // (u, v), rows k-2, k-1, k
+  float2 f0 = c0, f1 = c0, f2_ = c0;                   // filtered (u, v), rows k-6, k-5, k-4
+  float2 uvv = c0, fd = c0;                            // filtered (uu, vv), (Pxx, Pyy), row k-5
+  float uvt = 0.f, fo = 0.f;                           // filtered uv, Pxy, row k-5
+  float2 ha[5], hb[5], hc[5];                          // column sums of (u, v), (uu, vv), (Pxx, Pyy)
+  float hd[5], he[5];                                  // and of uv, Pxy: rows k-6 .. k-2
+  float sm[7];                                         // |S|, rows k-7 .. k-1
+  float2 l[3][3];                                      // (LM, MM), rows k-8 .. k-6, columns j-1 .. j+1
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    ha[q] = hb[q] = hc[q] = c0;
+    hd[q] = he[q] = 0.f;
   }
-  float c = alm / (amm + 1e-8f);
-  c = fminf(fmaxf(c, 0.0f), 0.2f);
-  nsg[k] = c * delta2 * smag[k];
-  if (cd) cd[k] = c;
+#pragma unroll
+  for (int q = 0; q < 7; ++q) sm[q] = 0.f;
+#pragma unroll
+  for (int q = 0; q < 9; ++q) l[q / 3][q % 3] = c0;
+  float2 *uv0 = S.uv[0], *uv1 = S.uv[1], *uv2 = S.uv[2];     // rows k-2, k-1, k
+  const int steps = r1 - r0 + DY_HALO + DY_LEAD;
+#pragma unroll 5
+  for (int n = 0; n < steps; ++n) {                    // row k = r0 - 5 + n is in c2
+    const int a = n & 1, b = a ^ 1;                    // this step's slot, the last one's
+    const float2 ahead = next();
+    uv2[t] = c2;
+    // strain at row k - 1
+    float2 pd;
+    float po;
+    {
+      const float2 yp = uv1[t + 1], ym = uv1[t - 1];
+      const float du_dx = (c2.x - c0.x) * h2x, dv_dx = (c2.y - c0.y) * h2x;
+      const float du_dy = (yp.x - ym.x) * h2y, dv_dy = (yp.y - ym.y) * h2y;
+      const float sxy = 0.5f * (du_dy + dv_dx);
+      const float smag =
+          sqrtf(2.0f * (du_dx * du_dx + dv_dy * dv_dy + 2.0f * sxy * sxy) + 1e-10f);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) sm[q] = sm[q + 1];
+      sm[6] = smag;
+      pd = make_float2(smag * du_dx, smag * dv_dy);
+      po = smag * sxy;
+    }
+    // column sums at row k - 2
+    {
+      float2 sa = make_float2(0.f, 0.f), sb = sa, sc = sa;
+      float sd = 0.f, se = 0.f;
+#pragma unroll
+      for (int d = -2; d <= 2; ++d) {
+        const float2 w = uv0[t + d];
+        sa = add2(sa, w);
+        sb = fma2(w, w, sb);
+        sd = fmaf(w.x, w.y, sd);
+        sc = add2(sc, S.pd[b][t + d]);
+        se += S.po[b][t + d];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        ha[q] = ha[q + 1];
+        hb[q] = hb[q + 1];
+        hc[q] = hc[q + 1];
+        hd[q] = hd[q + 1];
+        he[q] = he[q + 1];
+      }
+      ha[4] = sa;
+      hb[4] = sb;
+      hc[4] = sc;
+      hd[4] = sd;
+      he[4] = se;
+    }
+    S.pd[a][t] = pd;
+    S.po[a][t] = po;
+    // LM and MM at row k - 5, from the filtered rows k - 6 .. k - 4
+    f0 = f1;
+    f1 = f2_;
+    const float2 uvv1 = uvv, fd1 = fd;
+    const float uvt1 = uvt, fo1 = fo;
+    {
+      float2 sa = make_float2(0.f, 0.f), sb = sa, sc = sa;
+      float sd = 0.f, se = 0.f;
+#pragma unroll
+      for (int d = 0; d < 5; ++d) {
+        sa = add2(sa, ha[d]);
+        sb = add2(sb, hb[d]);
+        sc = add2(sc, hc[d]);
+        sd += hd[d];
+        se += he[d];
+      }
+      const float2 i2 = f2(inv);
+      f2_ = mul2(sa, i2);
+      uvv = mul2(sb, i2);
+      fd = mul2(sc, i2);
+      uvt = __fmul_rn(sd, inv);
+      fo = __fmul_rn(se, inv);
+    }
+    float2 lmv;
+    {
+      const float2 yp = S.ft[b][t + 1], ym = S.ft[b][t - 1];
+      const float du_dx = (f2_.x - f0.x) * h2x, dv_dx = (f2_.y - f0.y) * h2x;
+      const float du_dy = (yp.x - ym.x) * h2y, dv_dy = (yp.y - ym.y) * h2y;
+      const float sxy = 0.5f * (du_dy + dv_dx);
+      const float smag =
+          sqrtf(2.0f * (du_dx * du_dx + dv_dy * dv_dy + 2.0f * sxy * sxy) + 1e-10f);
+      const float u_ = f1.x, v_ = f1.y;
+      const float L11 = u_ * u_ - uvv1.x, L12 = u_ * v_ - uvt1, L22 = v_ * v_ - uvv1.y;
+      const float M11 = a2 * smag * du_dx - fd1.x;
+      const float M12 = a2 * smag * sxy - fo1;
+      const float M22 = a2 * smag * dv_dy - fd1.y;
+      lmv.x = L11 * M11 + L12 * M12 + L22 * M22;
+      lmv.y = M11 * M11 + M12 * M12 + M22 * M22;
+    }
+    S.ft[a][t] = f2_;
+    // the average at row k - 7, from LM and MM of rows k - 8 .. k - 6
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      l[0][q] = l[1][q];
+      l[1][q] = l[2][q];
+      l[2][q] = S.lm[b][t - 1 + q];
+    }
+    S.lm[a][t] = lmv;
+    const int g = r0 - DY_HALO + n - DY_LEAD;
+    if (mine && g >= r0) {
+      float2 m = make_float2(0.f, 0.f);
+      if (inside && g > 0 && g < nx - 1) {
+#pragma unroll
+        for (int q = 0; q < 9; ++q) m = add2(m, l[q / 3][q % 3]);
+        m = mul2(m, f2(1.0f / 9.0f));
+      }
+      float c = m.x / (m.y + 1e-8f);
+      c = fminf(fmaxf(c, 0.0f), 0.2f);
+      const long k = (long)g * ny + j;
+      nsg[k] = c * delta2 * sm[0];
+      if (cd) cd[k] = c;
+    }
+    c0 = c1;
+    c1 = c2;
+    c2 = ahead;
+    float2* w = uv0;
+    uv0 = uv1;
+    uv1 = uv2;
+    uv2 = w;
+    __syncthreads();
+  }
 }
 
 int launch_les(const AjStepParams& p, const Layout& L, void* ws, int model, const float* u,
@@ -385,8 +433,8 @@ int launch_les(const AjStepParams& p, const Layout& L, void* ws, int model, cons
     return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
   }
   if (mac_input) {
-    float* uc = D + 14 * n;
-    float* vc = D + 15 * n;
+    float* uc = D;
+    float* vc = D + n;
     launch_pdl(true, k_mac_to_center, dim3(grd), dim3(blk), 0, st, u, v, uc, vc, nx, ny);
     uu = uc;
     vv = vc;
@@ -396,18 +444,10 @@ int launch_les(const AjStepParams& p, const Layout& L, void* ws, int model, cons
     launch_pdl(true, k_les_const, dim3(grd), dim3(blk), 0, st, uu, vv, nsg, nx, ny, h2x, h2y,
                (float)(c * c));
   } else if (model == AJ_LES_DYNAMIC) {
-    float *smag = D, *sxx = D + n, *sxy = D + 2 * n, *syy = D + 3 * n;
-    float *ut = D + 4 * n, *vt = D + 5 * n, *uut = D + 6 * n, *uvt = D + 7 * n, *vvt = D + 8 * n;
-    float *fxx = D + 9 * n, *fxy = D + 10 * n, *fyy = D + 11 * n;
-    float *lm = D + 12 * n, *mm = D + 13 * n;
-    launch_pdl(true, k_dyn_strain, dim3(grd), dim3(blk), 0, st, uu, vv, nx, ny, h2x, h2y, smag, sxx,
-               sxy, syy);
-    launch_pdl(true, k_dyn_filter, dim3(grd), dim3(blk), 0, st, uu, vv, sxx, sxy, syy, nx, ny, ut,
-               vt, uut, uvt, vvt, fxx, fxy, fyy);
-    launch_pdl(true, k_dyn_lm, dim3(grd), dim3(blk), 0, st, ut, vt, uut, uvt, vvt, fxx, fxy, fyy,
-               nx, ny, h2x, h2y, 4.0f, lm, mm);
-    launch_pdl(true, k_dyn_final, dim3(grd), dim3(blk), 0, st, lm, mm, smag, nx, ny,
-               (float)(delta * delta), nsg, cd);
+    const int strips = (int)cdiv(ny, DY_THREADS - 2 * DY_HALO), width = (int)cdiv(ny, strips);
+    const int run = dyn_rows(nx, strips);
+    launch_pdl(true, k_dyn, dim3(strips, cdiv(nx, run)), dim3((width + 2 * DY_HALO + 31) / 32 * 32), 0,
+               st, uu, vv, nx, ny, width, run, h2x, h2y, 4.0f, (float)(delta * delta), nsg, cd);
   } else {
     return AJ_ERR_PARAM;
   }

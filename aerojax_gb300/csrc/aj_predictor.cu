@@ -247,8 +247,9 @@ constexpr int DY_THREADS = 256, DY_HALO = 5, DY_LEAD = 7;   // rows from load to
 // 256x64 5.8 / 5.8 (6.2), 512x128 7.5 / 8.3 (7.3), 1024x256 16.5 / 11.4 (12.6),
 // 2048x512 19.5 at 304 (36), 4096x2048 106 at 304, 112 at 608 (294).
 static int dyn_rows(int nx, int strips) {
-  const int one = (int)cdiv((long)nx * strips, 152);
-  return one <= 4 ? std::max(one, 2) : (int)cdiv((long)nx * strips, 304);
+  auto rows = [&](int blocks) { return (int)cdiv(nx, std::max(1, blocks / strips)); };
+  const int one = rows(152);
+  return one <= 4 ? std::max(one, 2) : rows(304);
 }
 struct DynRow {
   float2 uv[3][DY_THREADS + 4], pd[2][DY_THREADS + 4], ft[2][DY_THREADS + 4], lm[2][DY_THREADS + 4];

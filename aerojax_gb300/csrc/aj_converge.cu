@@ -33,6 +33,7 @@
 // g = (theta - 1) / theta, theta = (1 - 2^-l) / 2).  The oracle is
 // oracle/ref_np.py mg_converge (FP64 throughout).
 #include "aj_internal.cuh"
+#include <algorithm>
 #include <math.h>
 #include <string.h>
 #include <map>
@@ -1100,8 +1101,14 @@ __global__ void __launch_bounds__(256) k_cv_init(const float* __restrict__ p0,
   }
 }
 
-// residual of the reference operator before the first cycle (double-FP32)
-// and the FP64 norms of r and b; a block per 8 rows
+// Residual of the reference operator before the first cycle (double-FP32)
+// and the FP64 norms of r and b; a thread a column pair over four rows with
+// 8-byte reads and paired arithmetic, a block bands of 32 rows by 64 columns.
+// What bounds it: a band's chain of reads and double-FP32 arithmetic at 24 warps
+// an SM.  Cold, a thread one column over eight rows -> this: 2048x512 13.4 -> 12
+// us, 4096x2048 60 -> 43 (51 with a block for every band).
+constexpr int CVR_ROWS = 4;
+constexpr unsigned CVR_BLOCKS = 456;   // three an SM
 __global__ void __launch_bounds__(256) k_cv_resid(const float* __restrict__ ps,
                                                   const float* __restrict__ b,
                                                   float* __restrict__ r, int n, int m, DfCoef co,
@@ -1109,63 +1116,69 @@ __global__ void __launch_bounds__(256) k_cv_resid(const float* __restrict__ ps,
   pdl_wait();
   const long N = (long)n * m;
   const df ax{co.axh, co.axl}, ay{co.ayh, co.ayl};
-  float acc = 0.f, accb = 0.f;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < m) {
-    const int i0 = blockIdx.y * CV_ROWS;
-    // all loads first: the state at rows i0-1 .. i0+CV_ROWS (column j), the
-    // column neighbours j-1, j+1 and b at rows i0 .. i0+CV_ROWS-1
-    float ch[CV_ROWS + 2], cl[CV_ROWS + 2], yph[CV_ROWS], ypl[CV_ROWS], ymh[CV_ROWS],
-        yml[CV_ROWS], bv[CV_ROWS];
+  df sum{0.f, 0.f}, sumb{0.f, 0.f};
+  const int j = 2 * (blockIdx.x * 32 + (threadIdx.x & 31));
+  // a block walks bands of 32 rows: its three atomics on the scalars, and not
+  // its loads, set the time when every band had a block of its own
+  for (int i0 = (blockIdx.y * 8 + (threadIdx.x >> 5)) * CVR_ROWS; j < m && i0 < n;
+       i0 += gridDim.y * 8 * CVR_ROWS) {
+    float acc = 0.f, accb = 0.f;
+    auto pair = [&](const float* f, long k) { return *reinterpret_cast<const float2*>(f + k); };
+    // all loads first: the state at rows i0 - 1 .. i0 + 4, the pair's column
+    // neighbours and b
+    df2 c[CVR_ROWS + 2];
+    df lf[CVR_ROWS], rt[CVR_ROWS];
+    float2 bv[CVR_ROWS];
 #pragma unroll
-    for (int q = 0; q < CV_ROWS + 2; ++q) {
+    for (int q = 0; q < CVR_ROWS + 2; ++q) {
       const int i = i0 - 1 + q;
-      ch[q] = cl[q] = 0.f;
+      c[q].hi = c[q].lo = f2(0.f);
       if (i >= 0 && i < n) {
         const long k = (long)i * m + j;
-        ch[q] = ps[k];
-        cl[q] = ps[N + k];
+        c[q].hi = pair(ps, k);
+        c[q].lo = pair(ps, N + k);
       }
     }
 #pragma unroll
-    for (int q = 0; q < CV_ROWS; ++q) {
-      const int i = i0 + q;
-      yph[q] = ypl[q] = ymh[q] = yml[q] = bv[q] = 0.f;
-      if (i < n - 1) {
-        const long k = (long)i * m + j;
-        if (j + 1 < m) {
-          yph[q] = ps[k + 1];
-          ypl[q] = ps[N + k + 1];
-        }
-        if (j > 0) {
-          ymh[q] = ps[k - 1];
-          yml[q] = ps[N + k - 1];
-        }
-        bv[q] = b[k];
+    for (int q = 0; q < CVR_ROWS; ++q) {
+      const long k = (long)(i0 + q) * m + j;
+      bv[q] = f2(0.f);
+      lf[q] = rt[q] = df{0.f, 0.f};
+      if (i0 + q < n - 1) {
+        bv[q] = pair(b, k);
+        if (j > 0) lf[q] = df{ps[k - 1], ps[N + k - 1]};
+        if (j + 2 < m) rt[q] = df{ps[k + 2], ps[N + k + 2]};
       }
     }
 #pragma unroll
-    for (int q = 0; q < CV_ROWS; ++q) {
+    for (int q = 0; q < CVR_ROWS; ++q) {
       const int i = i0 + q;
       if (i >= n) break;
-      const long k = (long)i * m + j;
-      float rr = 0.f;
+      float2 rr = f2(0.f);
       if (i != n - 1) {
-        const df c{ch[q + 1], cl[q + 1]};
-        const df xp{ch[q + 2], cl[q + 2]};
-        const df xm = i > 0 ? df{ch[q], cl[q]} : c;
-        const df yp = j + 1 < m ? df{yph[q], ypl[q]} : c;
-        const df ym = j > 0 ? df{ymh[q], yml[q]} : c;
-        const df res = df_residual(bv[q], c, xp, xm, yp, ym, ax, ay);
-        rr = res.hi + res.lo;
-        accb = fmaf(bv[q], bv[q], accb);
+        const df2 x = c[q + 1], xm = i > 0 ? c[q] : x;
+        // the neighbours' edge ghosts are the cell itself
+        const df2 yp{make_float2(x.hi.y, j + 2 < m ? rt[q].hi : x.hi.y),
+                     make_float2(x.lo.y, j + 2 < m ? rt[q].lo : x.lo.y)};
+        const df2 ym{make_float2(j > 0 ? lf[q].hi : x.hi.x, x.hi.x),
+                     make_float2(j > 0 ? lf[q].lo : x.lo.x, x.lo.x)};
+        const df2 res = df2_residual(bv[q], x, c[q + 2], xm, yp, ym, ax, ay);
+        rr = add2(res.hi, res.lo);
+        accb = fmaf(bv[q].x, bv[q].x, accb);
+        accb = fmaf(bv[q].y, bv[q].y, accb);
       }
-      r[k] = rr;
-      acc = fmaf(rr, rr, acc);
+      cp_st2(r + (long)i * m + j, rr);
+      acc = fmaf(rr.x, rr.x, acc);
+      acc = fmaf(rr.y, rr.y, acc);
     }
+    sum = df_add(sum, df{acc, 0.f});
+    sumb = df_add(sumb, df{accb, 0.f});
   }
-  block_sum_atomic_f(acc, &sc->acc[0]);
-  block_sum_atomic_f(accb, &sc->acc[1]);
+  const double t = block_sum_df(sum), tb = block_sum_df(sumb);
+  if (threadIdx.x == 0) {
+    atomicAdd(&sc->acc[0], t);
+    atomicAdd(&sc->acc[1], tb);
+  }
   // the last block: commit the history rotation, reset the solve's counters
   // and run the test before the first cycle (the guess may already satisfy rtol)
   __shared__ int am_last;
@@ -1208,19 +1221,33 @@ __global__ void __launch_bounds__(256) k_cv_resid(const float* __restrict__ ps,
 }
 
 // p = hi + lo; with a history, the state also goes to the free slot (the
-// next solve's k_cv_resid makes it the latest); thread 0 files the statistics
-__global__ void k_cv_out(PState ps, DevScalars* sc, float* __restrict__ p, long N, float* hist,
-                         AjStats* stats) {
+// next solve's k_cv_resid makes it the latest); thread 0 files the statistics.
+// V: floats a thread, 4 where p is 16-byte aligned (N is a multiple of 4).
+template <int V>
+__global__ void __launch_bounds__(256) k_cv_out(PState ps, DevScalars* sc, float* __restrict__ p,
+                                                long N, float* hist, AjStats* stats) {
   pdl_wait();
-  long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const long k = (blockIdx.x * (long)blockDim.x + threadIdx.x) * V;
   const float* src = sc->pcur ? ps.b : ps.a;
   if (k < N) {
-    const float hi = src[k], lo = src[N + k];
-    p[k] = hi + lo;
+    alignas(16) float hi[V], lo[V], out[V];
+    auto get = [](float* v, const float* f) {
+      if constexpr (V == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(f);
+      else v[0] = f[0];
+    };
+    auto put = [](float* f, const float* v) {
+      if constexpr (V == 4) *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(v);
+      else f[0] = v[0];
+    };
+    get(hi, src + k);
+    get(lo, src + N + k);
+#pragma unroll
+    for (int q = 0; q < V; ++q) out[q] = hi[q] + lo[q];
+    put(p + k, out);
     if (hist) {
       float* dst = hist + (long)(1 - sc->hist_cur) * 2 * N;
-      dst[k] = hi;
-      dst[N + k] = lo;
+      put(dst + k, hi);
+      put(dst + N + k, lo);
     }
   }
   if (k == 0) {
@@ -1444,7 +1471,9 @@ int converge_solve(const AjStepParams& p, const Layout& L, void* ws, const float
     const int rc = nn_correct_state(p, L, ws, at<float>(ws, L.b0), *nn, ps.a, st);
     if (rc != AJ_OK) return rc;
   }
-  launch_pdl(true, k_cv_resid, dim3(rgrid), dim3(256), 0, st, ps.a, at<float>(ws, L.b0),
+  launch_pdl(true, k_cv_resid, dim3(cdiv(p.ny, 64), std::min<unsigned>(cdiv(p.nx, 8 * CVR_ROWS),
+                                                             std::max(1u, CVR_BLOCKS / (unsigned)cdiv(p.ny, 64)))),
+             dim3(256), 0, st, ps.a, at<float>(ws, L.b0),
              at<float>(ws, L.B[0]), p.nx, p.ny, df_coef(1.0 / (p.dx * p.dx), 1.0 / (p.dy * p.dy)),
              sc, p.mg_rtol);
 
@@ -1494,8 +1523,11 @@ int converge_solve(const AjStepParams& p, const Layout& L, void* ws, const float
     cudaGraph_t out;
     if (cudaStreamEndCapture(side, &out) != cudaSuccess) return AJ_ERR_CUDA;
   }
-  launch_pdl(true, k_cv_out, dim3(cdiv(N, 256)), dim3(256), 0, st, ps, sc, pout, N,
-             extrap ? at<float>(ws, L.hist) : nullptr, stats);
+  float* hist = extrap ? at<float>(ws, L.hist) : nullptr;
+  if (N % 4 == 0 && (reinterpret_cast<uintptr_t>(pout) & 15) == 0)
+    launch_pdl(true, k_cv_out<4>, dim3(cdiv(N, 1024)), dim3(256), 0, st, ps, sc, pout, N, hist, stats);
+  else
+    launch_pdl(true, k_cv_out<1>, dim3(cdiv(N, 256)), dim3(256), 0, st, ps, sc, pout, N, hist, stats);
   return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
 }
 

@@ -743,7 +743,8 @@ int32_t aj_kernel_count(const AjStepParams* prm, int32_t cycles) {
     n += parity_kernel_count(p, L);
   } else {
     int body = 2 * L.lc + 1 + (L.ld > 0 ? 2 : 0);               // downs, coarse solve, ups
-    n += 2 + (cycles > 1 ? cycles : 1) * body + 1;              // init, resid, loop, out+stats
+    const int least = converge_inline_cycles(p);                // launched whether needed or not
+    n += 2 + (cycles > least ? cycles : least) * body + 1;      // init, resid, loop, out+stats
   }
   n += 1;                                                       // correction
   // features, scales, the convolutions (12, or 10 with the two

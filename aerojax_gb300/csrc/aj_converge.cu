@@ -1433,6 +1433,9 @@ static void cv_body(const AjStepParams& p, const Layout& L, void* ws,
 // nearly every solve runs: two from a warm start (two or three run), four
 // from zero (four or five).
 constexpr int CV_INLINE_WARM = 2, CV_INLINE_ZERO = 4;
+int converge_inline_cycles(const AjStepParams& p) {
+  return std::min(p.warm_start == AJ_WARM_ZERO ? CV_INLINE_ZERO : CV_INLINE_WARM, p.max_cycles);
+}
 
 static cudaStream_t side_stream() {
   static cudaStream_t s = nullptr;
@@ -1497,8 +1500,7 @@ int converge_solve(const AjStepParams& p, const Layout& L, void* ws, const float
     cudaGraphConditionalHandle h;
     if (cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) != cudaSuccess)
       return AJ_ERR_CUDA;
-    const int inline_cycles = p.warm_start == AJ_WARM_ZERO ? CV_INLINE_ZERO : CV_INLINE_WARM;
-    for (int k = 0; k < inline_cycles && k < p.max_cycles; ++k) cv_body(p, L, ws, h, 1, st);
+    for (int k = 0; k < converge_inline_cycles(p); ++k) cv_body(p, L, ws, h, 1, st);
     if (cudaStreamGetCaptureInfo(st, &cs, &id, &g, &deps, &ed, &nd) != cudaSuccess)
       return AJ_ERR_CUDA;
     // the params union has no default constructor: zero-initialised storage

@@ -37,7 +37,9 @@ struct DevScalars {
   int hist_pending;    // a solve finished since the last k_cv_begin
   float dt_last;       // dt of the last finished solve
   float dt_prev;       // dt of the latest solution in the history
-  unsigned int pad_[3];
+  float nn_ir, nn_ip;  // learned warm start: 1 / nn_rms_r, 1 / nn_rms_p
+  float nn_os_hi, nn_os_lo;   // nn_out_scale as two floats
+  unsigned int pad_[1];
 };
 
 struct Layout {

@@ -302,8 +302,8 @@ __device__ __forceinline__ void conv_tile(const ConvArgs& cv, int t, int co0,
     const int Hc = H >> 1, Wc = W >> 1;
     float ir = 1.f, ip = 1.f;
     if (cv.norm) {
-      ir = (float)(1.0 / cv.norm->nn_rms_r);
-      ip = (float)(1.0 / cv.norm->nn_rms_p);
+      ir = cv.norm->nn_ir;
+      ip = cv.norm->nn_ip;
     }
     for (int e0 = tid; e0 < CT_HALO * C8; e0 += XB * CONV_THREADS) {
       float4 xa[XB], xb[XB], ca[XB], cb[XB];
@@ -575,8 +575,8 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv_pair(PairArgs a) {
     const int Hc = H >> 1, Wc = W >> 1;
     float ir = 1.f, ip = 1.f;
     if (a.norm) {
-      ir = (float)(1.0 / a.norm->nn_rms_r);
-      ip = (float)(1.0 / a.norm->nn_rms_p);
+      ir = a.norm->nn_ir;
+      ip = a.norm->nn_ip;
     }
     for (int e0 = tid; e0 < S::HIN * C8; e0 += XB * CONV_THREADS) {
       float4 xa[XB], xb[XB], ca[XB], cb[XB];
@@ -1336,15 +1336,120 @@ __global__ void __launch_bounds__(256) k_nn_feat(const float* __restrict__ b,
   }
 }
 
+// The same four columns a thread with 16-byte reads (ny is a multiple of 16):
+// 13 reads for four cells where each cell read 12.  Every cell's expressions
+// and every window's order of additions are k_nn_feat's.  What bounds it: the
+// reads' round trip, then L2.  Cold at 2048x512, F = 8, right-hand side formed here:
+// 12.4 -> 7.0 us.
+template <int F>
+__global__ void __launch_bounds__(256) k_nn_feat4(const float* __restrict__ b,
+                                                  const float* __restrict__ mask,
+                                                  const float* __restrict__ pp, int nx, int ny,
+                                                  float ax, float ay, float* __restrict__ x,
+                                                  RhsSrc rs) {
+  pdl_wait();
+  constexpr int S = F == 2 ? 2 : 1;   // window sums a thread takes part in
+  __shared__ float red[3][S][8][32];
+  const int lane = threadIdx.x, row = threadIdx.y;
+  const int j = 4 * (blockIdx.x * 32 + lane), i = blockIdx.y * 8 + row;
+  struct F4 {
+    float v[4];
+  };
+  auto ld = [](const float* p) {
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    return F4{t.x, t.y, t.z, t.w};
+  };
+  const F4 zero{0.f, 0.f, 0.f, 0.f};
+  F4 vr = zero, vm = zero, vp = zero;
+  if (i < nx && j < ny) {
+    const long k = (long)i * ny + j;
+    vp = ld(pp + k);
+    vm = ld(mask + k);
+    F4 bk;
+    if (rs.us) {
+      const F4 up = ld(rs.us + k + ny), um = ld(rs.us + k);
+      const float* v = rs.vs + (long)i * (ny + 1) + j;
+      float w[5];
+#pragma unroll
+      for (int q = 0; q < 5; ++q) w[q] = ldg(v + q);
+      const float dt = rs.sc->dt;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float du = (up.v[q] - um.v[q]) * rs.idx;
+        const float dv = (w[q + 1] - w[q]) * rs.idy;
+        const float out = ((du + dv) / dt) * vm.v[q];
+        bk.v[q] = (rs.outlet && i == nx - 1) ? 0.f : out;
+      }
+      *reinterpret_cast<float4*>(rs.b_out + k) = make_float4(bk.v[0], bk.v[1], bk.v[2], bk.v[3]);
+    } else {
+      bk = ld(b + k);
+    }
+    if (i != nx - 1) {
+      const F4 xp = ld(pp + k + ny), xm = i > 0 ? ld(pp + k - ny) : vp;
+      const float c[6] = {j > 0 ? pp[k - 1] : vp.v[0], vp.v[0], vp.v[1], vp.v[2], vp.v[3],
+                          j + 4 < ny ? pp[k + 4] : vp.v[3]};
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        vr.v[q] = bk.v[q] - (ax * ((xp.v[q] - c[q + 1]) + (xm.v[q] - c[q + 1])) +
+                             ay * ((c[q + 2] - c[q + 1]) + (c[q] - c[q + 1])));
+    }
+  }
+  auto sums = [&](int f, const F4& v) {
+    const float a = v.v[0] + v.v[1], c = v.v[2] + v.v[3];
+    if (F == 2) {
+      red[f][0][row][lane] = a;
+      red[f][S - 1][row][lane] = c;
+    } else {
+      float t = a + c;
+      if (F == 8) t += __shfl_xor_sync(0xffffffffu, t, 1);
+      red[f][0][row][lane] = t;
+    }
+  };
+  sums(0, vr);
+  sums(1, vm);
+  sums(2, vp);
+  __syncthreads();
+  if (row % F || i >= nx || j >= ny || (F == 8 && (lane & 1))) return;
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    float a[3] = {0.f, 0.f, 0.f};
+    for (int q = 0; q < F; ++q)
+#pragma unroll
+      for (int f = 0; f < 3; ++f) a[f] += red[f][s][row + q][lane];
+    const float inv = 1.f / (float)(F * F);
+    float4* o = reinterpret_cast<float4*>(x) + ((long)(i / F) * (ny / F) + (j + 2 * s) / F) * 4;
+    o[0] = make_float4(a[0] * inv, a[1] * inv, a[2] * inv, 0.f);
+    o[1] = o[2] = o[3] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+
 // per-sample scales: RMS of channels 0 and 2 over the network grid and the
 // output scale rms_r * lmin^2 / 10 (a correction solving A dp = r has that
 // magnitude).  Each block files its FP64 partial sums in part[2 b], part[2 b
 // + 1]; the last block to finish adds them in block order, so the scales -
 // and the correction - are bit-reproducible.
+// Both sums go through one pair of barriers, the warps' totals added by a warp:
+// one sum after the other, each with a serial loop over the warps, 11.7 us
+// cold at 256x64 cells;
+// this 9.7.
+__device__ __forceinline__ void block_sum2(double& a, double& b) {
+  __shared__ double2 wp[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  a = warp_sum(a);
+  b = warp_sum(b);
+  if (lane == 0) wp[w] = make_double2(a, b);
+  __syncthreads();
+  if (w == 0) {
+    const double2 t = lane < nw ? wp[lane] : make_double2(0.0, 0.0);
+    a = warp_sum(t.x);
+    b = warp_sum(t.y);
+  }
+  __syncthreads();
+}
 constexpr int NN_SCALE_BLOCKS = 32;
 static_assert(2 * NN_SCALE_BLOCKS <= kPartials, "the partial sums live in the workspace's part");
 __global__ void __launch_bounds__(512) k_nn_scale(const float* __restrict__ x, long cells,
-                                                  DevScalars* sc, double lmin2, double* part) {
+                                                  DevScalars* sc, double out_fac, double* part) {
   pdl_wait();
   float sr = 0.f, sp = 0.f;
   const long stride = (long)gridDim.x * blockDim.x;
@@ -1354,8 +1459,8 @@ __global__ void __launch_bounds__(512) k_nn_scale(const float* __restrict__ x, l
     sr = fmaf(r, r, sr);
     sp = fmaf(q, q, sp);
   }
-  const double br = block_sum((double)sr);
-  const double bp = block_sum((double)sp);
+  double br = (double)sr, bp = (double)sp;
+  block_sum2(br, bp);
   __shared__ int am_last;
   if (threadIdx.x == 0) {
     part[2 * blockIdx.x] = br;
@@ -1374,15 +1479,30 @@ __global__ void __launch_bounds__(512) k_nn_scale(const float* __restrict__ x, l
     lr += __ldcg(part + 2 * b);
     lp += __ldcg(part + 2 * b + 1);
   }
-  const double tr = block_sum(lr);
-  const double tp = block_sum(lp);
-  if (threadIdx.x == 0) {
-    const double rr = sqrt(tr / (double)cells), rp = sqrt(tp / (double)cells);
-    const double rrc = rr > 1e-30 ? rr : 1e-30, rpc = rp > 1e-30 ? rp : 1e-30;
-    sc->nn_rms_r = rrc;
-    sc->nn_rms_p = rpc;
-    sc->nn_out_scale = rrc * lmin2 / 10.0;
-    sc->red_count = 0u;
+  double tr = lr, tp = lp;
+  block_sum2(tr, tp);
+  if (threadIdx.x < 32) {
+    // lane 0 the residual's scale, lane 1 the pressure's, in one chain of FP64
+    // operations; the reciprocals and the split that every later block needs
+    // are formed once here
+    tp = __shfl_sync(0xffffffffu, tp, 0);
+    const int lane = threadIdx.x;
+    const double rms = sqrt((lane == 0 ? tr : tp) / (double)cells);
+    const double r = rms > 1e-30 ? rms : 1e-30;
+    const float inv = (float)(1.0 / r);
+    if (lane == 0) {
+      const double os = r * out_fac;
+      const float hi = (float)os;
+      sc->nn_rms_r = r;
+      sc->nn_ir = inv;
+      sc->nn_out_scale = os;
+      sc->nn_os_hi = hi;
+      sc->nn_os_lo = (float)(os - (double)hi);
+      sc->red_count = 0u;
+    } else if (lane == 1) {
+      sc->nn_rms_p = r;
+      sc->nn_ip = inv;
+    }
   }
 }
 
@@ -1392,7 +1512,7 @@ __global__ void k_nn_norm(float* __restrict__ x, float* __restrict__ x3, long ce
   pdl_wait();
   const long c = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (c >= cells) return;
-  const float ir = (float)(1.0 / sc->nn_rms_r), ip = (float)(1.0 / sc->nn_rms_p);
+  const float ir = sc->nn_ir, ip = sc->nn_ip;
   float* o = x + c * 16;
   o[0] *= ir;
   o[2] *= ip;
@@ -1419,40 +1539,65 @@ __global__ void k_nn_target(const float* __restrict__ pt, const float* __restric
   target[(long)I * w + J] = (float)((double)(a / (float)(F * F)) / sc->nn_out_scale);
 }
 
-// the correction at fine cell (i, j): bilinear prolongation of the network
-// output (channel 0 of 16 on the grid F times coarser) times out_scale
-__device__ __forceinline__ float nn_corr_at(const float* __restrict__ y, int nx, int ny, int F,
-                                            double out_scale, int i, int j) {
+// The correction at four columns j .. j + 3 of fine row i (ny is a multiple of
+// 16): bilinear prolongation of the network output (channel 0 of 16 on the
+// grid F times coarser) times out_scale, the product in double-FP32 (hi, lo: an
+// FP64 product and two conversions a cell set the kernel's time).
+__device__ __forceinline__ float4 nn_corr4(const float* __restrict__ y, int nx, int ny, int F,
+                                           float hi, float lo, int i, int j) {
   const int h = nx / F, w = ny / F;
-  const float xi = (i + 0.5f) / F - 0.5f, xj = (j + 0.5f) / F - 0.5f;
-  int i0 = (int)floorf(xi), j0 = (int)floorf(xj);
-  const float ti = xi - i0, tj = xj - j0;
-  const int i1 = min(max(i0 + 1, 0), h - 1), j1 = min(max(j0 + 1, 0), w - 1);
+  const float xi = (i + 0.5f) / F - 0.5f;
+  int i0 = (int)floorf(xi);
+  const float ti = xi - i0;
+  const int i1 = min(max(i0 + 1, 0), h - 1);
   i0 = min(max(i0, 0), h - 1);
-  j0 = min(max(j0, 0), w - 1);
-  const float v00 = y[((long)i0 * w + j0) * 16], v01 = y[((long)i0 * w + j1) * 16];
-  const float v10 = y[((long)i1 * w + j0) * 16], v11 = y[((long)i1 * w + j1) * 16];
-  const float v = (1.f - ti) * ((1.f - tj) * v00 + tj * v01) + ti * ((1.f - tj) * v10 + tj * v11);
-  return (float)(v * out_scale);
+  float v00 = 0.f, v01 = 0.f, v10 = 0.f, v11 = 0.f, o[4];
+  int have = -2;   // the window column that the four values belong to
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float xj = (j + q + 0.5f) / F - 0.5f;
+    const int jf = (int)floorf(xj);
+    const float tj = xj - jf;
+    if (jf != have) {
+      const int j1 = min(max(jf + 1, 0), w - 1), j0 = min(max(jf, 0), w - 1);
+      v00 = y[((long)i0 * w + j0) * 16], v01 = y[((long)i0 * w + j1) * 16];
+      v10 = y[((long)i1 * w + j0) * 16], v11 = y[((long)i1 * w + j1) * 16];
+      have = jf;
+    }
+    const float v = (1.f - ti) * ((1.f - tj) * v00 + tj * v01) + ti * ((1.f - tj) * v10 + tj * v11);
+    const float p = v * hi;
+    o[q] = p + fmaf(v, lo, fmaf(v, hi, -p));
+  }
+  return make_float4(o[0], o[1], o[2], o[3]);
 }
 
 // state += the correction, added to the double-FP32 state (hi: N floats, lo:
-// N floats) with Knuth's TwoSum; the outlet row stays pinned at 0
-__global__ void k_nn_apply(const float* __restrict__ y, int nx, int ny, int F,
-                           float* __restrict__ state, const DevScalars* sc) {
+// N floats) with Knuth's TwoSum; the outlet row stays pinned at 0.  2048x512,
+// cold: 9.1 us with a cell a thread and its FP64 product -> 6.0.
+__global__ void __launch_bounds__(256) k_nn_apply(const float* __restrict__ y, int nx, int ny,
+                                                  int F, float* __restrict__ state,
+                                                  const DevScalars* sc) {
   pdl_wait();
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= nx - 1 || j >= ny) return;
   const long N = (long)nx * ny;
-  const long k = (long)i * ny + j;
-  const float c = nn_corr_at(y, nx, ny, F, sc->nn_out_scale, i, j);
-  const float hi = state[k], lo = state[N + k];
-  const float s = hi + c, bb = s - hi;
-  const float e = (hi - (s - bb)) + (c - bb) + lo;
-  const float s2 = s + e;
-  state[k] = s2;
-  state[N + k] = e - (s2 - s);
+  float4* hp = reinterpret_cast<float4*>(state + (long)i * ny + j);
+  float4* lp = reinterpret_cast<float4*>(state + N + (long)i * ny + j);
+  float4 hi = *hp, lo = *lp;
+  const float4 c = nn_corr4(y, nx, ny, F, sc->nn_os_hi, sc->nn_os_lo, i, j);
+  auto add = [](float& h, float& l, float c) {
+    const float s = h + c, bb = s - h;
+    const float e = (h - (s - bb)) + (c - bb) + l;
+    h = s + e;
+    l = e - (h - s);
+  };
+  add(hi.x, lo.x, c.x);
+  add(hi.y, lo.y, c.y);
+  add(hi.z, lo.z, c.z);
+  add(hi.w, lo.w, c.w);
+  *hp = hi;
+  *lp = lo;
 }
 
 // p0 = p_prev + the correction in FP32 (aj_nn_warmstart); the outlet row is
@@ -1461,11 +1606,14 @@ __global__ void k_nn_apply_guess(const float* __restrict__ y, int nx, int ny, in
                                  const float* __restrict__ pp, float* __restrict__ p0,
                                  const DevScalars* sc) {
   pdl_wait();
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= nx || j >= ny) return;
   const long k = (long)i * ny + j;
-  p0[k] = i == nx - 1 ? 0.f : pp[k] + nn_corr_at(y, nx, ny, F, sc->nn_out_scale, i, j);
+  const float4 c = nn_corr4(y, nx, ny, F, sc->nn_os_hi, sc->nn_os_lo, i, j);
+  const float v[4] = {c.x, c.y, c.z, c.w};   // (pp and p0 are the caller's: any alignment)
+#pragma unroll
+  for (int q = 0; q < 4; ++q) p0[k + q] = i == nx - 1 ? 0.f : pp[k + q] + v[q];
 }
 
 // [n][h][w][3] -> [n][h][w][16] (zeros beyond the features), four channels a
@@ -1506,11 +1654,21 @@ int nn_features(const AjStepParams& p, void* ws, double* part, const float* b, c
     rs.sc = sc;
     rs.b_out = const_cast<float*>(b);
   }
-  launch_pdl(pdl, k_nn_feat, dim3(cdiv(p.ny, 32), cdiv(p.nx, 8)), blk, 0, st, b, mask, pp, p.nx,
-             p.ny, F, (float)(1.0 / (p.dx * p.dx)), (float)(1.0 / (p.dy * p.dy)), x16, rs);
+  const float ax = (float)(1.0 / (p.dx * p.dx)), ay = (float)(1.0 / (p.dy * p.dy));
+  const dim3 g4(cdiv(p.ny, 128), cdiv(p.nx, 8));
+  uintptr_t bits = 0;   // all but vs, whose rows are not 16-byte strided
+  for (const void* q : {(const void*)b, (const void*)mask, (const void*)pp, (const void*)us,
+                        (const void*)rs.b_out, (const void*)x16})
+    bits |= reinterpret_cast<uintptr_t>(q);
+  if (bits & 15)
+    launch_pdl(pdl, k_nn_feat, dim3(cdiv(p.ny, 32), cdiv(p.nx, 8)), blk, 0, st, b, mask, pp, p.nx,
+               p.ny, F, ax, ay, x16, rs);
+  else if (F == 8) launch_pdl(pdl, k_nn_feat4<8>, g4, blk, 0, st, b, mask, pp, p.nx, p.ny, ax, ay, x16, rs);
+  else if (F == 4) launch_pdl(pdl, k_nn_feat4<4>, g4, blk, 0, st, b, mask, pp, p.nx, p.ny, ax, ay, x16, rs);
+  else launch_pdl(pdl, k_nn_feat4<2>, g4, blk, 0, st, b, mask, pp, p.nx, p.ny, ax, ay, x16, rs);
   const double lx = p.nx * p.dx, ly = p.ny * p.dy, lmin = lx < ly ? lx : ly;
   launch_pdl(pdl, k_nn_scale, dim3(NN_SCALE_BLOCKS), dim3(512), 0, st, x16, (long)h * w, sc,
-             lmin * lmin, part);
+             lmin * lmin / 10.0, part);
   if (normalise)
     launch_pdl(pdl, k_nn_norm, dim3(cdiv((long)h * w, 256)), dim3(256), 0, st, x16, x3,
                (long)h * w, (const DevScalars*)sc);
@@ -1535,7 +1693,7 @@ int nn_correct_state(const AjStepParams& p, const Layout& L, void* ws, const flo
   NnW W{reinterpret_cast<const __nv_bfloat16*>(nn.packed), nn.master};
   rc = nn_forward(1, h, w, W, A, st, false, at<DevScalars>(ws, 0));
   if (rc != AJ_OK) return rc;
-  dim3 blk(32, 8), grd(cdiv(p.ny, 32), cdiv(p.nx, 8));
+  dim3 blk(32, 8), grd(cdiv(p.ny, 128), cdiv(p.nx, 8));
   launch_pdl(true, k_nn_apply, grd, blk, 0, st, (const float*)A.y, p.nx, p.ny, F, state,
              (const DevScalars*)at<DevScalars>(ws, 0));
   return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;
@@ -1667,7 +1825,7 @@ int32_t aj_nn_warmstart(const AjStepParams* prm, const float* rhs, const float* 
   const NnW W{reinterpret_cast<const __nv_bfloat16*>(nn_packed), nn_master};
   rc = nn_forward(1, h, w, W, A, st, false, sc);
   if (rc != AJ_OK) return rc;
-  const dim3 blk(32, 8), grd(cdiv(p.ny, 32), cdiv(p.nx, 8));
+  const dim3 blk(32, 8), grd(cdiv(p.ny, 128), cdiv(p.nx, 8));
   launch_pdl(true, k_nn_apply_guess, grd, blk, 0, st, (const float*)A.y, p.nx, p.ny, F, p_prev, p0,
              (const DevScalars*)sc);
   return cudaGetLastError() == cudaSuccess ? AJ_OK : AJ_ERR_CUDA;

@@ -127,6 +127,38 @@ def test_weight_gradient_ragged_tiles(dev, n, h, w):
         assert _rel(gp[name][1], rp[name][1]) < 1e-4, (name, "b", _rel(gp[name][1], rp[name][1]))
 
 
+@pytest.mark.parametrize("F,nx,ny", [(2, 48, 32), (4, 64, 160), (8, 64, 128), (8, 192, 320)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_features_wide(dev, F, nx, ny, offset):
+    """The features of every factor on partial and whole blocks of 128 columns,
+    with aligned fields and with fields one float off the 16-byte boundary (a
+    cell a thread), against the oracle."""
+    from aerojax_gb300.params import StepConfig
+    from aerojax_gb300.solver import Plan
+    from aerojax_gb300._lib import lib, check
+    import ctypes
+    rng = np.random.default_rng(F + nx)
+    dx, dy = 0.02, 0.03
+    def field(scale):
+        a = (scale * rng.standard_normal((nx, ny))).astype(np.float32)
+        t = torch.zeros(nx * ny + 4, device=dev)[offset:offset + nx * ny]
+        t.copy_(torch.as_tensor(a.ravel()))
+        return a, t
+    (b, tb), (m, tm), (pp, tp) = field(2.0), field(1.0), field(0.1)
+    cfg = StepConfig(nx=nx, ny=ny, dx=dx, dy=dy, nu=1e-3, grid_type="mac", variant="gui",
+                     mg_mode="converge", nn_factor=F)
+    plan = Plan(cfg, dev)
+    h, w = nx // F, ny // F
+    x3 = torch.zeros(h * w * 3, device=dev)
+    st = torch.cuda.current_stream().cuda_stream
+    plan.ws.zero_()
+    check("aj_nn_features", lib().aj_nn_features(
+        ctypes.byref(plan.params), tb.data_ptr(), tm.data_ptr(), tp.data_ptr(), None,
+        x3.data_ptr(), None, plan.ws.data_ptr(), plan.nbytes, st))
+    x, _, _ = N.features(b, m, pp, dx, dy, F)
+    assert _rel(x3.cpu().numpy().reshape(h, w, 3), x[..., :3]) < 1e-4
+
+
 @pytest.mark.parametrize("n,h,w", [(9, 72, 40), (19, 64, 8)])
 def test_batched_convolution_runs(dev, n, h, w):
     """Batches whose layers walk runs of 16x8 tiles: partial tiles in both

@@ -59,6 +59,47 @@ def test_multigrid_parity_bands(cuda_lib, nx, ny, guess):
         assert st["cycles"] == 3 and st["err"] == 0
 
 
+@pytest.mark.parametrize("nx,ny", [(512, 256), (528, 272)])
+def test_mac_step_wide(cuda_lib, nx, ny):
+    """The right-hand side and the correction four columns a thread (from 2^17
+    cells; whole and partial blocks of 128 columns), through a MAC step against
+    the oracle; the fields one float off the 16-byte boundary take the kernels of
+    a cell a thread and give the same bits."""
+    import torch
+    from aerojax_gb300.params import StepConfig
+    from aerojax_gb300.solver import Plan, run_step
+    from oracle import ref_np as R
+    rng = np.random.default_rng(nx)
+    f = lambda n, m, a, s: (a + s * rng.standard_normal((n, m))).astype(np.float32)
+    u, v = f(nx + 1, ny, 1.0, 0.2), f(nx, ny + 1, 0.0, 0.2)
+    mask = (rng.random((nx, ny)) > 0.02).astype(np.float32)
+    cfg = StepConfig(nx=nx, ny=ny, dx=0.02, dy=0.025, nu=1e-3, grid_type="mac", variant="gui",
+                     v_cycles=2, brinkman_eta=1e-3, dt=2e-3)
+    outs = []
+    for off in (0, 1):
+        def place(a):
+            t = torch.zeros(a.size + 4, device="cuda")[off:off + a.size].view(a.shape)
+            t.copy_(torch.as_tensor(a))
+            return t
+        m = place(mask)
+        plan = Plan(cfg, m.device)
+        plan.prepare(m)
+        out = tuple(place(np.zeros(s, np.float32)) for s in ((nx + 1, ny), (nx, ny + 1), (nx, ny)))
+        outs.append([t.clone() for t in run_step(plan, place(u), place(v), m, out=out)])
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+    d = lambda a: a.astype(np.float64)
+    us, vs = R.rk_step_unified_mac(d(u), d(v), 2e-3, 1e-3, 0.02, 0.025, d(mask), U_inf=1.0,
+                                   slip_walls=True, brinkman_eta=1e-3)
+    p = d(outs[0][2].cpu().numpy())
+    dpx = np.zeros((nx + 1, ny))
+    dpx[1:-1] = (p[1:] - p[:-1]) / 0.02
+    dpy = np.zeros((nx, ny + 1))
+    dpy[:, 1:-1] = (p[:, 1:] - p[:, :-1]) / 0.025
+    assert rel(outs[0][0][2:-2, 2:-2], (us - 2e-3 * dpx)[2:-2, 2:-2]) < TOL
+    assert rel(outs[0][1][2:-2, 2:-2], (vs - 2e-3 * dpy)[2:-2, 2:-2]) < TOL
+
+
 @pytest.mark.parametrize("nx,ny", [(7, 6), (31, 246), (160, 247), (309, 40), (611, 493)])
 def test_dynamic_smagorinsky_strips(cuda_lib, nx, ny):
     """The dynamic model's strips of columns (one full, one column more, three)

@@ -742,7 +742,8 @@ int32_t aj_kernel_count(const AjStepParams* prm, int32_t cycles) {
   if (p.mg_mode == AJ_MG_PARITY) {
     n += parity_kernel_count(p, L);
   } else {
-    int body = 2 * L.lc + 1 + (L.ld > 0 ? 2 : 0);               // downs, coarse solve, ups
+    // downs, coarse solve, ups, test
+    int body = 2 * L.lc + 1 + (L.ld > 0 ? 2 : 0) + converge_check_apart(L);
     const int least = converge_inline_cycles(p);                // launched whether needed or not
     n += 2 + (cycles > least ? cycles : least) * body + 1;      // init, resid, loop, out+stats
   }

@@ -15,7 +15,8 @@
 //                      a developed flow it ends in as many cycles as V(2,2)
 //                      with a halo of 3 instead of 5), then p += e, the
 //                      residual r = b - A p for the next iteration, its FP64
-//                      norm, and (last block) the convergence test that sets
+//                      norm, and (k_cv_check, or the last block beside
+//                      other instances) the convergence test that sets
 //                      the while node's condition with cudaGraphSetConditional
 //
 // Precision.  The V-cycle runs in FP32.  The refinement state p and the
@@ -422,6 +423,7 @@ struct CvCheck {
   int max_cycles;
   int use_handle;
   cudaGraphConditionalHandle h;
+  int apart = 0;   // the test runs in a kernel of its own (k_cv_check)
 };
 
 // convergence bookkeeping after a V-cycle (device scalars; one thread).  All
@@ -472,7 +474,7 @@ struct PState {
 
 // level 0: e + P(e_coarse), post-smoothing, p += e (double-FP32, ping-pong), the
 // residual of the reference operator for the next iteration (double-FP32), its
-// FP64 norm, and the convergence test in the last block to finish.  The
+// FP64 norm, and the convergence test (k_cv_check, or the last block).  The
 // residual ping-pongs with the pressure (rs.a pairs with ps.a): a block reads
 // the current residual over its region while its neighbours write the next
 // one, so the two must never share a buffer.  The pressure of the region goes
@@ -582,6 +584,7 @@ __global__ void __launch_bounds__(32 * G, CP_THREADS_SM / (32 * G)) k_cv_up0(
   const df total = sum_lanes<32>(t.tx < G ? ws[t.tx] : df{0.f, 0.f});
   if (t.tx == 0) {
     atomicAdd(&sc->acc[0], (double)total.hi + (double)total.lo);
+    if (ck.apart) return;
     __threadfence();
     if (atomicAdd(&sc->red_count, 1u) == gridDim.x * gridDim.y - 1) {
       __threadfence();
@@ -590,6 +593,15 @@ __global__ void __launch_bounds__(32 * G, CP_THREADS_SM / (32 * G)) k_cv_up0(
       cv_check_body(sc, ck);
     }
   }
+}
+
+// the convergence test of a cycle whose k_cv_up0 left it out; nothing to do
+// where the target was met before the cycle (k_cv_up0 ended the loop itself)
+__global__ void k_cv_check(DevScalars* sc, CvCheck ck) {
+  pdl_wait();
+  if (sc->mg_done) return;
+  sc->pcur = 1 - sc->pcur;
+  cv_check_body(sc, ck);
 }
 
 struct CvBlock {
@@ -1396,6 +1408,16 @@ static void level_up(const CvLvl& c, const Layout& L, void* ws, int l, const int
 }
 
 // one refinement iteration
+// Whether a cycle's test has a kernel of its own.  In the last block of
+// k_cv_up0 it makes every block wait at its end for a fence and a counter, and
+// the next cycle for that block's chain.  Four cycles in line, us, in the last
+// block -> apart: 256x64 80.7 -> 80.3, 512x128 86.7 -> 82.4, 1024x256 99.0 ->
+// 94.9, 2048x512 163 -> 160, 4096x1024 386 -> 377, 4096x2048 641 -> 632.  Beside
+// other instances (crowd) the extra launch costs what it saves.  (The sums on
+// 64 addresses instead of one: slower, 1024x256 103, 4096x2048 638 - the FP64
+// sum of the 64 outweighs the atomics.)
+int converge_check_apart(const Layout& L) { return L.crowd <= 1.f; }
+
 static void cv_body(const AjStepParams& p, const Layout& L, void* ws,
                     cudaGraphConditionalHandle h, int use_handle, cudaStream_t st) {
   DevScalars* sc = at<DevScalars>(ws, 0);
@@ -1423,8 +1445,9 @@ static void cv_body(const AjStepParams& p, const Layout& L, void* ws,
     if (sh == 1) level_up<8>(c, L, ws, l, done, st);
     else level_up<12>(c, L, ws, l, done, st);
   }
-  CvCheck ck{p.max_cycles, use_handle, h};
+  const CvCheck ck{p.max_cycles, use_handle, h, converge_check_apart(L)};
   level0_up_s(sh0, p, c0, L, ws, sc, ck, 0, st);
+  if (ck.apart) launch_pdl(true, k_cv_check, dim3(1), dim3(1), 0, st, sc, ck);
 }
 
 // Cycles recorded in line before the while node.  An iteration of the node

@@ -388,6 +388,7 @@ int converge_prepare(const AjStepParams& p, const Layout& L, void* ws, cudaStrea
 int converge_solve(const AjStepParams& p, const Layout& L, void* ws, const float* p0,
                    float* pout, cudaStream_t st, const NnWarm* nn = nullptr,
                    AjStats* stats = nullptr, bool init_done = false);
+int converge_check_apart(const Layout& L);   // 1: a cycle's test is a launch of its own
 int converge_inline_cycles(const AjStepParams& p);   // cycles recorded before the while node
 int converge_init(const AjStepParams& p, const Layout& L, void* ws, const float* p0,
                   cudaStream_t st);

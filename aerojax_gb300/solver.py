@@ -142,11 +142,16 @@ _plan_fields = attrgetter(*(f.name for f in fields(StepConfig) if f.name not in 
 
 
 def get_plan(cfg: StepConfig, device) -> Plan:
+    """The plan of a configuration, kept for later calls.  Configurations that
+    differ in ``dt`` alone share one; it has the dt of the latest call (this
+    one, or run_step's argument)."""
     key = (repr(_plan_fields(cfg)), str(device))
     plan = _PLANS.get(key)
     if plan is None:
         plan = Plan(cfg, device)
         _PLANS[key] = plan
+    elif not cfg.cfl_dt:
+        plan.params.dt = cfg.dt
     return plan
 
 

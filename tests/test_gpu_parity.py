@@ -165,6 +165,39 @@ def test_multigrid_parity_unaligned(cuda_lib):
     assert torch.equal(*out) and float(out[0].abs().max()) > 0
 
 
+@pytest.mark.parametrize("mac", [False, True])
+def test_predictor_takes_each_calls_dt(cuda_lib, mac):
+    """Calls that differ in their time step alone (they share a workspace), there
+    and back, each against the oracle at its own dt."""
+    import aerojax_gb300 as aj
+    from oracle import ref_np as R
+    nx, ny = 66, 38
+    rng = np.random.default_rng(21)
+    f = lambda n, m, a: (a + 0.1 * rng.standard_normal((n, m))).astype(np.float32)
+    u, v = (f(nx + 1, ny, 1.0), f(nx, ny + 1, 0.0)) if mac else (f(nx, ny, 1.0), f(nx, ny, 0.0))
+    mask = np.ones((nx, ny), np.float32)
+    gpu = aj.rk_step_unified_mac if mac else aj.rk_step_unified
+    ref = R.rk_step_unified_mac if mac else R.rk_step_unified
+    d = lambda a: a.astype(np.float64)
+    for dt in (1e-3, 4e-3, 1e-3):
+        got = gpu(T(u), T(v), dt, 4e-3, 1 / 64, 1 / 48, T(mask), brinkman_eta=1e-3)
+        want = ref(d(u), d(v), dt, 4e-3, 1 / 64, 1 / 48, d(mask), brinkman_eta=1e-3)
+        assert rel(got[0], want[0]) < TOL
+        assert rel(got[1], want[1]) < TOL
+
+
+def test_plan_takes_each_configurations_dt(cuda_lib):
+    """A step through get_plan's plan runs with the dt of the configuration asked
+    for, whichever came before it."""
+    import aerojax_gb300 as aj
+    u, v, mask = T(np.ones((64, 48))), T(np.zeros((64, 48))), T(np.ones((64, 48)))
+    for dt in (2e-3, 3e-3, 2e-3):
+        plan = aj.get_plan(aj.StepConfig(nx=64, ny=48, dx=0.02, dy=0.02, nu=1e-3, dt=dt), u.device)
+        plan.prepare(mask)
+        aj.run_step(plan, u, v, mask)
+        assert plan.stats()["dt"] == np.float32(dt)
+
+
 @pytest.mark.parametrize("name", ["rk3", "rk2", "rk3_hyper", "rk3_field"])
 def test_predictor_collocated(cuda_lib, name):
     import aerojax_gb300 as aj

@@ -251,9 +251,10 @@ def rollout_vjp(initial_state: SimState, mask, params: dict, num_steps: int, g_u
     # the two histories as one tensor, where differentiable_rollout made them:
     # one copy stages a step's u and v.  The cotangents stay in place.
     hist = hu._base if hu._base is not None and hu._base is hv._base else None
-    if hist is not None and not (hist.shape == (2, *hu.shape) and
-                                 hist[0].data_ptr() == hu.data_ptr() and
-                                 hist[1].data_ptr() == hv.data_ptr()):
+    same = lambda a, b: (a.dtype == b.dtype and a.shape == b.shape and a.stride() == b.stride()
+                         and a.data_ptr() == b.data_ptr())
+    if hist is not None and not (hist.shape == (2, *hu.shape) and same(hist[0], hu)
+                                 and same(hist[1], hv)):
         hist = None
     for k in range(num_steps - 1, -1, -1):
         if k > 0 and hist is not None:

@@ -140,6 +140,27 @@ def test_rollout_vjp_matches_oracle(dev):
     assert _scalar_ok(got["U_inf"], ref, "U_inf", 2e-4), (got["U_inf"], ref["U_inf"])
 
 
+def test_rollout_vjp_takes_transposed_history(dev):
+    """A history whose rows lie transposed in memory, in one tensor of the shape
+    that differentiable_rollout makes: the same gradient."""
+    from aerojax_gb300 import adjoint as ADJ
+    from aerojax_gb300.params import SimState
+    n = 3
+    u, v, mask, s, rng = _case(64, 64, 17)
+    gu, gv = (_t(rng.standard_normal((64, 64)).astype(np.float32), dev) for _ in range(2))
+    params = {"dx": DX, "dy": DX, "nu": NU, "U_inf": U, "sdf": _t(s, dev)}
+    st = SimState(u=_t(u, dev), v=_t(v, dev), p=None, u_prev=None, v_prev=None, c=None, dt=DT,
+                  iteration=0)
+    m = _t(mask, dev)
+    _, (hu, hv) = ADJ.differentiable_rollout(st, m, params, n)
+    other = torch.stack([hu, hv]).transpose(2, 3).contiguous()
+    want = ADJ.rollout_vjp(st, m, params, n, gu, gv, history=(hu, hv))
+    got = ADJ.rollout_vjp(st, m, params, n, gu, gv,
+                          history=(other[0].transpose(1, 2), other[1].transpose(1, 2)))
+    for k in ("u", "v", "sdf"):
+        assert torch.equal(got[k], want[k]), k
+
+
 @pytest.mark.parametrize("fast,hyper,slip,use_sdf,cycles", [
     (False, 0.05, True, True, 2), (True, 0.0, False, True, 1), (False, 0.05, False, False, 5)])
 def test_gui_step_vjp_matches_oracle(dev, fast, hyper, slip, use_sdf, cycles):

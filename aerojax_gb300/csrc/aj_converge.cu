@@ -577,13 +577,14 @@ __global__ void __launch_bounds__(32 * G, CP_THREADS_SM / (32 * G)) k_cv_up0(
   }
   if (profile) return;
   __shared__ df ws[G];
-  const df s = sum_lanes<32>(df{acc, 0.f});
+  const df s = warp_sum_df(df{acc, 0.f});
   if (t.tx == 0) ws[t.ty] = s;
   __syncthreads();
   if (t.ty > 0) return;
-  const df total = sum_lanes<32>(t.tx < G ? ws[t.tx] : df{0.f, 0.f});
+  static_assert(G <= 16, "half a warp adds the warps");
+  const double total = warp_sum<16>(t.tx < G ? df_double(ws[t.tx]) : 0.0);
   if (t.tx == 0) {
-    atomicAdd(&sc->acc[0], (double)total.hi + (double)total.lo);
+    atomicAdd(&sc->acc[0], total);
     if (ck.apart) return;
     __threadfence();
     if (atomicAdd(&sc->red_count, 1u) == gridDim.x * gridDim.y - 1) {

@@ -123,8 +123,10 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned int* addr, float v) {
   atomicMax(addr, __float_as_uint(v));
 }
 
+template <int LANES = 32>
 __device__ __forceinline__ double warp_sum(double v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
@@ -190,36 +192,32 @@ __device__ __forceinline__ df df_add(df a, df b) {
   return quick_two_sum(s.hi, s.lo);
 }
 
-// Sums as (hi, lo) pairs whose lo collects the TwoSum errors of hi: a third of
-// df_add's operations where terms of one sign are added (and FP64 runs at
-// 1/64 of the FP32 rate); the sum of LANES neighbouring lanes in each of them
-__device__ __forceinline__ df sum_add(df a, df b) {
-  const df t = two_sum(a.hi, b.hi);
-  return {t.hi, t.lo + (a.lo + b.lo)};
-}
-template <int LANES>
-__device__ __forceinline__ df sum_lanes(df s) {
-#pragma unroll
-  for (int o = LANES / 2; o > 0; o >>= 1)
-    s = sum_add(s, df{__shfl_xor_sync(~0u, s.hi, o), __shfl_xor_sync(~0u, s.lo, o)});
-  return s;
-}
-
-// Block-wide sum of one double-FP32 value per thread, in a fixed order (the
-// result is bit-reproducible): a TwoSum butterfly inside each warp, one FP64
-// value per warp, the warps summed by thread 0, which gets the total.  Every
-// thread of the block must call it (it synchronises).
-__device__ __forceinline__ double block_sum_df(df v) {
-  __shared__ double wd_[32];
+// The warp's sum of one double-FP32 value per lane, in every lane: a TwoSum
+// butterfly.  What is added further, warps and blocks, is added in FP64
+// (df_double, by one warp: conversions and additions run at 1/64 of the FP32
+// rate): with pairs of FP32 numbers to the end, their low word not even
+// renormalised, the norms' largest error was 6e-15 relative, so it is 2e-15
+// (blocks of 8 to 32 warps, random fields).
+__device__ __forceinline__ df warp_sum_df(df v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float h = __shfl_xor_sync(0xffffffffu, v.hi, o);
     const float l = __shfl_xor_sync(0xffffffffu, v.lo, o);
     v = df_add(v, df{h, l});
   }
+  return v;
+}
+__device__ __forceinline__ double df_double(df v) { return (double)v.hi + (double)v.lo; }
+
+// Block-wide sum of one double-FP32 value per thread, in a fixed order (the
+// result is bit-reproducible): the warps' sums added by thread 0, which gets
+// the total.  Every thread of the block must call it (it synchronises).
+__device__ __forceinline__ double block_sum_df(df v) {
+  __shared__ double wd_[32];
+  v = warp_sum_df(v);
   const int nthreads = blockDim.x * blockDim.y;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-  if ((tid & 31) == 0) wd_[tid >> 5] = (double)v.hi + (double)v.lo;
+  if ((tid & 31) == 0) wd_[tid >> 5] = df_double(v);
   __syncthreads();
   double t = 0.0;
   if (tid == 0)

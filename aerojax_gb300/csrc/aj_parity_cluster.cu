@@ -119,8 +119,9 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
   const int rank = (int)cl.block_rank(), C = (int)cl.num_blocks();
   cl.barrier_arrive();             // no remote store before every block has started
   extern __shared__ __align__(16) float pcs[];
-  __shared__ df nrm[2 * PC_MAX_CTAS];
+  __shared__ double nrm[2 * PC_MAX_CTAS];
   __shared__ df wsum[2 * PC_WARPS];
+  __shared__ double sq[2];   // sum r^2 and sum b^2
   __shared__ int stop;
   const int lt = a.lt, nl = a.nl, tid = threadIdx.x;
   auto r0 = [&](int l) { return rank * a.lv[l].R; };
@@ -145,7 +146,6 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
   __syncthreads();
   cl.barrier_wait();
   int cycles = 0;
-  double rsq = 0.0, bsq = 0.0;   // thread 0: sum r^2 and sum b^2
   for (int cyc = 0; cyc < a.cycles; ++cyc) {
     // down: two pre-sweeps (the second resets the outlet row), the residual
     // and its 2x2 average onto the coarser level
@@ -301,35 +301,26 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
       });
     }
     if (!a.whole) break;   // the coarsest level alone
-    // the early-exit test, the blocks' sums added by every block alike
-    // (FP32 pairs throughout: FP64 runs at 1/64 of the FP32 rate, and 512
-    // threads adding doubles took 7 us a cycle)
-    rr = sum_lanes<32>(rr);
-    if (cyc == 0) bb = sum_lanes<32>(bb);
-    if ((tid & 31) == 0) {
-      wsum[tid >> 5] = rr;
-      wsum[PC_WARPS + (tid >> 5)] = bb;
+    // the early-exit test, the blocks' sums added by every block alike (FP64
+    // in one warp only: it runs at 1/64 of the FP32 rate)
+#pragma unroll 1
+    for (int q = 0; q < (cyc == 0 ? 2 : 1); ++q) {
+      const df s = warp_sum_df(q ? bb : rr);
+      if ((tid & 31) == 0) wsum[q * PC_WARPS + (tid >> 5)] = s;
     }
     __syncthreads();
-    if (tid < 32) {   // the warps' sums; lane q files the block's in block q
-      rr = sum_lanes<32>(wsum[tid]);
-      if (cyc == 0) bb = sum_lanes<32>(wsum[PC_WARPS + tid]);
-      if (tid < C) {
-        df* d = cl.map_shared_rank(nrm, tid);
-        d[rank] = rr;
-        d[PC_MAX_CTAS + rank] = bb;
-      }
+    // the residual's by warp 0, b's by warp 1 (first cycle)
+    const int which = tid >> 5, lane = tid & 31;
+    const bool adds = tid < (cyc == 0 ? 64 : 32);
+    if (adds) {   // the warps' sums; lane q files the block's in block q
+      const double t = warp_sum(df_double(wsum[tid]));
+      if (lane < C) cl.map_shared_rank(nrm, lane)[which * PC_MAX_CTAS + rank] = t;
     }
     cl.sync();
-    if (tid < 32) {
-      const df t = sum_lanes<PC_MAX_CTAS>(tid < C ? nrm[tid] : df{0.f, 0.f});
-      if (cyc == 0)
-        bb = sum_lanes<PC_MAX_CTAS>(tid < C ? nrm[PC_MAX_CTAS + tid] : df{0.f, 0.f});
-      if (tid == 0) {
-        if (cyc == 0) bsq = (double)bb.hi + (double)bb.lo;
-        rsq = (double)t.hi + (double)t.lo;
-        stop = rsq * a.dxdy < a.tol2;
-      }
+    if (adds) {
+      const double t = warp_sum<PC_MAX_CTAS>(lane < C ? nrm[which * PC_MAX_CTAS + lane] : 0.0);
+      if (lane == 0) sq[which] = t;
+      if (tid == 0) stop = t * a.dxdy < a.tol2;
     }
     cycles = cyc + 1;
     __syncthreads();
@@ -343,6 +334,7 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_par_cluster(const __grid_cons
   if (a.whole && rank == 0 && tid == 0) {
     DevScalars* sc = a.sc;
     const float dt = sc->dt;
+    const double rsq = sq[0], bsq = sq[1];
     const int conv = stop, err = isfinite(rsq) ? AJ_OK : AJ_ERR_NONFINITE;
     const double bnorm = sqrt(bsq), abs_sq = rsq * a.dxdy;
     const double rel = bnorm > 0.0 ? sqrt(rsq) / bnorm : sqrt(rsq);

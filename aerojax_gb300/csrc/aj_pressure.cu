@@ -367,28 +367,31 @@ __global__ void __launch_bounds__(32 * G, 1024 / (32 * G)) k_par_up(ParTile a) {
   if constexpr (NORM) {
     pair_store<PT_RUN>(geo, o, A, x);
     __syncthreads();
-    df rr{0.f, 0.f}, bb{0.f, 0.f};
-    if (o.mine)
-      pair_resid<PT_RUN>(a.co, geo, o, A, b, outlet, x, [&](int r, float2 v) {
-        // (b - A p) in FP32 as the reference evaluates it; its square exactly
-        rr = pair_add_sq(rr, v);
-        if (a.also_b) bb = pair_add_sq(bb, b[r]);
-      });
     __shared__ df ws[2 * G];
-    rr = sum_lanes<32>(rr);
-    if (a.also_b) bb = sum_lanes<32>(bb);
-    if (threadIdx.x == 0) {
-      ws[threadIdx.y] = rr;
-      ws[G + threadIdx.y] = bb;
+    df s{0.f, 0.f};
+    if (o.mine)
+      pair_resid<PT_RUN>(a.co, geo, o, A, b, outlet, x, [&](int, float2 v) {
+        // (b - A p) in FP32 as the reference evaluates it; its square exactly
+        s = pair_add_sq(s, v);
+      });
+    s = warp_sum_df(s);
+    if (threadIdx.x == 0) ws[threadIdx.y] = s;
+    if (a.also_b) {
+      s = df{0.f, 0.f};
+#pragma unroll
+      for (int r = 0; r < PT_RUN; ++r)
+        if (o.mine && r < o.cnt) s = pair_add_sq(s, b[r]);
+      s = warp_sum_df(s);
+      if (threadIdx.x == 0) ws[G + threadIdx.y] = s;
     }
     __syncthreads();
     if (threadIdx.y > 0) return;
     const int l = threadIdx.x;
-    rr = sum_lanes<G>(ws[l % G]);
-    if (a.also_b) bb = sum_lanes<G>(ws[G + l % G]);
+    const double tr = warp_sum<G>(df_double(ws[l % G])),
+                 tb = a.also_b ? warp_sum<G>(df_double(ws[G + l % G])) : 0.0;
     if (l == 0) {
-      atomicAdd(&a.sc->acc[0], (double)rr.hi + (double)rr.lo);
-      if (a.also_b) atomicAdd(&a.sc->acc[1], (double)bb.hi + (double)bb.lo);
+      atomicAdd(&a.sc->acc[0], tr);
+      if (a.also_b) atomicAdd(&a.sc->acc[1], tb);
       __threadfence();
       // every block's sums are in: the early-exit test
       if (atomicAdd(&a.sc->red_count, 1u) == gridDim.x * gridDim.y - 1) {

@@ -198,6 +198,21 @@ def test_plan_takes_each_configurations_dt(cuda_lib):
         assert plan.stats()["dt"] == np.float32(dt)
 
 
+@pytest.mark.parametrize("nx,ny,step,count", [(288, 48, 16, 17), (448, 304, 4, 6)])
+@pytest.mark.parametrize("mac", [False, True])
+def test_rhs_norm_is_a_double_sum(cuda_lib, nx, ny, step, count, mac):
+    """The V-cycle's norms (the whole solve on the cluster; one block of the tiled
+    level-0 kernel) are FP64 sums of the warps' totals: 1, 2^-24 and a few times
+    2^-52 from as many warps add up without a rounding, which a pair of FP32
+    numbers cannot hold."""
+    import aerojax_gb300 as aj
+    rhs = np.zeros((nx, ny), np.float32)
+    rhs[step * np.arange(count), 5] = [1.0, 2.0 ** -12] + [2.0 ** -26] * (count - 2)
+    fn = aj.poisson_multigrid_mac if mac else aj.poisson_multigrid
+    _, st = fn(T(rhs), T(np.ones((nx, ny))), 0.02, 0.025, v_cycles=1, return_stats=True)
+    assert st["rhs_norm"] == np.sqrt(1.0 + 2.0 ** -24 + (count - 2) * 2.0 ** -52)
+
+
 @pytest.mark.parametrize("name", ["rk3", "rk2", "rk3_hyper", "rk3_field"])
 def test_predictor_collocated(cuda_lib, name):
     import aerojax_gb300 as aj

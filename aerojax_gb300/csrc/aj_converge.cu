@@ -1661,7 +1661,7 @@ int profile_pressure_kernel(const AjStepParams& p, const Layout& L, void* ws, in
                             cudaStream_t st) {
   if (p.mg_mode != AJ_MG_CONVERGE) return AJ_ERR_PARAM;
   DevScalars* sc = at<DevScalars>(ws, 0);
-  const int* never = reinterpret_cast<const int*>(&sc->pad_[0]);   // always 0
+  const int* never = reinterpret_cast<const int*>(&sc->zero);
   CvLvl c = cv_level(p, L, 0);
   const int sh = variant_shape(tile_variant(p.nx, p.ny), c);
   if (which == 0) {
@@ -1714,7 +1714,7 @@ int converge_autotune(const AjStepParams& p, const Layout& L, void* ws, int reps
                       int* chosen, cudaStream_t st) {
   if (p.mg_mode != AJ_MG_CONVERGE) return AJ_ERR_PARAM;
   DevScalars* sc = at<DevScalars>(ws, 0);
-  const int* never = reinterpret_cast<const int*>(&sc->pad_[0]);   // always 0
+  const int* never = reinterpret_cast<const int*>(&sc->zero);
   const CvLvl c = cv_level(p, L, 0);
   const CvCheck ck{p.max_cycles, 0, 0};
   cudaEvent_t e0, e1;

@@ -39,7 +39,7 @@ struct DevScalars {
   float dt_prev;       // dt of the latest solution in the history
   float nn_ir, nn_ip;  // learned warm start: 1 / nn_rms_r, 1 / nn_rms_p
   float nn_os_hi, nn_os_lo;   // nn_out_scale as two floats
-  unsigned int pad_[1];
+  unsigned int zero;          // always 0, written by no kernel
 };
 
 struct Layout {

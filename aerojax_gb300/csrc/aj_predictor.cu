@@ -59,11 +59,11 @@ int launch_set_dt(const AjStepParams& p, void* ws, cudaStream_t st) {
 // stage writes it for the kernels after it.
 struct StageDt {
   DevScalars* write = nullptr;   // first stage of a fixed-dt step
-  const DevScalars* sc = nullptr;
+  const float* src = nullptr;    // the device's dt; when known, a word that nothing writes
   float dt = 0.f, dtc = 0.f;
   int known = 0;
 };
-__device__ __forceinline__ float stage_dt(const StageDt& d) { return d.known ? d.dt : d.sc->dt; }
+__device__ __forceinline__ float stage_dt(const StageDt& d) { return d.known ? d.dt : *d.src; }
 // (the large kernels do it on their edge blocks' branch: before the loads it
 // cost the staggered upwind stages at 4096x2048 223 -> 281 us)
 __device__ __forceinline__ void stage_dt_write(const StageDt& d) {
@@ -1488,10 +1488,11 @@ __global__ void __launch_bounds__(256, MacRows<ADV>::BLOCKS) k_rk_mac_rows(RkMac
   using M = MacRows<ADV>;
   constexpr int HB = M::HB, R = M::R;
   const int nx = a.nx, ny = a.ny, nyv = ny + 1;
-  // upwind reads the device's dt even where it is not used: without that read
-  // the compiler orders the loads after it differently, and three stages at
+  // upwind reads src even where the host knows dt (src is then not the scalars'
+  // dt, which the first stage's edge block writes): without that read the
+  // compiler orders the loads after it differently, and three stages at
   // 4096x2048 take 285 us instead of 223
-  const float read = ADV == AJ_ADV_WENO5 ? 0.f : a.dt.sc->dt;
+  const float read = ADV == AJ_ADV_WENO5 ? 0.f : *a.dt.src;
   const float dt = ADV == AJ_ADV_WENO5 ? stage_dt(a.dt) : (a.dt.known ? a.dt.dt : read);
   const int edge = M::edge_blocks(nx, ny);
   if ((int)blockIdx.x < edge) {
@@ -1607,8 +1608,9 @@ int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const flo
                      const float* v, const float* mask, const float* nsg, int double_count,
                      float* us, float* vs, cudaStream_t st, DtFrom dt) {
   StageDt sdt;
-  sdt.sc = at<DevScalars>(ws, 0);
   sdt.known = dt != DtFrom::device;
+  DevScalars* sc = at<DevScalars>(ws, 0);
+  sdt.src = sdt.known ? reinterpret_cast<const float*>(&sc->zero) : &sc->dt;
   sdt.dt = (float)p.dt;
   sdt.dtc = (float)p.dt_correction;
   const int nx = p.nx, ny = p.ny;
@@ -1650,7 +1652,7 @@ int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const flo
     for (int s = 1; s <= nstage; ++s) {
       a.stage = s;
       a.dt = sdt;
-      if (s == 1 && dt == DtFrom::host) a.dt.write = at<DevScalars>(ws, 0);
+      if (s == 1 && dt == DtFrom::host) a.dt.write = sc;
       a.uin = in_u;
       a.vin = in_v;
       bool last = s == nstage;
@@ -1696,7 +1698,7 @@ int launch_predictor(const AjStepParams& p, const Layout& L, void* ws, const flo
     for (int s = 1; s <= nstage; ++s) {
       a.stage = s;
       a.dt = sdt;
-      if (s == 1 && dt == DtFrom::host) a.dt.write = at<DevScalars>(ws, 0);
+      if (s == 1 && dt == DtFrom::host) a.dt.write = sc;
       a.uin = in_u;
       a.vin = in_v;
       bool last = s == nstage;

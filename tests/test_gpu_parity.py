@@ -213,6 +213,26 @@ def test_rhs_norm_is_a_double_sum(cuda_lib, nx, ny, step, count, mac):
     assert st["rhs_norm"] == np.sqrt(1.0 + 2.0 ** -24 + (count - 2) * 2.0 ** -52)
 
 
+@pytest.mark.parametrize("nx,ny", [(2048, 512), (64, 8192), (64, 32768)])
+def test_multigrid_parity_wide_coarsest(cuda_lib, nx, ny):
+    """Two levels below the finest on grids whose coarsest bands do not fit the
+    V-cycle's cluster: the coarsest sweeps on a cluster of their own, and, where
+    not even that holds them (64x32768), a launch a sweep."""
+    import aerojax_gb300 as aj
+    from oracle import ref_np as R
+    rng = np.random.default_rng(nx + ny)
+    dx, dy = 0.02, 0.025
+    rhs = rng.standard_normal((nx, ny)).astype(np.float32)
+    mask = (rng.random((nx, ny)) > 0.05).astype(np.float32)
+    d = lambda a: a.astype(np.float64)
+    for mac in (False, True):
+        fn = aj.poisson_multigrid_mac if mac else aj.poisson_multigrid
+        p, st = fn(T(rhs), T(mask), dx, dy, levels=2, v_cycles=2, return_stats=True)
+        ref = R.poisson_multigrid(d(rhs), d(mask), dx, dy, levels=2, v_cycles=2, mac=mac)
+        assert rel(p, ref) < TOL, (mac, rel(p, ref))
+        assert st["cycles"] == 2 and st["err"] == 0
+
+
 @pytest.mark.parametrize("name", ["rk3", "rk2", "rk3_hyper", "rk3_field"])
 def test_predictor_collocated(cuda_lib, name):
     import aerojax_gb300 as aj

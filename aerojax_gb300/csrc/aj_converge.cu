@@ -1424,10 +1424,10 @@ static void cv_body(const AjStepParams& p, const Layout& L, void* ws,
   DevScalars* sc = at<DevScalars>(ws, 0);
   const int* done = &sc->mg_done;
   const int lc = L.lc;
-  // level 0: the autotuned shape, but beside other instances the rule's
+  // level 0: the shape that the autotuner took instead of the rule's, or the rule's
   const CvLvl c0 = cv_level(p, L, 0);
-  const int sh0 = L.crowd > 1.f ? cv_shape(c0.n, c0.m, L.crowd)
-                                : variant_shape(tile_variant(p.nx, p.ny), c0);
+  const int tuned = tile_variant(p.nx, p.ny);
+  const int sh0 = tuned ? variant_shape(tuned, c0) : cv_shape(c0.n, c0.m, L.crowd);
   for (int l = 0; l < lc; ++l) {
     CvLvl c = cv_level(p, L, l);
     const int sh = cv_shape(c.n, c.m, L.crowd);

@@ -9,7 +9,8 @@ converging multigrid to a 1e-6 relative residual.  Each instance is the
 collocated step_pure step (solver/pure_functions/step.py:49-467) of the
 cylinder channel (grid spacing 1/64, inlet U = 1, slip walls), the flow of
 solver/params.py:308-413's presets at its Re.  The level-0 multigrid tile
-shape of every grid size comes from the autotuner (aj_autotune).
+shape of every grid size comes from the autotuner (aj_autotune), or, where that
+finds no faster one than the default, from the rule for instances side by side.
 """
 from __future__ import annotations
 

@@ -360,9 +360,11 @@ int32_t aj_release_graphs(void);
    (converging mode, after aj_prepare on this workspace): times each
    candidate `reps` times (level-0 pre- and post-smoothing kernels on the
    workspace's current contents), keeps the fastest for every later call on
-   this grid shape in this process, and returns the per-candidate times (host
-   array of AJ_TILE_VARIANTS floats, ms, nullable) and the choice (host,
-   nullable).  Synchronises the stream.  No reference counterpart. */
+   this grid shape in this process (an ensemble's instances too, unless the
+   default is the fastest: their default goes by what runs beside them), and
+   returns the per-candidate times (host array of AJ_TILE_VARIANTS floats, ms,
+   nullable) and the choice (host, nullable).  Synchronises the stream.  No
+   reference counterpart. */
 #define AJ_TILE_VARIANTS 3
 int32_t aj_autotune(const AjStepParams* prm, void* workspace, size_t workspace_bytes,
                     int32_t reps, float* times_ms, int32_t* chosen, void* stream);

@@ -78,27 +78,6 @@ __device__ __forceinline__ df df_mul(df a, df b) {
   p.lo += a.hi * b.lo + a.lo * b.hi;
   return quick_two_sum(p.hi, p.lo);
 }
-__device__ __forceinline__ df df_add_f(df a, float b) {
-  df s = two_sum(a.hi, b);
-  s.lo += a.lo;
-  return quick_two_sum(s.hi, s.lo);
-}
-// Dekker's addition with one TwoSum: error <= ~2^-47 max(|a|, |b|), which in
-// the residual below stays ~1e-14 |p| ax, far under the 1e-6 |b| targets
-__device__ __forceinline__ df df_add_s(df a, df b) {
-  df s = two_sum(a.hi, b.hi);
-  s.lo += a.lo + b.lo;
-  return quick_two_sum(s.hi, s.lo);
-}
-// r = b - (ax ((xp + xm) - 2c) + ay ((yp + ym) - 2c)), all double-FP32 (-2c is
-// exact, so each second difference costs two additions, not three)
-__device__ __forceinline__ df df_residual(float b, df c, df xp, df xm, df yp, df ym, df ax, df ay) {
-  const df c2{-2.f * c.hi, -2.f * c.lo};
-  const df sx = df_add_s(df_add_s(xp, xm), c2);
-  const df sy = df_add_s(df_add_s(yp, ym), c2);
-  const df ap = df_add_s(df_mul(ax, sx), df_mul(ay, sy));
-  return df_add_f(df_neg(ap), b);
-}
 
 // ---------------------------------------------------------------- paired double-FP32
 // Two double-FP32 values side by side (a thread's two columns of a tile row)
@@ -116,12 +95,14 @@ __device__ __forceinline__ df2 quick_two_sum2(float2 a, float2 b) {
   const float2 s = add2(a, b);
   return {s, sub2(b, sub2(s, a))};
 }
-__device__ __forceinline__ df2 df2_add_s(df2 a, df2 b) {   // as df_add_s
+// Dekker's addition with one TwoSum: error <= ~2^-47 max(|a|, |b|), which in
+// the residual below stays ~1e-14 |p| ax, far under the 1e-6 |b| targets
+__device__ __forceinline__ df2 df2_add_s(df2 a, df2 b) {
   df2 s = two_sum2(a.hi, b.hi);
   s.lo = add2(s.lo, add2(a.lo, b.lo));
   return quick_two_sum2(s.hi, s.lo);
 }
-__device__ __forceinline__ df2 df2_add_f(df2 a, float2 b) {   // as df_add_f
+__device__ __forceinline__ df2 df2_add_f(df2 a, float2 b) {
   df2 s = two_sum2(a.hi, b);
   s.lo = add2(s.lo, a.lo);
   return quick_two_sum2(s.hi, s.lo);
@@ -135,15 +116,15 @@ __device__ __forceinline__ df2 df2_mul_u(df a, df2 b) {
   const float2 cross = __ffma2_rn(ah, b.lo, __fmul2_rn(f2(a.lo), b.hi));
   return quick_two_sum2(p, sub2(cross, en));
 }
-// b - a: df_add_f(df_neg(a), b) with the signs carried through (negation
-// is exact, so every rounding is the scalar form's)
+// b - a: TwoSum of b and -a.hi with the signs carried through
 __device__ __forceinline__ df2 df2_rsub_f(float2 b, df2 a) {
   const float2 s = sub2(b, a.hi);
   const float2 bb = add2(s, a.hi);
   const float2 e = sub2(sub2(b, bb), add2(a.hi, sub2(s, bb)));
   return quick_two_sum2(s, sub2(e, a.lo));
 }
-// df_residual for two cells
+// r = b - (ax ((xp + xm) - 2c) + ay ((yp + ym) - 2c)), all double-FP32 (-2c is
+// exact, so each second difference costs two additions, not three)
 __device__ __forceinline__ df2 df2_residual(float2 b, df2 c, df2 xp, df2 xm, df2 yp, df2 ym,
                                             df ax, df ay) {
   const df2 c2{__fmul2_rn(c.hi, f2(-2.f)), __fmul2_rn(c.lo, f2(-2.f))};
@@ -848,8 +829,9 @@ int converge_direct_level(const Layout& L) {
 // by row products).  16 x 32 output tiles, 2 outputs a thread: at 512 x 128
 // that is 128 blocks, and since the three kernels of this solve are bound by
 // their own latency (one block's staging round, its product and a launch),
-// more and lighter blocks win: 32 x 32 tiles with 4-byte reads took 8 us each
-// cold, 16-byte reads of both panels and of the shared rows 5.2 -> TIME us.
+// more and lighter blocks win: 32 x 32 tiles with 4-byte reads took 8.0 and 8.3
+// us cold, these with 16-byte reads of both panels and of the shared rows 6.6
+// and 6.9.
 // The basis is staged before the wait for the previous kernel.
 constexpr int CV_DI = 16, CV_DC = 32;
 constexpr int CV_DK = CV_DIRECT_MAX_M + 4;   // row stride: 16-byte rows, free of bank conflicts

@@ -31,13 +31,13 @@ struct DevScalars {
   unsigned int red_count;
   int loops;           // converging mode: executions of the while body
   int pcur;            // converging mode: which FP64 pressure buffer is current
-  double nn_rms_r, nn_rms_p, nn_out_scale;   // learned warm start: per-sample scales
+  double nn_out_scale;       // learned warm start: the correction's scale, per sample
   int hist_n;          // converging mode: solutions held in the history (0..2)
   int hist_cur;        // history slot of the latest solution
   int hist_pending;    // a solve finished since the last k_cv_begin
   float dt_last;       // dt of the last finished solve
   float dt_prev;       // dt of the latest solution in the history
-  float nn_ir, nn_ip;  // learned warm start: 1 / nn_rms_r, 1 / nn_rms_p
+  float nn_ir, nn_ip;  // learned warm start: reciprocal RMS of the residual, the pressure
   float nn_os_hi, nn_os_lo;   // nn_out_scale as two floats
   unsigned int zero;          // always 0, written by no kernel
 };
@@ -70,8 +70,6 @@ struct Layout {
   float crowd = 1.f;            // instances of this size running side by side
 };
 
-// Number of dynamic-LES temporaries (nx*ny floats each).
-constexpr int kDynFields = 12;
 constexpr int kPartials = 4096;
 
 bool make_layout(const AjStepParams& p, Layout& L);
@@ -224,32 +222,6 @@ __device__ __forceinline__ double block_sum_df(df v) {
     for (int k = 0; k < (nthreads >> 5); ++k) t += wd_[k];
   __syncthreads();
   return t;
-}
-
-// Block-wide sum of one float per thread added atomically to *dst by one
-// thread: a double-FP32 TwoSum butterfly in each warp (the FP32 pipes; the
-// FP64 butterfly of block_sum_atomic costs ~10 FP64 operations per thread on
-// GB300's 1/64-rate FP64 pipe), one FP64 value per warp.  Every thread of the
-// block must call it (it synchronises).
-__device__ __forceinline__ void block_sum_atomic_f(float v, double* dst) {
-  __shared__ double wf_[32];
-  df s{v, 0.f};
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float h = __shfl_xor_sync(0xffffffffu, s.hi, o);
-    const float l = __shfl_xor_sync(0xffffffffu, s.lo, o);
-    s = df_add(s, df{h, l});
-  }
-  const int nthreads = blockDim.x * blockDim.y;
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-  if ((tid & 31) == 0) wf_[tid >> 5] = (double)s.hi + (double)s.lo;
-  __syncthreads();
-  if (tid == 0) {
-    double t = 0.0;
-    for (int k = 0; k < (nthreads >> 5); ++k) t += wf_[k];
-    atomicAdd(dst, t);
-  }
-  __syncthreads();
 }
 
 // Block-wide sum of one double per thread in a fixed order (the result is

@@ -1493,14 +1493,12 @@ __global__ void __launch_bounds__(512) k_nn_scale(const float* __restrict__ x, l
     if (lane == 0) {
       const double os = r * out_fac;
       const float hi = (float)os;
-      sc->nn_rms_r = r;
       sc->nn_ir = inv;
       sc->nn_out_scale = os;
       sc->nn_os_hi = hi;
       sc->nn_os_lo = (float)(os - (double)hi);
       sc->red_count = 0u;
     } else if (lane == 1) {
-      sc->nn_rms_p = r;
       sc->nn_ip = inv;
     }
   }
@@ -1542,7 +1540,8 @@ __global__ void k_nn_target(const float* __restrict__ pt, const float* __restric
 // The correction at four columns j .. j + 3 of fine row i (ny is a multiple of
 // 16): bilinear prolongation of the network output (channel 0 of 16 on the
 // grid F times coarser) times out_scale, the product in double-FP32 (hi, lo: an
-// FP64 product and two conversions a cell set the kernel's time).
+// FP64 product and two conversions a cell set the kernel's time) and rounded
+// to FP32: the FP64 product's rounding in each of 2e7 random ones.
 __device__ __forceinline__ float4 nn_corr4(const float* __restrict__ y, int nx, int ny, int F,
                                            float hi, float lo, int i, int j) {
   const int h = nx / F, w = ny / F;

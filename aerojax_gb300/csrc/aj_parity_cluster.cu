@@ -8,9 +8,12 @@
 // memory and fills a fraction of the SMs.  Here block k of the cluster keeps
 // a band of rows of every level in shared memory for the whole cycle:
 //   - bands nest: R rows of the coarsest level, 2R of the next finer, ...;
-//   - a level's band carries a halo deep enough (3 rows) that its two sweeps
-//     and the residual are computed redundantly without any exchange, and the
-//     coarsest level's halo (11 rows) covers all of its ten sweeps;
+//   - a level's band carries a halo deep enough that its two sweeps and the
+//     residual (3 rows) are computed redundantly without any exchange, and the
+//     coarsest level's covers its nine sweeps after the first, which starts from
+//     zero, and the two rows that the finer level's prolongation reads (11);
+//     both are kept one row deeper (PC_HALO, PC_HALO_COARSE), even, so that a
+//     2x2 block stays in one thread;
 //   - a block stores what its neighbours' halos need (the restricted residual
 //     going down, the corrected iterate going up) straight into their shared
 //     memory, and one cluster barrier per level and direction publishes it.

@@ -22,7 +22,8 @@ inline PairCoef parity_coef(const AjStepParams& p) {
 
 // s / den for the sweeps' constant divisor: s rden and one Newton correction
 // of the quotient by its exact residual (Markstein 1990), three operations
-// instead of a division per cell
+// instead of a division per cell, and the division's quotient short of under-
+// and overflow (an infinite s gives NaN: the norm ends as non-finite either way)
 __device__ __forceinline__ float pair_div(float s, const PairCoef& a) {
   const float q = s * a.rden;
   return fmaf(fmaf(-q, a.den, s), a.rden, q);

@@ -601,8 +601,10 @@ extern "C" int32_t aj_geometry(int32_t nx, int32_t ny, double lx, double ly, int
 namespace aj {
 
 // s / d for a divisor known on the host, r = 1 / d: s r corrected once by its
-// exact residual (Markstein 1990), the correctly rounded quotient in four
-// operations instead of a division; where s r is not finite it stands as it is.
+// exact residual (Markstein 1990), four operations instead of a division.
+// Short of under- and overflow it is the division's quotient (compared for
+// 6000 divisors and every significand of s); where s r is not finite it
+// stands as it is.
 struct Quot {
   float d, r;
 };

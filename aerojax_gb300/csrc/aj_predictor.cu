@@ -678,9 +678,14 @@ __device__ __forceinline__ float stage_val(const RkArgs& a, const float* f, cons
                                            const float* k1, float* k1_out, int i, int j,
                                            float dt) {
   long k = (long)i * a.ny + j;
-  float r = rhs_comp<PER, HYPER, ADV>(a, f, i, j);
+  // the cell's own reads beside the stencil's: after the store of k1 the
+  // compiler leaves them behind it, a round trip of their own (three upwind
+  // stages at 3001x1503 157 us, so 123)
+  const float x0 = ldg(f0 + k), chi = ldg(a.chi + k);
+  const float g = a.rk2 && a.stage == 2 ? ldg(k1 + k) : 0.f;
+  const float r = rhs_comp<PER, HYPER, ADV>(a, f, i, j);
   if (a.rk2 && a.stage == 1 && k1_out) k1_out[k] = r;
-  return stage_sum(a, ldg(f0 + k), r, ldg(a.chi + k), a.rk2 && a.stage == 2 ? ldg(k1 + k) : 0.f, dt);
+  return stage_sum(a, x0, r, chi, g, dt);
 }
 
 // one stage of component COMP at (i, j).  The last stage applies the hard mask
@@ -719,9 +724,16 @@ __device__ __forceinline__ void rk_col_one(const RkArgs& a, int i, int j, float 
 }
 template <bool PER, bool HYPER, int ADV>
 __device__ __forceinline__ void rk_col_cell(const RkArgs& a, int i, int j, float dt) {
-  if (ADV != AJ_ADV_WENO5 && (a.rk2 ? a.stage != 2 : a.stage != 3)) {
-    // both components in one scope share their loads
+  const bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
+  if (!last || PER) {   // no boundary conditions
+    // both components in one scope share their loads (a periodic grid's last
+    // stage apart, with one component a branch: three stages at 3001x1503,
+    // upwind, 142 us, so 135; WENO5 1000x252 28, so 25)
     const long k = (long)i * a.ny + j;
+    if (last && !(ldg(a.mask + k) > 0.5f)) {
+      a.uout[k] = a.vout[k] = 0.f;
+      return;
+    }
     a.uout[k] = stage_val<PER, HYPER, ADV>(a, a.uin, a.u0, a.k1u, a.k1u_out, i, j, dt);
     a.vout[k] = stage_val<PER, HYPER, ADV>(a, a.vin, a.v0, a.k1v, a.k1v_out, i, j, dt);
     return;
@@ -1441,6 +1453,51 @@ __device__ __forceinline__ void rk_mac_one(const RkMac& a, int i, int j, float d
   (COMP == 0 ? a.uout : a.vout)[(long)i * (COMP == 0 ? a.ny : a.ny + 1) + j] = o;
 }
 
+// The same for the kernel of a cell a thread.  Here the evaluation stands at
+// each branch: with rk_mac_face's one for all, and the two components' interior
+// reads apart, three stages took 66 us with WENO5 and hyperviscosity at
+// 1000x252, so 63; upwind with hyperviscosity at 3001x1503 227, so 222; WENO5
+// between no-slip walls there 805, so 756.  (Where threads share a block of edge
+// cells, as in k_rk_mac_rows, the one call site wins.)
+template <int COMP, bool HYPER, int ADV>
+__device__ __forceinline__ void rk_mac_branch(const RkMac& a, int i, int j, float dt) {
+  const int nx = a.nx, ny = a.ny, m = COMP == 0 ? ny : ny + 1;
+  if (i >= (COMP == 0 ? nx + 1 : nx) || j >= m) return;
+  const bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
+  constexpr int HB = ADV == AJ_ADV_WENO5 ? 4 : 2;
+  const int ei = COMP == 0 ? nx - HB : nx - 1 - HB, ej = COMP == 0 ? ny - 1 - HB : ny - HB;
+  float* k1o = last ? nullptr : (COMP == 0 ? a.k1u_out : a.k1v_out);
+  auto stage = [&](int ii, int jj) {
+    return stage_mac_any<COMP, HYPER, ADV>(a, ii, jj, dt, k1o);
+  };
+  float o = 0.f;
+  if (a.flow == AJ_FLOW_VON_KARMAN && a.slip && i >= HB && i <= ei && j >= HB && j <= ej) {
+    if constexpr (ADV == AJ_ADV_WENO5) o = stage_mac_any<COMP, HYPER, ADV, true>(a, i, j, dt, k1o);
+    else if constexpr (COMP == 0) o = stage_mac_u_int<HYPER>(a, i, j, dt, k1o);
+    else o = stage_mac_v_int<HYPER>(a, i, j, dt, k1o);
+  } else if (!last) {
+    o = stage(i, j);
+  } else if (a.flow == AJ_FLOW_VON_KARMAN) {
+    if (COMP == 0) {
+      if (!a.slip && (j == 0 || j == ny - 1)) o = 0.f;
+      else if (i == 0) o = a.U;
+      else o = stage(i == nx ? nx - 1 : i, a.slip ? (j == 0 ? 1 : (j == ny - 1 ? ny - 2 : j)) : j);
+    } else if (i != 0 && j != 0 && j != ny) {
+      o = stage(i == nx - 1 ? nx - 2 : i, j);
+    }
+  } else if (a.flow == AJ_FLOW_LID_DRIVEN_CAVITY) {
+    if (COMP == 0) {
+      if (i == 0 || i == nx || j == 0) o = 0.f;
+      else o = j == ny - 1 ? a.U : stage(i, j);
+    } else if (i != 0 && i != nx - 1 && j != 0 && j != ny) {
+      o = stage(i, j);
+    }
+  } else {
+    o = stage(i, j);
+  }
+  (COMP == 0 ? a.uout : a.vout)[(long)i * m + j] = o;
+}
+
 template <bool HYPER, int ADV>
 __global__ void __launch_bounds__(256) k_rk_mac(RkMac a) {
   pdl_wait();
@@ -1448,18 +1505,27 @@ __global__ void __launch_bounds__(256) k_rk_mac(RkMac a) {
   const int i = blockIdx.y * blockDim.y + threadIdx.y;
   const float dt = stage_dt(a.dt);
   stage_dt_write(a.dt);
-  if (ADV != AJ_ADV_WENO5 && !HYPER && a.flow == AJ_FLOW_VON_KARMAN && a.slip && i >= 2 &&
-      i <= a.nx - 3 && j >= 2 && j <= a.ny - 3) {
-    // both faces of an interior cell share the paired FP32 instructions
+  if (ADV != AJ_ADV_WENO5 && a.flow == AJ_FLOW_VON_KARMAN && a.slip && i >= 2 && i <= a.nx - 3 &&
+      j >= 2 && j <= a.ny - 3) {
+    // both faces of an interior cell in one scope: without hyperviscosity they
+    // share the paired FP32 instructions, with it their loads
     const bool last = a.rk2 ? a.stage == 2 : a.stage == 3;
-    const float2 o = stage_mac_uv_int(a, i, j, dt, last ? nullptr : a.k1u_out,
-                                      last ? nullptr : a.k1v_out);
-    a.uout[(long)i * a.ny + j] = o.x;
-    a.vout[(long)i * (a.ny + 1) + j] = o.y;
+    float uo, vo;
+    if (HYPER) {
+      uo = stage_mac_u_int<HYPER>(a, i, j, dt, last ? nullptr : a.k1u_out);
+      vo = stage_mac_v_int<HYPER>(a, i, j, dt, last ? nullptr : a.k1v_out);
+    } else {
+      const float2 o = stage_mac_uv_int(a, i, j, dt, last ? nullptr : a.k1u_out,
+                                        last ? nullptr : a.k1v_out);
+      uo = o.x;
+      vo = o.y;
+    }
+    a.uout[(long)i * a.ny + j] = uo;
+    a.vout[(long)i * (a.ny + 1) + j] = vo;
     return;
   }
-  rk_mac_one<0, HYPER, ADV>(a, i, j, dt);
-  rk_mac_one<1, HYPER, ADV>(a, i, j, dt);
+  rk_mac_branch<0, HYPER, ADV>(a, i, j, dt);
+  rk_mac_branch<1, HYPER, ADV>(a, i, j, dt);
 }
 
 // The stage of the slip-wall von Karman channel a run of rows a thread: the

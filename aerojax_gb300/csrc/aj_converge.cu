@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(32 * G, CP_THREADS_SM / (32 * G)) k_cv_up0(
   }
   if (profile) return;
   __shared__ df ws[G];
-  const df s = warp_sum_df(df{acc, 0.f});
+  const df s = warp_sum_df(acc);
   if (t.tx == 0) ws[t.ty] = s;
   __syncthreads();
   if (t.ty > 0) return;

@@ -196,14 +196,19 @@ __device__ __forceinline__ df df_add(df a, df b) {
 // rate): with pairs of FP32 numbers to the end, their low word not even
 // renormalised, the norms' largest error was 6e-15 relative, so it is 2e-15
 // (blocks of 8 to 32 warps, random fields).
+template <int FIRST = 16>
 __device__ __forceinline__ df warp_sum_df(df v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = FIRST; o > 0; o >>= 1) {
     const float h = __shfl_xor_sync(0xffffffffu, v.hi, o);
     const float l = __shfl_xor_sync(0xffffffffu, v.lo, o);
     v = df_add(v, df{h, l});
   }
   return v;
+}
+// of one float per lane: the first addition is a TwoSum alone
+__device__ __forceinline__ df warp_sum_df(float v) {
+  return warp_sum_df<8>(two_sum(v, __shfl_xor_sync(0xffffffffu, v, 16)));
 }
 __device__ __forceinline__ double df_double(df v) { return (double)v.hi + (double)v.lo; }
 

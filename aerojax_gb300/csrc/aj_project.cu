@@ -738,6 +738,11 @@ __global__ void k_diagnostics(const float* __restrict__ u, const float* __restri
 // it: HBM, three fields in and four out.  4096x2048: 91 -> 46 us (2.6 -> 5.1
 // TB/s); one cell a thread with ten divisions a cell was bound by issue.
 constexpr int POST_ROWS = 4;
+// Below, its few blocks' chains over their rows set the time.  Warm, a cell a
+// thread / this, us, diagnostics (with dye): 512x128 2.3 (2.6) / 3.9 (4.9),
+// 1024x256 2.8 (3.7) / 4.9 (6.0), 1536x512 5.1 (7.2) / 5.6 (7.2), 2048x512 6.3
+// (9.0) / 5.6 (7.2), 4096x2048 59 (80) / 32 (44).
+constexpr long POST4_MIN_CELLS = 3 << 18;
 template <bool PER>
 __global__ void __launch_bounds__(256) k_post4(const float* __restrict__ u,
                                                const float* __restrict__ v, int nx, int ny,
@@ -846,7 +851,7 @@ static int post_step(const AjStepParams* prm, const float* u, const float* v, co
   const Dye dye{c_in, c_out, dt, diffusivity, quot((float)(prm->dx * prm->dx)),
                 quot((float)(prm->dy * prm->dy))};
   cudaStream_t st = (cudaStream_t)stream;
-  bool wide = !mac && ny % 4 == 0;   // k_post4's alignment
+  bool wide = !mac && ny % 4 == 0 && (long)nx * ny >= POST4_MIN_CELLS;   // k_post4's alignment
   for (const void* q : {(const void*)u, (const void*)v, (const void*)c_in, (const void*)c_out,
                         (const void*)vort, (const void*)div, (const void*)speed})
     wide = wide && (reinterpret_cast<uintptr_t>(q) & 15) == 0;

@@ -314,6 +314,14 @@ def test_post_step_shapes(cuda_lib, shape, flow, grid):
     assert torch.equal(alone, out[0])
 
 
+@pytest.mark.parametrize("shape", [(3, 262148), (1027, 772)])
+@pytest.mark.parametrize("flow", ["von_karman", "taylor_green"])
+def test_post_step_large_shapes(cuda_lib, shape, flow):
+    """The same from the size on that takes four columns and four rows a thread:
+    runs of rows and blocks of columns cut by the grid's ends."""
+    test_post_step_shapes(cuda_lib, shape, flow, "collocated")
+
+
 def test_training_data_file(cuda_lib, tmp_path):
     """generate_training_data writes the reference's .npz layout
     (training_utils.py:12-81) and the recorded fields are the solver's."""

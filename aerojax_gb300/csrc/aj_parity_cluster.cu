@@ -28,7 +28,7 @@
 // What bounds it: the chain of short passes (a block barrier each) and the
 // cluster barriers (~0.3 us) on 16 SMs - hence the limit on a thread's run:
 // above it the tiled kernels, which use all SMs, are the faster ones.
-// Measured: a step_pure step at 512x96 with 3 cycles 130 -> 73 us (the solve
+// Measured: a step_pure step at 512x96 with 3 cycles 130 -> 70 us (the solve
 // in one launch instead of 28); a cycle at 256x64 38.7 -> 16.8 us, at 512x128
 // 39.0 -> 19.5 us.
 #include "aj_parity_pair.cuh"
@@ -434,9 +434,11 @@ static int pc_ctas(const Layout& L) {
 // level 0 fits (a cycle, collocated: 384x96 18.4 us against 20.5 us with tiled
 // level-0 kernels, 512x128 19.5 against 20.4); else the levels whose bands,
 // halo included, are at most PC_TAIL_CELLS cells: below that a level's two
-// launches cost more than its share of the cluster's time (limits of 1000 /
-// 1800 / none: 1008x368 25.8 / 25.8 / 28.3 us a cycle, 2048x512 37.1 / 35.7 /
-// 35.9).
+// launches cost more than its share of the cluster's time.  Limits of 1000 /
+// 1800 / 3600 / none, us a cycle, collocated: 96x2048 25.4 / 25.4 / 24.6 / 27.5,
+// 640x256 21.8 / 21.1 / 21.1 / 20.8, 1008x368 24.2 / 24.2 / 24.0 / 26.7, 1024x512
+// 27.9 / 26.2 / 26.2 / 26.2, 768x768 28.2 / 27.0 / 27.1 / 27.3, 2048x512 36.9 /
+// 35.6 / 35.6 / 36.5, 4096x1024 72.6 / 72.3 / 72.3 / 71.4 (MAC alike).
 constexpr int PC_TAIL_CELLS = 1800;
 int parity_cluster_level(const AjStepParams& p, const Layout& L) {
   const int C = pc_ctas(L), nl = L.nlev;
